@@ -625,14 +625,6 @@ int ch3d_create(const ch3d_config* cfg, const double* yp, ch3d_ctx** out) {
   if (e != cudaSuccess) { int r = fail(CH3D_ERR_CUDA, "stream: %s", cudaGetErrorString(e)); delete c; return r; }
   if (cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess)
     return cleanup(fail(CH3D_ERR_CUDA, "event create failed"));
-  if (c->fp32) {
-    int lo = 0, hi = 0;
-    if (cudaDeviceGetStreamPriorityRange(&lo, &hi) != cudaSuccess ||
-        cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, hi) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess)
-      return cleanup(fail(CH3D_ERR_CUDA, "side stream create failed"));
-  }
   rc = c->fp32 ? alloc_fields<float>(c) : alloc_fields<double>(c);
   if (rc) return cleanup(rc);
   {
@@ -673,21 +665,20 @@ int ch3d_create(const ch3d_config* cfg, const double* yp, ch3d_ctx** out) {
     // Poisson y-solve (Thomas) factors per (kx, |kz|), computed once
     const size_t nrow = (size_t)(c->nz / 2 + 1) * c->ny * c->nxh;
     const size_t fw = c->fp32 ? sizeof(float) : sizeof(double);
-    if (cudaMalloc(&c->yRM, nrow * fw) != cudaSuccess || cudaMalloc(&c->yCP, nrow * fw) != cudaSuccess)
-      return cleanup(fail(CH3D_ERR_NOMEM, "Poisson factors"));
-    c->bytes += (long long)(2 * nrow) * fw;
+    if (cudaMalloc(&c->yRM, nrow * fw) != cudaSuccess) return cleanup(fail(CH3D_ERR_NOMEM, "Poisson factors"));
+    c->bytes += (long long)nrow * fw;
     if (c->fp32) {
       const size_t lr = (size_t)(c->KL + 1) * c->ny * c->TSy;
       const size_t ls = (size_t)(2 * c->KL + 1) * c->TSy * c->ny * 2;  // FP64 complex sweep scratch
       if (cudaMalloc(&c->yRM64, lr * sizeof(double)) != cudaSuccess ||
-          cudaMalloc(&c->yCP64, lr * sizeof(double)) != cudaSuccess ||
-          cudaMalloc(&c->ylow, ls * sizeof(double)) != cudaSuccess)
+          (!ysolve_chunked(c->ny) && cudaMalloc(&c->ylow, ls * sizeof(double)) != cudaSuccess))
         return cleanup(fail(CH3D_ERR_NOMEM, "Poisson low-mode factors"));
     }
     if (y_periodic(c)) {
-      if (cudaMalloc(&c->yA2, nrow * sizeof(double)) != cudaSuccess)
+      if (cudaMalloc(&c->yCP, nrow * sizeof(double)) != cudaSuccess ||
+          cudaMalloc(&c->yA2, nrow * sizeof(double)) != cudaSuccess)
         return cleanup(fail(CH3D_ERR_NOMEM, "Poisson factors"));
-      c->bytes += (long long)nrow * sizeof(double);
+      c->bytes += (long long)(2 * nrow) * sizeof(double);
     }
     e = launch_ysolve_factors(c);
     if (e != cudaSuccess) return cleanup(fail(CH3D_ERR_CUDA, "Poisson factors: %s", cudaGetErrorString(e)));
@@ -738,14 +729,11 @@ int ch3d_destroy(ch3d_ctx* c) {
   void* mbufs[] = {c->mlp_params, c->mlp_packed, c->mlp_status, c->sgs_tau, c->sgs_f, c->spec2,
                    c->specacc};
   for (void* b : mbufs) if (b) cudaFree(b);
-  void* bufs[] = {c->hfac, c->mtab, c->yRM, c->yCP, c->ylow, c->yA2, c->yRM64, c->yCP64, c->spec, c->met, c->met64, c->wave, c->twx, c->twr, c->twz, c->sc, c->part, c->part2,
+  void* bufs[] = {c->hfac, c->mtab, c->yRM, c->yCP, c->ylow, c->yA2, c->yRM64, c->spec, c->met, c->met64, c->wave, c->twx, c->twr, c->twz, c->sc, c->part, c->part2,
                   c->red1, c->red2, c->stat, c->statpart};
   for (void* b : bufs) if (b) cudaFree(b);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
-  if (c->ev_fork) cudaEventDestroy(c->ev_fork);
-  if (c->ev_join) cudaEventDestroy(c->ev_join);
-  if (c->side) cudaStreamDestroy(c->side);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
   return CH3D_OK;

@@ -17,10 +17,6 @@ struct ch3d_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-  // mixed path: a high-priority side stream for the FP64 low-mode Poisson y solves,
-  // forked from and joined to `stream` around the FP32 solves
-  cudaStream_t side = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   double last_ms = 0;
 
   // Runge-Kutta constants (src/CFD_2nd/m_Parameters.f90:291-306)
@@ -49,11 +45,11 @@ struct ch3d_ctx {
   int* mlp_status = nullptr;
   double* sgs_tau = nullptr;     // 6 N stresses at the cell centres
   double* sgs_f = nullptr;       // 3 N stress-divergence forces at the velocity points
-  void* yRM = nullptr;       // Poisson y-solve Thomas factors per mode (fixed for the run);
-  void* yCP = nullptr;       // FP64, or FP32 in the mixed path
+  void* yRM = nullptr;       // Poisson y-solve elimination factors per mode (fixed for the run), FP64, or FP32 in
+                             // the mixed path; periodic y: those of the cyclic systems
+  void* yCP = nullptr;       // periodic y: the cyclic systems' second factor
   double* yRM64 = nullptr;   // mixed path: FP64 factors of the low modes (kx < TSy, |kz| <= KL)
-  double* yCP64 = nullptr;
-  double* ylow = nullptr;    // mixed path: FP64 forward-sweep scratch of the low modes
+  double* ylow = nullptr;    // mixed path, columns beyond the chunked solve: FP64 sweep scratch of the low modes
   double* yA2 = nullptr;     // periodic y: the Poisson cyclic solve's closure vector per mode
   bool gsub = false;         // the march stops at g; divergence and projection substitute u*
   int KL = 8;
@@ -119,6 +115,8 @@ cudaError_t launch_helm_factors(ch3d_ctx* c);
 cudaError_t launch_prsrc_xfft(ch3d_ctx* c, int mode);  // mode 0: div(u*)/pmAlpha, 1: div(u), 2: source in phi,
                                                        // 3: div(u*) in phi's array, /pmAlpha (register FFT only)
 cudaError_t launch_poisson_spectral(ch3d_ctx* c);      // z fwd, y solve, z inv
+cudaError_t launch_ysolve(ch3d_ctx* c);                // the y systems (ch3d_ysolve.cu)
+bool ysolve_chunked(int ny);                           // they run as the chunked kernel (no scratch)
 cudaError_t launch_xifft(ch3d_ctx* c);
 // register-resident FFT kernels for the lengths with a plan (ch3d_rfft.cu);
 // false: no plan, nothing launched

@@ -718,318 +718,6 @@ __global__ void __launch_bounds__(256) k_ysolve(Geo<T> g, Metrics<double> m, con
 }
 
 // ---------------------------------------------------------------------------
-// y solve with per-mode factors precomputed once per run (the Poisson matrix
-// of mode (kx,kz) does not change during a run).  Factors depend on kz only
-// through WaveNumZ, which is even in kz, so modes kz and nz-kz share them;
-// the grid visits kz and nz-kz back to back so that the second read hits L2.
-// Layout (FP64): RM[(kzh*ny + j)*nxh + kx], CP likewise (chunk-local LU),
-// IFD[((kzh*Q + q)*6 + c)*nxh + kx] (interface block factors Minv, l, v).
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ int kz_of_block(int y, int nz) {
-  return y == 0 ? 0 : ((y & 1) ? (y + 1) / 2 : nz - y / 2);
-}
-
-// Factors of the Thomas elimination of the Poisson y systems
-// [am2Pr, ac2Pr + wx(kx) + wz(kz), ap2Pr] (src/CFD_2nd/m_Poisson.f90:1126-1150,
-// InverseTridiagonal, m_Tools.f90:224-251), one thread per (kx, |kz|) column:
-// rm_j = 1 / (b_j - a_j cp_{j-1}), cp_j = c_j rm_j; row 1 of the (0,0) system
-// is replaced by phi = 0 (:1136-1140).  They depend on the grid only and are
-// computed once per run, in FP64 and stored in precision R, layout
-// ((kzh * ny) + j) * ldx + kx.
-template <class R>
-__global__ void __launch_bounds__(128) k_ythomas_factors(Metrics<double> m, const double* __restrict__ wave, int nx,
-                                                         int ny, R* __restrict__ RMf, R* __restrict__ CPf, int ldx,
-                                                         int kxn) {
-  const int kx = blockIdx.x * blockDim.x + threadIdx.x, kzh = blockIdx.y;
-  if (kx >= kxn) return;
-  const double lam = wave[kx] + wave[nx + kzh];
-  const bool pin = (kx == 0 && kzh == 0);
-  double cp = 0.0;
-  for (int j = 0; j < ny; ++j) {
-    const int jc = j + 1;
-    double a = m.am2Pr[jc], c = m.ap2Pr[jc], b = m.ac2Pr[jc] + lam;
-    if (pin && j == 0) { a = 0.0; b = 1.0; c = 0.0; }
-    const double rm = 1.0 / (j == 0 ? b : b - a * cp);
-    cp = c * rm;
-    const size_t o = ((size_t)kzh * ny + j) * ldx + kx;
-    RMf[o] = (R)rm;
-    CPf[o] = (R)cp;
-  }
-}
-
-template <class R> struct Vec2Of;
-template <> struct Vec2Of<double> { typedef double2 type; };
-template <> struct Vec2Of<float> { typedef float2 type; };
-
-// Poisson y solve, Thomas across threads: one thread per (kx, kz) column,
-// threads numbered kx fastest so that a warp reads 32 consecutive kx of one
-// row of the (kx, j, kz) spectrum.  The forward sweep keeps d_j in place in
-// the spectrum (the FP64 low modes of the mixed path in an FP64 scratch
-// array, layout [j][low column]), the backward sweep overwrites it with the
-// solution.  Rows are processed in batches of YB: the batch's loads are all
-// issued before its dependent recurrence, so YB rows of every column are in
-// flight at once.  YB is 16 in the FP64 kernel and 8 in the mixed one (whose
-// FP64 low-mode sweeps share the FP32 sweeps' register budget); at 768x384x576
-// the spectral group takes 2.51 ms FP64 with 16 rows against 2.61 with 8, mixed
-// 1.65 with 8 against 1.73 with 16; refilling each row's slot as soon as it is
-// consumed instead of whole batches was slower in both.
-
-template <class R, class CT, int YB, class LD, class ST, class STD, class LDD>
-__device__ __forceinline__ void thomas_column(int ny, bool pin, const R* __restrict__ rm, const R* __restrict__ cp,
-                                              size_t fst, const double* __restrict__ am, LD load, ST store,
-                                              STD store_d, LDD load_d) {
-  R dx = (R)0, dy = (R)0;
-  for (int j0 = 0; j0 < ny; j0 += YB) {
-    R fx[YB], fy[YB], r[YB], a[YB];
-#pragma unroll
-    for (int u = 0; u < YB; ++u) {
-      const int j = j0 + u;
-      if (j < ny) {
-        const CT f = load(j);
-        fx[u] = (R)f.x; fy[u] = (R)f.y;
-        r[u] = __ldg(rm + fst * j);
-        a[u] = (R)__ldg(am + j + 1);
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < YB; ++u) {
-      const int j = j0 + u;
-      if (j < ny) {
-        if (j == 0) {
-          dx = pin ? (R)0 : fx[u] * r[u];
-          dy = pin ? (R)0 : fy[u] * r[u];
-        } else {
-          dx = (fx[u] - a[u] * dx) * r[u];
-          dy = (fy[u] - a[u] * dy) * r[u];
-        }
-        store_d(j, dx, dy);
-      }
-    }
-  }
-  store(ny - 1, dx, dy);
-  for (int j1 = ny - 2; j1 >= 0; j1 -= YB) {
-    R ex[YB], ey[YB], c[YB];
-#pragma unroll
-    for (int u = 0; u < YB; ++u) {
-      const int j = j1 - u;
-      if (j >= 0) {
-        const CT v = load_d(j);
-        ex[u] = (R)v.x; ey[u] = (R)v.y;
-        c[u] = __ldg(cp + fst * j);
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < YB; ++u) {
-      const int j = j1 - u;
-      if (j >= 0) {
-        dx = ex[u] - c[u] * dx;
-        dy = ey[u] - c[u] * dy;
-        store(j, dx, dy);
-      }
-    }
-  }
-}
-
-// All columns in the precision of the field (FP64 path), or in the mixed
-// path the FP32 columns: the low modes kx < KX, |kz| <= KL are skipped
-// (KX = 0: none) and solved by k_ythomas_low.
-template <class T, class R, int YB>
-__global__ void __launch_bounds__(128) k_ythomas(Geo<T> g, Metrics<double> m, const R* __restrict__ RMf,
-                                                 const R* __restrict__ CPf, typename CplxOf<T>::type* __restrict__ spec,
-                                                 int KL, int KX, const DevScalars* __restrict__ sc) {
-  typedef typename CplxOf<T>::type CT;
-  if (sc->status) return;
-  const int nxh = g.nxh, ny = g.ny, nz = g.nz;
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)nxh * nz) return;
-  const int kx = (int)(t % nxh), kz = (int)(t / nxh);
-  const int kzh = kz <= nz - kz ? kz : nz - kz;
-  if (kx < KX && kzh <= KL) return;
-  const size_t st = (size_t)nxh;
-  CT* col = spec + kx + st * ny * kz;
-  const R* rm = RMf + (size_t)kzh * ny * st + kx;
-  const R* cp = CPf + (size_t)kzh * ny * st + kx;
-  auto load = [&](int j) { return col[st * j]; };
-  auto store = [&](int j, R x, R y) { col[st * j] = mk((T)x, (T)y); };
-  thomas_column<R, CT, YB>(ny, kx == 0 && kz == 0, rm, cp, st, m.am2Pr, load, store, store, load);
-}
-
-// Mixed path: the low modes kx < KX, |kz| <= KL (column zi = kz for kz <= KL,
-// KL + nz - kz above) in FP64 with FP64 factors, their forward sweep kept in
-// the FP64 scratch [j][low column].
-template <class T>
-__global__ void __launch_bounds__(128) k_ythomas_low(Geo<T> g, Metrics<double> m, const double* __restrict__ RM64,
-                                                     const double* __restrict__ CP64,
-                                                     typename CplxOf<T>::type* __restrict__ spec,
-                                                     double2* __restrict__ scr, int KL, int KX,
-                                                     const DevScalars* __restrict__ sc) {
-  typedef typename CplxOf<T>::type CT;
-  if (sc->status) return;
-  const int nxh = g.nxh, ny = g.ny, nz = g.nz;
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= (2 * KL + 1) * KX) return;
-  const int zi = q / KX, kx = q - zi * KX;
-  const int kz = zi <= KL ? zi : nz - (zi - KL);
-  if (kx >= nxh || (zi > KL && kz <= KL)) return;
-  const int kzh = kz <= nz - kz ? kz : nz - kz;
-  const size_t st = (size_t)nxh;
-  CT* col = spec + kx + st * ny * kz;
-  const size_t nlow = (size_t)(2 * KL + 1) * KX;
-  double2* w = scr + (size_t)zi * KX + kx;  // [j][low column]
-  auto load = [&](int j) { const CT v = col[st * j]; return make_double2(v.x, v.y); };
-  auto store = [&](int j, double x, double y) { col[st * j] = mk((T)x, (T)y); };
-  auto store_d = [&](int j, double x, double y) { w[nlow * j] = make_double2(x, y); };
-  auto load_d = [&](int j) { return w[nlow * j]; };
-  thomas_column<double, double2, 16>(ny, kx == 0 && kz == 0, RM64 + (size_t)kzh * ny * KX + kx,
-                                     CP64 + (size_t)kzh * ny * KX + kx, (size_t)KX, m.am2Pr, load, store, store_d,
-                                     load_d);
-}
-
-// ---------------------------------------------------------------------------
-// Periodic y (clcPPE_z1_periodic, src/CFD_2nd/m_Poisson.f90:954-1073): the
-// systems [am2Pr, ac2Pr + wx(kx) + wz(kz), ap2Pr] are cyclic, solved by
-// InversePeriodicTridiagonal (src/CFD_2nd/m_Tools.f90:109-162), with row 1
-// of the (0,0) system replaced by phi = 0 (:1012-1029).  Its coefficient
-// recurrences depend on the mode only and are computed once per run, one
-// thread per (kx, |kz|), FP64, layout ((kzh * ny) + j) * nxh + kx:
-//   PP_0 = b_1 (row 1 divides), PP_j = 1 / (b + a arrmn1_{j-1}) (ppj),
-//   A1_j = arrmn1_j, A1_{n-1} = the closing denominator,
-//   A2_j = arrmn2_j after the backward pass.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_ycyclic_factors(Metrics<double> m, const double* __restrict__ wave, int nx,
-                                                         int ny, int nxh, double* __restrict__ PP,
-                                                         double* __restrict__ A1, double* __restrict__ A2) {
-  const int kx = blockIdx.x * blockDim.x + threadIdx.x, kzh = blockIdx.y;
-  if (kx >= nxh) return;
-  const double lam = wave[kx] + wave[nx + kzh];
-  const bool pin = (kx == 0 && kzh == 0);
-  const size_t st = (size_t)nxh, o = (size_t)kzh * ny * st + kx;
-  auto coef = [&](int j, double& a, double& b, double& c) {
-    a = m.am2Pr[j + 1]; c = m.ap2Pr[j + 1]; b = m.ac2Pr[j + 1] + lam;
-    if (pin && j == 0) { a = 0.0; b = 1.0; c = 0.0; }
-  };
-  double a, b, c;
-  coef(0, a, b, c);
-  double v1 = -c / b, v2 = -a / b;
-  PP[o] = b; A1[o] = v1; A2[o] = v2;
-  for (int j = 1; j <= ny - 2; ++j) {
-    coef(j, a, b, c);
-    const double ppj = 1.0 / (b + a * v1);
-    v1 = -c * ppj;
-    v2 = -a * v2 * ppj;
-    PP[o + st * j] = ppj; A1[o + st * j] = v1; A2[o + st * j] = v2;
-  }
-  // backward pass: arrmn2_n = 1, arrmn2_j += arrmn1_j arrmn2_{j+1}
-  double w = 1.0;
-  A2[o + st * (ny - 1)] = w;
-  for (int j = ny - 2; j >= 0; --j) {
-    w = A2[o + st * j] + A1[o + st * j] * w;
-    A2[o + st * j] = w;
-  }
-  coef(ny - 1, a, b, c);
-  A1[o + st * (ny - 1)] = c * A2[o] + a * A2[o + st * (ny - 2)] + b;
-}
-
-// One thread per (kx, kz) column of the (kx, j, kz) spectrum (kx fastest, so
-// a warp reads 32 consecutive kx of one row), FP64, in place: forward
-// elimination, the backward pass of the right-hand side (arrmn3), the closure
-// of row n, and the back substitution f_j = f_n arrmn2_j + arrmn3_j.  Each
-// pass loads YB rows (and their factors) before its dependent recurrence, so
-// YB loads of every column are in flight at once.
-template <class T, int YB>
-__global__ void __launch_bounds__(128) k_ycyclic(Geo<T> g, Metrics<double> m, const double* __restrict__ PP,
-                                                 const double* __restrict__ A1, const double* __restrict__ A2,
-                                                 typename CplxOf<T>::type* __restrict__ spec,
-                                                 const DevScalars* __restrict__ sc) {
-  typedef typename CplxOf<T>::type CT;
-  if (sc->status) return;
-  const int nxh = g.nxh, ny = g.ny, nz = g.nz;
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)nxh * nz) return;
-  const int kx = (int)(t % nxh), kz = (int)(t / nxh);
-  const int kzh = kz <= nz - kz ? kz : nz - kz;
-  const size_t st = (size_t)nxh;
-  CT* col = spec + kx + st * ny * kz;
-  const size_t o = (size_t)kzh * ny * st + kx;
-  const bool pin = (kx == 0 && kz == 0);
-  // forward elimination, rows 1..n-1 (0-based 0..ny-2); row 1 divides by b_1
-  double dx = 0.0, dy = 0.0;
-  for (int j0 = 0; j0 <= ny - 2; j0 += YB) {
-    double fx[YB], fy[YB], pp[YB], am[YB];
-#pragma unroll
-    for (int u = 0; u < YB; ++u) {
-      const int j = j0 + u;
-      if (j <= ny - 2) {
-        const CT f = col[st * j];
-        fx[u] = (double)f.x; fy[u] = (double)f.y;
-        pp[u] = PP[o + st * j];
-        am[u] = m.am2Pr[j + 1];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < YB; ++u) {
-      const int j = j0 + u;
-      if (j <= ny - 2) {
-        if (j == 0) {
-          dx = pin ? 0.0 : fx[u] / pp[u];
-          dy = pin ? 0.0 : fy[u] / pp[u];
-        } else {
-          dx = (fx[u] - am[u] * dx) * pp[u];
-          dy = (fy[u] - am[u] * dy) * pp[u];
-        }
-        col[st * j] = mk((T)dx, (T)dy);
-      }
-    }
-  }
-  // backward pass: arrmn3_n = 0, arrmn3_j = f_j + arrmn1_j arrmn3_{j+1}
-  double ex = 0.0, ey = 0.0, lx = 0.0, ly = 0.0;
-  for (int j1 = ny - 2; j1 >= 0; j1 -= YB) {
-    double vx[YB], vy[YB], a1[YB];
-#pragma unroll
-    for (int u = 0; u < YB; ++u) {
-      const int j = j1 - u;
-      if (j >= 0) {
-        const CT f = col[st * j];
-        vx[u] = (double)f.x; vy[u] = (double)f.y;
-        a1[u] = A1[o + st * j];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < YB; ++u) {
-      const int j = j1 - u;
-      if (j >= 0) {
-        ex = vx[u] + a1[u] * ex;
-        ey = vy[u] + a1[u] * ey;
-        col[st * j] = mk((T)ex, (T)ey);
-        if (j == ny - 2) { lx = ex; ly = ey; }
-      }
-    }
-  }
-  // closure of row n, then f_j = f_n arrmn2_j + arrmn3_j
-  const double an = m.am2Pr[ny], cn = m.ap2Pr[ny], den = A1[o + st * (ny - 1)];
-  const CT fl = col[st * (ny - 1)];
-  const double fnx = ((double)fl.x - cn * ex - an * lx) / den, fny = ((double)fl.y - cn * ey - an * ly) / den;
-  col[st * (ny - 1)] = mk((T)fnx, (T)fny);
-  for (int j0 = 0; j0 <= ny - 2; j0 += YB) {
-    double vx[YB], vy[YB], a2[YB];
-#pragma unroll
-    for (int u = 0; u < YB; ++u) {
-      const int j = j0 + u;
-      if (j <= ny - 2) {
-        const CT f = col[st * j];
-        vx[u] = (double)f.x; vy[u] = (double)f.y;
-        a2[u] = A2[o + st * j];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < YB; ++u) {
-      const int j = j0 + u;
-      if (j <= ny - 2) col[st * j] = mk((T)(fnx * a2[u] + vx[u]), (T)(fny * a2[u] + vy[u]));
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
 // inverse x transform (complex-to-real, unnormalised as FFTW's HC2R) * normfft
 // (src/CFD_2nd/m_Poisson.f90:1194-1200) -> phi.
 // ---------------------------------------------------------------------------
@@ -1476,31 +1164,7 @@ template <class T> static cudaError_t spectral_t(ch3d_ctx* c) {
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
-  const unsigned gy = (unsigned)(((long long)c->nxh * c->nz + 127) / 128);
-  if (y_periodic(c)) {  // periodic y (FP64 only): the cyclic systems
-    k_ycyclic<T, 16><<<gy, 128, 0, c->stream>>>(make_geo<T>(c), c->m64full, (const double*)c->yRM,
-                                                (const double*)c->yCP, c->yA2, (CT*)c->spec, c->sc);
-  } else if (!c->fp32) {
-    k_ythomas<T, double, 16><<<gy, 128, 0, c->stream>>>(make_geo<T>(c), c->m64full, (const double*)c->yRM,
-                                                        (const double*)c->yCP, (CT*)c->spec, 0, 0, c->sc);
-  } else {
-    // mixed: FP32 systems and factors; the low modes near kx = kz = 0 in FP64 on the
-    // high-priority side stream, overlapping the FP32 sweeps (a fork and a join in
-    // the captured step graph)
-    const int nlow = (2 * c->KL + 1) * c->TSy;
-    if ((e = cudaEventRecord(c->ev_fork, c->stream)) != cudaSuccess) return e;
-    if ((e = cudaStreamWaitEvent(c->side, c->ev_fork, 0)) != cudaSuccess) return e;
-    k_ythomas_low<T><<<(nlow + 127) / 128, 128, 0, c->side>>>(make_geo<T>(c), c->m64full, c->yRM64, c->yCP64,
-                                                              (CT*)c->spec, (double2*)c->ylow, c->KL, c->TSy, c->sc);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = cudaEventRecord(c->ev_join, c->side)) != cudaSuccess) return e;
-    k_ythomas<T, float, 16><<<gy, 128, 0, c->stream>>>(make_geo<T>(c), c->m64full, (const float*)c->yRM,
-                                                       (const float*)c->yCP, (CT*)c->spec, c->KL, c->TSy, c->sc);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    e = cudaStreamWaitEvent(c->stream, c->ev_join, 0);
-  }
-  e = e != cudaSuccess ? e : cudaGetLastError();
-  if (e != cudaSuccess) return e;
+  if ((e = launch_ysolve(c)) != cudaSuccess) return e;
   if (launch_zfft_r(c, 1, &e)) return e;
   k_zfft<T><<<gz, nthrz, smemz, c->stream>>>(make_geo<T>(c), (CT*)c->spec, c->planz, (const CT*)c->twz, TKX, 1, c->sc);
   return cudaGetLastError();
@@ -1523,27 +1187,6 @@ template <class T> static cudaError_t zfft_fwd_t(ch3d_ctx* c) {
   return cudaGetLastError();
 }
 cudaError_t launch_zfft_forward(ch3d_ctx* c) { return c->fp32 ? zfft_fwd_t<float>(c) : zfft_fwd_t<double>(c); }
-
-template <class T> static cudaError_t yfactors_t(ch3d_ctx* c) {
-  const dim3 g((c->nxh + 127) / 128, c->nz / 2 + 1);
-  if (y_periodic(c)) {  // periodic y (FP64 only)
-    k_ycyclic_factors<<<g, 128, 0, c->stream>>>(c->m64full, c->wave, c->nx, c->ny, c->nxh, (double*)c->yRM,
-                                                (double*)c->yCP, c->yA2);
-  } else if (!c->fp32) {
-    k_ythomas_factors<double><<<g, 128, 0, c->stream>>>(c->m64full, c->wave, c->nx, c->ny, (double*)c->yRM,
-                                                        (double*)c->yCP, c->nxh, c->nxh);
-  } else {
-    k_ythomas_factors<float><<<g, 128, 0, c->stream>>>(c->m64full, c->wave, c->nx, c->ny, (float*)c->yRM,
-                                                       (float*)c->yCP, c->nxh, c->nxh);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    k_ythomas_factors<double><<<dim3(1, c->KL + 1), 128, 0, c->stream>>>(c->m64full, c->wave, c->nx, c->ny, c->yRM64,
-                                                                        c->yCP64, c->TSy,
-                                                                        c->nxh < c->TSy ? c->nxh : c->TSy);
-  }
-  return cudaGetLastError();
-}
-cudaError_t launch_ysolve_factors(ch3d_ctx* c) { return c->fp32 ? yfactors_t<float>(c) : yfactors_t<double>(c); }
 
 cudaError_t launch_poisson_spectral(ch3d_ctx* c) { return c->fp32 ? spectral_t<float>(c) : spectral_t<double>(c); }
 
