@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(ch3d_mlp::TILE, 6)
   }
   float y[NOUT];
   bool ok = false;
-  if (fwd_inputs(smem, x)) ok = fwd_layers(smem, y, nullptr, nullptr, c, valid, N);
+  if (fwd_inputs(smem, x)) ok = fwd_layers(smem, y);
   else fwd_abort(smem);
   if (!ok && threadIdx.x == 0) atomicExch(mstatus, 1);
   if (!valid) return;

@@ -11,7 +11,8 @@
 // offset 16R between the two 8-wide K halves of one K=16 instruction and
 // stride-byte offset 128 between 8-row groups.  D = A * B^T with A [M x K]
 // and B [N x K] both K-major, so a linear layer y = x W^T takes B = W
-// (out x in, the PyTorch weight layout) and the backward dX = dY W takes B = W^T.
+// (out x in, the PyTorch weight layout).  The backward GEMMs read the same
+// tiles with the indices exchanged, as MN-major operands (gemm_issue_t, _bt).
 // Eight consecutive k of one row are 16 contiguous bytes, so a thread that
 // owns a row writes it with 16-byte stores.
 //
@@ -156,6 +157,29 @@ __device__ __forceinline__ void gemm_issue(uint32_t d_tmem, const unsigned char*
   }
 }
 
+// D[features x N] (+)= A^T B with A [128 points x 64 features] and B [128 points
+// x N], both stored as K-major tiles with points as rows and read as MN-major
+// operands (instruction descriptor bits 15, 16): within an 8 x 8 core matrix
+// the 8 contiguous elements are features, the 16-byte rows points; feature
+// groups are 16 * TILE bytes apart (stride offset), point groups 128 bytes
+// (leading offset).  M = 128: rows 64.. of D come from the memory after A.
+__device__ __forceinline__ void gemm_issue_t(uint32_t d_tmem, const unsigned char* A, const unsigned char* B, int N,
+                                             uint32_t accumulate) {
+  const uint32_t idesc = idesc_bf16(TILE, N) | (1u << 15) | (1u << 16);
+  for (int kk = 0; kk < TILE / 16; ++kk)
+    mma_bf16(d_tmem, sdesc(A + kk * 256, 128, 16 * TILE), sdesc(B + kk * 256, 128, 16 * TILE), idesc,
+             kk > 0 ? 1u : accumulate);
+}
+// D[points x N] = A[points x K] * W[K x N] with W the forward operand (its K rows
+// out of R, N inputs contiguous), read as an MN-major B
+__device__ __forceinline__ void gemm_issue_bt(uint32_t d_tmem, const unsigned char* A, const unsigned char* W, int N,
+                                              int K, int R) {
+  const uint32_t idesc = idesc_bf16(TILE, N) | (1u << 16);
+  for (int kk = 0; kk < K / 16; ++kk)
+    mma_bf16(d_tmem, sdesc(A + kk * 2 * 16 * TILE, 16 * TILE, 128), sdesc(W + kk * 256, 128, 16 * R), idesc,
+             kk > 0 ? 1u : 0u);
+}
+
 // GELU in its tanh form (Hendrycks & Gimpel 2016): 0.5 x (1 + tanh u),
 // u = sqrt(2/pi) (x + 0.044715 x^3).  With r = 1 / (1 + exp(2u)),
 // 1 + tanh u = 2 (1 - r), so gelu = x - x r.  exp(2u) = 2^(2u log2 e) with
@@ -212,20 +236,6 @@ __device__ __forceinline__ void stage_w(unsigned char* t, const float* __restric
     st_bf16x8(t, n, k0, NP, v);
   }
 }
-// B = W^T: N = cols (padded to NP), K = rows (padded to KP), the backward operand
-__device__ __forceinline__ void stage_wt(unsigned char* t, const float* __restrict__ W, int rows, int cols, int NP,
-                                         int KP) {
-  const int kq = KP >> 3;
-  for (int e = threadIdx.x; e < NP * kq; e += blockDim.x) {
-    int n, k0;
-    stage_index(e, kq, n, k0);
-    float v[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) v[q] = (n < cols && k0 + q < rows) ? __ldg(W + (k0 + q) * cols + n) : 0.f;
-    st_bf16x8(t, n, k0, NP, v);
-  }
-}
-
 struct Smem {
   uint64_t bar;   // tensor-core completion
   uint64_t wbar;  // arrival of the packed parameters (fwd_prologue_packed)
@@ -340,12 +350,9 @@ __device__ __forceinline__ void fwd_abort(unsigned char* smem) {
 }
 
 // The four layers on the staged tile: y[0..5] = network output of this
-// thread's point.  Training mode (Z != nullptr) also stores the
-// pre-activations Z1..Z3 (FP32) and activations H1..H3 (BF16) of valid
-// points, [B x 64] each.  Returns false (uniformly over the CTA) when a
-// wait on the tensor cores expired; the tensor memory is released either way.
-__device__ __forceinline__ bool fwd_layers(unsigned char* smem, float* y, float* __restrict__ Z,
-                                           __nv_bfloat16* __restrict__ H, long long pt, bool valid, long long B) {
+// thread's point.  Returns false (uniformly over the CTA) when a wait on the
+// tensor cores expired; the tensor memory is released either way.
+__device__ __forceinline__ bool fwd_layers(unsigned char* smem, float* y) {
   Smem* S = (Smem*)smem;
   const int tid = threadIdx.x, warp = tid >> 5;
   unsigned char* HA = smem + FwdSmem::HA;
@@ -380,14 +387,7 @@ __device__ __forceinline__ bool fwd_layers(unsigned char* smem, float* y, float*
 #pragma unroll
         for (int q = 0; q < 16; q += 4) *reinterpret_cast<float4*>(bq + q) = *reinterpret_cast<const float4*>(bs + l * NH + c0 + q);
 #pragma unroll
-        for (int q = 0; q < 16; ++q) {
-          const float z = acc[q] + bq[q];
-          h[q] = gelu(z);
-          if (Z != nullptr && valid) {
-            Z[(long long)l * B * NH + pt * NH + c0 + q] = z;
-            H[(long long)l * B * NH + pt * NH + c0 + q] = __float2bfloat16_rn(h[q]);
-          }
-        }
+        for (int q = 0; q < 16; ++q) h[q] = gelu(acc[q] + bq[q]);
         st_bf16x8(HA, tid, c0, TILE, h);
         st_bf16x8(HA, tid, c0 + 8, TILE, h + 8);
       }
