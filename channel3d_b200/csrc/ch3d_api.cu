@@ -84,19 +84,39 @@ void mesh_section(double* yp1, int id1, int id2, double c1, double c2, int Stret
   yp[id1] = c1; yp[id2] = c2;
 }
 
+// Plan of an n-point transform, n a product of 2 and 3: the fewest passes of
+// radix at most 16, the largest radix as small as they allow, smaller radices first.
 bool factor23(int n, FFTPlanDev& pl) {
   pl.n = n; pl.npass = 0;
   int m = n;
-  while (m % 4 == 0) { pl.radix[pl.npass++] = 4; m /= 4; }
-  while (m % 2 == 0) { pl.radix[pl.npass++] = 2; m /= 2; }
-  while (m % 3 == 0) { pl.radix[pl.npass++] = 3; m /= 3; }
+  while (m % 2 == 0) m /= 2;
+  while (m % 3 == 0) m /= 3;
+  if (m != 1 || n >= (1 << 16)) return false;
+  static const int radices[] = {2, 3, 4, 6, 8, 9, 12, 16};
+  for (int np = 1; n > 1 && pl.npass == 0; ++np)
+    for (int top : radices) {  // np ascending radices up to top
+      int r[CH3D_MAX_PASSES] = {0};
+      auto search = [&](auto&& self, int p, int rest, int hi) -> bool {
+        if (p == 0) return rest == 1;
+        for (int q = 7; q >= 0; --q) {
+          r[p - 1] = radices[q];
+          if (radices[q] <= hi && rest % radices[q] == 0 && self(self, p - 1, rest / radices[q], radices[q])) return true;
+        }
+        return false;
+      };
+      if (!search(search, np, n, top)) continue;
+      for (int p = 0; p < np; ++p) pl.radix[p] = r[p];
+      pl.npass = np;
+      break;
+    }
   int Ns = 1;
   for (int p = 0; p < pl.npass; ++p) {
     pl.mNB[p] = fdiv_magic((unsigned)(n / pl.radix[p]));
     pl.mNs[p] = fdiv_magic((unsigned)Ns);
+    pl.Ns[p] = Ns;
     Ns *= pl.radix[p];
   }
-  return m == 1 && pl.npass <= CH3D_MAX_PASSES && n < (1 << 16);
+  return true;
 }
 
 template <class CT>
@@ -1202,7 +1222,7 @@ int ch3d_poisson_noalloc(int nxc, int nyc, int nzc, double xlx, double zlz, cons
   if (need > (size_t)CH3D_NOALLOC_SCRATCH_BYTES)
     return fail(CH3D_ERR_INVALID, "grid %d x %d x %d needs %zu bytes of scratch, more than the %u bytes of "
                 "CH3D_NOALLOC_SCRATCH_BYTES", nxc, nyc, nzc, need, (unsigned)CH3D_NOALLOC_SCRATCH_BYTES);
-  const size_t smem = noalloc_smem(nxc, nyc, nzc);
+  const size_t smem = noalloc_smem(nyc, px, pz);
   if (smem > noalloc_smem_limit())
     return fail(CH3D_ERR_UNSUPPORTED, "grid %d x %d x %d: a transform or y-solve block of the allocation-free solve "
                 "needs %zu bytes of shared memory, more than its %zu-byte limit", nxc, nyc, nzc, smem,

@@ -129,7 +129,7 @@ cudaError_t launch_zfft_forward(ch3d_ctx* c);          // forward z transform of
 cudaError_t launch_spectra(ch3d_ctx* c, int jfor1, int jfor2);  // one sample of the 4th-order 1-D spectra
 // allocation-free Poisson solve (static device scratch, ch3d_step.cu)
 size_t noalloc_bytes(int nx, int ny, int nz);
-size_t noalloc_smem(int nx, int ny, int nz);
+size_t noalloc_smem(int ny, const FFTPlanDev& planx, const FFTPlanDev& planz);
 size_t noalloc_smem_limit();
 cudaError_t noalloc_scratch_address(int dev, void** out);
 cudaError_t poisson_noalloc(int nx, int ny, int nz, double xlx, double zlz, const double* yp, int bclo, int bchi,

@@ -1,0 +1,287 @@
+// ch3d_fft.cu -- the Poisson transforms for line lengths without a
+// register-resident plan (ch3d_rfft.cu), any product of 2 and 3, with the
+// shared-memory passes of fft.cuh:
+//   k_xfft_g   clcPrSrcOther (src/CFD_2nd/m_TScheme.f90:213-241) fused with the
+//              forward x R2C transform (m_Poisson.f90:241-333, R2HC)
+//   k_zfft_g   z transform of the spectrum, in place
+//   k_xifft_g  inverse x C2R transform * normfft -> phi (m_Poisson.f90:1194-1200)
+// The first pass forms or loads its points in registers and the last one
+// stores them (k_xfft_g: after the real-to-complex split), so global memory is
+// touched once and shared memory only between passes.
+#include "ch3d_fft.cuh"
+
+namespace ch3d {
+
+// Position of point n of a line in shared memory: one gap per 2^sh points
+// (against bank conflicts of the first pass's strided stores), none with sh = 31.
+__device__ __forceinline__ int xpad(int n, int sh) { return n + (n >> sh); }
+
+// src = div(u)/pmAlpha (modes 0, 1), packed as z_n = src_2n + i src_2n+1, complex
+// FFT of length nx/2, then the real-to-complex split
+// X_k = (Z_k + conj Z_{M-k})/2 - i W_nx^k (Z_k - conj Z_{M-k})/2, k = 0..M.
+// SRC: 0 2nd-order divergence, 1 4th-order divergence, 2 the source (mode 2), the
+// divergence (mode 3) or a field (mode 4) as it stands in the first array.
+template <class T, int SRC>
+__global__ void __launch_bounds__(256) k_xfft_g(Geo<T> g, Metrics<T> m, const T* __restrict__ ux,
+                                                const T* __restrict__ uy, const T* __restrict__ uz,
+                                                typename CplxOf<T>::type* __restrict__ spec, FFTPlanDev pl,
+                                                const typename CplxOf<T>::type* __restrict__ tw,
+                                                const typename CplxOf<T>::type* __restrict__ twr, int LPB, int LP, int sh,
+                                                int mode, DevScalars* __restrict__ sc, T* __restrict__ pr) {
+  typedef typename CplxOf<T>::type CT;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  if (sc->status) return;
+  const int nx = g.nx, ny = g.ny, nz = g.nz, M = nx / 2, nxh = g.nxh;
+  const int nlines = ny * nz;
+  const int line0 = blockIdx.x * LPB;
+  const int nl = min(LPB, nlines - line0);
+  CT* src = (CT*)smem_raw;
+  CT* dst = src + (size_t)LPB * LP;
+  const T sudtal = mode == 0 || mode == 3 ? (T)(1.0 / sc->pmAlpha) : (T)1;
+  const T rdx = g.rdx, rdz = g.rdz;
+  double dmax = 0.0;
+  auto form = [&](int l, int n) -> CT {
+    const int line = line0 + l;
+    const long long base = (long long)nx * line;
+    const int i0 = 2 * n;
+    T r0, r1;
+    if constexpr (SRC == 2) {
+      const CT s01 = __ldg(reinterpret_cast<const CT*>(ux + base + i0));  // (i0, i0+1): nx and i0 even
+      r0 = s01.x; r1 = s01.y;
+    } else {
+      const int k = line / ny, j = line - k * ny;
+      const T sucaj = m.rdyp[j + 1];
+      if constexpr (SRC == 1) {
+        const C4<T> c4(g);
+        r0 = div4_cell(g, c4, sucaj, ux, uy, uz, i0, j, k);
+        r1 = div4_cell(g, c4, sucaj, ux, uy, uz, i0 + 1, j, k);
+      } else {
+        const int i2 = i0 + 2 == nx ? 0 : i0 + 2;
+        const long long basep = k + 1 == nz ? base - (long long)nx * ny * (nz - 1) : base + (long long)nx * ny;
+        const CT u01 = __ldg(reinterpret_cast<const CT*>(ux + base + i0));
+        const T u2 = __ldg(ux + base + i2);
+        const CT v01 = __ldg(reinterpret_cast<const CT*>(uy + base + i0));
+        // uy at j+1: the next row, above the top row the wall value or, periodic in y, row 0
+        const CT v01p = j + 1 < ny ? __ldg(reinterpret_cast<const CT*>(uy + base + nx + i0))
+                        : (g.bc.hi == 0 ? __ldg(reinterpret_cast<const CT*>(uy + base - (long long)(ny - 1) * nx + i0))
+                                        : mk((T)g.bc.uy_hi, (T)g.bc.uy_hi));
+        const CT w01 = __ldg(reinterpret_cast<const CT*>(uz + base + i0));
+        const CT w01p = __ldg(reinterpret_cast<const CT*>(uz + basep + i0));
+        r0 = (u01.y - u01.x) * rdx + (v01p.x - v01.x) * sucaj + (w01p.x - w01.x) * rdz;
+        r1 = (u2 - u01.y) * rdx + (v01p.y - v01.y) * sucaj + (w01p.y - w01.y) * rdz;
+        if (mode == 0 && g.implicit == 2) {  // clcPrSrc_FIMP: pressure += -xnu/2 div (m_TScheme.f90:271)
+          const T xnuhm = -(T)0.5 * g.xnu;
+          CT* p01 = reinterpret_cast<CT*>(pr + base + i0);
+          const CT p = *p01;
+          *p01 = mk(p.x + xnuhm * r0, p.y + xnuhm * r1);
+        }
+      }
+    }
+    dmax = fmax(dmax, fmax(fabs((double)r0), fabs((double)r1)));
+    return mk(sudtal * r0, sudtal * r1);
+  };
+  fft_pass<CT, false>(pl, 0, nl, tw, form, [&](int l, int n, CT v) { src[l * LP + xpad(n, sh)] = v; });
+  __syncthreads();
+  for (int p = 1; p < pl.npass; ++p) {
+    fft_pass<CT, false>(pl, p, nl, tw, [&](int l, int n) { return src[l * LP + xpad(n, sh)]; },
+                        [&](int l, int n, CT v) { dst[l * LP + xpad(n, sh)] = v; });
+    __syncthreads();
+    CT* t = src; src = dst; dst = t;
+  }
+  const T hf = (T)0.5;
+  const unsigned long long mM1 = fdiv_magic((unsigned)(M + 1));
+  for (int t = threadIdx.x; t < nl * (M + 1); t += blockDim.x) {
+    const int l = fdiv(t, mM1), kk = t - l * (M + 1);
+    const CT a = src[l * LP + xpad(kk == M ? 0 : kk, sh)];
+    const CT b = cconj(src[l * LP + xpad(kk == 0 ? 0 : M - kk, sh)]);
+    const CT e = mk(hf * (a.x + b.x), hf * (a.y + b.y));
+    const CT dd = csub(a, b);
+    const CT o = mk(hf * dd.y, -hf * dd.x);  // (a-b)/(2i)
+    spec[(long long)nxh * (line0 + l) + kk] = cadd(e, cmul(__ldg(twr + kk), o));
+  }
+  if (mode >= 3) return;  // mode 3: its maximum was taken where the divergence was formed; 4: a plain transform
+  __shared__ double wred[8];
+  for (int o = 16; o > 0; o >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
+  if ((threadIdx.x & 31) == 0) wred[threadIdx.x >> 5] = dmax;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double v = wred[0];
+    for (int w = 1; w < (int)blockDim.x / 32; ++w) v = fmax(v, wred[w]);
+    atomic_max_nonneg(&sc->divmax1, v);
+  }
+}
+
+// z transform of the spectrum, in place: layout (kx, j, kz), lines over kz.
+// Block = up to TKX consecutive kx at one j; point n of line l at n * TKX + l.
+template <class T>
+__global__ void __launch_bounds__(256) k_zfft_g(Geo<T> g, typename CplxOf<T>::type* __restrict__ spec, FFTPlanDev pl,
+                                                const typename CplxOf<T>::type* __restrict__ tw, int TKX, int inverse,
+                                                const DevScalars* __restrict__ sc) {
+  typedef typename CplxOf<T>::type CT;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  if (sc->status) return;
+  const int nz = g.nz, nxh = g.nxh;
+  const int kx0 = blockIdx.x * TKX, nl = min(TKX, nxh - kx0);
+  const long long zs = (long long)nxh * g.ny;
+  CT* const col = spec + kx0 + (long long)nxh * blockIdx.y;
+  CT* src = (CT*)smem_raw;
+  CT* dst = src + (size_t)TKX * nz;  // used from three passes on
+  auto ldg = [&](int l, int n) { const CT v = col[zs * n + l]; return inverse ? cconj(v) : v; };
+  auto stg = [&](int l, int n, CT v) { col[zs * n + l] = inverse ? cconj(v) : v; };
+  auto lds = [&](int l, int n) { return src[n * TKX + l]; };
+  const int last = pl.npass - 1;
+  if (last == 0) {
+    fft_pass<CT, true>(pl, 0, nl, tw, ldg, stg);
+    return;
+  }
+  fft_pass<CT, true>(pl, 0, nl, tw, ldg, [&](int l, int n, CT v) { src[n * TKX + l] = v; });
+  __syncthreads();
+  for (int p = 1; p < last; ++p) {
+    fft_pass<CT, true>(pl, p, nl, tw, lds, [&](int l, int n, CT v) { dst[n * TKX + l] = v; });
+    __syncthreads();
+    CT* t = src; src = dst; dst = t;
+  }
+  fft_pass<CT, true>(pl, last, nl, tw, lds, stg);
+}
+
+// inverse x transform (complex-to-real, unnormalised as FFTW's HC2R) * normfft -> phi
+template <class T>
+__global__ void __launch_bounds__(256) k_xifft_g(Geo<T> g, const typename CplxOf<T>::type* __restrict__ spec,
+                                                 T* __restrict__ phi, FFTPlanDev pl,
+                                                 const typename CplxOf<T>::type* __restrict__ tw,
+                                                 const typename CplxOf<T>::type* __restrict__ twr, int LPB, int LP,
+                                                 int sh, T normfft, const DevScalars* __restrict__ sc) {
+  typedef typename CplxOf<T>::type CT;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  if (sc->status) return;
+  const int nx = g.nx, M = nx / 2, nxh = g.nxh;
+  const int nlines = g.ny * g.nz;
+  const int line0 = blockIdx.x * LPB;
+  const int nl = min(LPB, nlines - line0);
+  CT* src = (CT*)smem_raw;
+  CT* dst = src + (size_t)LPB * LP;
+  auto unsplit = [&](int l, int kk) -> CT {
+    const CT* X = spec + (long long)nxh * (line0 + l);
+    const CT a = X[kk];
+    const CT b = cconj(X[M - kk]);
+    const CT e = cadd(a, b);
+    const CT o = cmul(csub(a, b), cconj(__ldg(twr + kk)));
+    return cconj(mk(e.x - o.y, e.y + o.x));  // Z_k = e + i o, conjugated for the forward-transform-based inverse
+  };
+  auto out = [&](int l, int n, CT v) {
+    reinterpret_cast<CT*>(phi + (long long)nx * (line0 + l))[n] = mk(v.x * normfft, -v.y * normfft);
+  };
+  auto lds = [&](int l, int n) { return src[l * LP + xpad(n, sh)]; };
+  const int last = pl.npass - 1;
+  if (last == 0) {
+    fft_pass<CT, false>(pl, 0, nl, tw, unsplit, out);
+    return;
+  }
+  fft_pass<CT, false>(pl, 0, nl, tw, unsplit, [&](int l, int n, CT v) { src[l * LP + xpad(n, sh)] = v; });
+  __syncthreads();
+  for (int p = 1; p < last; ++p) {
+    fft_pass<CT, false>(pl, p, nl, tw, lds, [&](int l, int n, CT v) { dst[l * LP + xpad(n, sh)] = v; });
+    __syncthreads();
+    CT* t = src; src = dst; dst = t;
+  }
+  fft_pass<CT, false>(pl, last, nl, tw, lds, out);
+}
+
+// ---------------------------------------------------------------------------
+// launchers
+// ---------------------------------------------------------------------------
+constexpr int kFftSmemLimit = 200 * 1024;
+
+template <class T> static cudaError_t limits_t() {
+  const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  cudaError_t r = cudaFuncSetAttribute(k_xfft_g<T, 0>, a, kFftSmemLimit);
+  if (r == cudaSuccess) r = cudaFuncSetAttribute(k_xfft_g<T, 1>, a, kFftSmemLimit);
+  if (r == cudaSuccess) r = cudaFuncSetAttribute(k_xfft_g<T, 2>, a, kFftSmemLimit);
+  if (r == cudaSuccess) r = cudaFuncSetAttribute(k_zfft_g<T>, a, kFftSmemLimit);
+  if (r == cudaSuccess) r = cudaFuncSetAttribute(k_xifft_g<T>, a, kFftSmemLimit);
+  return r;
+}
+cudaError_t fft_generic_setup(int device) {
+  static PerDevice site;
+  return once_per_device(site, device, [] {
+    const cudaError_t r = limits_t<double>();
+    return r == cudaSuccess ? limits_t<float>() : r;
+  });
+}
+
+// Lines per x block: one round of 128 tasks in the first pass, at most 16 lines.
+template <class T> static XShape x_shape(int M, int R0) {
+  XShape s;
+  s.LPB = 128 * R0 / M < 1 ? 1 : (128 * R0 / M > 16 ? 16 : 128 * R0 / M);
+  s.sh = sizeof(T) == 8 ? 3 : 4;
+  s.LP = M + (M >> s.sh);
+  s.smem = (size_t)2 * s.LPB * s.LP * sizeof(typename CplxOf<T>::type);
+  if (s.smem > (size_t)kFftSmemLimit) {  // very long lines: no padding
+    s.sh = 31;
+    s.LP = M;
+    s.smem = (size_t)2 * s.LPB * s.LP * sizeof(typename CplxOf<T>::type);
+  }
+  s.threads = M / R0 > 128 ? 256 : 128;
+  return s;
+}
+
+template <class T>
+cudaError_t xfft_generic(const Geo<T>& g, const Metrics<T>& m, const T* a, const T* b, const T* c,
+                         typename CplxOf<T>::type* spec, const FFTPlanDev& pl, const typename CplxOf<T>::type* tw,
+                         const typename CplxOf<T>::type* twr, int mode, DevScalars* sc, T* pr, cudaStream_t st) {
+  const XShape s = x_shape<T>(g.nx / 2, pl.radix[0]);
+  const int nlines = g.ny * g.nz, grid = (nlines + s.LPB - 1) / s.LPB;
+  auto go = [&](auto kern) {
+    kern<<<grid, s.threads, s.smem, st>>>(g, m, a, b, c, spec, pl, tw, twr, s.LPB, s.LP, s.sh, mode, sc, pr);
+  };
+  if (mode >= 2) go(k_xfft_g<T, 2>);
+  else if (g.order == 4) go(k_xfft_g<T, 1>);
+  else go(k_xfft_g<T, 0>);
+  return cudaGetLastError();
+}
+
+// kx lines per z block: 128-byte segments per kz (FP32: 64-byte ones for long
+// lines), fewer where shared memory asks for it
+template <class T>
+cudaError_t zfft_generic(const Geo<T>& g, typename CplxOf<T>::type* spec, const FFTPlanDev& pl,
+                         const typename CplxOf<T>::type* tw, int inverse, const DevScalars* sc, cudaStream_t st) {
+  typedef typename CplxOf<T>::type CT;
+  const int nbuf = pl.npass <= 1 ? 0 : (pl.npass == 2 ? 1 : 2);
+  int TKX = sizeof(T) == 8 || g.nz > 256 ? 8 : 16;
+  while (TKX > 1 && (size_t)nbuf * TKX * g.nz * sizeof(CT) > (size_t)kFftSmemLimit / 2) TKX >>= 1;
+  k_zfft_g<T><<<dim3((g.nxh + TKX - 1) / TKX, g.ny), g.nz > 256 ? 256 : 128, (size_t)nbuf * TKX * g.nz * sizeof(CT),
+                st>>>(g, spec, pl, tw, TKX, inverse, sc);
+  return cudaGetLastError();
+}
+
+template <class T>
+cudaError_t xifft_generic(const Geo<T>& g, const typename CplxOf<T>::type* spec, T* phi, const FFTPlanDev& pl,
+                          const typename CplxOf<T>::type* tw, const typename CplxOf<T>::type* twr, T normfft,
+                          const DevScalars* sc, cudaStream_t st) {
+  const XShape s = x_shape<T>(g.nx / 2, pl.radix[0]);
+  const int nlines = g.ny * g.nz;
+  k_xifft_g<T><<<(nlines + s.LPB - 1) / s.LPB, s.threads, s.smem, st>>>(g, spec, phi, pl, tw, twr, s.LPB, s.LP, s.sh,
+                                                                        normfft, sc);
+  return cudaGetLastError();
+}
+
+// Largest dynamic shared memory (bytes) a transform of an nx x nz plane's lines asks for in FP64
+size_t fft_generic_smem(const FFTPlanDev& planx, const FFTPlanDev& planz) {
+  const size_t sx = x_shape<double>(planx.n, planx.radix[0]).smem;
+  const size_t sz = planz.npass <= 1 ? 0 : (size_t)(planz.npass == 2 ? 1 : 2) * planz.n * sizeof(double2);
+  return sx > sz ? sx : sz;
+}
+
+#define CH3D_FFT_INST(T)                                                                                             \
+  template cudaError_t xfft_generic<T>(const Geo<T>&, const Metrics<T>&, const T*, const T*, const T*,                \
+                                       CplxOf<T>::type*, const FFTPlanDev&, const CplxOf<T>::type*,                   \
+                                       const CplxOf<T>::type*, int, DevScalars*, T*, cudaStream_t);                   \
+  template cudaError_t zfft_generic<T>(const Geo<T>&, CplxOf<T>::type*, const FFTPlanDev&, const CplxOf<T>::type*,    \
+                                       int, const DevScalars*, cudaStream_t);                                         \
+  template cudaError_t xifft_generic<T>(const Geo<T>&, const CplxOf<T>::type*, T*, const FFTPlanDev&,                 \
+                                        const CplxOf<T>::type*, const CplxOf<T>::type*, T, const DevScalars*,         \
+                                        cudaStream_t);
+CH3D_FFT_INST(double)
+CH3D_FFT_INST(float)
+
+}  // namespace ch3d

@@ -1,0 +1,28 @@
+// ch3d_fft.cuh -- launchers of the generic-length Poisson transforms
+// (ch3d_fft.cu); fft_generic_setup(device) once before the first launch.
+#pragma once
+#include "ch3d_dev.cuh"
+
+namespace ch3d {
+
+struct XShape {
+  int LPB, LP, sh, threads;  // lines per block, padded line length, padding shift
+  size_t smem;
+};
+
+cudaError_t fft_generic_setup(int device);
+size_t fft_generic_smem(const FFTPlanDev& planx, const FFTPlanDev& planz);
+// mode: 0 div(u*)/pmAlpha of (a, b, c), 1 div(u), 2 source in a, 3 divergence in a, /pmAlpha, 4 field in a
+template <class T>
+cudaError_t xfft_generic(const Geo<T>& g, const Metrics<T>& m, const T* a, const T* b, const T* c,
+                         typename CplxOf<T>::type* spec, const FFTPlanDev& pl, const typename CplxOf<T>::type* tw,
+                         const typename CplxOf<T>::type* twr, int mode, DevScalars* sc, T* pr, cudaStream_t st);
+template <class T>
+cudaError_t zfft_generic(const Geo<T>& g, typename CplxOf<T>::type* spec, const FFTPlanDev& pl,
+                         const typename CplxOf<T>::type* tw, int inverse, const DevScalars* sc, cudaStream_t st);
+template <class T>
+cudaError_t xifft_generic(const Geo<T>& g, const typename CplxOf<T>::type* spec, T* phi, const FFTPlanDev& pl,
+                          const typename CplxOf<T>::type* tw, const typename CplxOf<T>::type* twr, T normfft,
+                          const DevScalars* sc, cudaStream_t st);
+
+}  // namespace ch3d

@@ -21,6 +21,7 @@
 #include <vector>
 #include "ch3d_ctx.h"
 #include "ch3d_dev.cuh"
+#include "ch3d_fft.cuh"
 
 namespace ch3d {
 
@@ -479,124 +480,6 @@ __global__ void __launch_bounds__(256) k_uhat_pimp(Geo<T> g, const double* __res
 }
 
 // ---------------------------------------------------------------------------
-// clcPrSrcOther (src/CFD_2nd/m_TScheme.f90:213-241) fused with the forward
-// x transform: src = div(u)/pmAlpha, packed as z_n = src_2n + i src_2n+1,
-// complex FFT of length nx/2, then the real-to-complex split
-// X_k = (Z_k + conj Z_{M-k})/2 - i W_nx^k (Z_k - conj Z_{M-k})/2, k = 0..M.
-// ---------------------------------------------------------------------------
-template <class T>
-__global__ void __launch_bounds__(256) k_prsrc_xfft(Geo<T> g, Metrics<T> m, const T* __restrict__ ux,
-                                                    const T* __restrict__ uy, const T* __restrict__ uz,
-                                                    typename CplxOf<T>::type* __restrict__ spec, FFTPlanDev pl,
-                                                    const typename CplxOf<T>::type* __restrict__ tw,
-                                                    const typename CplxOf<T>::type* __restrict__ twr, int LPB, int mode,
-                                                    DevScalars* __restrict__ sc, T* __restrict__ pr) {
-  typedef typename CplxOf<T>::type CT;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  if (sc->status) return;
-  const int nx = g.nx, ny = g.ny, nz = g.nz, M = nx / 2, nxh = g.nxh;
-  const int nlines = ny * nz;
-  const int line0 = blockIdx.x * LPB;
-  const int nl = min(LPB, nlines - line0);
-  CT* A = (CT*)smem_raw;
-  CT* B = A + (size_t)LPB * M;
-  const T sudtal = mode == 0 ? (T)(1.0 / sc->pmAlpha) : (T)1;
-  const T rdx = g.rdx, rdz = g.rdz;
-  double dmax = 0.0;
-  for (int t = threadIdx.x; t < nl * M; t += blockDim.x) {
-    const int l = t / M, n = t % M;
-    const int line = line0 + l;
-    const int j = line % ny, k = line / ny;
-    const int kp = wrapp(k, nz);
-    const int i0 = 2 * n, i1 = 2 * n + 1, i2 = wrapp(i1, nx);
-    const long long base = (long long)nx * (j + (long long)ny * k);
-    const T sucaj = m.rdyp[j + 1];
-    const T u0 = ux[base + i0], u1 = ux[base + i1], u2 = ux[base + i2];
-    const T v0 = uy[base + i0], v1 = uy[base + i1];
-    const T v0p = fld(uy, g, 1, i0, j + 1, k), v1p = fld(uy, g, 1, i1, j + 1, k);
-    const long long basep = (long long)nx * (j + (long long)ny * kp);
-    const T w0 = uz[base + i0], w1 = uz[base + i1];
-    const T w0p = uz[basep + i0], w1p = uz[basep + i1];
-    T r0 = (u1 - u0) * rdx + (v0p - v0) * sucaj + (w0p - w0) * rdz;
-    T r1 = (u2 - u1) * rdx + (v1p - v1) * sucaj + (w1p - w1) * rdz;
-    if (g.order == 4) {
-      const C4<T> c4(g);
-      r0 = div4_cell(g, c4, sucaj, ux, uy, uz, i0, j, k);
-      r1 = div4_cell(g, c4, sucaj, ux, uy, uz, i1, j, k);
-    }
-    if (mode == 2 || mode == 4) { r0 = u0; r1 = u1; }  // ux carries the source (standalone Poisson) or the field
-    if (mode == 0 && g.implicit == 2) {     // clcPrSrc_FIMP: pressure += -xnu/2 div (m_TScheme.f90:271)
-      const T xnuhm = -(T)0.5 * g.xnu;
-      pr[base + i0] = pr[base + i0] + xnuhm * r0;
-      pr[base + i1] = pr[base + i1] + xnuhm * r1;
-    }
-    dmax = fmax(dmax, fmax(fabs((double)r0), fabs((double)r1)));
-    A[l * M + n] = mk(sudtal * r0, sudtal * r1);
-  }
-  // block max of |div| (any block size up to 1024)
-  {
-    __shared__ double wred[32];
-    for (int o = 16; o > 0; o >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
-    if ((threadIdx.x & 31) == 0) wred[threadIdx.x >> 5] = dmax;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      double v = threadIdx.x < (blockDim.x + 31) / 32 ? wred[threadIdx.x] : 0.0;
-      for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-      if (threadIdx.x == 0 && mode != 4) atomic_max_nonneg(&sc->divmax1, v);
-    }
-    __syncthreads();
-  }
-  const CT* Z = fft_lines<CT, false>(A, B, pl, nl, M, 1, tw);
-  const T hf = (T)0.5;
-  for (int t = threadIdx.x; t < nl * (M + 1); t += blockDim.x) {
-    const int l = t / (M + 1), kk = t % (M + 1);
-    const CT a = Z[l * M + (kk == M ? 0 : kk)];
-    const CT b = cconj(Z[l * M + (kk == 0 ? 0 : M - kk)]);
-    const CT e = mk(hf * (a.x + b.x), hf * (a.y + b.y));
-    const CT dd = csub(a, b);
-    const CT o = mk(hf * dd.y, -hf * dd.x);  // (a-b)/(2i)
-    const CT w = __ldg(twr + kk);
-    spec[(long long)nxh * (line0 + l) + kk] = cadd(e, cmul(w, o));
-  }
-}
-
-// ---------------------------------------------------------------------------
-// z transform of the spectrum, in place: layout (kx, j, kz), lines over kz.
-// Block = TKX consecutive kx at one j; lines interleaved in shared memory.
-// ---------------------------------------------------------------------------
-template <class T>
-__global__ void __launch_bounds__(256) k_zfft(Geo<T> g, typename CplxOf<T>::type* __restrict__ spec, FFTPlanDev pl,
-                                              const typename CplxOf<T>::type* __restrict__ tw, int TKX, int inverse,
-                                              const DevScalars* __restrict__ sc) {
-  typedef typename CplxOf<T>::type CT;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  if (sc->status) return;
-  const int nz = g.nz, ny = g.ny, nxh = g.nxh;
-  const int kx0 = blockIdx.x * TKX, j = blockIdx.y;
-  CT* A = (CT*)smem_raw;
-  CT* B = A + (size_t)TKX * nz;
-  const long long zs = (long long)nxh * ny;
-  for (int t = threadIdx.x; t < TKX * nz; t += blockDim.x) {
-    const int l = t % TKX, kz = t / TKX;
-    const int kx = kx0 + l;
-    CT v = mk((T)0, (T)0);
-    if (kx < nxh) v = spec[kx + (long long)nxh * j + zs * kz];
-    if (inverse) v = cconj(v);
-    A[kz * TKX + l] = v;
-  }
-  __syncthreads();
-  const CT* Z = fft_lines<CT, true>(A, B, pl, TKX, 1, TKX, tw);
-  for (int t = threadIdx.x; t < TKX * nz; t += blockDim.x) {
-    const int l = t % TKX, kz = t / TKX;
-    const int kx = kx0 + l;
-    if (kx >= nxh) continue;
-    CT v = Z[kz * TKX + l];
-    if (inverse) v = cconj(v);
-    spec[kx + (long long)nxh * j + zs * kz] = v;
-  }
-}
-
-// ---------------------------------------------------------------------------
 // y tridiagonal per (kx,kz) (src/CFD_2nd/m_Poisson.f90:1114-1156):
 // [am2Pr, ac2Pr + WaveNumX + WaveNumZ, ap2Pr], with the (kx,kz)=(0,0) system's
 // first row replaced by the identity and zero right-hand side.  Solved in FP64
@@ -714,47 +597,6 @@ __global__ void __launch_bounds__(256) k_ysolve(Geo<T> g, Metrics<double> m, con
     if (p > 0) { const double al = AL[t]; x.x += al * G[2 * (p - 1)].x; x.y += al * G[2 * (p - 1)].y; }
     if (p < P - 1) { const double be = CP[t]; x.x += be * G[2 * p + 1].x; x.y += be * G[2 * p + 1].y; }
     spec[kx + (long long)nxh * j + zs * kz] = mk((T)x.x, (T)x.y);
-  }
-}
-
-// ---------------------------------------------------------------------------
-// inverse x transform (complex-to-real, unnormalised as FFTW's HC2R) * normfft
-// (src/CFD_2nd/m_Poisson.f90:1194-1200) -> phi.
-// ---------------------------------------------------------------------------
-template <class T>
-__global__ void __launch_bounds__(256) k_xifft(Geo<T> g, const typename CplxOf<T>::type* __restrict__ spec,
-                                               T* __restrict__ phi, FFTPlanDev pl,
-                                               const typename CplxOf<T>::type* __restrict__ tw,
-                                               const typename CplxOf<T>::type* __restrict__ twr, int LPB, T normfft,
-                                               const DevScalars* __restrict__ sc) {
-  typedef typename CplxOf<T>::type CT;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  if (sc->status) return;
-  const int nx = g.nx, ny = g.ny, nz = g.nz, M = nx / 2, nxh = g.nxh;
-  const int nlines = ny * nz;
-  const int line0 = blockIdx.x * LPB;
-  const int nl = min(LPB, nlines - line0);
-  CT* A = (CT*)smem_raw;
-  CT* B = A + (size_t)LPB * M;
-  for (int t = threadIdx.x; t < nl * M; t += blockDim.x) {
-    const int l = t / M, kk = t % M;
-    const CT* X = spec + (long long)nxh * (line0 + l);
-    const CT a = X[kk];
-    const CT b = cconj(X[M - kk]);
-    const CT e = cadd(a, b);
-    const CT o = cmul(csub(a, b), cconj(__ldg(twr + kk)));
-    // Z_k = e + i o ; stored conjugated for the forward-transform-based inverse
-    const CT z = mk(e.x - o.y, e.y + o.x);
-    A[l * M + kk] = cconj(z);
-  }
-  __syncthreads();
-  const CT* Z = fft_lines<CT, false>(A, B, pl, nl, M, 1, tw);
-  for (int t = threadIdx.x; t < nl * M; t += blockDim.x) {
-    const int l = t / M, n = t % M;
-    const CT z = cconj(Z[l * M + n]);
-    const long long base = (long long)nx * (line0 + l);
-    phi[base + 2 * n] = z.x * normfft;
-    phi[base + 2 * n + 1] = z.y * normfft;
   }
 }
 
@@ -1111,101 +953,43 @@ template <class T> static cudaError_t uhat_t(ch3d_ctx* c) {
 cudaError_t launch_uhat(ch3d_ctx* c) { return c->fp32 ? uhat_t<float>(c) : uhat_t<double>(c); }
 
 
-// Shared-memory budget of one FFT block (two ping-pong buffers): three
-// blocks of 256 threads fit in an SM.
-static const int kFFTSmem = 74 * 1024;
-
-template <class T> static int lines_per_block(int M) {
-  int lpb = kFFTSmem / (2 * M * (int)sizeof(typename CplxOf<T>::type));
-  if (lpb > 16) lpb = 16;
-  if (lpb < 1) lpb = 1;
-  return lpb;
-}
-
+// The register-resident transforms where the length has a plan, else the generic ones (ch3d_fft.cu).
 template <class T> static cudaError_t prsrc_t(ch3d_ctx* c, int mode) {
   typedef typename CplxOf<T>::type CT;
   cudaError_t e;
-  if (launch_prsrc_xfft_r(c, mode, &e)) return e;  // register FFT when the length has a plan
+  if (launch_prsrc_xfft_r(c, mode, &e)) return e;
+  if ((e = fft_generic_setup(c->device)) != cudaSuccess) return e;
   T** f = (T**)c->f;
-  const int M = c->nx / 2;
-  const int LPB = lines_per_block<T>(M);
-  const int nlines = c->ny * c->nz;
-  size_t smem = (size_t)2 * LPB * M * sizeof(CT);
-  static PerDevice attr;  // per precision (template instance)
-  if ((e = smem_limit_once(attr, c->device, k_prsrc_xfft<T>, 200 * 1024)) != cudaSuccess) return e;
-  const int nthr = 256;
-  T* a = mode == 2 || mode == 4 ? f[10] : (mode == 1 ? f[0] : f[12]);
-  T* b = mode == 1 ? f[1] : f[13];
-  T* cz = mode == 1 ? f[2] : f[14];
-  k_prsrc_xfft<T><<<(nlines + LPB - 1) / LPB, nthr, smem, c->stream>>>(make_geo<T>(c), metrics_of<T>(c), a, b, cz,
-                                                                      (CT*)c->spec, c->planx, (const CT*)c->twx,
-                                                                      (const CT*)c->twr, LPB, mode, c->sc, f[3]);
-  return cudaGetLastError();
+  const T* a = mode >= 2 ? f[10] : (mode == 1 ? f[0] : f[12]);
+  return xfft_generic<T>(make_geo<T>(c), metrics_of<T>(c), a, mode == 1 ? f[1] : f[13], mode == 1 ? f[2] : f[14],
+                         (CT*)c->spec, c->planx, (const CT*)c->twx, (const CT*)c->twr, mode, c->sc, f[3], c->stream);
 }
 cudaError_t launch_prsrc_xfft(ch3d_ctx* c, int mode) { return c->fp32 ? prsrc_t<float>(c, mode) : prsrc_t<double>(c, mode); }
 
-template <class T> static cudaError_t spectral_t(ch3d_ctx* c) {
-  typedef typename CplxOf<T>::type CT;
-  const int nz = c->nz;
-  cudaError_t e;
-  const bool zr = launch_zfft_r(c, 0, &e);  // register FFT when nz has a plan
-  if (zr && e != cudaSuccess) return e;
-  int TKX = kFFTSmem / (2 * nz * (int)sizeof(CT));
-  int t = 1;
-  while (t * 2 <= TKX && t * 2 <= 16) t *= 2;
-  TKX = t;
-  size_t smemz = (size_t)2 * TKX * nz * sizeof(CT);
-  const int nthrz = 256;
-  static PerDevice attr;  // per precision (template instance)
-  if ((e = smem_limit_once(attr, c->device, k_zfft<T>, 200 * 1024)) != cudaSuccess) return e;
-  dim3 gz((c->nxh + TKX - 1) / TKX, c->ny);
-  if (!zr) {
-    k_zfft<T><<<gz, nthrz, smemz, c->stream>>>(make_geo<T>(c), (CT*)c->spec, c->planz, (const CT*)c->twz, TKX, 0, c->sc);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
-  if ((e = launch_ysolve(c)) != cudaSuccess) return e;
-  if (launch_zfft_r(c, 1, &e)) return e;
-  k_zfft<T><<<gz, nthrz, smemz, c->stream>>>(make_geo<T>(c), (CT*)c->spec, c->planz, (const CT*)c->twz, TKX, 1, c->sc);
-  return cudaGetLastError();
-}
-// Forward z transform of the spectrum alone (the first step of the spectral solve).
-template <class T> static cudaError_t zfft_fwd_t(ch3d_ctx* c) {
+template <class T> static cudaError_t zfft_t(ch3d_ctx* c, int inverse) {
   typedef typename CplxOf<T>::type CT;
   cudaError_t e;
-  if (launch_zfft_r(c, 0, &e)) return e;
-  const int nz = c->nz;
-  int TKX = kFFTSmem / (2 * nz * (int)sizeof(CT));
-  int t = 1;
-  while (t * 2 <= TKX && t * 2 <= 16) t *= 2;
-  TKX = t;
-  static PerDevice attr;  // per precision (template instance)
-  if ((e = smem_limit_once(attr, c->device, k_zfft<T>, 200 * 1024)) != cudaSuccess) return e;
-  dim3 gz((c->nxh + TKX - 1) / TKX, c->ny);
-  k_zfft<T><<<gz, 256, (size_t)2 * TKX * nz * sizeof(CT), c->stream>>>(make_geo<T>(c), (CT*)c->spec, c->planz,
-                                                                      (const CT*)c->twz, TKX, 0, c->sc);
-  return cudaGetLastError();
+  if (launch_zfft_r(c, inverse, &e)) return e;
+  if ((e = fft_generic_setup(c->device)) != cudaSuccess) return e;
+  return zfft_generic<T>(make_geo<T>(c), (CT*)c->spec, c->planz, (const CT*)c->twz, inverse, c->sc, c->stream);
 }
-cudaError_t launch_zfft_forward(ch3d_ctx* c) { return c->fp32 ? zfft_fwd_t<float>(c) : zfft_fwd_t<double>(c); }
+static cudaError_t zfft(ch3d_ctx* c, int inverse) { return c->fp32 ? zfft_t<float>(c, inverse) : zfft_t<double>(c, inverse); }
+// forward z transform of the spectrum alone (the first step of the spectral solve)
+cudaError_t launch_zfft_forward(ch3d_ctx* c) { return zfft(c, 0); }
 
-cudaError_t launch_poisson_spectral(ch3d_ctx* c) { return c->fp32 ? spectral_t<float>(c) : spectral_t<double>(c); }
+cudaError_t launch_poisson_spectral(ch3d_ctx* c) {
+  cudaError_t e = zfft(c, 0);
+  if (e == cudaSuccess) e = launch_ysolve(c);
+  return e == cudaSuccess ? zfft(c, 1) : e;
+}
 
 template <class T> static cudaError_t xifft_t(ch3d_ctx* c) {
   typedef typename CplxOf<T>::type CT;
   cudaError_t e;
-  if (launch_xifft_r(c, &e)) return e;  // register FFT when the length has a plan
-  T** f = (T**)c->f;
-  const int M = c->nx / 2;
-  const int LPB = lines_per_block<T>(M);
-  const int nlines = c->ny * c->nz;
-  size_t smem = (size_t)2 * LPB * M * sizeof(CT);
-  static PerDevice attr;  // per precision (template instance)
-  if ((e = smem_limit_once(attr, c->device, k_xifft<T>, 200 * 1024)) != cudaSuccess) return e;
-  const int nthr = 256;
-  k_xifft<T><<<(nlines + LPB - 1) / LPB, nthr, smem, c->stream>>>(make_geo<T>(c), (const CT*)c->spec, f[10], c->planx,
-                                                                 (const CT*)c->twx, (const CT*)c->twr, LPB,
-                                                                 (T)c->normfft, c->sc);
-  return cudaGetLastError();
+  if (launch_xifft_r(c, &e)) return e;
+  if ((e = fft_generic_setup(c->device)) != cudaSuccess) return e;
+  return xifft_generic<T>(make_geo<T>(c), (const CT*)c->spec, (T*)c->f[10], c->planx, (const CT*)c->twx,
+                          (const CT*)c->twr, (T)c->normfft, c->sc, c->stream);
 }
 cudaError_t launch_xifft(ch3d_ctx* c) { return c->fp32 ? xifft_t<float>(c) : xifft_t<double>(c); }
 
@@ -1470,10 +1254,8 @@ cudaError_t noalloc_scratch_address(int dev, void** out) {
     cudaError_t r = cudaGetSymbolAddress(&p, g_noalloc_scratch);
     if (r != cudaSuccess) return r;
     const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    if ((r = cudaFuncSetAttribute(k_prsrc_xfft<double>, a, kNoallocSmemLimit)) != cudaSuccess) return r;
-    if ((r = cudaFuncSetAttribute(k_zfft<double>, a, kNoallocSmemLimit)) != cudaSuccess) return r;
+    if ((r = fft_generic_setup(dev)) != cudaSuccess) return r;
     if ((r = cudaFuncSetAttribute(k_ysolve<double>, a, kNoallocSmemLimit)) != cudaSuccess) return r;
-    if ((r = cudaFuncSetAttribute(k_xifft<double>, a, kNoallocSmemLimit)) != cudaSuccess) return r;
     g_noalloc_addr[dev] = p;
     return cudaSuccess;
   });
@@ -1481,40 +1263,29 @@ cudaError_t noalloc_scratch_address(int dev, void** out) {
   return e;
 }
 
-// Launch shapes of the allocation-free solve: x-transform lines per block,
-// z-transform kx lines per block, y-solve threads per system, and the dynamic
-// shared memory of the x, z and y kernels.
+// Launch shape of the allocation-free solve's y kernel: threads per system,
+// systems per block and its dynamic shared memory.
 struct NoallocShape {
-  int LPB, TKX, P, TS;
-  size_t smx, smz, smy;
+  int P, TS;
+  size_t smy;
 };
-static NoallocShape noalloc_shape(int nx, int ny, int nz) {
+static NoallocShape noalloc_shape(int ny) {
   NoallocShape s;
-  const int M = nx / 2;
-  s.LPB = lines_per_block<double>(M);
-  int TKX = kFFTSmem / (2 * nz * (int)sizeof(double2));
-  int tk = 1;
-  while (tk * 2 <= TKX && tk * 2 <= 16) tk *= 2;
-  s.TKX = tk;
   int P = 16;
   while (P > 1 && ny < 2 * P) P >>= 1;
   s.P = P;
   s.TS = 8;
   const int Q = P - 1;
-  s.smx = (size_t)2 * s.LPB * M * sizeof(double2);
-  s.smz = (size_t)2 * s.TKX * nz * sizeof(double2);
   s.smy = (size_t)ny * s.TS * (sizeof(double2) + 2 * sizeof(double)) +
           (size_t)s.TS * (Q > 0 ? Q : 1) * (2 * sizeof(double2) + 5 * sizeof(double)) + 16;
   return s;
 }
 
-// Largest dynamic shared memory (bytes) one kernel of the solve of an
-// nx x ny x nz grid asks for; the solve runs only where it is within
-// noalloc_smem_limit().
-size_t noalloc_smem(int nx, int ny, int nz) {
-  const NoallocShape s = noalloc_shape(nx, ny, nz);
-  size_t m = s.smx > s.smz ? s.smx : s.smz;
-  return m > s.smy ? m : s.smy;
+// Largest dynamic shared memory (bytes) one kernel of the solve asks for; the
+// solve runs only where it is within noalloc_smem_limit().
+size_t noalloc_smem(int ny, const FFTPlanDev& planx, const FFTPlanDev& planz) {
+  const size_t f = fft_generic_smem(planx, planz), y = noalloc_shape(ny).smy;
+  return f > y ? f : y;
 }
 size_t noalloc_smem_limit() { return (size_t)kNoallocSmemLimit; }
 
@@ -1602,20 +1373,16 @@ cudaError_t poisson_noalloc(int nx, int ny, int nz, double xlx, double zlz, cons
   const double2* twz = tw + 2 * M + 1;
 
   // forward x transform of the source (mode 2: the source is read as is)
-  const NoallocShape sh = noalloc_shape(nx, ny, nz);
-  const int LPB = sh.LPB, TKX = sh.TKX, P = sh.P, TS = sh.TS;
-  const int nlines = ny * nz;
-  k_prsrc_xfft<double><<<(nlines + LPB - 1) / LPB, 256, sh.smx, st>>>(g, m, d_src, d_src, d_src, spec, planx, twx,
-                                                                      twr, LPB, 2, sc, nullptr);
-  dim3 gz((nxh + TKX - 1) / TKX, ny);
-  k_zfft<double><<<gz, 256, sh.smz, st>>>(g, spec, planz, twz, TKX, 0, sc);
-  k_ysolve<double><<<dim3((nxh + TS - 1) / TS, nz), TS * P < 64 ? 64 : TS * P, sh.smy, st>>>(g, m, wave, spec, TS, P,
-                                                                                              sc);
-  k_zfft<double><<<gz, 256, sh.smz, st>>>(g, spec, planz, twz, TKX, 1, sc);
-  k_xifft<double><<<(nlines + LPB - 1) / LPB, 256, sh.smx, st>>>(g, spec, d_phi, planx, twx, twr, LPB,
-                                                                 1.0 / ((double)nx * (double)nz), sc);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
+  const NoallocShape sh = noalloc_shape(ny);
+  if ((e = xfft_generic<double>(g, m, d_src, d_src, d_src, spec, planx, twx, twr, 2, sc, nullptr, st)) != cudaSuccess ||
+      (e = zfft_generic<double>(g, spec, planz, twz, 0, sc, st)) != cudaSuccess)
+    return e;
+  k_ysolve<double><<<dim3((nxh + sh.TS - 1) / sh.TS, nz), sh.TS * sh.P < 64 ? 64 : sh.TS * sh.P, sh.smy, st>>>(
+      g, m, wave, spec, sh.TS, sh.P, sc);
+  if ((e = cudaGetLastError()) != cudaSuccess ||
+      (e = zfft_generic<double>(g, spec, planz, twz, 1, sc, st)) != cudaSuccess ||
+      (e = xifft_generic<double>(g, spec, d_phi, planx, twx, twr, 1.0 / ((double)nx * (double)nz), sc, st)) != cudaSuccess)
+    return e;
   // the host tables above are pageable and local to this call
   return cudaStreamSynchronize(st);
 }

@@ -17,60 +17,6 @@
 
 namespace ch3d {
 
-// multiply by the constant (c, s) = cos - i sin pattern of a twiddle
-template <class CT, class RT> __device__ __forceinline__ CT cmulk(CT a, RT c, RT s) {
-  return mk(a.x * c - a.y * s, a.x * s + a.y * c);
-}
-
-// forward radix-8: two radix-4 transforms of the even and odd points, W8 = exp(-i pi/4)
-template <class CT> struct Bfly<CT, 8> {
-  static __device__ __forceinline__ void run(CT* v) {
-    typedef decltype(v[0].x) RT;
-    const RT h = (RT)0.70710678118654752440084436210484903928;  // sqrt(1/2)
-    CT e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
-    Bfly<CT, 4>::run(e);
-    Bfly<CT, 4>::run(o);
-    const CT o1 = mk(h * (o[1].x + o[1].y), h * (o[1].y - o[1].x));   // W8^1 o1
-    const CT o2 = mk(o[2].y, -o[2].x);                                // W8^2 o2 = -i o2
-    const CT o3 = mk(h * (o[3].y - o[3].x), -h * (o[3].x + o[3].y));  // W8^3 o3
-    v[0] = cadd(e[0], o[0]); v[4] = csub(e[0], o[0]);
-    v[1] = cadd(e[1], o1);   v[5] = csub(e[1], o1);
-    v[2] = cadd(e[2], o2);   v[6] = csub(e[2], o2);
-    v[3] = cadd(e[3], o3);   v[7] = csub(e[3], o3);
-  }
-};
-
-// forward radix-12 as 4 x 3: n = 3 n1 + n2, k = k1 + 4 k2; radix-4 over n1,
-// twiddle W12^(n2 k1), radix-3 over n2
-template <class CT> struct Bfly<CT, 12> {
-  static __device__ __forceinline__ void run(CT* v) {
-    typedef decltype(v[0].x) RT;
-    const RT s3 = (RT)0.86602540378443864676372317075293618;  // sqrt(3)/2
-    const RT hf = (RT)0.5;
-    CT y[3][4];
-#pragma unroll
-    for (int n2 = 0; n2 < 3; ++n2) {
-#pragma unroll
-      for (int n1 = 0; n1 < 4; ++n1) y[n2][n1] = v[3 * n1 + n2];
-      Bfly<CT, 4>::run(y[n2]);
-    }
-    // W12^1 = (s3, -1/2), W12^2 = (1/2, -s3), W12^3 = -i, W12^4 = (-1/2, -s3), W12^6 = -1
-    y[1][1] = cmulk(y[1][1], s3, -hf);
-    y[1][2] = cmulk(y[1][2], hf, -s3);
-    y[1][3] = mk(y[1][3].y, -y[1][3].x);
-    y[2][1] = cmulk(y[2][1], hf, -s3);
-    y[2][2] = cmulk(y[2][2], -hf, -s3);
-    y[2][3] = mk(-y[2][3].x, -y[2][3].y);
-#pragma unroll
-    for (int k1 = 0; k1 < 4; ++k1) {
-      CT w[3] = {y[0][k1], y[1][k1], y[2][k1]};
-      Bfly<CT, 3>::run(w);
-#pragma unroll
-      for (int k2 = 0; k2 < 3; ++k2) v[k1 + 4 * k2] = w[k2];
-    }
-  }
-};
-
 struct WarpSync {
   __device__ __forceinline__ void operator()() const { __syncwarp(); }
 };
