@@ -485,12 +485,11 @@ static bool march_path(const ch3d_ctx* c) {
 }
 
 int record_step(ch3d_ctx* c) {
-  CU(launch_step_begin(c));
-  if (c->cfg.LES_type > 0) CU(launch_sgs_nut(c));  // once per step, after the CFL (m_ChannelSystem.f90:89)
+  if (c->cfg.LES_type > 0) CU(launch_sgs_nut(c));  // once per step (m_ChannelSystem.f90:89)
   const bool o4 = c->cfg.order == 4, fimp = c->cfg.order == 2 && c->cfg.IsImplicit == 2;
   for (int ns = 1; ns <= c->iadvance; ++ns) {
     if (o4) CU(launch_visc4_partials(c));
-    CU(launch_substep_setup(c, ns));
+    CU(launch_substep_setup(c, ns, true));
     if (march_path(c)) {  // RHS + y solves as one column march, its own Thomas factors
       CU(launch_rhs_march(c));
     } else if (c->cfg.LES_type > 0) {  // the LES y solves form their own coefficients (FEXP: none)
@@ -519,7 +518,6 @@ int record_step(ch3d_ctx* c) {
     CU(launch_poisson_spectral(c));
     CU(launch_xifft(c));
     if (ns == c->iadvance && march_diag_fusable(c)) {  // CheckDivergence etc. ride on the last projection
-      CU(launch_diag_reset(c));
       CU(c->gsub ? launch_proj_bsub(c, true) : launch_proj_diag(c));
     } else {
       CU(c->gsub ? launch_proj_bsub(c, false) : launch_proj(c, 0));
@@ -857,7 +855,7 @@ int ch3d_stage(ch3d_ctx* c, int stage, int ns) {
   switch (stage) {
     case 0:
       if (c->cfg.order == 4) CU(launch_visc4_partials(c));  // forcing of clcRhsXYZ from the current ux
-      CU(launch_substep_setup(c, ns));
+      CU(launch_substep_setup(c, ns, false));
       break;
     case 1:
       if (c->cfg.LES_type > 0) CU(launch_rhs_les(c));
@@ -1147,11 +1145,11 @@ int ch3d_kernel_times(ch3d_ctx* c, int nsteps, double* out, int nout) {
   auto mark = [&](int g) { grp.push_back(g); return cudaEventRecord(ev[q++], c->stream); };
   auto done = [&]() { return cudaEventRecord(ev[q++], c->stream); };
   for (int s = 0; s < nsteps; ++s) {
-    CU(mark(6)); CU(launch_step_begin(c)); if (c->cfg.LES_type > 0) CU(launch_sgs_nut(c)); CU(done());
+    CU(mark(6)); if (c->cfg.LES_type > 0) CU(launch_sgs_nut(c)); CU(done());
     for (int ns = 1; ns <= c->iadvance; ++ns) {
       CU(mark(6));
       if (c->cfg.order == 4) CU(launch_visc4_partials(c));
-      CU(launch_substep_setup(c, ns));
+      CU(launch_substep_setup(c, ns, true));
       if (!march_path(c) && c->cfg.order != 4 && c->cfg.LES_type == 0 && !y_periodic(c) && c->cfg.IsImplicit != 0)
         CU(launch_helm_factors(c));
       CU(done());
@@ -1182,8 +1180,7 @@ int ch3d_kernel_times(ch3d_ctx* c, int nsteps, double* out, int nout) {
       CU(mark(3)); CU(launch_poisson_spectral(c)); CU(done());
       CU(mark(4)); CU(launch_xifft(c)); CU(done());
       if (ns == c->iadvance && march_diag_fusable(c)) {
-        CU(mark(5)); CU(launch_diag_reset(c));
-        CU(c->gsub ? launch_proj_bsub(c, true) : launch_proj_diag(c)); CU(done());
+        CU(mark(5)); CU(c->gsub ? launch_proj_bsub(c, true) : launch_proj_diag(c)); CU(done());
       } else {
         CU(mark(5)); CU(c->gsub ? launch_proj_bsub(c, false) : launch_proj(c, 0)); CU(done());
       }

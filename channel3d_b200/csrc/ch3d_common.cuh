@@ -89,7 +89,8 @@ struct DevScalars {
   double cflmp, uxm, s1tot1;
   double utau;                                          // LES: wall friction velocity of the step
   unsigned long long divmax1, divmax2, vmax[3], uddx;  // bit patterns of non-negative doubles
-  int itime, status, ns, pad;
+  int itime, status, ns;
+  unsigned ticket;                                      // blocks of the scalar kernels that have finished
 };
 
 // Metric vectors (FP64 master copies; FP32 copies for the mixed path).

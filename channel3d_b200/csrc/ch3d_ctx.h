@@ -94,8 +94,8 @@ namespace ch3d {
 // y periodic (BcOption(3:4) = 0): the triply periodic steps (FIMP_000, PIMP_0)
 inline bool y_periodic(const ch3d_ctx* c) { return c->cfg.BcOption[2] == 0; }
 // launchers (ch3d_step.cu)
-cudaError_t launch_substep_setup(ch3d_ctx* c, int ns);
-cudaError_t launch_step_begin(ch3d_ctx* c);
+cudaError_t launch_substep_setup(ch3d_ctx* c, int ns, bool whole_step);  // whole_step: with the step's CFL and dt (ns 1)
+                                                                         // and the reset of its maxima (last ns)
 cudaError_t launch_step_end(ch3d_ctx* c);
 cudaError_t launch_rhs(ch3d_ctx* c);
 cudaError_t launch_uhat(ch3d_ctx* c);                  // stage path: Rhs arrays -> u*
@@ -137,7 +137,6 @@ cudaError_t poisson_noalloc(int nx, int ny, int nz, double xlx, double zlz, cons
                             const FFTPlanDev& planz);
 cudaError_t launch_proj(ch3d_ctx* c, int mode);        // mode 0: u = u* - a grad phi, p update; 1: u -= grad phi
 cudaError_t launch_proj_diag(ch3d_ctx* c);             // last substep: projection + step diagnostics (march path)
-cudaError_t launch_diag_reset(ch3d_ctx* c);
 cudaError_t launch_bulk_partials(ch3d_ctx* c);
 cudaError_t launch_diag(ch3d_ctx* c);
 int diag_npart(const ch3d_ctx* c);                     // partial sums k_diag writes to part2

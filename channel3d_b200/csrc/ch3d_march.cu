@@ -20,95 +20,9 @@
 // file substitute u* themselves (13 values of global traffic per cell: ux uy
 // uz p, Hist x3 read + written, g x3 written).  Where the march substitutes
 // itself, g is read back and u* written as well (19 values).
-#include "ch3d_ctx.h"
-#include "ch3d_dev.cuh"
+#include "ch3d_march.cuh"
 
 namespace ch3d {
-
-// Row table of the march (precision T, MT_W values per row j = 0..ny-1):
-// the y metrics at jc = j + 1 and the Thomas factors a, 1/m, c/m of the two
-// Helmholtz sets (set 0: ux and uz, set 1: uy; m_TSchemePIMP_inc.f90:392-430,
-// 542-589, 702-740).  cp of the last row is stored as 0 (it has no upper neighbour).
-enum {
-  MT_IY1, MT_IY3, MT_RDYP, MT_RDYC, MT_AP2C, MT_AC2C, MT_AM2C, MT_AP2P, MT_AC2P, MT_AM2P,
-  MT_A0, MT_RM0, MT_CP0, MT_A1, MT_RM1, MT_CP1, MT_W
-};
-// Second table for the twisted march (lower half eliminated upwards, upper half
-// downwards): the downward factors c, 1/m', a/m' of both sets, with
-// m'_{ny-1} = b, m'_j = b_j - c_j aq_{j+1}; rows of MD_W values.
-enum { MD_C0, MD_RQ0, MD_AQ0, MD_C1, MD_RQ1, MD_AQ1, MD_W = 8 };
-
-// Layout of the march table buffer (values of precision T at the start of a
-// buffer sized for FP64): the row tables of the RK substeps ns = 1..3 (ny * MT_W
-// values each), their downward tables (ny * MD_W each), then per substep the
-// pmBeta its factors were computed for (FP64 bit patterns; all ones = not yet
-// computed).
-constexpr int kMarchTables = 3;
-size_t march_table_bytes(int ny) {
-  return (size_t)kMarchTables * ny * (MT_W + MD_W) * sizeof(double) + kMarchTables * sizeof(unsigned long long);
-}
-static unsigned long long* march_beta_slots(void* mtab, int ny) {
-  return (unsigned long long*)((char*)mtab + (size_t)kMarchTables * ny * (MT_W + MD_W) * sizeof(double));
-}
-template <class T> static T* march_down_tables(void* mtab, int ny) { return (T*)mtab + (size_t)kMarchTables * ny * MT_W; }
-cudaError_t march_table_reset(ch3d_ctx* c) {
-  return cudaMemsetAsync(march_beta_slots(c->mtab, c->ny), 0xff, kMarchTables * sizeof(unsigned long long),
-                         c->stream);
-}
-
-// Table of substep sc->ns; skipped when it already holds the factors of this
-// pmBeta (constant dt: computed once per substep of the run).
-template <class T>
-__global__ void k_march_table(HelmCoef hc, Metrics<T> m, int ny, T* __restrict__ tabs, T* __restrict__ dtabs,
-                              unsigned long long* __restrict__ beta_slot, const DevScalars* __restrict__ sc) {
-  if (sc->status) return;
-  const int q = sc->ns - 1;
-  const unsigned long long bits = (unsigned long long)__double_as_longlong(sc->pmBeta);
-  if (beta_slot[q] == bits) return;  // uniform across the block
-  T* tab = tabs + (size_t)q * ny * MT_W;
-  if (threadIdx.x == 0 || threadIdx.x == 32) {  // one thread per Helmholtz set, sequential in j
-    const int set = threadIdx.x == 0 ? 0 : 1;
-    const double pmBeta = sc->pmBeta;
-    T* col = tab + (set ? MT_A1 : MT_A0);
-    double cpp = 0.0;
-    for (int j = 0; j < ny; ++j) {
-      double a, b, c;
-      helm_abc(hc, set, pmBeta, j, a, b, c);
-      const double rm = 1.0 / (j == 0 ? b : b - a * cpp);
-      const double cp = c * rm;
-      col[(size_t)j * MT_W + 0] = (T)a;
-      col[(size_t)j * MT_W + 1] = (T)rm;
-      col[(size_t)j * MT_W + 2] = j == ny - 1 ? (T)0 : (T)cp;
-      cpp = cp;
-    }
-  }
-  if (threadIdx.x == 64 || threadIdx.x == 96) {  // downward elimination, sequential from the top
-    const int set = threadIdx.x == 64 ? 0 : 1;
-    const double pmBeta = sc->pmBeta;
-    T* col = dtabs + (size_t)q * ny * MD_W + (set ? MD_C1 : MD_C0);
-    double aqn = 0.0;
-    for (int j = ny - 1; j >= 0; --j) {
-      double a, b, c;
-      helm_abc(hc, set, pmBeta, j, a, b, c);
-      const double rq = 1.0 / (j == ny - 1 ? b : b - c * aqn);
-      const double aq = a * rq;
-      col[(size_t)j * MD_W + 0] = (T)c;
-      col[(size_t)j * MD_W + 1] = (T)rq;
-      col[(size_t)j * MD_W + 2] = (T)aq;
-      aqn = aq;
-    }
-  }
-  for (int j = threadIdx.x; j < ny; j += blockDim.x) {
-    const int jc = j + 1;
-    T* row = tab + (size_t)j * MT_W;
-    row[MT_IY1] = m.yinterp[jc]; row[MT_IY3] = m.yinterp[jc + 1];
-    row[MT_RDYP] = m.rdyp[jc]; row[MT_RDYC] = m.rdyc[jc];
-    row[MT_AP2C] = m.ap2c[jc]; row[MT_AC2C] = m.ac2c[jc]; row[MT_AM2C] = m.am2c[jc];
-    row[MT_AP2P] = m.ap2p[jc]; row[MT_AC2P] = m.ac2p[jc]; row[MT_AM2P] = m.am2p[jc];
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) beta_slot[q] = bits;
-}
 
 // Staging geometry: x halo H rounded up to whole copy vectors of VW points, and
 // points per staged row of a 32 x BZ tile.
@@ -1045,9 +959,6 @@ template <class T, bool O4> static cudaError_t rhs_march_t(ch3d_ctx* c) {
   constexpr int BZ = S::BZ, D = S::D, RS = S::RS;
   const size_t smem = S::smem;
   T** f = (T**)c->f;
-  k_march_table<T><<<1, 128, 0, c->stream>>>(helm_coef(c), metrics_of<T>(c), c->ny, (T*)c->mtab,
-                                             march_down_tables<T>(c->mtab, c->ny),
-                                             march_beta_slots(c->mtab, c->ny), c->sc);
   auto kern = k_rhs_march<T, O4, false, true, 1, BZ, D, RS>;
   auto kern_tw = k_rhs_march<T, O4, true, true, 1, BZ, D, RS>;
   const bool tw = march_twisted_t<T, O4>(c);  // also sets the twisted kernel's shared-memory limit

@@ -26,96 +26,6 @@
 namespace ch3d {
 
 // ---------------------------------------------------------------------------
-// scalar kernels
-// ---------------------------------------------------------------------------
-
-// src/CFD_2nd/m_ChannelSystem.f90:81-88 (CalcMaxCFL result -> cflmp, dt)
-__global__ void k_step_begin(DevScalars* sc, int iCFL, double CFLc, double dtMax) {
-  if (sc->status) return;
-  double uddx = __longlong_as_double((long long)sc->uddx);
-  sc->itime += 1;
-  sc->cflmp = uddx * sc->dt;
-  if (iCFL == 1) {
-    double d = CFLc / uddx;
-    sc->dt = d < dtMax ? d : dtMax;
-  } else {
-    sc->dt = dtMax;
-  }
-}
-
-// src/CFD_2nd/m_Parameters.f90:329-342 (PMcoeUpdate) and the bulk constraint of
-// src/CFD_2nd/m_TSchemePIMP_inc.f90:60-74 from the partial sums of the current ux.
-// 4th order (order == 4): the partial sums are those of the mean viscous stress
-// and the forcing follows src/CFD_4th/m_TScheme.f90:364-377.
-__global__ void k_substep_setup(DevScalars* sc, const double* __restrict__ part, int npart, int ns, double gam,
-                                double the, double alp, double xnu, int IsUxConst, double ubulk, double norm_bulk,
-                                int order, double nxnz, double yly) {
-  __shared__ double red[256];
-  if (sc->status) return;
-  double s = 0;
-  for (int q = threadIdx.x; q < npart; q += blockDim.x) s += part[q];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    double dt = sc->dt;
-    sc->pmGamma = gam * dt;
-    sc->pmTheta = the * dt;
-    sc->pmAlpha = alp * dt;
-    sc->pmBeta = 0.5 * alp * xnu * dt;
-    sc->SimTime = sc->SimTime + dt * alp;
-    sc->pmAlphaC = alp;
-    sc->pmBetaT = 0.5 * alp * dt;
-    if (ns == 1) sc->PrGradAver = 0.0;
-    sc->ns = ns;
-    sc->divmax1 = 0ull;
-    if (IsUxConst && order == 4) {
-      const double dpm = xnu * red[0] / nxnz / yly;
-      sc->PrGradNow = dpm;
-      sc->dpmdxns = -(sc->pmAlpha * dpm);  // RhsX - pmAlpha*dpmdxns
-      sc->PrGradAver = sc->PrGradAver + dpm * alp;
-    } else if (IsUxConst) {
-      double s1tot1 = red[0] * norm_bulk;
-      sc->s1tot1 = s1tot1;
-      sc->dpmdxns = alp * (ubulk - s1tot1);
-      sc->PrGradNow = (ubulk - s1tot1) / dt;
-      sc->PrGradAver = sc->PrGradAver + alp * sc->PrGradNow;
-    } else {
-      sc->dpmdxns = 0.0;
-    }
-  }
-}
-
-// src/CFD_2nd/m_ChannelSystem.f90:127-130 (limit checks after the step) and
-// CalcUxAver (src/CFD_2nd/m_Tools.f90:250-270) from partial sums.
-__global__ void k_step_end(DevScalars* sc, const double* __restrict__ part, int npart, double norm_uxm, double div_limit,
-                           double vel_limit) {
-  __shared__ double red[256];
-  if (sc->status) return;
-  double s = 0;
-  for (int q = threadIdx.x; q < npart; q += blockDim.x) s += part[q];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    sc->uxm = red[0] * norm_uxm;
-    double d2 = __longlong_as_double((long long)sc->divmax2);
-    double v0 = __longlong_as_double((long long)sc->vmax[0]);
-    double v1 = __longlong_as_double((long long)sc->vmax[1]);
-    double v2 = __longlong_as_double((long long)sc->vmax[2]);
-    double vmin = fmin(v0, fmin(v1, v2));
-    if (!(d2 <= div_limit)) sc->status = 1;        // NaN trips too
-    else if (!(vmin <= vel_limit)) sc->status = 2;
-  }
-}
-
-// ---------------------------------------------------------------------------
 // clcRhsX/Y/Z_PIMP  (src/CFD_2nd/m_TSchemePIMP_inc.f90:7-75, 161-209, 277-325)
 // at one cell: returns the three right-hand sides and updates HistX/Y/Z.
 // The mean pressure gradient dpmdxns (:61-74) is added by the callers.
@@ -794,11 +704,6 @@ __global__ void __launch_bounds__(128) k_diag(Geo<T> g, Metrics<T> m, const T* _
   }
 }
 
-__global__ void k_diag_reset(DevScalars* sc) {
-  if (sc->status) return;
-  sc->divmax2 = 0ull; sc->vmax[0] = 0ull; sc->vmax[1] = 0ull; sc->vmax[2] = 0ull; sc->uddx = 0ull;
-}
-
 // max |div u| of the current field into *slot (for ch3d_project)
 template <class T>
 __global__ void __launch_bounds__(256) k_divmax(Geo<T> g, Metrics<T> m, const T* __restrict__ ux,
@@ -833,54 +738,6 @@ __global__ void __launch_bounds__(256) k_divmax(Geo<T> g, Metrics<T> m, const T*
 static dim3 cell_grid(const ch3d_ctx* c) { return dim3((c->nx + 31) / 32, (c->ny + 7) / 8, c->nz); }
 static dim3 cell_block() { return dim3(32, 8, 1); }
 
-
-cudaError_t launch_step_begin(ch3d_ctx* c) {
-  k_step_begin<<<1, 1, 0, c->stream>>>(c->sc, c->cfg.iCFL, c->cfg.CFLc, c->cfg.dtMax);
-  return cudaGetLastError();
-}
-
-// first level of the deterministic two-level sum of block partials
-__global__ void __launch_bounds__(256) k_reduce_partials(const double* __restrict__ in, int n, double* __restrict__ out) {
-  __shared__ double red[256];
-  const int nb = gridDim.x;
-  const int chunk = (n + nb - 1) / nb;
-  const int lo = blockIdx.x * chunk, hi = min(n, lo + chunk);
-  double s = 0.0;
-  for (int q = lo + threadIdx.x; q < hi; q += blockDim.x) s += in[q];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[blockIdx.x] = red[0];
-}
-
-cudaError_t launch_reduce_partials(ch3d_ctx* c, const double* in, int n, double* out) {
-  k_reduce_partials<<<CH3D_NRED, 256, 0, c->stream>>>(in, n, out);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_substep_setup(ch3d_ctx* c, int ns) {
-  // the partials of the bulk sums (march projection or k_bulk_partial), or of the
-  // 4th-order viscous sum (k_visc4_partial)
-  const int np = c->cfg.order == 4 ? visc4_npart(c) : (c->march ? c->npart_m : c->npart);
-  k_reduce_partials<<<CH3D_NRED, 256, 0, c->stream>>>(c->part, np, c->red1);
-  const double norm_bulk = 1.0 / ((double)c->nx * (double)c->nz) / (c->cfg.ybulk2 - c->cfg.ybulk1);
-  k_substep_setup<<<1, 256, 0, c->stream>>>(c->sc, c->red1, CH3D_NRED, ns, c->gam[ns - 1], c->the[ns - 1],
-                                            c->alp[ns - 1], c->cfg.xnu, c->cfg.IsUxConst, c->cfg.ubulk, norm_bulk,
-                                            c->cfg.order, (double)(c->nx * c->nz), c->cfg.yly);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_step_end(ch3d_ctx* c) {
-  const double norm = 1.0 / ((double)c->nx * (double)c->nz) / c->cfg.yly;
-  // part2: written by the fused projection (march layout) or by k_diag
-  k_reduce_partials<<<CH3D_NRED, 256, 0, c->stream>>>(c->part2, march_diag_fusable(c) ? c->npart_m : diag_npart(c),
-                                                       c->red2);
-  k_step_end<<<1, 256, 0, c->stream>>>(c->sc, c->red2, CH3D_NRED, norm, c->cfg.div_limit, c->cfg.vel_limit);
-  return cudaGetLastError();
-}
 
 template <class T> static cudaError_t rhs_t(ch3d_ctx* c) {
   T** f = (T**)c->f;
@@ -1003,11 +860,6 @@ template <class T> static cudaError_t proj_t(ch3d_ctx* c, int mode) {
 }
 cudaError_t launch_proj(ch3d_ctx* c, int mode) { return c->fp32 ? proj_t<float>(c, mode) : proj_t<double>(c, mode); }
 cudaError_t launch_proj_diag(ch3d_ctx* c) { return launch_proj_march(c, 0, true); }
-cudaError_t launch_diag_reset(ch3d_ctx* c) {
-  k_diag_reset<<<1, 1, 0, c->stream>>>(c->sc);
-  return cudaGetLastError();
-}
-
 template <class T> static cudaError_t bulk_t(ch3d_ctx* c) {
   if (c->march) return launch_bulk_march(c);
   T** f = (T**)c->f;
@@ -1035,7 +887,6 @@ int diag_npart(const ch3d_ctx* c) {
 
 template <class T> static cudaError_t diag_t(ch3d_ctx* c) {
   T** f = (T**)c->f;
-  k_diag_reset<<<1, 1, 0, c->stream>>>(c->sc);
   k_diag<T><<<diag_grid(c), 128, 0, c->stream>>>(make_geo<T>(c), metrics_of<T>(c), f[0], f[1], f[2], c->part2, c->sc,
                                                  diag_rows(c));
   return cudaGetLastError();

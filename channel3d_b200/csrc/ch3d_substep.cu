@@ -1,0 +1,289 @@
+// ch3d_substep.cu -- the scalar work between the field kernels: one launch at
+// the start of each substep (the step's CFL number and dt, PMcoeUpdate, the
+// bulk constraint from the partial sums, the line solves' coefficient tables)
+// and one at its end (the bulk mean, the limit checks).
+//
+// Few partial sums are reduced by one block; many by CH3D_NRED blocks, the
+// last of which to finish sums the blocks' results in block order and does the
+// scalar work, so the result does not depend on the order the blocks run in.
+#include "ch3d_march.cuh"
+
+namespace ch3d {
+
+constexpr int kSetupThreads = 256;
+constexpr int kStagedRows = 1024;  // rows whose coefficient vectors fit in the shared memory of the setup block
+
+// Sum of part[0..n) over the grid, valid in every thread of the block for which
+// the function returns true (the only block, or the last one to finish).
+__device__ __forceinline__ bool grid_sum(const double* __restrict__ part, int n, double* __restrict__ red,
+                                         unsigned* ticket, double* sh /* kSetupThreads */, double& sum) {
+  const int nb = gridDim.x, chunk = (n + nb - 1) / nb;
+  const int lo = blockIdx.x * chunk, hi = min(n, lo + chunk);
+  auto block_sum = [&](double v) {
+    sh[threadIdx.x] = v;
+    __syncthreads();
+    for (int w = kSetupThreads / 2; w > 0; w >>= 1) {
+      if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
+      __syncthreads();
+    }
+    const double r = sh[0];
+    __syncthreads();
+    return r;
+  };
+  double s = 0.0;
+  for (int q = lo + (int)threadIdx.x; q < hi; q += kSetupThreads) s += part[q];
+  sum = block_sum(s);
+  if (nb == 1) return true;
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    red[blockIdx.x] = sum;
+    __threadfence();
+    last = atomicInc(ticket, nb - 1) == (unsigned)nb - 1;  // back to 0 for the next launch
+  }
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  s = 0.0;
+  for (int q = threadIdx.x; q < nb; q += kSetupThreads) s += __ldcg(red + q);
+  sum = block_sum(s);
+  return true;
+}
+
+struct SubstepPar {
+  int ns, begin, last;  // begin: the step starts here; last: the step's diagnostics follow
+  double gam, the, alp;
+  int iCFL, IsUxConst, order;
+  double CFLc, dtMax, xnu, ubulk, norm_bulk, nxnz, yly;
+};
+
+// Elimination factors of the row table for pmBeta (see ch3d_march.cuh), one
+// thread per Helmholtz set and direction, sequential in j; skipped when the
+// table already holds those of this pmBeta (constant dt).  The coefficient
+// vectors come through shared memory (co, 5 (ny + 1) values) where they fit: read
+// from global memory row by row they cost 49 us at 64 rows.
+template <class T>
+__device__ void update_row_table(const HelmCoef& hg, const Metrics<T>& m, int ny, T* __restrict__ tab,
+                                 T* __restrict__ dtab, double pmBeta, double* co) {
+  HelmCoef hc = hg;
+  if (co) {
+    const double* src[5] = {hg.ap2cForCN, hg.am2cForCN, hg.ap2p, hg.ac2p, hg.am2p};
+    const double** dst[5] = {&hc.ap2cForCN, &hc.am2cForCN, &hc.ap2p, &hc.ac2p, &hc.am2p};
+    for (int v = 0; v < 5; ++v) {
+      double* o = co + (size_t)v * (ny + 1);
+      for (int q = threadIdx.x; q <= ny; q += blockDim.x) o[q] = src[v][q];
+      *dst[v] = o;
+    }
+    __syncthreads();
+  }
+  const int who = threadIdx.x >> 5;
+  if ((threadIdx.x & 31) == 0 && who < 4) {
+    const int set = who & 1;
+    if (who < 2) {  // upwards: a, 1/m, c/m
+      T* col = tab + (set ? MT_A1 : MT_A0);
+      double cpp = 0.0;
+      for (int j = 0; j < ny; ++j) {
+        double a, b, c;
+        helm_abc(hc, set, pmBeta, j, a, b, c);
+        const double rm = 1.0 / (j == 0 ? b : b - a * cpp);
+        const double cp = c * rm;
+        col[(size_t)j * MT_W + 0] = (T)a;
+        col[(size_t)j * MT_W + 1] = (T)rm;
+        col[(size_t)j * MT_W + 2] = j == ny - 1 ? (T)0 : (T)cp;
+        cpp = cp;
+      }
+    } else if (dtab) {  // downwards (twisted march): c, 1/m', a/m'
+      T* col = dtab + (set ? MD_C1 : MD_C0);
+      double aqn = 0.0;
+      for (int j = ny - 1; j >= 0; --j) {
+        double a, b, c;
+        helm_abc(hc, set, pmBeta, j, a, b, c);
+        const double rq = 1.0 / (j == ny - 1 ? b : b - c * aqn);
+        const double aq = a * rq;
+        col[(size_t)j * MD_W + 0] = (T)c;
+        col[(size_t)j * MD_W + 1] = (T)rq;
+        col[(size_t)j * MD_W + 2] = (T)aq;
+        aqn = aq;
+      }
+    }
+  }
+  for (int j = threadIdx.x; j < ny; j += blockDim.x) {
+    const int jc = j + 1;
+    T* row = tab + (size_t)j * MT_W;
+    row[MT_IY1] = m.yinterp[jc]; row[MT_IY3] = m.yinterp[jc + 1];
+    row[MT_RDYP] = m.rdyp[jc]; row[MT_RDYC] = m.rdyc[jc];
+    row[MT_AP2C] = m.ap2c[jc]; row[MT_AC2C] = m.ac2c[jc]; row[MT_AM2C] = m.am2c[jc];
+    row[MT_AP2P] = m.ap2p[jc]; row[MT_AC2P] = m.ac2p[jc]; row[MT_AM2P] = m.am2p[jc];
+  }
+}
+
+template <class T> struct TableArgs {
+  HelmCoef hc;
+  Metrics<T> m;
+  int ny;
+  T* tab;                     // row tables of the substeps (null: none)
+  T* dtab;                    // their downward tables (null: not used)
+  unsigned long long* slots;  // pmBeta the tables of each substep hold (all ones: none)
+};
+
+template <class T>
+__global__ void __launch_bounds__(kSetupThreads) k_substep(DevScalars* sc, const double* __restrict__ part, int npart,
+                                                           double* __restrict__ red, SubstepPar p, TableArgs<T> ta) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double sh[kSetupThreads];
+  __shared__ double beta;
+  if (sc->status) return;
+  double s1;
+  if (!grid_sum(part, npart, red, &sc->ticket, sh, s1)) return;
+  if (threadIdx.x == 0) {
+    if (p.begin) {  // src/CFD_2nd/m_ChannelSystem.f90:81-88 (CalcMaxCFL result -> cflmp, dt)
+      const double uddx = __longlong_as_double((long long)sc->uddx);
+      sc->itime += 1;
+      sc->cflmp = uddx * sc->dt;
+      if (p.iCFL == 1) {
+        const double d = p.CFLc / uddx;
+        sc->dt = d < p.dtMax ? d : p.dtMax;
+      } else {
+        sc->dt = p.dtMax;
+      }
+    }
+    // src/CFD_2nd/m_Parameters.f90:329-342 (PMcoeUpdate)
+    const double dt = sc->dt;
+    sc->pmGamma = p.gam * dt;
+    sc->pmTheta = p.the * dt;
+    sc->pmAlpha = p.alp * dt;
+    beta = 0.5 * p.alp * p.xnu * dt;
+    sc->pmBeta = beta;
+    sc->SimTime = sc->SimTime + dt * p.alp;
+    sc->pmAlphaC = p.alp;
+    sc->pmBetaT = 0.5 * p.alp * dt;
+    if (p.ns == 1) sc->PrGradAver = 0.0;
+    sc->ns = p.ns;
+    sc->divmax1 = 0ull;
+    if (p.IsUxConst && p.order == 4) {
+      // the partial sums are those of the mean viscous stress (src/CFD_4th/m_TScheme.f90:364-377)
+      const double dpm = p.xnu * s1 / p.nxnz / p.yly;
+      sc->PrGradNow = dpm;
+      sc->dpmdxns = -(sc->pmAlpha * dpm);  // RhsX - pmAlpha*dpmdxns
+      sc->PrGradAver = sc->PrGradAver + dpm * p.alp;
+    } else if (p.IsUxConst) {
+      // the bulk constraint of src/CFD_2nd/m_TSchemePIMP_inc.f90:60-74 from the sums of the current ux
+      const double s1tot1 = s1 * p.norm_bulk;
+      sc->s1tot1 = s1tot1;
+      sc->dpmdxns = p.alp * (p.ubulk - s1tot1);
+      sc->PrGradNow = (p.ubulk - s1tot1) / dt;
+      sc->PrGradAver = sc->PrGradAver + p.alp * sc->PrGradNow;
+    } else {
+      sc->dpmdxns = 0.0;
+    }
+    if (p.last) {  // the maxima the diagnostics of this step accumulate
+      sc->divmax2 = 0ull;
+      sc->vmax[0] = sc->vmax[1] = sc->vmax[2] = 0ull;
+      sc->uddx = 0ull;
+    }
+  }
+  if (!ta.tab) return;
+  __syncthreads();
+  const int q = p.ns - 1;
+  const unsigned long long bits = (unsigned long long)__double_as_longlong(beta);
+  if (ta.slots[q] == bits) return;  // uniform: every thread reads it before thread 0 writes below
+  __syncthreads();
+  update_row_table(ta.hc, ta.m, ta.ny, ta.tab + (size_t)q * ta.ny * MT_W,
+                   ta.dtab ? ta.dtab + (size_t)q * ta.ny * MD_W : nullptr, beta,
+                   ta.ny <= kStagedRows ? reinterpret_cast<double*>(smem_raw) : nullptr);
+  __syncthreads();
+  if (threadIdx.x == 0) ta.slots[q] = bits;
+}
+
+// src/CFD_2nd/m_ChannelSystem.f90:127-130 (limit checks after the step) and
+// CalcUxAver (src/CFD_2nd/m_Tools.f90:250-270) from partial sums.
+__global__ void __launch_bounds__(kSetupThreads) k_step_end(DevScalars* sc, const double* __restrict__ part, int npart,
+                                                            double* __restrict__ red, double norm_uxm, double div_limit,
+                                                            double vel_limit) {
+  __shared__ double sh[kSetupThreads];
+  if (sc->status) return;
+  double s;
+  if (!grid_sum(part, npart, red, &sc->ticket, sh, s) || threadIdx.x != 0) return;
+  sc->uxm = s * norm_uxm;
+  const double d2 = __longlong_as_double((long long)sc->divmax2);
+  const double v0 = __longlong_as_double((long long)sc->vmax[0]);
+  const double v1 = __longlong_as_double((long long)sc->vmax[1]);
+  const double v2 = __longlong_as_double((long long)sc->vmax[2]);
+  const double vmin = fmin(v0, fmin(v1, v2));
+  if (!(d2 <= div_limit)) sc->status = 1;        // NaN trips too
+  else if (!(vmin <= vel_limit)) sc->status = 2;
+}
+
+// first level of the deterministic two-level sum of block partials
+__global__ void __launch_bounds__(256) k_reduce_partials(const double* __restrict__ in, int n, double* __restrict__ out) {
+  __shared__ double red[256];
+  const int nb = gridDim.x;
+  const int chunk = (n + nb - 1) / nb;
+  const int lo = blockIdx.x * chunk, hi = min(n, lo + chunk);
+  double s = 0.0;
+  for (int q = lo + threadIdx.x; q < hi; q += blockDim.x) s += in[q];
+  red[threadIdx.x] = s;
+  __syncthreads();
+  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
+    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) out[blockIdx.x] = red[0];
+}
+
+// ---------------------------------------------------------------------------
+// launchers
+// ---------------------------------------------------------------------------
+size_t march_table_bytes(int ny) {
+  return (size_t)kMarchTables * ny * (MT_W + MD_W) * sizeof(double) + kMarchTables * sizeof(unsigned long long);
+}
+cudaError_t march_table_reset(ch3d_ctx* c) {
+  return cudaMemsetAsync(march_beta_slots(c->mtab, c->ny), 0xff, kMarchTables * sizeof(unsigned long long),
+                         c->stream);
+}
+
+cudaError_t launch_reduce_partials(ch3d_ctx* c, const double* in, int n, double* out) {
+  k_reduce_partials<<<CH3D_NRED, 256, 0, c->stream>>>(in, n, out);
+  return cudaGetLastError();
+}
+
+// One block up to 4096 partial sums (16 per thread), else CH3D_NRED.
+static unsigned setup_blocks(int n) { return n <= 16 * kSetupThreads ? 1u : (unsigned)CH3D_NRED; }
+
+template <class T> static cudaError_t substep_t(ch3d_ctx* c, int ns, bool whole_step) {
+  SubstepPar p;
+  p.ns = ns;
+  p.begin = whole_step && ns == 1;
+  p.last = whole_step && ns == c->iadvance;
+  p.gam = c->gam[ns - 1]; p.the = c->the[ns - 1]; p.alp = c->alp[ns - 1];
+  p.iCFL = c->cfg.iCFL; p.IsUxConst = c->cfg.IsUxConst; p.order = c->cfg.order;
+  p.CFLc = c->cfg.CFLc; p.dtMax = c->cfg.dtMax; p.xnu = c->cfg.xnu; p.ubulk = c->cfg.ubulk;
+  p.norm_bulk = 1.0 / ((double)c->nx * (double)c->nz) / (c->cfg.ybulk2 - c->cfg.ybulk1);
+  p.nxnz = (double)(c->nx * c->nz);
+  p.yly = c->cfg.yly;
+  TableArgs<T> ta;
+  ta.hc = helm_coef(c);
+  ta.m = metrics_of<T>(c);
+  ta.ny = c->ny;
+  ta.tab = c->march || c->cfg.order == 4 ? (T*)c->mtab : nullptr;
+  ta.dtab = ta.tab && march_twisted(c) ? march_down_tables<T>(c->mtab, c->ny) : nullptr;
+  ta.slots = march_beta_slots(c->mtab, c->ny);
+  // the partials of the bulk sums (projection or k_bulk_partial), or of the
+  // 4th-order viscous sum (k_visc4_partial)
+  const int np = c->cfg.order == 4 ? visc4_npart(c) : (c->march ? c->npart_m : c->npart);
+  const size_t smem = ta.tab && c->ny <= kStagedRows ? (size_t)5 * (c->ny + 1) * sizeof(double) : 0;
+  k_substep<T><<<setup_blocks(np), kSetupThreads, smem, c->stream>>>(c->sc, c->part, np, c->red1, p, ta);
+  return cudaGetLastError();
+}
+cudaError_t launch_substep_setup(ch3d_ctx* c, int ns, bool whole_step) {
+  return c->fp32 ? substep_t<float>(c, ns, whole_step) : substep_t<double>(c, ns, whole_step);
+}
+
+cudaError_t launch_step_end(ch3d_ctx* c) {
+  const double norm = 1.0 / ((double)c->nx * (double)c->nz) / c->cfg.yly;
+  // part2: written by the fused projection (march layout) or by k_diag
+  const int np = march_diag_fusable(c) ? c->npart_m : diag_npart(c);
+  k_step_end<<<setup_blocks(np), kSetupThreads, 0, c->stream>>>(c->sc, c->part2, np, c->red2, norm, c->cfg.div_limit, c->cfg.vel_limit);
+  return cudaGetLastError();
+}
+
+}  // namespace ch3d
