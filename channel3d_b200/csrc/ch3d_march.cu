@@ -491,12 +491,21 @@ __global__ void __launch_bounds__(32 * BZ * (TW ? 2 : 1),
 // ---------------------------------------------------------------------------
 // FluidVelUpdate (src/CFD_2nd/m_TScheme.f90:281-306) + PressureUpdate_PIMP
 // (src/CFD_2nd/m_TSchemePIMP_inc.f90:852-873) as a march: a thread owns one
-// (i, k) column over a chunk of MJ rows and keeps phi at j-1, j, j+1 in
+// (i, k) column over a chunk of `rows` rows and keeps phi at j-1, j, j+1 in
 // registers (Neumann ghosts of SetBC_and_UpdateHalo_pr at the walls).  The
 // block's sum of ux * s1coe (the next substep's bulk constraint, clcRhsX_PIMP
 // :60-74) goes to part[block].  mode 1: projection only (pmAlpha = 1, p kept).
 // ---------------------------------------------------------------------------
-constexpr int MJ = 32;  // rows per block of the march projection
+// Rows per block of the march projection: 32 where the grid fills the GPU anyway,
+// else as few as give about four blocks per SM (at least 4: a block's first and
+// last row read phi of the rows next to them).  64^3: 17.2 us with 32 rows (64
+// blocks), 9.4 us with 4.
+static int proj_rows(const ch3d_ctx* c) {
+  const long long cols = (long long)((c->nx + 31) / 32) * ((c->nz + 3) / 4);
+  int rows = 32;
+  while (rows > 4 && cols * ((c->ny + rows - 1) / rows) < 4LL * sm_count(c->device)) rows >>= 1;
+  return rows;
+}
 
 __device__ __forceinline__ double block_sum128(double v, double* sh /* 4 */) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -515,13 +524,14 @@ template <class T, bool DIAG>
 __global__ void __launch_bounds__(128) k_proj_march(Geo<T> g, Metrics<T> m, const T* uxs, const T* uys,
                                                     const T* uzs, T* ux, T* uy, T* uz, T* __restrict__ pr,
                                                     const T* __restrict__ phi, double* __restrict__ part,
-                                                    double* __restrict__ part2, int mode, DevScalars* __restrict__ sc) {
+                                                    double* __restrict__ part2, int mode, int rows,
+                                                    DevScalars* __restrict__ sc) {
   __shared__ double red[7][4];
   if (sc->status) return;
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const long long plane = (long long)nx * ny;
   const int i = blockIdx.x * 32 + (threadIdx.x & 31), k = blockIdx.y * 4 + (threadIdx.x >> 5);
-  const int j0 = blockIdx.z * MJ, j1 = min(j0 + MJ, ny);
+  const int j0 = blockIdx.z * rows, j1 = min(j0 + rows, ny);
   double s = 0.0, s2 = 0.0, dv = 0.0, v0 = 0.0, v1 = 0.0, v2 = 0.0, cf = 0.0;
   if (i < nx && k < nz) {
     const long long col = i + plane * k;
@@ -634,11 +644,11 @@ __global__ void __launch_bounds__(128) k_proj_march(Geo<T> g, Metrics<T> m, cons
 // the same partial sums of ux * s1coe for a freshly uploaded field
 template <class T>
 __global__ void __launch_bounds__(128) k_bulk_march(Geo<T> g, Metrics<T> m, const T* __restrict__ ux,
-                                                    double* __restrict__ part) {
+                                                    double* __restrict__ part, int rows) {
   __shared__ double red[4];
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const int i = blockIdx.x * 32 + (threadIdx.x & 31), k = blockIdx.y * 4 + (threadIdx.x >> 5);
-  const int j0 = blockIdx.z * MJ, j1 = min(j0 + MJ, ny);
+  const int j0 = blockIdx.z * rows, j1 = min(j0 + rows, ny);
   double s = 0.0;
   if (i < nx && k < nz) {
     const long long col = i + (long long)nx * ny * k;
@@ -855,7 +865,10 @@ __global__ void __launch_bounds__(128) k_proj_bsub(Geo<T> g, Metrics<T> m, const
   }
 }
 
-static dim3 march_proj_grid(const ch3d_ctx* c) { return dim3((c->nx + 31) / 32, (c->nz + 3) / 4, (c->ny + MJ - 1) / MJ); }
+static dim3 march_proj_grid(const ch3d_ctx* c) {
+  const int rows = proj_rows(c);
+  return dim3((c->nx + 31) / 32, (c->nz + 3) / 4, (c->ny + rows - 1) / rows);
+}
 int march_npart(const ch3d_ctx* c) {
   const dim3 g = march_proj_grid(c);
   return (int)(g.x * g.y * g.z);
@@ -869,11 +882,11 @@ template <class T> static cudaError_t proj_march_t(ch3d_ctx* c, int mode, bool d
   if (diag)
     k_proj_march<T, true><<<march_proj_grid(c), 128, 0, c->stream>>>(make_geo<T>(c), metrics_of<T>(c), in[0], in[1],
                                                                       in[2], f[0], f[1], f[2], f[3], f[10], c->part,
-                                                                      c->part2, mode, c->sc);
+                                                                      c->part2, mode, proj_rows(c), c->sc);
   else
     k_proj_march<T, false><<<march_proj_grid(c), 128, 0, c->stream>>>(make_geo<T>(c), metrics_of<T>(c), in[0], in[1],
                                                                        in[2], f[0], f[1], f[2], f[3], f[10], c->part,
-                                                                       c->part2, mode, c->sc);
+                                                                       c->part2, mode, proj_rows(c), c->sc);
   return cudaGetLastError();
 }
 cudaError_t launch_proj_march(ch3d_ctx* c, int mode, bool diag) {
@@ -881,7 +894,8 @@ cudaError_t launch_proj_march(ch3d_ctx* c, int mode, bool diag) {
 }
 template <class T> static cudaError_t bulk_march_t(ch3d_ctx* c) {
   T** f = (T**)c->f;
-  k_bulk_march<T><<<march_proj_grid(c), 128, 0, c->stream>>>(make_geo<T>(c), metrics_of<T>(c), f[0], c->part);
+  k_bulk_march<T><<<march_proj_grid(c), 128, 0, c->stream>>>(make_geo<T>(c), metrics_of<T>(c), f[0], c->part,
+                                                          proj_rows(c));
   return cudaGetLastError();
 }
 cudaError_t launch_bulk_march(ch3d_ctx* c) { return c->fp32 ? bulk_march_t<float>(c) : bulk_march_t<double>(c); }
