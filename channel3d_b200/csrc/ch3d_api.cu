@@ -11,7 +11,7 @@
 #include <string>
 #include <vector>
 #include "../../include/ch3d_mlp.h"
-#include "ch3d_ctx.h"
+#include "ch3d_march.cuh"
 
 using namespace ch3d;
 
@@ -294,7 +294,7 @@ int alloc_fields(ch3d_ctx* c) {
     c->bytes += (long long)c->N * 9 * 8;
   }
   if ((c->cfg.order == 2 && c->cfg.IsImplicit == 2) || y_periodic(c)) {
-    const size_t nb = ptri_factor_doubles(c->nx, c->ny, c->nz) * sizeof(double);
+    const size_t nb = kMarchTables * ptri_doubles(c->nx, c->ny, c->nz) * sizeof(double);
     CU(cudaMalloc(&c->pfac, nb));
     CU(cudaMemsetAsync(c->pfac, 0, nb, c->stream));
     c->bytes += (long long)nb;
@@ -484,31 +484,30 @@ static bool march_path(const ch3d_ctx* c) {
   return c->cfg.LES_type == 0 && c->cfg.order == 2 && c->cfg.IsImplicit == 1 && !y_periodic(c);
 }
 
+// u -> u* of one substep: right-hand sides, Hist and the Crank-Nicolson solves
+cudaError_t launch_ustar(ch3d_ctx* c) {
+  const ch3d_config& g = c->cfg;
+  cudaError_t e;
+  if (c->march && !march_rows_path(c)) return launch_rhs_march(c);  // one column march
+  if (g.order == 4) return launch_rhs_march(c);  // the same with the 4th-order stencils
+  if (les_const(c)) return (e = launch_rhs_les_const(c)) != cudaSuccess ? e : launch_uhat(c);
+  if (g.LES_type > 0) {  // the LES y solves form their own coefficients (FEXP: none)
+    if ((e = launch_rhs_les(c)) != cudaSuccess) return e;
+    return g.IsImplicit == 0 ? launch_uhat_fexp(c) : launch_uhat_les(c);
+  }
+  if (g.IsImplicit == 0) return launch_ustar_fexp(c);  // explicit right-hand sides, u* = u + Rhs
+  if ((e = launch_rhs(c)) != cudaSuccess) return e;
+  if (g.IsImplicit == 2 && (e = launch_ptri_xz(c)) != cudaSuccess) return e;
+  return y_periodic(c) ? launch_ptri_y(c) : launch_uhat(c);  // FIMP_000 or PIMP_0, else between walls
+}
+
 int record_step(ch3d_ctx* c) {
   if (c->cfg.LES_type > 0) CU(launch_sgs_nut(c));  // once per step (m_ChannelSystem.f90:89)
-  const bool o4 = c->cfg.order == 4, fimp = c->cfg.order == 2 && c->cfg.IsImplicit == 2;
+  const bool o4 = c->cfg.order == 4;
   for (int ns = 1; ns <= c->iadvance; ++ns) {
     if (o4) CU(launch_visc4_partials(c));
     CU(launch_substep_setup(c, ns, true));
-    if (march_path(c)) {  // RHS + y solves as one column march, its own Thomas factors
-      CU(launch_rhs_march(c));
-    } else if (c->cfg.LES_type > 0) {  // the LES y solves form their own coefficients (FEXP: none)
-      CU(launch_rhs_les(c));
-      CU(c->cfg.IsImplicit == 0 ? launch_uhat_fexp(c) : launch_uhat_les(c));
-    } else if (fimp) {
-      if (!y_periodic(c)) CU(launch_helm_factors(c));
-      CU(launch_rhs_fimp(c));
-      CU(launch_ptri_xz(c));
-      CU(y_periodic(c) ? launch_ptri_y(c) : launch_uhat(c));  // FIMP_000 or FIMP_010
-    } else if (c->cfg.IsImplicit == 0) {  // FEXP: explicit right-hand sides, u* = u + Rhs
-      CU(launch_rhs_fimp(c));
-      CU(launch_uhat_fexp(c));
-    } else if (y_periodic(c)) {  // PIMP_0: the periodic y sweep alone
-      CU(launch_rhs(c));
-      CU(launch_ptri_y(c));
-    } else {
-      CU(launch_rhs_march(c));  // 4th order: the same column march with the 4th-order stencils
-    }
+    CU(launch_ustar(c));
     if (c->gsub) {
       CU(launch_div_bsub(c));
       CU(launch_prsrc_xfft(c, 3));
@@ -662,15 +661,7 @@ int ch3d_create(const ch3d_config* cfg, const double* yp, ch3d_ctx** out) {
   else c->m32 = Metrics<float>();
   if (!c->fp32) c->m64 = metrics_ptrs<double>((const double*)c->met, c->ny);
   c->TSy = 8;  // kx extent of the FP64 low modes of the mixed path
-  // chunks of the partitioned Helmholtz solves: the power of two nearest below
-  // sqrt(ny) (2..32), balancing the chunk sweeps (2 ny / P rows) against the
-  // serial interface solve (P - 1 steps)
-  c->Pv = 2;
-  while (c->Pv < 32 && 4 * c->Pv * c->Pv <= c->ny) c->Pv <<= 1;
-  while (c->Pv > 1 && c->ny < 2 * c->Pv) c->Pv >>= 1;
   {
-    size_t nf = (size_t)2 * (5 * c->ny + 6 * (c->Pv > 1 ? c->Pv - 1 : 1));
-    if (cudaMalloc(&c->hfac, nf * sizeof(double)) != cudaSuccess) return cleanup(fail(CH3D_ERR_NOMEM, "hfac"));
     if (cudaMalloc(&c->mtab, march_table_bytes(c->ny)) != cudaSuccess)
       return cleanup(fail(CH3D_ERR_NOMEM, "march table"));
     if (march_table_reset(c) != cudaSuccess) return cleanup(fail(CH3D_ERR_CUDA, "march table"));
@@ -706,7 +697,7 @@ int ch3d_create(const ch3d_config* cfg, const double* yp, ch3d_ctx** out) {
     c->npart = (int)(g.x * g.y * g.z);
     c->march = march_path(c);
     // large 2nd-order grids: the march stops at g, the divergence and projection substitute
-    c->gsub = c->march && !march_twisted(c) && xplan_exists(c->nx / 2);
+    c->gsub = c->march && !march_rows_path(c) && !march_twisted(c) && xplan_exists(c->nx / 2);
     c->npart_m = march_npart(c);
     if (c->npart_m > c->npart) c->npart = c->npart_m;
     if (diag_npart(c) > c->npart) c->npart = diag_npart(c);
@@ -747,7 +738,7 @@ int ch3d_destroy(ch3d_ctx* c) {
   void* mbufs[] = {c->mlp_params, c->mlp_packed, c->mlp_status, c->sgs_tau, c->sgs_f, c->spec2,
                    c->specacc};
   for (void* b : mbufs) if (b) cudaFree(b);
-  void* bufs[] = {c->hfac, c->mtab, c->yRM, c->yCP, c->ylow, c->yA2, c->yRM64, c->spec, c->met, c->met64, c->wave, c->twx, c->twr, c->twz, c->sc, c->part, c->part2,
+  void* bufs[] = {c->mtab, c->yRM, c->yCP, c->ylow, c->yA2, c->yRM64, c->spec, c->met, c->met64, c->wave, c->twx, c->twr, c->twz, c->sc, c->part, c->part2,
                   c->red1, c->red2, c->stat, c->statpart};
   for (void* b : bufs) if (b) cudaFree(b);
   if (c->ev0) cudaEventDestroy(c->ev0);
@@ -859,14 +850,13 @@ int ch3d_stage(ch3d_ctx* c, int stage, int ns) {
       break;
     case 1:
       if (c->cfg.LES_type > 0) CU(launch_rhs_les(c));
-      else CU(c->cfg.order == 4 ? launch_rhs4(c) : (c->cfg.IsImplicit != 1 ? launch_rhs_fimp(c) : launch_rhs(c)));
+      else CU(c->cfg.order == 4 ? launch_rhs4(c) : launch_rhs(c));
       break;
     case 2:
       if (c->cfg.IsImplicit == 0) { CU(launch_uhat_fexp(c)); break; }
       if (c->cfg.LES_type > 0) { CU(launch_uhat_les(c)); break; }
       if (c->cfg.order == 2 && c->cfg.IsImplicit == 2) CU(launch_ptri_xz(c));
       if (y_periodic(c)) { CU(launch_ptri_y(c)); break; }
-      CU(launch_helm_factors(c));
       CU(launch_uhat(c));
       break;
     case 3: break;  // clcPrSrc is fused into the forward x transform of stage 4
@@ -1131,7 +1121,7 @@ int ch3d_memory_bytes(ch3d_ctx* c, long long* bytes) {
 // Runs `nsteps` steps kernel group by kernel group with CUDA events between
 // the groups on the context's stream; out[q] = mean milliseconds per launch of
 // group q: 0 rhs, 1 uhat, 2 prsrc+x FFT, 3 z FFT + y solve + z iFFT,
-// 4 x iFFT, 5 projection, 6 scalar/reduction kernels.
+// 4 x iFFT, 5 projection, 6 scalar/reduction kernels.  Group 0 holds u -> u*.
 int ch3d_kernel_times(ch3d_ctx* c, int nsteps, double* out, int nout) {
   if (!c || !out || nout < 7 || nsteps < 1) return fail(CH3D_ERR_INVALID, "bad argument");
   CU(cudaSetDevice(c->device));
@@ -1150,28 +1140,9 @@ int ch3d_kernel_times(ch3d_ctx* c, int nsteps, double* out, int nout) {
       CU(mark(6));
       if (c->cfg.order == 4) CU(launch_visc4_partials(c));
       CU(launch_substep_setup(c, ns, true));
-      if (!march_path(c) && c->cfg.order != 4 && c->cfg.LES_type == 0 && !y_periodic(c) && c->cfg.IsImplicit != 0)
-        CU(launch_helm_factors(c));
       CU(done());
-      if (march_path(c)) {
-        CU(mark(0)); CU(launch_rhs_march(c)); CU(done());
-        CU(mark(1)); CU(done());
-      } else if (c->cfg.LES_type > 0) {
-        CU(mark(0)); CU(launch_rhs_les(c)); CU(done());
-        CU(mark(1)); CU(c->cfg.IsImplicit == 0 ? launch_uhat_fexp(c) : launch_uhat_les(c)); CU(done());
-      } else if (c->cfg.order == 2 && c->cfg.IsImplicit == 2) {
-        CU(mark(0)); CU(launch_rhs_fimp(c)); CU(done());
-        CU(mark(1)); CU(launch_ptri_xz(c)); CU(y_periodic(c) ? launch_ptri_y(c) : launch_uhat(c)); CU(done());
-      } else if (c->cfg.IsImplicit == 0) {
-        CU(mark(0)); CU(launch_rhs_fimp(c)); CU(done());
-        CU(mark(1)); CU(launch_uhat_fexp(c)); CU(done());
-      } else if (y_periodic(c)) {
-        CU(mark(0)); CU(launch_rhs(c)); CU(done());
-        CU(mark(1)); CU(launch_ptri_y(c)); CU(done());
-      } else {
-        CU(mark(0)); CU(launch_rhs_march(c)); CU(done());
-        CU(mark(1)); CU(done());
-      }
+      CU(mark(0)); CU(launch_ustar(c)); CU(done());
+      CU(mark(1)); CU(done());
       if (c->gsub) {
         CU(mark(2)); CU(launch_div_bsub(c)); CU(launch_prsrc_xfft(c, 3)); CU(done());
       } else {
@@ -1260,7 +1231,7 @@ int ch3d_path_flags(ch3d_ctx* c, int* flags) {
   if (!c || !flags) return fail(CH3D_ERR_INVALID, "NULL argument");
   CU(cudaSetDevice(c->device));
   const bool march = march_path(c) || c->cfg.order == 4;
-  *flags = (march ? CH3D_PATH_MARCH : 0) | (march && march_twisted(c) ? CH3D_PATH_TWISTED : 0) |
+  *flags = (march ? CH3D_PATH_MARCH : 0) | (march && !march_rows_path(c) && march_twisted(c) ? CH3D_PATH_TWISTED : 0) |
            (c->gsub ? CH3D_PATH_GSUB : 0);
   return CH3D_OK;
 }

@@ -33,9 +33,8 @@ struct ch3d_ctx {
   // device buffers
   void* f[15] = {nullptr};   // ux uy uz p hx hy hz rx ry rz phi nut u*x u*y u*z (precision T)
   void* ih[6] = {nullptr};   // 4th order: uxhx uyhx uzhx uxhz uyhz uzhz (precision T)
-  double* hfac = nullptr;    // Helmholtz chunk/interface factors of the current substep
-  void* mtab = nullptr;      // column-march row table of the current substep (precision T)
-  double* pfac = nullptr;    // FIMP or periodic y: periodic x/z/y sweep factors of the current substep
+  void* mtab = nullptr;      // row tables of the substeps (precision T)
+  double* pfac = nullptr;    // FIMP or periodic y: periodic x/z/y sweep factors of the substeps
   double* les_delta = nullptr;  // LES: DeltaCell (ny+2) | wall distance of the cell centres (ny+2)
   // learned closure (LES_type CH3D_LES_MLP)
   float* mlp_params = nullptr;   // CH3D_MLP_NPARAM FP32
@@ -54,7 +53,6 @@ struct ch3d_ctx {
   bool gsub = false;         // the march stops at g; divergence and projection substitute u*
   int KL = 8;
   int TSy = 8;               // kx extent of the FP64 low modes
-  int Pv = 32;               // chunks of the partitioned velocity Helmholtz solves
   void* spec = nullptr;      // complex spectrum (kx,j,kz)
   void* met = nullptr;       // packed metric vectors (precision T)
   double* met64 = nullptr;   // FP64 copy (always)
@@ -93,14 +91,19 @@ namespace ch3d {
 
 // y periodic (BcOption(3:4) = 0): the triply periodic steps (FIMP_000, PIMP_0)
 inline bool y_periodic(const ch3d_ctx* c) { return c->cfg.BcOption[2] == 0; }
+// learned closure with the partially implicit step: the total viscosity is xnu everywhere
+inline bool les_const(const ch3d_ctx* c) { return c->cfg.LES_type == CH3D_LES_MLP && c->cfg.IsImplicit == 1; }
 // launchers (ch3d_step.cu)
 cudaError_t launch_substep_setup(ch3d_ctx* c, int ns, bool whole_step);  // whole_step: with the step's CFL and dt (ns 1)
                                                                          // and the reset of its maxima (last ns)
 cudaError_t launch_step_end(ch3d_ctx* c);
-cudaError_t launch_rhs(ch3d_ctx* c);
+cudaError_t launch_rhs(ch3d_ctx* c);                   // 2nd order: the scheme's right-hand sides -> RhsX/Y/Z
+cudaError_t launch_ustar_fexp(ch3d_ctx* c);            // explicit scheme: right-hand sides and u* in one pass
+cudaError_t launch_rhs_les_const(ch3d_ctx* c);         // learned closure: constant viscosity and the stress force
 cudaError_t launch_uhat(ch3d_ctx* c);                  // stage path: Rhs arrays -> u*
 // 2nd-order PIMP step: RHS + y solves as a column march (ch3d_march.cu)
-cudaError_t launch_rhs_march(ch3d_ctx* c);             // u -> u*, Hist, with its row table
+cudaError_t launch_rhs_march(ch3d_ctx* c);             // u -> u*, Hist
+bool march_rows_path(const ch3d_ctx* c);               // few columns: right-hand sides by chunks of rows, then the y sweep
 size_t march_table_bytes(int ny);
 cudaError_t march_table_reset(ch3d_ctx* c);           // forget the cached factors
 cudaError_t launch_proj_march(ch3d_ctx* c, int mode, bool diag);  // projection + pressure update + bulk partials
@@ -111,7 +114,6 @@ bool xplan_exists(int m);                               // the register x FFT ha
 bool march_diag_fusable(const ch3d_ctx* c);            // the step diagnostics can ride on the last projection
 cudaError_t launch_bulk_march(ch3d_ctx* c);            // bulk partials of an uploaded field
 int march_npart(const ch3d_ctx* c);
-cudaError_t launch_helm_factors(ch3d_ctx* c);
 cudaError_t launch_prsrc_xfft(ch3d_ctx* c, int mode);  // mode 0: div(u*)/pmAlpha, 1: div(u), 2: source in phi,
                                                        // 3: div(u*) in phi's array, /pmAlpha (register FFT only)
 cudaError_t launch_poisson_spectral(ch3d_ctx* c);      // z fwd, y solve, z inv
@@ -151,12 +153,10 @@ cudaError_t launch_visc4_partials(ch3d_ctx* c);        // mean viscous stress pa
 int visc4_npart(const ch3d_ctx* c);                   // their count
 cudaError_t launch_dissipation(ch3d_ctx* c, int* npart);  // CalcDissipationRate partials -> part2
 cudaError_t launch_reduce_partials(ch3d_ctx* c, const double* in, int n, double* out);  // CH3D_NRED sums
-// fully implicit and explicit 2nd-order steps (ch3d_step.cu, ch3d_fimp.cu)
-cudaError_t launch_rhs_fimp(ch3d_ctx* c);              // clcRhsX/Y/Z_FIMP (or _FEXP) -> RhsX/Y/Z
+// fully implicit and explicit 2nd-order steps (ch3d_step.cu, ch3d_sweep.cu)
 cudaError_t launch_uhat_fexp(ch3d_ctx* c);             // clcU1/2/3Hat_FEXP: u* = u + RhsX/Y/Z
 cudaError_t launch_ptri_xz(ch3d_ctx* c);               // periodic x and z sweeps of RhsX/Y/Z, in place
 cudaError_t launch_ptri_y(ch3d_ctx* c);                // periodic y sweep (y periodic, FIMP or PIMP): u* = u + solution
-size_t ptri_factor_doubles(int nx, int ny, int nz);
 // LES (ch3d_les.cu), FP64
 cudaError_t launch_mlp_pack(ch3d_ctx* c);              // parameter image of the closure's network
 cudaError_t launch_fill_nut(ch3d_ctx* c);              // nut = xnu (learned closure)

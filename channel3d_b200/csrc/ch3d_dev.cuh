@@ -122,7 +122,7 @@ template <class T> __device__ __forceinline__ void nbr_next_row(Nbr& n, const Ge
 }
 
 // ---------------------------------------------------------------------------
-// Partitioned tridiagonal solve (used by clcU*Hat and the Poisson y solve).
+// Partitioned tridiagonal solve (the allocation-free Poisson y solve).
 // A system of n rows is cut into P chunks.  Each chunk is solved locally
 // (Thomas) for the data and for two "spikes" (its response to the unknown
 // just left of and just right of it); the 2(P-1) interface unknowns then
@@ -167,40 +167,6 @@ inline HelmCoef helm_coef(const ch3d_ctx* c) {
   hc.ap2p = M + 7 * L; hc.ac2p = M + 8 * L; hc.am2p = M + 9 * L;
   hc.ap2cForCN = M + 14 * L; hc.am2cForCN = M + 15 * L;
   return hc;
-}
-
-// Factor layout of one set: RM | AA | CP | AL | BE (ny each), then per
-// interface q: M00 M01 M10 M11 l v (6 each).
-__host__ __device__ inline int helm_set_stride(int ny, int P) { return 5 * ny + 6 * (P > 1 ? P - 1 : 1); }
-
-// Interface (reduced) block-tridiagonal solve of one column, with the
-// precomputed factors; F: chunk-local solutions of the column (stride fs).
-template <class T, class FT>
-__device__ __forceinline__ void helm_interfaces(const FT* __restrict__ IFD, const T* F, int fs, int ny, int P,
-                                                T* G /* 2*(P-1) */) {
-  const int Q = P - 1;
-  T gu = (T)0, gw = (T)0;
-  for (int q = 0; q < Q; ++q) {
-    const int eq = chunk_hi(q, ny, P), sq1 = chunk_lo(q + 1, ny, P);
-    const FT* R = IFD + 6 * q;
-    const T ru = F[eq * fs] - (q > 0 ? (T)R[4] * gu : (T)0);
-    const T rw = F[sq1 * fs];
-    gu = (T)R[0] * ru + (T)R[1] * rw;
-    gw = (T)R[2] * ru + (T)R[3] * rw;
-    G[2 * q] = gu;
-    G[2 * q + 1] = gw;
-  }
-  if (Q < 1) return;
-  T zw = G[2 * (Q - 1) + 1];
-  for (int q = Q - 2; q >= 0; --q) {
-    const FT* R = IFD + 6 * q;
-    const T f = (T)R[5] * zw;
-    const T zu = G[2 * q] - (T)R[1] * f;
-    const T zwn = G[2 * q + 1] - (T)R[3] * f;
-    G[2 * q] = zu;
-    G[2 * q + 1] = zwn;
-    zw = zwn;
-  }
 }
 
 template <class T> Geo<T> make_geo(const ch3d_ctx* c) {

@@ -227,61 +227,19 @@ __global__ void __launch_bounds__(32 * BZ * (TW ? 2 : 1),
       const T* P0 = &ring[3][slot(j - 1)][c0];
       const T* P1 = &ring[3][slot(j)][c0];
 
-      ux_c = X1[0]; const T ux_ip = X1[1], ux_im = X1[-1]; ux_jp = X2[0]; ux_jm = X0[0];
-      const T ux_kp = X1[SX], ux_km = X1[-SX], ux_ip_jm = X0[1], ux_ip_km = X1[1 - SX];
-      uy_c = Y1[0]; uy_jp = Y2[0]; uy_jm = Y0[0]; const T uy_ip = Y1[1], uy_im = Y1[-1];
-      const T uy_im_jp = Y2[-1], uy_kp = Y1[SX], uy_km = Y1[-SX], uy_jp_km = Y2[-SX];
-      uz_c = Z1[0]; uz_jp = Z2[0]; uz_jm = Z0[0]; const T uz_ip = Z1[1], uz_im = Z1[-1];
-      const T uz_kp = Z1[SX], uz_km = Z1[-SX], uz_im_kp = Z1[SX - 1], uz_jm_kp = Z0[SX];
-      const T p_c = P1[0], p_im = P1[-1], p_jm = P0[0], p_km = P1[-SX];
-
-      const T IY1 = tr[MT_IY1], IY2 = one - IY1;
-      const T IY3 = tr[MT_IY3], IY4 = one - IY3;
-      {  // RhsX (clcRhsX_PIMP, m_TSchemePIMP_inc.f90:7-75)
-        const T qdx1 = quarter * rdx, qdx3 = quarter * rdz;
-        const T sucaj = half * tr[MT_RDYP];
-        T h11 = ((ux_ip + ux_c) * (ux_ip + ux_c) - (ux_c + ux_im) * (ux_c + ux_im)) * qdx1;
-        T h12 = ((uy_jp + uy_im_jp) * (IY3 * ux_c + IY4 * ux_jp) - (uy_c + uy_im) * (IY1 * ux_jm + IY2 * ux_c)) * sucaj;
-        T h13 = ((uz_kp + uz_im_kp) * (ux_kp + ux_c) - (uz_c + uz_im) * (ux_c + ux_km)) * qdx3;
-        T d11q1 = (ux_ip - two * ux_c + ux_im) * rdx2;
-        T d22q1 = tr[MT_AP2C] * ux_jp + tr[MT_AC2C] * ux_c + tr[MT_AM2C] * ux_jm;
-        T d33q1 = g.ap3c * ux_kp + g.ac3c * ux_c + g.am3c * ux_km;
-        T dcq13 = d11q1 + d33q1;
-        T gradp1 = (p_c - p_im) * rdx;
-        T convEd1 = -h11 - h12 - h13 + xnu * dcq13 + g.g1;
-        rx = pmGamma * convEd1 + pmTheta * hxo - pmAlpha * gradp1 + two * pmBeta * d22q1;
-        hx[idx] = convEd1;
-      }
-      {  // RhsY (clcRhsY_PIMP, :161-209)
-        const T hdx1 = half * rdx, hdx3 = half * rdz;
-        const T sucac = tr[MT_RDYC], qsucac = quarter * sucac;
-        T h21 = ((IY1 * ux_ip_jm + IY2 * ux_ip) * (uy_ip + uy_c) - (IY1 * ux_jm + IY2 * ux_c) * (uy_c + uy_im)) * hdx1;
-        T h22 = ((uy_jp + uy_c) * (uy_jp + uy_c) - (uy_c + uy_jm) * (uy_c + uy_jm)) * qsucac;
-        T h23 = ((IY1 * uz_jm_kp + IY2 * uz_kp) * (uy_kp + uy_c) - (IY1 * uz_jm + IY2 * uz_c) * (uy_c + uy_km)) * hdx3;
-        T d11q2 = g.ap1c * uy_ip + g.ac1c * uy_c + g.am1c * uy_im;
-        T d22q2 = tr[MT_AP2P] * uy_jp + tr[MT_AC2P] * uy_c + tr[MT_AM2P] * uy_jm;
-        T d33q2 = g.ap3c * uy_kp + g.ac3c * uy_c + g.am3c * uy_km;
-        T dcq13 = d11q2 + d33q2;
-        T gradp2 = (p_c - p_jm) * sucac;
-        T convEd2 = -h21 - h22 - h23 + xnu * dcq13 + g.g2;
-        ry = pmGamma * convEd2 + pmTheta * hyo - pmAlpha * gradp2 + two * pmBeta * d22q2;
-        hy[idx] = convEd2;
-      }
-      {  // RhsZ (clcRhsZ_PIMP, :277-325)
-        const T qdx1 = quarter * rdx, qdx3 = quarter * rdz;
-        const T sucaj = half * tr[MT_RDYP];
-        T h31 = ((ux_ip + ux_ip_km) * (uz_ip + uz_c) - (ux_c + ux_km) * (uz_c + uz_im)) * qdx1;
-        T h32 = ((uy_jp + uy_jp_km) * (IY3 * uz_c + IY4 * uz_jp) - (uy_c + uy_km) * (IY1 * uz_jm + IY2 * uz_c)) * sucaj;
-        T h33 = ((uz_kp + uz_c) * (uz_kp + uz_c) - (uz_c + uz_km) * (uz_c + uz_km)) * qdx3;
-        T d11q3 = g.ap1c * uz_ip + g.ac1c * uz_c + g.am1c * uz_im;
-        T d22q3 = tr[MT_AP2C] * uz_jp + tr[MT_AC2C] * uz_c + tr[MT_AM2C] * uz_jm;
-        T d33q3 = (uz_kp - two * uz_c + uz_km) * rdz2;
-        T dcq13 = d11q3 + d33q3;
-        T gradp3 = (p_c - p_km) * rdz;
-        T convEd3 = -h31 - h32 - h33 + xnu * dcq13 + g.g3;
-        rz = pmGamma * convEd3 + pmTheta * hzo - pmAlpha * gradp3 + two * pmBeta * d22q3;
-        hz[idx] = convEd3;
-      }
+      const Sten2<T> s = {X1[0], X1[1], X1[-1], X2[0], X0[0], X1[SX], X1[-SX], X0[1], X1[1 - SX],
+                          Y1[0], Y1[1], Y1[-1], Y2[0], Y0[0], Y1[SX], Y1[-SX], Y2[-1], Y2[-SX],
+                          Z1[0], Z1[1], Z1[-1], Z2[0], Z0[0], Z1[SX], Z1[-SX], Z1[SX - 1], Z0[SX],
+                          P1[0], P1[-1], P0[0], P1[-SX]};
+      ux_c = s.ux_c; ux_jp = s.ux_jp; ux_jm = s.ux_jm;
+      uy_c = s.uy_c; uy_jp = s.uy_jp; uy_jm = s.uy_jm;
+      uz_c = s.uz_c; uz_jp = s.uz_jp; uz_jm = s.uz_jm;
+      const T ho[3] = {hxo, hyo, hzo};
+      const RhsCoef<T> pm = {pmGamma, pmTheta, pmAlpha, pmBeta};
+      T r[3], h[3];
+      rhs2_cell<RHS_PIMP>(g, tr, s, ho, pm, r, h);
+      rx = r[0]; ry = r[1]; rz = r[2];
+      hx[idx] = h[0]; hy[idx] = h[1]; hz[idx] = h[2];
       } else {
         // 4th order: row r, x offset dx, z offset dz of staged array a
         auto V = [&](int a, int r, int dx, int dz) -> T { return ring[a][slot(r)][c0 + dx + dz * SX]; };
@@ -1020,6 +978,15 @@ template <class T, bool O4> static cudaError_t rhs_march_t(ch3d_ctx* c) {
     if (!done) args(kern, grid, 32 * BZ, smem);
   }
   return cudaGetLastError();
+}
+// Grids with few columns: a column march's time is set by its dependent rows per
+// thread, however few columns there are; the right-hand sides by chunks of rows
+// and the y sweep as its own pass cost 6 more arrays of (L2) traffic instead.
+// Step with the march / by rows: 64^3 (4096 columns) 239 / 150 us, 96^3 414 / 337,
+// 128^3 (16384) 588 / 563, 192 x 64 x 96 mixed (18432) 282 / 311, 192^3 (36864)
+// 1613 / 1960: the line lies between the last two groups, at 120 columns per SM.
+bool march_rows_path(const ch3d_ctx* c) {
+  return c->march && (long long)c->nx * c->nz <= 120LL * sm_count(c->device);
 }
 cudaError_t launch_rhs_march(ch3d_ctx* c) {
   if (c->cfg.order == 4) return c->fp32 ? rhs_march_t<float, true>(c) : rhs_march_t<double, true>(c);

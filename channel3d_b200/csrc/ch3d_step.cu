@@ -26,370 +26,6 @@
 namespace ch3d {
 
 // ---------------------------------------------------------------------------
-// clcRhsX/Y/Z_PIMP  (src/CFD_2nd/m_TSchemePIMP_inc.f90:7-75, 161-209, 277-325)
-// at one cell: returns the three right-hand sides and updates HistX/Y/Z.
-// The mean pressure gradient dpmdxns (:61-74) is added by the callers.
-// ---------------------------------------------------------------------------
-template <class T>
-__device__ __forceinline__ void rhs_point(const Geo<T>& g, const Metrics<T>& m, const T* __restrict__ ux,
-                                          const T* __restrict__ uy, const T* __restrict__ uz,
-                                          const T* __restrict__ pr, T* __restrict__ hx, T* __restrict__ hy,
-                                          T* __restrict__ hz, int i, int j, int k, T pmGamma, T pmTheta, T pmAlpha,
-                                          T pmBeta, T& rxo, T& ryo, T& rzo) {
-  const int nx = g.nx, ny = g.ny, nz = g.nz;
-  const int im = wrapm(i, nx), ip = wrapp(i, nx), km = wrapm(k, nz), kp = wrapp(k, nz);
-  const int jc = j + 1;
-  const T two = (T)2, half = (T)0.5, quarter = (T)0.25, one = (T)1;
-  const long long idx = i + (long long)nx * (j + (long long)ny * k);
-
-  const T ux_c = __ldg(ux + idx);
-  const T ux_ip = fld(ux, g, 0, ip, j, k), ux_im = fld(ux, g, 0, im, j, k);
-  const T ux_jp = fld(ux, g, 0, i, j + 1, k), ux_jm = fld(ux, g, 0, i, j - 1, k);
-  const T ux_kp = fld(ux, g, 0, i, j, kp), ux_km = fld(ux, g, 0, i, j, km);
-  const T ux_ip_jm = fld(ux, g, 0, ip, j - 1, k), ux_ip_km = fld(ux, g, 0, ip, j, km);
-  const T uy_c = __ldg(uy + idx);
-  const T uy_ip = fld(uy, g, 1, ip, j, k), uy_im = fld(uy, g, 1, im, j, k);
-  const T uy_jp = fld(uy, g, 1, i, j + 1, k), uy_jm = fld(uy, g, 1, i, j - 1, k);
-  const T uy_im_jp = fld(uy, g, 1, im, j + 1, k);
-  const T uy_kp = fld(uy, g, 1, i, j, kp), uy_km = fld(uy, g, 1, i, j, km);
-  const T uy_jp_km = fld(uy, g, 1, i, j + 1, km);
-  const T uz_c = __ldg(uz + idx);
-  const T uz_ip = fld(uz, g, 2, ip, j, k), uz_im = fld(uz, g, 2, im, j, k);
-  const T uz_jp = fld(uz, g, 2, i, j + 1, k), uz_jm = fld(uz, g, 2, i, j - 1, k);
-  const T uz_kp = fld(uz, g, 2, i, j, kp), uz_km = fld(uz, g, 2, i, j, km);
-  const T uz_im_kp = fld(uz, g, 2, im, j, kp), uz_jm_kp = fld(uz, g, 2, i, j - 1, kp);
-  const T p_c = __ldg(pr + idx);
-  const T p_im = fld(pr, g, 3, im, j, k), p_jm = fld(pr, g, 3, i, j - 1, k), p_km = fld(pr, g, 3, i, j, km);
-  const T hx_o = hx[idx], hy_o = hy[idx], hz_o = hz[idx];
-
-  const T rdx = g.rdx, rdz = g.rdz, rdx2 = g.rdx2, rdz2 = g.rdz2, xnu = g.xnu;
-  const T IY1 = m.yinterp[jc], IY2 = one - IY1;
-  const T IY3 = m.yinterp[jc + 1], IY4 = one - IY3;
-  {  // RhsX
-    const T qdx1 = quarter * rdx, qdx3 = quarter * rdz;
-    const T sucaj = half * m.rdyp[jc];
-    T h11 = ((ux_ip + ux_c) * (ux_ip + ux_c) - (ux_c + ux_im) * (ux_c + ux_im)) * qdx1;
-    T h12 = ((uy_jp + uy_im_jp) * (IY3 * ux_c + IY4 * ux_jp) - (uy_c + uy_im) * (IY1 * ux_jm + IY2 * ux_c)) * sucaj;
-    T h13 = ((uz_kp + uz_im_kp) * (ux_kp + ux_c) - (uz_c + uz_im) * (ux_c + ux_km)) * qdx3;
-    T d11q1 = (ux_ip - two * ux_c + ux_im) * rdx2;
-    T d22q1 = m.ap2c[jc] * ux_jp + m.ac2c[jc] * ux_c + m.am2c[jc] * ux_jm;
-    T d33q1 = g.ap3c * ux_kp + g.ac3c * ux_c + g.am3c * ux_km;
-    T dcq13 = d11q1 + d33q1;
-    T gradp1 = (p_c - p_im) * rdx;
-    T convEd1 = -h11 - h12 - h13 + xnu * dcq13 + g.g1;
-    rxo = pmGamma * convEd1 + pmTheta * hx_o - pmAlpha * gradp1 + two * pmBeta * d22q1;
-    hx[idx] = convEd1;
-  }
-  {  // RhsY
-    const T hdx1 = half * rdx, hdx3 = half * rdz;
-    const T sucac = m.rdyc[jc], qsucac = quarter * sucac;
-    T h21 = ((IY1 * ux_ip_jm + IY2 * ux_ip) * (uy_ip + uy_c) - (IY1 * ux_jm + IY2 * ux_c) * (uy_c + uy_im)) * hdx1;
-    T h22 = ((uy_jp + uy_c) * (uy_jp + uy_c) - (uy_c + uy_jm) * (uy_c + uy_jm)) * qsucac;
-    T h23 = ((IY1 * uz_jm_kp + IY2 * uz_kp) * (uy_kp + uy_c) - (IY1 * uz_jm + IY2 * uz_c) * (uy_c + uy_km)) * hdx3;
-    T d11q2 = g.ap1c * uy_ip + g.ac1c * uy_c + g.am1c * uy_im;
-    T d22q2 = m.ap2p[jc] * uy_jp + m.ac2p[jc] * uy_c + m.am2p[jc] * uy_jm;
-    T d33q2 = g.ap3c * uy_kp + g.ac3c * uy_c + g.am3c * uy_km;
-    T dcq13 = d11q2 + d33q2;
-    T gradp2 = (p_c - p_jm) * sucac;
-    T convEd2 = -h21 - h22 - h23 + xnu * dcq13 + g.g2;
-    ryo = pmGamma * convEd2 + pmTheta * hy_o - pmAlpha * gradp2 + two * pmBeta * d22q2;
-    hy[idx] = convEd2;
-  }
-  {  // RhsZ
-    const T qdx1 = quarter * rdx, qdx3 = quarter * rdz;
-    const T sucaj = half * m.rdyp[jc];
-    T h31 = ((ux_ip + ux_ip_km) * (uz_ip + uz_c) - (ux_c + ux_km) * (uz_c + uz_im)) * qdx1;
-    T h32 = ((uy_jp + uy_jp_km) * (IY3 * uz_c + IY4 * uz_jp) - (uy_c + uy_km) * (IY1 * uz_jm + IY2 * uz_c)) * sucaj;
-    T h33 = ((uz_kp + uz_c) * (uz_kp + uz_c) - (uz_c + uz_km) * (uz_c + uz_km)) * qdx3;
-    T d11q3 = g.ap1c * uz_ip + g.ac1c * uz_c + g.am1c * uz_im;
-    T d22q3 = m.ap2c[jc] * uz_jp + m.ac2c[jc] * uz_c + m.am2c[jc] * uz_jm;
-    T d33q3 = (uz_kp - two * uz_c + uz_km) * rdz2;
-    T dcq13 = d11q3 + d33q3;
-    T gradp3 = (p_c - p_km) * rdz;
-    T convEd3 = -h31 - h32 - h33 + xnu * dcq13 + g.g3;
-    rzo = pmGamma * convEd3 + pmTheta * hz_o - pmAlpha * gradp3 + two * pmBeta * d22q3;
-    hz[idx] = convEd3;
-  }
-}
-
-// One component of clcRhsX/Y/Z_PIMP (or _FIMP, _FEXP) at one cell (C = 0, 1, 2),
-// with its Hist update.
-template <class T, int C>
-__device__ __forceinline__ T rhs_comp(const Geo<T>& g, const Metrics<T>& m, const T* __restrict__ ux,
-                                      const T* __restrict__ uy, const T* __restrict__ uz, const T* __restrict__ pr,
-                                      T* __restrict__ h, int i, int j, int k, T pmGamma, T pmTheta, T pmAlpha,
-                                      T pmBeta) {
-  const Nbr n = make_nbr(g, i, j, k);
-  const int jc = j + 1;
-  const T two = (T)2, half = (T)0.5, quarter = (T)0.25, one = (T)1;
-  const T rdx = g.rdx, rdz = g.rdz, rdx2 = g.rdx2, rdz2 = g.rdz2, xnu = g.xnu;
-  const T IY1 = m.yinterp[jc], IY2 = one - IY1;
-  if (C == 0) {
-    const T ux_c = at(ux, n, 0), ux_ip = at(ux, n, n.xp), ux_im = at(ux, n, n.xm);
-    const T ux_jp = at_jp(ux, g, 0, n, 0), ux_jm = at_jm(ux, g, 0, n, 0);
-    const T ux_kp = at(ux, n, n.zp), ux_km = at(ux, n, n.zm);
-    const T uy_c = at(uy, n, 0), uy_im = at(uy, n, n.xm);
-    const T uy_jp = at_jp(uy, g, 1, n, 0), uy_im_jp = at_jp(uy, g, 1, n, n.xm);
-    const T uz_c = at(uz, n, 0), uz_im = at(uz, n, n.xm);
-    const T uz_kp = at(uz, n, n.zp), uz_im_kp = at(uz, n, n.zp + n.xm);
-    const T p_c = at(pr, n, 0), p_im = at(pr, n, n.xm);
-    const T h_o = h[n.c];
-    const T IY3 = m.yinterp[jc + 1], IY4 = one - IY3;
-    const T qdx1 = quarter * rdx, qdx3 = quarter * rdz;
-    const T sucaj = half * m.rdyp[jc];
-    T h11 = ((ux_ip + ux_c) * (ux_ip + ux_c) - (ux_c + ux_im) * (ux_c + ux_im)) * qdx1;
-    T h12 = ((uy_jp + uy_im_jp) * (IY3 * ux_c + IY4 * ux_jp) - (uy_c + uy_im) * (IY1 * ux_jm + IY2 * ux_c)) * sucaj;
-    T h13 = ((uz_kp + uz_im_kp) * (ux_kp + ux_c) - (uz_c + uz_im) * (ux_c + ux_km)) * qdx3;
-    T d11q1 = (ux_ip - two * ux_c + ux_im) * rdx2;
-    T d22q1 = m.ap2c[jc] * ux_jp + m.ac2c[jc] * ux_c + m.am2c[jc] * ux_jm;
-    T d33q1 = g.ap3c * ux_kp + g.ac3c * ux_c + g.am3c * ux_km;
-    T dcq13 = d11q1 + d33q1;
-    T gradp1 = (p_c - p_im) * rdx;
-    if (g.implicit == 0) {  // clcRhsX_FEXP (src/CFD_2nd/m_TSchemeFEXP_inc.f90:33-55)
-      T convEd1 = -h11 - h12 - h13 + xnu * (d11q1 + d22q1 + d33q1) + g.g1;
-      h[n.c] = convEd1;
-      return pmGamma * convEd1 + pmTheta * h_o - pmAlpha * gradp1;
-    }
-    if (g.implicit == 2) {  // clcRhsX_FIMP (src/CFD_2nd/m_TSchemeFIMP_inc.f90:45-55)
-      T convEd1 = -h11 - h12 - h13 + g.g1;
-      h[n.c] = convEd1;
-      return pmGamma * convEd1 + pmTheta * h_o - pmAlpha * gradp1 + two * pmBeta * (d11q1 + d22q1 + d33q1);
-    }
-    T convEd1 = -h11 - h12 - h13 + xnu * dcq13 + g.g1;
-    h[n.c] = convEd1;
-    return pmGamma * convEd1 + pmTheta * h_o - pmAlpha * gradp1 + two * pmBeta * d22q1;
-  } else if (C == 1) {
-    const T ux_c = at(ux, n, 0), ux_ip = at(ux, n, n.xp);
-    const T ux_jm = at_jm(ux, g, 0, n, 0), ux_ip_jm = at_jm(ux, g, 0, n, n.xp);
-    const T uy_c = at(uy, n, 0), uy_ip = at(uy, n, n.xp), uy_im = at(uy, n, n.xm);
-    const T uy_jp = at_jp(uy, g, 1, n, 0), uy_jm = at_jm(uy, g, 1, n, 0);
-    const T uy_kp = at(uy, n, n.zp), uy_km = at(uy, n, n.zm);
-    const T uz_c = at(uz, n, 0), uz_jm = at_jm(uz, g, 2, n, 0);
-    const T uz_kp = at(uz, n, n.zp), uz_jm_kp = at_jm(uz, g, 2, n, n.zp);
-    const T p_c = at(pr, n, 0), p_jm = at_jm(pr, g, 3, n, 0);
-    const T h_o = h[n.c];
-    const T hdx1 = half * rdx, hdx3 = half * rdz;
-    const T sucac = m.rdyc[jc], qsucac = quarter * sucac;
-    T h21 = ((IY1 * ux_ip_jm + IY2 * ux_ip) * (uy_ip + uy_c) - (IY1 * ux_jm + IY2 * ux_c) * (uy_c + uy_im)) * hdx1;
-    T h22 = ((uy_jp + uy_c) * (uy_jp + uy_c) - (uy_c + uy_jm) * (uy_c + uy_jm)) * qsucac;
-    T h23 = ((IY1 * uz_jm_kp + IY2 * uz_kp) * (uy_kp + uy_c) - (IY1 * uz_jm + IY2 * uz_c) * (uy_c + uy_km)) * hdx3;
-    T d11q2 = g.ap1c * uy_ip + g.ac1c * uy_c + g.am1c * uy_im;
-    T d22q2 = m.ap2p[jc] * uy_jp + m.ac2p[jc] * uy_c + m.am2p[jc] * uy_jm;
-    T d33q2 = g.ap3c * uy_kp + g.ac3c * uy_c + g.am3c * uy_km;
-    T dcq13 = d11q2 + d33q2;
-    T gradp2 = (p_c - p_jm) * sucac;
-    if (g.implicit == 0) {  // clcRhsY_FEXP (src/CFD_2nd/m_TSchemeFEXP_inc.f90:183-204)
-      T convEd2 = -h21 - h22 - h23 + xnu * (d11q2 + d22q2 + d33q2) + g.g2;
-      h[n.c] = convEd2;
-      return pmGamma * convEd2 + pmTheta * h_o - pmAlpha * gradp2;
-    }
-    if (g.implicit == 2) {  // clcRhsY_FIMP (src/CFD_2nd/m_TSchemeFIMP_inc.f90:104-115)
-      T convEd2 = -h21 - h22 - h23 + g.g2;
-      h[n.c] = convEd2;
-      return pmGamma * convEd2 + pmTheta * h_o - pmAlpha * gradp2 + two * pmBeta * (d11q2 + d22q2 + d33q2);
-    }
-    T convEd2 = -h21 - h22 - h23 + xnu * dcq13 + g.g2;
-    h[n.c] = convEd2;
-    return pmGamma * convEd2 + pmTheta * h_o - pmAlpha * gradp2 + two * pmBeta * d22q2;
-  } else {
-    const T ux_c = at(ux, n, 0), ux_ip = at(ux, n, n.xp);
-    const T ux_km = at(ux, n, n.zm), ux_ip_km = at(ux, n, n.zm + n.xp);
-    const T uy_c = at(uy, n, 0), uy_jp = at_jp(uy, g, 1, n, 0);
-    const T uy_km = at(uy, n, n.zm), uy_jp_km = at_jp(uy, g, 1, n, n.zm);
-    const T uz_c = at(uz, n, 0), uz_ip = at(uz, n, n.xp), uz_im = at(uz, n, n.xm);
-    const T uz_jp = at_jp(uz, g, 2, n, 0), uz_jm = at_jm(uz, g, 2, n, 0);
-    const T uz_kp = at(uz, n, n.zp), uz_km = at(uz, n, n.zm);
-    const T p_c = at(pr, n, 0), p_km = at(pr, n, n.zm);
-    const T h_o = h[n.c];
-    const T IY3 = m.yinterp[jc + 1], IY4 = one - IY3;
-    const T qdx1 = quarter * rdx, qdx3 = quarter * rdz;
-    const T sucaj = half * m.rdyp[jc];
-    T h31 = ((ux_ip + ux_ip_km) * (uz_ip + uz_c) - (ux_c + ux_km) * (uz_c + uz_im)) * qdx1;
-    T h32 = ((uy_jp + uy_jp_km) * (IY3 * uz_c + IY4 * uz_jp) - (uy_c + uy_km) * (IY1 * uz_jm + IY2 * uz_c)) * sucaj;
-    T h33 = ((uz_kp + uz_c) * (uz_kp + uz_c) - (uz_c + uz_km) * (uz_c + uz_km)) * qdx3;
-    T d11q3 = g.ap1c * uz_ip + g.ac1c * uz_c + g.am1c * uz_im;
-    T d22q3 = m.ap2c[jc] * uz_jp + m.ac2c[jc] * uz_c + m.am2c[jc] * uz_jm;
-    T d33q3 = (uz_kp - two * uz_c + uz_km) * rdz2;
-    T dcq13 = d11q3 + d33q3;
-    T gradp3 = (p_c - p_km) * rdz;
-    if (g.implicit == 0) {  // clcRhsZ_FEXP (src/CFD_2nd/m_TSchemeFEXP_inc.f90:299-320)
-      T convEd3 = -h31 - h32 - h33 + xnu * (d11q3 + d22q3 + d33q3) + g.g3;
-      h[n.c] = convEd3;
-      return pmGamma * convEd3 + pmTheta * h_o - pmAlpha * gradp3;
-    }
-    if (g.implicit == 2) {  // clcRhsZ_FIMP (src/CFD_2nd/m_TSchemeFIMP_inc.f90:161-172)
-      T convEd3 = -h31 - h32 - h33 + g.g3;
-      h[n.c] = convEd3;
-      return pmGamma * convEd3 + pmTheta * h_o - pmAlpha * gradp3 + two * pmBeta * (d11q3 + d22q3 + d33q3);
-    }
-    T convEd3 = -h31 - h32 - h33 + xnu * dcq13 + g.g3;
-    h[n.c] = convEd3;
-    return pmGamma * convEd3 + pmTheta * h_o - pmAlpha * gradp3 + two * pmBeta * d22q3;
-  }
-}
-
-// Stand-alone clcRhsX/Y/Z (one thread per cell); the stage-level entry point.
-template <class T>
-__global__ void __launch_bounds__(256) k_rhs_pimp(Geo<T> g, Metrics<T> m, const T* __restrict__ ux,
-                                                  const T* __restrict__ uy, const T* __restrict__ uz,
-                                                  const T* __restrict__ pr, T* __restrict__ hx, T* __restrict__ hy,
-                                                  T* __restrict__ hz, T* __restrict__ rx, T* __restrict__ ry,
-                                                  T* __restrict__ rz, const DevScalars* __restrict__ sc) {
-  if (sc->status) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = blockIdx.z;
-  if (i >= g.nx || j >= g.ny) return;
-  T a, b, c;
-  rhs_point(g, m, ux, uy, uz, pr, hx, hy, hz, i, j, k, (T)sc->pmGamma, (T)sc->pmTheta, (T)sc->pmAlpha,
-            (T)sc->pmBeta, a, b, c);
-  const long long idx = i + (long long)g.nx * (j + (long long)g.ny * k);
-  rx[idx] = a; ry[idx] = b; rz[idx] = c;
-}
-
-// clcRhsX/Y/Z_FIMP (src/CFD_2nd/m_TSchemeFIMP_inc.f90:6-177), or _FEXP
-// (src/CFD_2nd/m_TSchemeFEXP_inc.f90:6-324) when g.implicit = 0, one thread per
-// cell and component (blockIdx.z = component * nz + k: a thread holds one
-// component's stencil, so more threads fit an SM than with all three),
-// RhsX with the mean pressure gradient (:57-66) included.
-template <class T>
-__global__ void __launch_bounds__(256) k_rhs_fimp(Geo<T> g, Metrics<T> m, const T* __restrict__ ux,
-                                                  const T* __restrict__ uy, const T* __restrict__ uz,
-                                                  const T* __restrict__ pr, T* __restrict__ hx, T* __restrict__ hy,
-                                                  T* __restrict__ hz, T* __restrict__ rx, T* __restrict__ ry,
-                                                  T* __restrict__ rz, const DevScalars* __restrict__ sc) {
-  if (sc->status) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int comp = blockIdx.z / g.nz, k = blockIdx.z - comp * g.nz;
-  if (i >= g.nx || j >= g.ny) return;
-  const T pmGamma = (T)sc->pmGamma, pmTheta = (T)sc->pmTheta, pmAlpha = (T)sc->pmAlpha, pmBeta = (T)sc->pmBeta;
-  const long long idx = i + (long long)g.nx * (j + (long long)g.ny * k);
-  if (comp == 0)
-    rx[idx] = rhs_comp<T, 0>(g, m, ux, uy, uz, pr, hx, i, j, k, pmGamma, pmTheta, pmAlpha, pmBeta) + (T)sc->dpmdxns;
-  else if (comp == 1)
-    ry[idx] = rhs_comp<T, 1>(g, m, ux, uy, uz, pr, hy, i, j, k, pmGamma, pmTheta, pmAlpha, pmBeta);
-  else
-    rz[idx] = rhs_comp<T, 2>(g, m, ux, uy, uz, pr, hz, i, j, k, pmGamma, pmTheta, pmAlpha, pmBeta);
-}
-
-// Precomputes the chunk factors, spikes and interface block-Thomas factors of
-// both Helmholtz sets for the current pmBeta (once per substep; block = set).
-__global__ void k_helm_factors(HelmCoef hc, int ny, int P, double* __restrict__ fac,
-                               const DevScalars* __restrict__ sc) {
-  if (sc->status) return;
-  const int set = blockIdx.x;
-  double* F = fac + (size_t)set * helm_set_stride(ny, P);
-  double *RM = F, *AA = F + ny, *CP = F + 2 * ny, *AL = F + 3 * ny, *BE = F + 4 * ny, *IFD = F + 5 * ny;
-  const double pmBeta = sc->pmBeta;
-  const int Q = P - 1;
-  for (int p = threadIdx.x; p < P; p += blockDim.x) {
-    const int s = chunk_lo(p, ny, P), e = chunk_hi(p, ny, P);
-    double cpp = 0.0, dal = 0.0;
-    for (int j = s; j <= e; ++j) {
-      double a, b, c;
-      helm_abc(hc, set, pmBeta, j, a, b, c);
-      const double mm = (j == s) ? b : b - a * cpp;
-      const double rm = 1.0 / mm;
-      const double cp = c * rm;
-      dal = (j == s) ? -a * rm : -a * dal * rm;
-      RM[j] = rm; CP[j] = cp; AL[j] = (p == 0) ? 0.0 : dal; AA[j] = a;
-      cpp = cp;
-    }
-    BE[e] = (p == P - 1) ? 0.0 : -CP[e];
-    for (int j = e - 1; j >= s; --j) {
-      AL[j] = AL[j] - CP[j] * AL[j + 1];
-      BE[j] = -CP[j] * BE[j + 1];
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double m01p = 0.0, vprev = 0.0;
-    for (int q = 0; q < Q; ++q) {
-      const int eq = chunk_hi(q, ny, P), sq1 = chunk_lo(q + 1, ny, P);
-      const double l = -AL[eq], v = -BE[sq1];
-      double d00 = 1.0, d01 = -BE[eq], d10 = -AL[sq1], d11 = 1.0;
-      if (q > 0) d01 -= l * m01p * vprev;  // (L_q Minv_{q-1} U_{q-1}) has only a (0,1) entry
-      const double r = 1.0 / (d00 * d11 - d01 * d10);
-      double* R = IFD + 6 * q;
-      R[0] = d11 * r; R[1] = -d01 * r; R[2] = -d10 * r; R[3] = d00 * r; R[4] = l; R[5] = v;
-      m01p = R[1]; vprev = v;
-    }
-  }
-}
-
-// clcU1Hat/U2Hat/U3Hat_PIMP from RhsX/Y/Z in memory (stage-level entry point):
-// (I - pmBeta L_y) du = Rhs ; u* = u + du written to the u* buffers.
-// Block: TI consecutive i at one k, all j; threads = TI * P; blockIdx.z = component.
-template <class T, int TI>
-__global__ void __launch_bounds__(256) k_uhat_pimp(Geo<T> g, const double* __restrict__ fac, int P,
-                                                   const T* __restrict__ ux, const T* __restrict__ uy,
-                                                   const T* __restrict__ uz, const T* __restrict__ rx,
-                                                   const T* __restrict__ ry, const T* __restrict__ rz,
-                                                   T* __restrict__ uxs, T* __restrict__ uys, T* __restrict__ uzs,
-                                                   const DevScalars* __restrict__ sc) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  if (sc->status) return;
-  const int comp = blockIdx.z;
-  const T* u = comp == 0 ? ux : (comp == 1 ? uy : uz);
-  T* us = comp == 0 ? uxs : (comp == 1 ? uys : uzs);
-  const T* rhs = comp == 0 ? rx : (comp == 1 ? ry : rz);
-  const int nx = g.nx, ny = g.ny, k = blockIdx.y, i0 = blockIdx.x * TI, Q = P - 1;
-  const double* F64 = fac + (size_t)(comp == 1 ? 1 : 0) * helm_set_stride(ny, P);
-  const double *RM = F64, *AA = F64 + ny, *CP = F64 + 2 * ny, *AL = F64 + 3 * ny, *BE = F64 + 4 * ny,
-               *IFD = F64 + 5 * ny;
-  T* F = (T*)smem_raw;                    // ny * TI
-  T* IF = F + (size_t)ny * TI;            // TI * 2Q
-  // the 4th-order and FIMP RhsX already carry the forcing (k_rhs4, k_rhs_fimp)
-  const T add = (comp == 0 && g.order != 4 && g.implicit != 2) ? (T)sc->dpmdxns : (T)0;
-  const int tid = threadIdx.x;
-  // the block's right-hand sides (coalesced rows of TI values) by asynchronous
-  // copies, all in flight at once
-  for (int t = tid; t < ny * TI; t += blockDim.x) {
-    const int j = t / TI, ii = t % TI, i = i0 + ii;
-    if (i < nx) cp_async_el(F + t, rhs + i + (long long)nx * (j + (long long)ny * k));
-  }
-  cp_async_commit();
-  cp_async_wait<0>();  // this thread's copies (the slots it reads next)
-  for (int t = tid; t < ny * TI; t += blockDim.x) {
-    const int j = t / TI, ii = t % TI, i = i0 + ii;
-    T f = (T)0;
-    if (i < nx) f = F[t] + add;
-    if (comp == 1 && j == 0) f = (T)0;  // duy_ym: uy_ym is constant (Update_uy_ym_CH)
-    F[t] = f;
-  }
-  __syncthreads();
-  for (int t = tid; t < TI * P; t += blockDim.x) {
-    const int ii = t % TI, p = t / TI;
-    const int s = chunk_lo(p, ny, P), e = chunk_hi(p, ny, P);
-    T d = (T)0;
-    for (int j = s; j <= e; ++j) {
-      const T f = F[j * TI + ii];
-      d = (j == s) ? f * (T)RM[j] : (f - (T)AA[j] * d) * (T)RM[j];
-      F[j * TI + ii] = d;
-    }
-    for (int j = e - 1; j >= s; --j) {
-      d = F[j * TI + ii] - (T)CP[j] * d;
-      F[j * TI + ii] = d;
-    }
-  }
-  __syncthreads();
-  for (int t = tid; t < TI; t += blockDim.x) helm_interfaces<T>(IFD, F + t, TI, ny, P, IF + (size_t)t * 2 * (Q > 0 ? Q : 1));
-  __syncthreads();
-  for (int t = tid; t < ny * TI; t += blockDim.x) {
-    const int j = t / TI, ii = t % TI, i = i0 + ii;
-    if (i >= nx) continue;
-    const int p = chunk_of(j, ny, P);
-    const T* G = IF + (size_t)ii * 2 * (Q > 0 ? Q : 1);
-    T x = F[t];
-    if (p > 0) x += (T)AL[j] * G[2 * (p - 1)];
-    if (p < P - 1) x += (T)BE[j] * G[2 * p + 1];
-    const long long idx = i + (long long)nx * (j + (long long)ny * k);
-    us[idx] = u[idx] + x;
-  }
-}
-
-// ---------------------------------------------------------------------------
 // y tridiagonal per (kx,kz) (src/CFD_2nd/m_Poisson.f90:1114-1156):
 // [am2Pr, ac2Pr + WaveNumX + WaveNumZ, ap2Pr], with the (kx,kz)=(0,0) system's
 // first row replaced by the identity and zero right-hand side.  Solved in FP64
@@ -739,22 +375,6 @@ static dim3 cell_grid(const ch3d_ctx* c) { return dim3((c->nx + 31) / 32, (c->ny
 static dim3 cell_block() { return dim3(32, 8, 1); }
 
 
-template <class T> static cudaError_t rhs_t(ch3d_ctx* c) {
-  T** f = (T**)c->f;
-  k_rhs_pimp<T><<<cell_grid(c), cell_block(), 0, c->stream>>>(make_geo<T>(c), metrics_of<T>(c), f[0], f[1], f[2], f[3],
-                                                              f[4], f[5], f[6], f[7], f[8], f[9], c->sc);
-  return cudaGetLastError();
-}
-cudaError_t launch_rhs(ch3d_ctx* c) { return c->fp32 ? rhs_t<float>(c) : rhs_t<double>(c); }
-template <class T> static cudaError_t rhs_fimp_t(ch3d_ctx* c) {
-  T** f = (T**)c->f;
-  const dim3 grid((c->nx + 31) / 32, (c->ny + 7) / 8, 3 * c->nz);  // z: component * nz + k
-  k_rhs_fimp<T><<<grid, cell_block(), 0, c->stream>>>(make_geo<T>(c), metrics_of<T>(c), f[0], f[1], f[2], f[3],
-                                                              f[4], f[5], f[6], f[7], f[8], f[9], c->sc);
-  return cudaGetLastError();
-}
-cudaError_t launch_rhs_fimp(ch3d_ctx* c) { return c->fp32 ? rhs_fimp_t<float>(c) : rhs_fimp_t<double>(c); }
-
 // clcU1/2/3Hat_FEXP (src/CFD_2nd/m_TSchemeFEXP_inc.f90:391-488): u* = u + Rhs,
 // every cell; between walls the uy row on the lower wall then takes uy_ym,
 // as SetBC_and_UpdateHaloForPrSrc (src/CFD_2nd/m_BC_and_Halo.f90:349-405)
@@ -787,27 +407,6 @@ template <class T> static cudaError_t uhat_fexp_t(ch3d_ctx* c) {
 }
 cudaError_t launch_uhat_fexp(ch3d_ctx* c) { return c->fp32 ? uhat_fexp_t<float>(c) : uhat_fexp_t<double>(c); }
 
-cudaError_t launch_helm_factors(ch3d_ctx* c) {
-  k_helm_factors<<<2, 64, 0, c->stream>>>(helm_coef(c), c->ny, c->Pv, c->hfac, c->sc);
-  return cudaGetLastError();
-}
-
-template <class T> static cudaError_t uhat_t(ch3d_ctx* c) {
-  constexpr int TI = 16;
-  T** f = (T**)c->f;
-  const int P = c->Pv, Q = P - 1;
-  size_t smem = (size_t)c->ny * TI * sizeof(T) + (size_t)TI * 2 * (Q > 0 ? Q : 1) * sizeof(T) + 16;
-  static PerDevice attr;  // per precision (template instance)
-  auto kern = k_uhat_pimp<T, TI>;
-  cudaError_t e = smem_limit_once(attr, c->device, kern, 200 * 1024);
-  if (e != cudaSuccess) return e;
-  dim3 grid((c->nx + TI - 1) / TI, c->nz, 3);
-  int nthr = TI * P < 64 ? 64 : (TI * P > 256 ? 256 : TI * P);
-  kern<<<grid, nthr, smem, c->stream>>>(make_geo<T>(c), c->hfac, P, f[0], f[1], f[2], f[7], f[8], f[9], f[12], f[13],
-                                        f[14], c->sc);
-  return cudaGetLastError();
-}
-cudaError_t launch_uhat(ch3d_ctx* c) { return c->fp32 ? uhat_t<float>(c) : uhat_t<double>(c); }
 
 
 // The register-resident transforms where the length has a plan, else the generic ones (ch3d_fft.cu).

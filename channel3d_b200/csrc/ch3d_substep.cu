@@ -116,12 +116,40 @@ __device__ void update_row_table(const HelmCoef& hg, const Metrics<T>& m, int ny
   }
 }
 
+// Factor block of one periodic direction (layout: ch3d_march.cuh) for spacing r2 = 1/h^2
+__device__ void update_ptri_block(double* F, int n, double r2, double pmBeta) {
+  double *ppj = F, *v1 = F + (n + 1), *v2 = F + 2 * (n + 1), *abc = F + 3 * (n + 1);
+  const double a = -pmBeta * r2, c = -pmBeta * r2, b = pmBeta * r2 * 2.0 + 1.0;
+  double p1 = -c / b, p2 = -a / b;
+  v1[1] = p1;
+  v2[1] = p2;
+  v2[n] = 1.0;
+  ppj[1] = 0.0;
+  for (int j = 2; j <= n - 1; ++j) {
+    const double pp = 1.0 / (b + a * p1);
+    p1 = -c * pp;
+    p2 = -a * p2 * pp;
+    ppj[j] = pp;
+    v1[j] = p1;
+    v2[j] = p2;
+  }
+  double w = 1.0;
+  for (int j = n - 1; j >= 1; --j) {
+    w = v2[j] + v1[j] * w;
+    v2[j] = w;
+  }
+  abc[0] = a; abc[1] = b; abc[2] = c;
+  abc[3] = c * v2[1] + a * v2[n - 1] + b;
+}
+
 template <class T> struct TableArgs {
   HelmCoef hc;
   Metrics<T> m;
-  int ny;
+  int nx, ny, nz;
   T* tab;                     // row tables of the substeps (null: none)
   T* dtab;                    // their downward tables (null: not used)
+  double* pf;                 // periodic factor blocks of the substeps (null: none)
+  double r2x, r2y, r2z;       // 1/h^2 of the x, y and z sweeps; 0: no such sweep
   unsigned long long* slots;  // pmBeta the tables of each substep hold (all ones: none)
 };
 
@@ -187,6 +215,14 @@ __global__ void __launch_bounds__(kSetupThreads) k_substep(DevScalars* sc, const
   const unsigned long long bits = (unsigned long long)__double_as_longlong(beta);
   if (ta.slots[q] == bits) return;  // uniform: every thread reads it before thread 0 writes below
   __syncthreads();
+  if (ta.pf && threadIdx.x >= 128 && (threadIdx.x & 31) == 0) {  // warps 4, 5, 6: the x, z and y blocks
+    const int d = (threadIdx.x >> 5) - 4;
+    const double r2 = d == 0 ? ta.r2x : d == 1 ? ta.r2z : d == 2 ? ta.r2y : 0.0;
+    double* F = ta.pf + (size_t)q * ptri_doubles(ta.nx, ta.ny, ta.nz);
+    if (r2 > 0.0)
+      update_ptri_block(d == 0 ? F : d == 1 ? F + ptri_stride(ta.nx) : F + ptri_stride(ta.nx) + ptri_stride(ta.nz),
+                        d == 0 ? ta.nx : d == 1 ? ta.nz : ta.ny, r2, beta);
+  }
   update_row_table(ta.hc, ta.m, ta.ny, ta.tab + (size_t)q * ta.ny * MT_W,
                    ta.dtab ? ta.dtab + (size_t)q * ta.ny * MD_W : nullptr, beta,
                    ta.ny <= kStagedRows ? reinterpret_cast<double*>(smem_raw) : nullptr);
@@ -262,10 +298,18 @@ template <class T> static cudaError_t substep_t(ch3d_ctx* c, int ns, bool whole_
   p.yly = c->cfg.yly;
   TableArgs<T> ta;
   ta.hc = helm_coef(c);
-  ta.m = metrics_of<T>(c);
-  ta.ny = c->ny;
-  ta.tab = c->march || c->cfg.order == 4 ? (T*)c->mtab : nullptr;
-  ta.dtab = ta.tab && march_twisted(c) ? march_down_tables<T>(c->mtab, c->ny) : nullptr;
+  ta.m = c->cfg.LES_type == 0 ? metrics_of<T>(c) : Metrics<T>();
+  if constexpr (sizeof(T) == 8)
+    if (c->cfg.LES_type > 0) ta.m = c->m64full;
+  ta.nx = c->nx; ta.ny = c->ny; ta.nz = c->nz;
+  // the eddy-viscosity closures form their own coefficients
+  ta.tab = c->cfg.LES_type == 0 || les_const(c) ? (T*)c->mtab : nullptr;
+  ta.pf = c->pfac;
+  const bool fimp = c->cfg.order == 2 && c->cfg.IsImplicit == 2;
+  ta.r2x = fimp ? c->rdx2 : 0.0;
+  ta.r2z = fimp ? c->rdz2 : 0.0;
+  ta.r2y = y_periodic(c) ? c->rdy2 : 0.0;
+  ta.dtab = ta.tab && (c->march || c->cfg.order == 4) && march_twisted(c) ? march_down_tables<T>(c->mtab, c->ny) : nullptr;
   ta.slots = march_beta_slots(c->mtab, c->ny);
   // the partials of the bulk sums (projection or k_bulk_partial), or of the
   // 4th-order viscous sum (k_visc4_partial)
@@ -275,7 +319,8 @@ template <class T> static cudaError_t substep_t(ch3d_ctx* c, int ns, bool whole_
   return cudaGetLastError();
 }
 cudaError_t launch_substep_setup(ch3d_ctx* c, int ns, bool whole_step) {
-  return c->fp32 ? substep_t<float>(c, ns, whole_step) : substep_t<double>(c, ns, whole_step);
+  // LES: FP64 coefficients on either field type
+  return c->fp32 && c->cfg.LES_type == 0 ? substep_t<float>(c, ns, whole_step) : substep_t<double>(c, ns, whole_step);
 }
 
 cudaError_t launch_step_end(ch3d_ctx* c) {
