@@ -178,6 +178,21 @@ void build_metrics(ch3d_ctx* c) {
     if (c->yc[j] < g.ybulk1 || c->yc[j] >= g.ybulk2) w = 0.0;
     c->s1coe[j] = w;
   }
+  // 4th order: the forcing needs the mean viscous stress, the sum of (d11q1 + d33q1
+  // + d22q1) dyp over ux (src/CFD_4th/m_TScheme.f90:255-262, 364-377).  The x and z
+  // terms sum to zero over their periodic directions, so the sum is one of ux with
+  // a weight per row (zero up to rounding away from the walls) and a wall term.
+  if (g.order == 4) {
+    for (int j = 1; j <= nyc; ++j) {
+      double w = c->dyp[j] * c->ac2c[j];
+      if (j > 1) w += c->dyp[j - 1] * c->ap2c[j - 1];
+      if (j < nyc) w += c->dyp[j + 1] * c->am2c[j + 1];
+      if (j == 1) w -= c->dyp[1] * c->am2c[1];        // ghosts 2 u_wall - ux (no-slip walls)
+      if (j == nyc) w -= c->dyp[nyc] * c->ap2c[nyc];
+      c->s1coe[j] = w;
+    }
+    c->visc_wall = 2.0 * (g.uxBcValue[2] * c->dyp[1] * c->am2c[1] + g.uxBcValue[3] * c->dyp[nyc] * c->ap2c[nyc]);
+  }
   // x, z (uniform, periodic)
   c->dx = g.xlx / (double)c->nx; c->dz = g.zlz / (double)c->nz;
   c->rdx = (double)c->nx / g.xlx; c->rdz = (double)c->nz / g.zlz;
@@ -503,9 +518,7 @@ cudaError_t launch_ustar(ch3d_ctx* c) {
 
 int record_step(ch3d_ctx* c) {
   if (c->cfg.LES_type > 0) CU(launch_sgs_nut(c));  // once per step (m_ChannelSystem.f90:89)
-  const bool o4 = c->cfg.order == 4;
   for (int ns = 1; ns <= c->iadvance; ++ns) {
-    if (o4) CU(launch_visc4_partials(c));
     CU(launch_substep_setup(c, ns, true));
     CU(launch_ustar(c));
     if (c->gsub) {
@@ -701,7 +714,6 @@ int ch3d_create(const ch3d_config* cfg, const double* yp, ch3d_ctx** out) {
     c->npart_m = march_npart(c);
     if (c->npart_m > c->npart) c->npart = c->npart_m;
     if (diag_npart(c) > c->npart) c->npart = diag_npart(c);
-    if (visc4_npart(c) > c->npart) c->npart = visc4_npart(c);
     if (cudaMalloc(&c->part, (size_t)c->npart * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&c->part2, (size_t)c->npart * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&c->red1, CH3D_NRED * sizeof(double)) != cudaSuccess ||
@@ -845,7 +857,6 @@ int ch3d_stage(ch3d_ctx* c, int stage, int ns) {
   }
   switch (stage) {
     case 0:
-      if (c->cfg.order == 4) CU(launch_visc4_partials(c));  // forcing of clcRhsXYZ from the current ux
       CU(launch_substep_setup(c, ns, false));
       break;
     case 1:
@@ -1138,7 +1149,6 @@ int ch3d_kernel_times(ch3d_ctx* c, int nsteps, double* out, int nout) {
     CU(mark(6)); if (c->cfg.LES_type > 0) CU(launch_sgs_nut(c)); CU(done());
     for (int ns = 1; ns <= c->iadvance; ++ns) {
       CU(mark(6));
-      if (c->cfg.order == 4) CU(launch_visc4_partials(c));
       CU(launch_substep_setup(c, ns, true));
       CU(done());
       CU(mark(0)); CU(launch_ustar(c)); CU(done());

@@ -29,6 +29,7 @@ struct ch3d_ctx {
   std::vector<double> yp, yc, dyp, dyc, rdyp, rdyc, yinterp;
   std::vector<double> ap2c, ac2c, am2c, ap2p, ac2p, am2p, ap2Pr, ac2Pr, am2Pr;
   std::vector<double> am2cForCN, ap2cForCN, s1coe, WaveNumX, WaveNumZ;
+  double visc_wall = 0;      // 4th order: wall term of the mean viscous stress, per unit x-z area of cells
 
   // device buffers
   void* f[15] = {nullptr};   // ux uy uz p hx hy hz rx ry rz phi nut u*x u*y u*z (precision T)
@@ -150,8 +151,6 @@ cudaError_t launch_fill_row0(ch3d_ctx* c, int q, double v);  // field q: every j
 cudaError_t launch_convert(ch3d_ctx* c, const void* src, void* dst, long long n, int to_f32);  // FP64 <-> FP32
 // 4th-order solver (ch3d_step4.cu)
 cudaError_t launch_rhs4(ch3d_ctx* c);                  // stage path: interpolation + RhsX/Y/Z
-cudaError_t launch_visc4_partials(ch3d_ctx* c);        // mean viscous stress partial sums -> part
-int visc4_npart(const ch3d_ctx* c);                   // their count
 cudaError_t launch_dissipation(ch3d_ctx* c, int* npart);  // CalcDissipationRate partials -> part2
 cudaError_t launch_reduce_partials(ch3d_ctx* c, const double* in, int n, double* out);  // CH3D_NRED sums
 // fully implicit and explicit 2nd-order steps (ch3d_step.cu, ch3d_sweep.cu)

@@ -113,6 +113,29 @@ __device__ __forceinline__ T div4_cell(const Geo<T>& g, const C4<T>& c, T rdyp, 
                                        const T* __restrict__ uy, const T* __restrict__ uz, int i, int j, int k) {
   return div4_at(g, c, rdyp, ux, uy, uz, make_nbr(g, i, j, k));
 }
+// The same at the cells i0 and i0 + 1 (i0 even) of line `base` = nx (j + ny k),
+// read as aligned pairs; out[0], out[1] as div4_cell gives them.
+template <class T>
+__device__ __forceinline__ void div4_pair(const Geo<T>& g, const C4<T>& c, T rdyp, const T* __restrict__ ux,
+                                          const T* __restrict__ uy, const T* __restrict__ uz, long long base, int i0,
+                                          int j, int k, T (&out)[2]) {
+  typedef typename CplxOf<T>::type T2;
+  const int nx = g.nx;
+  const long long plane = (long long)nx * g.ny;
+  auto pair = [](const T* p) { return __ldg(reinterpret_cast<const T2*>(p)); };
+  const T2 um = pair(ux + base + (i0 == 0 ? nx - 2 : i0 - 2)), u0 = pair(ux + base + i0);
+  const T2 u2 = pair(ux + base + (i0 + 2 == nx ? 0 : i0 + 2));
+  const T2 v0 = pair(uy + base + i0);
+  const T2 v1 = j + 1 < g.ny ? pair(uy + base + nx + i0) : mk((T)g.bc.uy_hi, (T)g.bc.uy_hi);
+  const T* const wz = uz + i0;
+  const T2 wm = pair(wz + base + (k == 0 ? plane * (g.nz - 1) : -plane)), w0 = pair(wz + base);
+  const T2 w1 = pair(wz + base + (k + 1 >= g.nz ? plane * (1 - g.nz) : plane));
+  const T2 w2 = pair(wz + base + (k + 2 >= g.nz ? plane * (2 - g.nz) : 2 * plane));
+  out[0] = (c.dx1 * um.y + c.dx2 * u0.x + c.dx3 * u0.y + c.dx4 * u2.x) + (v1.x - v0.x) * rdyp +
+           (c.dz1 * wm.x + c.dz2 * w0.x + c.dz3 * w1.x + c.dz4 * w2.x);
+  out[1] = (c.dx1 * u0.x + c.dx2 * u0.y + c.dx3 * u2.x + c.dx4 * u2.y) + (v1.y - v0.y) * rdyp +
+           (c.dz1 * wm.y + c.dz2 * w0.y + c.dz3 * w1.y + c.dz4 * w2.y);
+}
 // move a neighbourhood one row up the same column (the x and z offsets do not
 // depend on j)
 template <class T> __device__ __forceinline__ void nbr_next_row(Nbr& n, const Geo<T>& g, int j) {

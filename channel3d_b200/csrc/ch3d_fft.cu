@@ -16,32 +16,25 @@ namespace ch3d {
 // (against bank conflicts of the first pass's strided stores), none with sh = 31.
 __device__ __forceinline__ int xpad(int n, int sh) { return n + (n >> sh); }
 
-// src = div(u)/pmAlpha (modes 0, 1), packed as z_n = src_2n + i src_2n+1, complex
-// FFT of length nx/2, then the real-to-complex split
-// X_k = (Z_k + conj Z_{M-k})/2 - i W_nx^k (Z_k - conj Z_{M-k})/2, k = 0..M.
+// The source of the forward transform, packed as z_n = src_2n + i src_2n+1:
+// div(u)/pmAlpha (modes 0, 1), with its largest magnitude in dmax.
 // SRC: 0 2nd-order divergence, 1 4th-order divergence, 2 the source (mode 2), the
 // divergence (mode 3) or a field (mode 4) as it stands in the first array.
-template <class T, int SRC>
-__global__ void __launch_bounds__(256) k_xfft_g(Geo<T> g, Metrics<T> m, const T* __restrict__ ux,
-                                                const T* __restrict__ uy, const T* __restrict__ uz,
-                                                typename CplxOf<T>::type* __restrict__ spec, FFTPlanDev pl,
-                                                const typename CplxOf<T>::type* __restrict__ tw,
-                                                const typename CplxOf<T>::type* __restrict__ twr, int LPB, int LP, int sh,
-                                                int mode, DevScalars* __restrict__ sc, T* __restrict__ pr) {
+template <class T, int SRC> struct XSource {
   typedef typename CplxOf<T>::type CT;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  if (sc->status) return;
-  const int nx = g.nx, ny = g.ny, nz = g.nz, M = nx / 2, nxh = g.nxh;
-  const int nlines = ny * nz;
-  const int line0 = blockIdx.x * LPB;
-  const int nl = min(LPB, nlines - line0);
-  CT* src = (CT*)smem_raw;
-  CT* dst = src + (size_t)LPB * LP;
-  const T sudtal = mode == 0 || mode == 3 ? (T)(1.0 / sc->pmAlpha) : (T)1;
-  const T rdx = g.rdx, rdz = g.rdz;
-  double dmax = 0.0;
-  auto form = [&](int l, int n) -> CT {
-    const int line = line0 + l;
+  const Geo<T>& g;
+  const Metrics<T>& m;
+  const T* __restrict__ ux;
+  const T* __restrict__ uy;
+  const T* __restrict__ uz;
+  T* __restrict__ pr;
+  int mode;
+  T sudtal;
+  double dmax;
+  // point n of line j + ny k
+  __device__ __forceinline__ CT operator()(int line, int n) {
+    const int nx = g.nx, ny = g.ny, nz = g.nz;
+    const T rdx = g.rdx, rdz = g.rdz;
     const long long base = (long long)nx * line;
     const int i0 = 2 * n;
     T r0, r1;
@@ -53,8 +46,9 @@ __global__ void __launch_bounds__(256) k_xfft_g(Geo<T> g, Metrics<T> m, const T*
       const T sucaj = m.rdyp[j + 1];
       if constexpr (SRC == 1) {
         const C4<T> c4(g);
-        r0 = div4_cell(g, c4, sucaj, ux, uy, uz, i0, j, k);
-        r1 = div4_cell(g, c4, sucaj, ux, uy, uz, i0 + 1, j, k);
+        T d[2];
+        div4_pair(g, c4, sucaj, ux, uy, uz, base, i0, j, k, d);
+        r0 = d[0]; r1 = d[1];
       } else {
         const int i2 = i0 + 2 == nx ? 0 : i0 + 2;
         const long long basep = k + 1 == nz ? base - (long long)nx * ny * (nz - 1) : base + (long long)nx * ny;
@@ -79,43 +73,80 @@ __global__ void __launch_bounds__(256) k_xfft_g(Geo<T> g, Metrics<T> m, const T*
     }
     dmax = fmax(dmax, fmax(fabs((double)r0), fabs((double)r1)));
     return mk(sudtal * r0, sudtal * r1);
-  };
-  fft_pass<CT, false>(pl, 0, nl, tw, form, [&](int l, int n, CT v) { src[l * LP + xpad(n, sh)] = v; });
+  }
+  // the block's largest |div| into sc->divmax1 (modes 0 to 2; mode 3: it was taken where the divergence was formed)
+  __device__ __forceinline__ void finish(DevScalars* sc) {
+    if (mode >= 3) return;
+    __shared__ double wred[16];
+    for (int o = 16; o > 0; o >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
+    if ((threadIdx.x & 31) == 0) wred[threadIdx.x >> 5] = dmax;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double v = wred[0];
+      for (int w = 1; w < (int)blockDim.x / 32; ++w) v = fmax(v, wred[w]);
+      atomic_max_nonneg(&sc->divmax1, v);
+    }
+  }
+};
+
+// real-to-complex split of a line Z (0..M-1): X_k = (Z_k + conj Z_{M-k})/2 - i W_nx^k (Z_k - conj Z_{M-k})/2, k = 0..M
+template <class CT> __device__ __forceinline__ CT r2c_split(CT a, CT zb, CT w) {
+  const auto hf = a.x * 0 + (decltype(a.x))0.5;
+  const CT b = cconj(zb);
+  const CT e = mk(hf * (a.x + b.x), hf * (a.y + b.y));
+  const CT dd = csub(a, b);
+  const CT o = mk(hf * dd.y, -hf * dd.x);  // (a-b)/(2i)
+  return cadd(e, cmul(w, o));
+}
+// and its inverse: Z_k = e + i o, conjugated for the forward-transform-based inverse
+template <class CT> __device__ __forceinline__ CT c2r_unsplit(CT a, CT xb, CT w) {
+  const CT b = cconj(xb);
+  const CT e = cadd(a, b);
+  const CT o = cmul(csub(a, b), cconj(w));
+  return cconj(mk(e.x - o.y, e.y + o.x));
+}
+
+// Forward x transform of LPB lines per block.
+template <class T, int SRC>
+__global__ void __launch_bounds__(256) k_xfft_g(Geo<T> g, Metrics<T> m, const T* __restrict__ ux,
+                                                const T* __restrict__ uy, const T* __restrict__ uz,
+                                                typename CplxOf<T>::type* __restrict__ spec, FFTPlanDev pl,
+                                                const typename CplxOf<T>::type* __restrict__ tw,
+                                                const typename CplxOf<T>::type* __restrict__ twr, int LPB, int LP, int sh,
+                                                unsigned long long mM1, int mode, DevScalars* __restrict__ sc,
+                                                T* __restrict__ pr) {
+  typedef typename CplxOf<T>::type CT;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  if (sc->status) return;
+  const int M = g.nx / 2, nxh = g.nxh;
+  const int line0 = blockIdx.x * LPB;
+  const int nl = min(LPB, g.ny * g.nz - line0);
+  CT* src = (CT*)smem_raw;
+  CT* dst = src + (size_t)LPB * LP;
+  XSource<T, SRC> form{g, m, ux, uy, uz, pr, mode, mode == 0 || mode == 3 ? (T)(1.0 / sc->pmAlpha) : (T)1, 0.0};
+  fft_pass<CT, false>(pl, 0, nl, 0ull, tw, [&](int l, int n) { return form(line0 + l, n); },
+                      [&](int l, int n, CT v) { src[l * LP + xpad(n, sh)] = v; });
   __syncthreads();
   for (int p = 1; p < pl.npass; ++p) {
-    fft_pass<CT, false>(pl, p, nl, tw, [&](int l, int n) { return src[l * LP + xpad(n, sh)]; },
+    fft_pass<CT, false>(pl, p, nl, 0ull, tw, [&](int l, int n) { return src[l * LP + xpad(n, sh)]; },
                         [&](int l, int n, CT v) { dst[l * LP + xpad(n, sh)] = v; });
     __syncthreads();
     CT* t = src; src = dst; dst = t;
   }
-  const T hf = (T)0.5;
-  const unsigned long long mM1 = fdiv_magic((unsigned)(M + 1));
   for (int t = threadIdx.x; t < nl * (M + 1); t += blockDim.x) {
     const int l = fdiv(t, mM1), kk = t - l * (M + 1);
-    const CT a = src[l * LP + xpad(kk == M ? 0 : kk, sh)];
-    const CT b = cconj(src[l * LP + xpad(kk == 0 ? 0 : M - kk, sh)]);
-    const CT e = mk(hf * (a.x + b.x), hf * (a.y + b.y));
-    const CT dd = csub(a, b);
-    const CT o = mk(hf * dd.y, -hf * dd.x);  // (a-b)/(2i)
-    spec[(long long)nxh * (line0 + l) + kk] = cadd(e, cmul(__ldg(twr + kk), o));
+    spec[(long long)nxh * (line0 + l) + kk] = r2c_split(src[l * LP + xpad(kk == M ? 0 : kk, sh)],
+                                                        src[l * LP + xpad(kk == 0 ? 0 : M - kk, sh)], __ldg(twr + kk));
   }
-  if (mode >= 3) return;  // mode 3: its maximum was taken where the divergence was formed; 4: a plain transform
-  __shared__ double wred[8];
-  for (int o = 16; o > 0; o >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
-  if ((threadIdx.x & 31) == 0) wred[threadIdx.x >> 5] = dmax;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double v = wred[0];
-    for (int w = 1; w < (int)blockDim.x / 32; ++w) v = fmax(v, wred[w]);
-    atomic_max_nonneg(&sc->divmax1, v);
-  }
+  form.finish(sc);
 }
 
 // z transform of the spectrum, in place: layout (kx, j, kz), lines over kz.
 // Block = up to TKX consecutive kx at one j; point n of line l at n * TKX + l.
 template <class T>
 __global__ void __launch_bounds__(256) k_zfft_g(Geo<T> g, typename CplxOf<T>::type* __restrict__ spec, FFTPlanDev pl,
-                                                const typename CplxOf<T>::type* __restrict__ tw, int TKX, int inverse,
+                                                const typename CplxOf<T>::type* __restrict__ tw, int TKX,
+                                                unsigned long long mT, unsigned long long mTail, int inverse,
                                                 const DevScalars* __restrict__ sc) {
   typedef typename CplxOf<T>::type CT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -126,22 +157,23 @@ __global__ void __launch_bounds__(256) k_zfft_g(Geo<T> g, typename CplxOf<T>::ty
   CT* const col = spec + kx0 + (long long)nxh * blockIdx.y;
   CT* src = (CT*)smem_raw;
   CT* dst = src + (size_t)TKX * nz;  // used from three passes on
+  const unsigned long long mL = nl == TKX ? mT : mTail;
   auto ldg = [&](int l, int n) { const CT v = col[zs * n + l]; return inverse ? cconj(v) : v; };
   auto stg = [&](int l, int n, CT v) { col[zs * n + l] = inverse ? cconj(v) : v; };
   auto lds = [&](int l, int n) { return src[n * TKX + l]; };
   const int last = pl.npass - 1;
   if (last == 0) {
-    fft_pass<CT, true>(pl, 0, nl, tw, ldg, stg);
+    fft_pass<CT, true>(pl, 0, nl, mL, tw, ldg, stg);
     return;
   }
-  fft_pass<CT, true>(pl, 0, nl, tw, ldg, [&](int l, int n, CT v) { src[n * TKX + l] = v; });
+  fft_pass<CT, true>(pl, 0, nl, mL, tw, ldg, [&](int l, int n, CT v) { src[n * TKX + l] = v; });
   __syncthreads();
   for (int p = 1; p < last; ++p) {
-    fft_pass<CT, true>(pl, p, nl, tw, lds, [&](int l, int n, CT v) { dst[n * TKX + l] = v; });
+    fft_pass<CT, true>(pl, p, nl, mL, tw, lds, [&](int l, int n, CT v) { dst[n * TKX + l] = v; });
     __syncthreads();
     CT* t = src; src = dst; dst = t;
   }
-  fft_pass<CT, true>(pl, last, nl, tw, lds, stg);
+  fft_pass<CT, true>(pl, last, nl, mL, tw, lds, stg);
 }
 
 // inverse x transform (complex-to-real, unnormalised as FFTW's HC2R) * normfft -> phi
@@ -160,13 +192,9 @@ __global__ void __launch_bounds__(256) k_xifft_g(Geo<T> g, const typename CplxOf
   const int nl = min(LPB, nlines - line0);
   CT* src = (CT*)smem_raw;
   CT* dst = src + (size_t)LPB * LP;
-  auto unsplit = [&](int l, int kk) -> CT {
+  auto unsplit = [&](int l, int kk) {
     const CT* X = spec + (long long)nxh * (line0 + l);
-    const CT a = X[kk];
-    const CT b = cconj(X[M - kk]);
-    const CT e = cadd(a, b);
-    const CT o = cmul(csub(a, b), cconj(__ldg(twr + kk)));
-    return cconj(mk(e.x - o.y, e.y + o.x));  // Z_k = e + i o, conjugated for the forward-transform-based inverse
+    return c2r_unsplit(X[kk], X[M - kk], __ldg(twr + kk));
   };
   auto out = [&](int l, int n, CT v) {
     reinterpret_cast<CT*>(phi + (long long)nx * (line0 + l))[n] = mk(v.x * normfft, -v.y * normfft);
@@ -174,17 +202,17 @@ __global__ void __launch_bounds__(256) k_xifft_g(Geo<T> g, const typename CplxOf
   auto lds = [&](int l, int n) { return src[l * LP + xpad(n, sh)]; };
   const int last = pl.npass - 1;
   if (last == 0) {
-    fft_pass<CT, false>(pl, 0, nl, tw, unsplit, out);
+    fft_pass<CT, false>(pl, 0, nl, 0ull, tw, unsplit, out);
     return;
   }
-  fft_pass<CT, false>(pl, 0, nl, tw, unsplit, [&](int l, int n, CT v) { src[l * LP + xpad(n, sh)] = v; });
+  fft_pass<CT, false>(pl, 0, nl, 0ull, tw, unsplit, [&](int l, int n, CT v) { src[l * LP + xpad(n, sh)] = v; });
   __syncthreads();
   for (int p = 1; p < last; ++p) {
-    fft_pass<CT, false>(pl, p, nl, tw, lds, [&](int l, int n, CT v) { dst[l * LP + xpad(n, sh)] = v; });
+    fft_pass<CT, false>(pl, p, nl, 0ull, tw, lds, [&](int l, int n, CT v) { dst[l * LP + xpad(n, sh)] = v; });
     __syncthreads();
     CT* t = src; src = dst; dst = t;
   }
-  fft_pass<CT, false>(pl, last, nl, tw, lds, out);
+  fft_pass<CT, false>(pl, last, nl, 0ull, tw, lds, out);
 }
 
 // ---------------------------------------------------------------------------
@@ -232,7 +260,7 @@ cudaError_t xfft_generic(const Geo<T>& g, const Metrics<T>& m, const T* a, const
   const XShape s = x_shape<T>(g.nx / 2, pl.radix[0]);
   const int nlines = g.ny * g.nz, grid = (nlines + s.LPB - 1) / s.LPB;
   auto go = [&](auto kern) {
-    kern<<<grid, s.threads, s.smem, st>>>(g, m, a, b, c, spec, pl, tw, twr, s.LPB, s.LP, s.sh, mode, sc, pr);
+    kern<<<grid, s.threads, s.smem, st>>>(g, m, a, b, c, spec, pl, tw, twr, s.LPB, s.LP, s.sh, fdiv_magic(g.nx / 2 + 1), mode, sc, pr);
   };
   if (mode >= 2) go(k_xfft_g<T, 2>);
   else if (g.order == 4) go(k_xfft_g<T, 1>);
@@ -249,8 +277,9 @@ cudaError_t zfft_generic(const Geo<T>& g, typename CplxOf<T>::type* spec, const 
   const int nbuf = pl.npass <= 1 ? 0 : (pl.npass == 2 ? 1 : 2);
   int TKX = sizeof(T) == 8 || g.nz > 256 ? 8 : 16;
   while (TKX > 1 && (size_t)nbuf * TKX * g.nz * sizeof(CT) > (size_t)kFftSmemLimit / 2) TKX >>= 1;
-  k_zfft_g<T><<<dim3((g.nxh + TKX - 1) / TKX, g.ny), g.nz > 256 ? 256 : 128, (size_t)nbuf * TKX * g.nz * sizeof(CT),
-                st>>>(g, spec, pl, tw, TKX, inverse, sc);
+  const int tail = g.nxh % TKX;
+  k_zfft_g<T><<<dim3((g.nxh + TKX - 1) / TKX, g.ny), g.nz > 256 ? 256 : 128, (size_t)nbuf * TKX * g.nz * sizeof(CT), st>>>(
+      g, spec, pl, tw, TKX, fdiv_magic(TKX), fdiv_magic(tail > 0 ? tail : 1), inverse, sc);
   return cudaGetLastError();
 }
 
@@ -260,8 +289,7 @@ cudaError_t xifft_generic(const Geo<T>& g, const typename CplxOf<T>::type* spec,
                           const DevScalars* sc, cudaStream_t st) {
   const XShape s = x_shape<T>(g.nx / 2, pl.radix[0]);
   const int nlines = g.ny * g.nz;
-  k_xifft_g<T><<<(nlines + s.LPB - 1) / s.LPB, s.threads, s.smem, st>>>(g, spec, phi, pl, tw, twr, s.LPB, s.LP, s.sh,
-                                                                        normfft, sc);
+  k_xifft_g<T><<<(nlines + s.LPB - 1) / s.LPB, s.threads, s.smem, st>>>(g, spec, phi, pl, tw, twr, s.LPB, s.LP, s.sh, normfft, sc);
   return cudaGetLastError();
 }
 

@@ -960,9 +960,7 @@ template <class T, bool O4> static cudaError_t rhs_march_t(ch3d_ctx* c) {
 // Grids with few columns: a column march's time is set by its dependent rows per
 // thread, however few columns there are; the right-hand sides by chunks of rows
 // and the y sweep as its own pass cost 6 more arrays of (L2) traffic instead.
-// Step with the march / by rows: 64^3 (4096 columns) 239 / 150 us, 96^3 414 / 337,
-// 128^3 (16384) 588 / 563, 192 x 64 x 96 mixed (18432) 282 / 311, 192^3 (36864)
-// 1613 / 1960: the line lies between the last two groups, at 120 columns per SM.
+// 64^3 (4096 columns): 50 us against 19; 192^3 (36864): 224 us against 335.
 bool march_rows_path(const ch3d_ctx* c) {
   return c->march && (long long)c->nx * c->nz <= 120LL * sm_count(c->device);
 }

@@ -75,8 +75,9 @@ __global__ void __launch_bounds__(32 * kXWarps, SRC ? 6 : (sizeof(T) == 4 ? 6 : 
           r0 = s01.x; r1 = s01.y;
         } else if (g.order == 4) {
           const C4<T> c4(g);
-          r0 = div4_cell(g, c4, sucaj, ux, uy, uz, i0, j, k);
-          r1 = div4_cell(g, c4, sucaj, ux, uy, uz, i0 + 1, j, k);
+          T d[2];
+          div4_pair(g, c4, sucaj, ux, uy, uz, base, i0, j, k, d);
+          r0 = d[0]; r1 = d[1];
         } else {
           // pairs (i0, i0+1) as one aligned vector load (nx and i0 even)
           typedef typename CplxOf<T>::type T2;

@@ -1,9 +1,9 @@
 // ch3d_step4.cu -- sm_100a kernels specific to the 4th-order solver
 // (src/CFD_4th/m_TScheme.f90): the interpolated velocities and the RHS of the
-// stage entry points, and the constant-flux forcing from the mean viscous
-// stress.  The step runs the RHS and y solves as the column march of
-// ch3d_march.cu (4th-order branch).  The pressure Poisson pipeline, projection and
-// diagnostics are the 2nd-order kernels with their 4th-order branches.
+// stage entry points, and the statistics.  The step runs the RHS and y solves as
+// the column march of ch3d_march.cu (4th-order branch).  The pressure Poisson
+// pipeline, projection and diagnostics are the 2nd-order kernels with their
+// 4th-order branches.
 #include "ch3d_ctx.h"
 #include "ch3d_dev.cuh"
 
@@ -149,55 +149,6 @@ __global__ void __launch_bounds__(256) k_rhs4(Geo<T> g, Metrics<T> m, Interp4 ih
   rz[idx] = rhs4_comp<T, 2>(g, m, ih, ux, uy, uz, pr, hz, i, j, k, pmGamma, pmTheta, pmAlpha, pmBeta);
 }
 
-// Block partial sums of (d11q1 + d33q1 + d22q1) * dyp over ux: the mean
-// viscous stress of the constant-flux forcing (src/CFD_4th/m_TScheme.f90:255-262,364-377).
-template <class T>
-__global__ void __launch_bounds__(128) k_visc4_partial(Geo<T> g, Metrics<T> m, const T* __restrict__ ux,
-                                                       double* __restrict__ part, int rows) {
-  __shared__ double red[4];
-  const int i = blockIdx.x * 32 + (threadIdx.x & 31), k = blockIdx.y * 4 + (threadIdx.x >> 5);
-  const int j0 = blockIdx.z * rows, j1 = min(j0 + rows, g.ny);
-  double s = 0.0;
-  if (i < g.nx && k < g.nz) {
-    const C4<T> c(g);
-    Nbr n = make_nbr(g, i, j0, k);
-#pragma unroll 4
-    for (int j = j0; j < j1; ++j) {
-      if (j > j0) nbr_next_row(n, g, j);
-      const int jc = j + 1;
-      const T ux_c = at(ux, n, 0);
-      const T d11 = c.dxx1 * at(ux, n, n.xm2) + c.dxx2 * at(ux, n, n.xm) + c.dxx3 * ux_c + c.dxx4 * at(ux, n, n.xp) +
-                    c.dxx5 * at(ux, n, n.xp2);
-      const T d22 = m.ap2c[jc] * at_jp(ux, g, 0, n, 0) + m.ac2c[jc] * ux_c + m.am2c[jc] * at_jm(ux, g, 0, n, 0);
-      const T d33 = c.dzz1 * at(ux, n, n.zm2) + c.dzz2 * at(ux, n, n.zm) + c.dzz3 * ux_c + c.dzz4 * at(ux, n, n.zp) +
-                    c.dzz5 * at(ux, n, n.zp2);
-      s += ((double)(d11 + d33) + (double)d22) * (double)m.dyp[jc];
-    }
-  }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0)
-    part[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)] = (red[0] + red[1]) + (red[2] + red[3]);
-}
-
-// rows per k_visc4_partial block: whole columns when the x-z plane alone gives
-// about eight blocks per SM, shorter chunks on small grids
-static int visc4_rows(const ch3d_ctx* c) {
-  const long long cols = (long long)((c->nx + 31) / 32) * ((c->nz + 3) / 4);
-  const long long chunks = (148LL * 8 + cols - 1) / cols;
-  const int rows = (int)((c->ny + chunks - 1) / chunks);
-  return rows < 8 ? 8 : rows;
-}
-static dim3 visc4_grid(const ch3d_ctx* c) {
-  const int rows = visc4_rows(c);
-  return dim3((c->nx + 31) / 32, (c->nz + 3) / 4, (c->ny + rows - 1) / rows);
-}
-int visc4_npart(const ch3d_ctx* c) {
-  const dim3 g = visc4_grid(c);
-  return (int)(g.x * g.y * g.z);
-}
-
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
@@ -228,21 +179,15 @@ template <class T> static cudaError_t rhs4_t(ch3d_ctx* c) {
 }
 cudaError_t launch_rhs4(ch3d_ctx* c) { return c->fp32 ? rhs4_t<float>(c) : rhs4_t<double>(c); }
 
-template <class T> static cudaError_t visc4_t(ch3d_ctx* c) {
-  T** f = (T**)c->f;
-  k_visc4_partial<T><<<visc4_grid(c), 128, 0, c->stream>>>(make_geo<T>(c), metrics_of<T>(c), f[0], c->part,
-                                                           visc4_rows(c));
-  return cudaGetLastError();
-}
-cudaError_t launch_visc4_partials(ch3d_ctx* c) { return c->fp32 ? visc4_t<float>(c) : visc4_t<double>(c); }
-
 // ---------------------------------------------------------------------------
 // Statistics of the 4th-order solver: the moments of clcStat
 // (src/CFD_4th/m_FlowCase.f90:330-640), SumStat(35,nyp) and the gradient
 // moments SumGrad(98,nyp) (HighOrderGradStat, defined at :17), FP64
 // accumulation in both precision modes.  One kernel per group of moments so
-// that a thread's accumulators stay in registers: group 0 the 35 SumStat
-// moments, groups 1..4 SumGrad(1..26), (27..50), (51..74), (75..98).
+// that a thread's accumulators stay in registers: groups 0 and 5 the SumStat
+// moments 1..23 and 24..35 (in one group they took 254 registers, eight warps
+// per SM), groups 1..4 SumGrad(1..26), (27..50), (51..74), (75..98).  The cells of
+// a chunk of z planes are spread over the block's threads whatever nx is.
 // Blocks (j, k-chunk); blockIdx.x == ny is the nyp row (:594-631).  The
 // partials are summed in a fixed order by k_stats4_finalize.
 // The reference's pressure array keeps zero in its planes x = nxc+2 and
@@ -250,11 +195,11 @@ cudaError_t launch_visc4_partials(ch3d_ctx* c) { return c->fp32 ? visc4_t<float>
 // m_BC_and_Halo.f90:42-45; the array starts at zero, m_Variables.f90:85), and
 // dpdxx / dpdzz of the last column and plane read it there; so do these.
 // ---------------------------------------------------------------------------
-constexpr int kStats4Lo[5] = {0, 0, 26, 50, 74};
-constexpr int kStats4N[5] = {35, 26, 24, 24, 24};
+constexpr int kStats4Lo[6] = {0, 0, 26, 50, 74, 23};
+constexpr int kStats4N[6] = {23, 26, 24, 24, 24, 12};
 
 template <class T, int GRP>
-__global__ void __launch_bounds__(256) k_stats4(Geo<T> g, Geo<double> gd, Metrics<double> m, const T* __restrict__ ux,
+__global__ void __launch_bounds__(256, 2) k_stats4(Geo<T> g, Geo<double> gd, Metrics<double> m, const T* __restrict__ ux,
                                                 const T* __restrict__ uy, const T* __restrict__ uz,
                                                 const T* __restrict__ pr, double* __restrict__ part, int kch) {
   constexpr int NQ = kStats4N[GRP], LO = kStats4Lo[GRP];
@@ -276,100 +221,107 @@ __global__ void __launch_bounds__(256) k_stats4(Geo<T> g, Geo<double> gd, Metric
   const double in1 = -1.0 / 16.0, in2 = 9.0 / 16.0, in3 = 9.0 / 16.0, in4 = -1.0 / 16.0;
   const double rdxt = rdx / 12.0, rdzt = rdz / 12.0;
   auto wx = [nx](int i) { return i < 0 ? i + nx : (i >= nx ? i - nx : i); };
-  auto wz = [nz](int k) { return k < 0 ? k + nz : (k >= nz ? k - nz : k); };
-  const int jc = j + 1, jm = j - 1, jp = j + 1;  // 0-based rows of jc, jc-1, jc+1
+  const int jc = j + 1;
   const double InterpY1 = m.yinterp[jc], InterpY2 = 1.0 - InterpY1;
   const double cac = m.rdyc[jc];
   if (j < ny) {
     const double cacU = m.rdyc[jc + 1], caj = m.rdyp[jc];
-    for (int k = k0; k < k1; ++k) {
-      const int ks = wz(k - 2), km = wz(k - 1), kp = wz(k + 1), ku = wz(k + 2);
-      for (int i = threadIdx.x; i < nx; i += blockDim.x) {
-        const int is = wx(i - 2), im = wx(i - 1), ip = wx(i + 1), iu = wx(i + 2);
-        auto U = [&](int a, int b, int c) { return (double)fld(ux, g, 0, a, b, c); };
-        auto V = [&](int a, int b, int c) { return (double)fld(uy, g, 1, a, b, c); };
-        auto W = [&](int a, int b, int c) { return (double)fld(uz, g, 2, a, b, c); };
-        auto P = [&](int a, int b, int c) { return (double)fld(pr, g, 3, a, b, c); };
-        const double uxloc = U(i, j, k), uyloc = V(i, j, k), uzloc = W(i, j, k), prloc = P(i, j, k);
-        const double dudy = (uxloc - U(i, jm, k)) * cac;
-        const double dvdx = dx1 * V(is, j, k) + dx2 * V(im, j, k) + dx3 * uyloc + dx4 * V(ip, j, k);
-        if constexpr (GRP == 0) {
-          const double uxCell = in1 * U(im, j, k) + in2 * uxloc + in3 * U(ip, j, k) + in4 * U(iu, j, k);
-          const double uyCell = (uyloc + V(i, jp, k)) * 0.5;
-          const double uy_xc = in1 * V(is, j, k) + in2 * V(im, j, k) + in3 * uyloc + in4 * V(ip, j, k);
-          const double uy_xp = in1 * V(is, jp, k) + in2 * V(im, jp, k) + in3 * V(i, jp, k) + in4 * V(ip, jp, k);
-          const double uzCell = in1 * W(i, j, km) + in2 * uzloc + in3 * W(i, j, kp) + in4 * W(i, j, ku);
-          const double prloc2 = InterpY1 * (in1 * P(is, jm, k) + in2 * P(im, jm, k) + in3 * P(i, jm, k) + in4 * P(ip, jm, k)) +
-                                InterpY2 * (in1 * P(is, j, k) + in2 * P(im, j, k) + in3 * prloc + in4 * P(ip, j, k));
-          const double dudx = dx1 * U(im, j, k) + dx2 * uxloc + dx3 * U(ip, j, k) + dx4 * U(iu, j, k);
-          const double dudz = dz1 * U(i, j, ks) + dz2 * U(i, j, km) + dz3 * uxloc + dz4 * U(i, j, kp);
-          const double dvdy = (V(i, jp, k) - uyloc) * caj;
-          const double dvdz = dz1 * V(i, j, ks) + dz2 * V(i, j, km) + dz3 * uyloc + dz4 * V(i, j, kp);
-          const double dwdx = dx1 * W(is, j, k) + dx2 * W(im, j, k) + dx3 * uzloc + dx4 * W(ip, j, k);
-          const double dwdy = (uzloc - W(i, jm, k)) * cac;
-          const double dwdz = dz1 * W(i, j, km) + dz2 * uzloc + dz3 * W(i, j, kp) + dz4 * W(i, j, ku);
-          const double dudxx = dxx1 * U(is, j, k) + dxx2 * U(im, j, k) + dxx3 * uxloc + dxx4 * U(ip, j, k) + dxx5 * U(iu, j, k);
-          const double dudyy = m.ap2c[jc] * U(i, jp, k) + m.ac2c[jc] * uxloc + m.am2c[jc] * U(i, jm, k);
-          const double dudzz = dzz1 * U(i, j, ks) + dzz2 * U(i, j, km) + dzz3 * uxloc + dzz4 * U(i, j, kp) + dzz5 * U(i, j, ku);
-          const double dvdxx = dxx1 * V(is, j, k) + dxx2 * V(im, j, k) + dxx3 * uyloc + dxx4 * V(ip, j, k) + dxx5 * V(iu, j, k);
-          const double dvdyy = m.ap2p[jc] * V(i, jp, k) + m.ac2p[jc] * uyloc + m.am2p[jc] * V(i, jm, k);
-          const double dvdzz = dzz1 * V(i, j, ks) + dzz2 * V(i, j, km) + dzz3 * uyloc + dzz4 * V(i, j, kp) + dzz5 * V(i, j, ku);
-          const double dwdxx = dxx1 * W(is, j, k) + dxx2 * W(im, j, k) + dxx3 * uzloc + dxx4 * W(ip, j, k) + dxx5 * W(iu, j, k);
-          const double dwdyy = m.ap2c[jc] * W(i, jp, k) + m.ac2c[jc] * uzloc + m.am2c[jc] * W(i, jm, k);
-          const double dwdzz = dzz1 * W(i, j, ks) + dzz2 * W(i, j, km) + dzz3 * uzloc + dzz4 * W(i, j, kp) + dzz5 * W(i, j, ku);
+    for (int t = threadIdx.x; t < nx * (k1 - k0); t += blockDim.x) {  // the chunk's cells, i fastest
+        const int kq = t / nx, i = t - kq * nx, k = k0 + kq;
+        const Nbr n = make_nbr(g, i, j, k);
+        const int is = n.xm2, im = n.xm, ip = n.xp, iu = n.xp2;             // offsets to i-2 .. i+2
+        const long long ks = n.zm2, km = n.zm, kp = n.zp, ku = n.zp2;       // offsets to k-2 .. k+2
+        auto val = [&](const T* a, int comp, int xo, int dj, long long zo) {  // row j + dj, with the wall ghosts
+          const long long o = xo + zo;
+          return (double)(dj == 0 ? at(a, n, o) : (dj < 0 ? at_jm(a, g, comp, n, o) : at_jp(a, g, comp, n, o)));
+        };
+        auto U = [&](int xo, int dj, long long zo) { return val(ux, 0, xo, dj, zo); };
+        auto V = [&](int xo, int dj, long long zo) { return val(uy, 1, xo, dj, zo); };
+        auto W = [&](int xo, int dj, long long zo) { return val(uz, 2, xo, dj, zo); };
+        auto P = [&](int xo, int dj, long long zo) { return val(pr, 3, xo, dj, zo); };
+        const double uxloc = U(0, 0, 0), uyloc = V(0, 0, 0), uzloc = W(0, 0, 0), prloc = P(0, 0, 0);
+        const double dudy = (uxloc - U(0, -1, 0)) * cac;
+        const double dvdx = dx1 * V(is, 0, 0) + dx2 * V(im, 0, 0) + dx3 * uyloc + dx4 * V(ip, 0, 0);
+        if constexpr (GRP == 0 || GRP == 5) {  // what a group does not sum is not computed
+          const double uxCell = in1 * U(im, 0, 0) + in2 * uxloc + in3 * U(ip, 0, 0) + in4 * U(iu, 0, 0);
+          const double uyCell = (uyloc + V(0, 1, 0)) * 0.5;
+          const double uy_xc = in1 * V(is, 0, 0) + in2 * V(im, 0, 0) + in3 * uyloc + in4 * V(ip, 0, 0);
+          const double uy_xp = in1 * V(is, 1, 0) + in2 * V(im, 1, 0) + in3 * V(0, 1, 0) + in4 * V(ip, 1, 0);
+          const double uzCell = in1 * W(0, 0, km) + in2 * uzloc + in3 * W(0, 0, kp) + in4 * W(0, 0, ku);
+          const double prloc2 = InterpY1 * (in1 * P(is, -1, 0) + in2 * P(im, -1, 0) + in3 * P(0, -1, 0) + in4 * P(ip, -1, 0)) +
+                                InterpY2 * (in1 * P(is, 0, 0) + in2 * P(im, 0, 0) + in3 * prloc + in4 * P(ip, 0, 0));
+          const double dudx = dx1 * U(im, 0, 0) + dx2 * uxloc + dx3 * U(ip, 0, 0) + dx4 * U(iu, 0, 0);
+          const double dudz = dz1 * U(0, 0, ks) + dz2 * U(0, 0, km) + dz3 * uxloc + dz4 * U(0, 0, kp);
+          const double dvdy = (V(0, 1, 0) - uyloc) * caj;
+          const double dvdz = dz1 * V(0, 0, ks) + dz2 * V(0, 0, km) + dz3 * uyloc + dz4 * V(0, 0, kp);
+          const double dwdx = dx1 * W(is, 0, 0) + dx2 * W(im, 0, 0) + dx3 * uzloc + dx4 * W(ip, 0, 0);
+          const double dwdy = (uzloc - W(0, -1, 0)) * cac;
+          const double dwdz = dz1 * W(0, 0, km) + dz2 * uzloc + dz3 * W(0, 0, kp) + dz4 * W(0, 0, ku);
+          const double dudxx = dxx1 * U(is, 0, 0) + dxx2 * U(im, 0, 0) + dxx3 * uxloc + dxx4 * U(ip, 0, 0) + dxx5 * U(iu, 0, 0);
+          const double dudyy = m.ap2c[jc] * U(0, 1, 0) + m.ac2c[jc] * uxloc + m.am2c[jc] * U(0, -1, 0);
+          const double dudzz = dzz1 * U(0, 0, ks) + dzz2 * U(0, 0, km) + dzz3 * uxloc + dzz4 * U(0, 0, kp) + dzz5 * U(0, 0, ku);
+          const double dvdxx = dxx1 * V(is, 0, 0) + dxx2 * V(im, 0, 0) + dxx3 * uyloc + dxx4 * V(ip, 0, 0) + dxx5 * V(iu, 0, 0);
+          const double dvdyy = m.ap2p[jc] * V(0, 1, 0) + m.ac2p[jc] * uyloc + m.am2p[jc] * V(0, -1, 0);
+          const double dvdzz = dzz1 * V(0, 0, ks) + dzz2 * V(0, 0, km) + dzz3 * uyloc + dzz4 * V(0, 0, kp) + dzz5 * V(0, 0, ku);
+          const double dwdxx = dxx1 * W(is, 0, 0) + dxx2 * W(im, 0, 0) + dxx3 * uzloc + dxx4 * W(ip, 0, 0) + dxx5 * W(iu, 0, 0);
+          const double dwdyy = m.ap2c[jc] * W(0, 1, 0) + m.ac2c[jc] * uzloc + m.am2c[jc] * W(0, -1, 0);
+          const double dwdzz = dzz1 * W(0, 0, ks) + dzz2 * W(0, 0, km) + dzz3 * uzloc + dzz4 * W(0, 0, kp) + dzz5 * W(0, 0, ku);
           const double vor_x = dwdy - dvdz, vor_y = dudz - dwdx, vor_z = dvdx - dudy;
-          const double dudxC = (-U(iu, j, k) + 8.0 * U(ip, j, k) - 8.0 * U(im, j, k) + U(is, j, k)) * rdxt;
-          const double dvdxU = dx1 * V(is, jp, k) + dx2 * V(im, jp, k) + dx3 * V(i, jp, k) + dx4 * V(ip, jp, k);
-          const double dudyU = (U(i, jp, k) - uxloc) * cacU;
-          const double dudzC = (InterpY1 * (-U(i, jm, ku) + 8.0 * U(i, jm, kp) - 8.0 * U(i, jm, km) + U(i, jm, ks)) +
-                                InterpY2 * (-U(i, j, ku) + 8.0 * U(i, j, kp) - 8.0 * U(i, j, km) + U(i, j, ks))) * rdzt;
-          auto dz4c = [&](int a) { return -V(a, j, ku) + 8.0 * V(a, j, kp) - 8.0 * V(a, j, km) + V(a, j, ks); };
-          const double dvdzC = (dz4c(is) * in1 + dz4c(im) * in2 + dz4c(i) * in3 + dz4c(ip) * in4) * rdzt;
-          A[0] += uxloc; A[1] += uyloc; A[2] += uzloc; A[3] += prloc;
-          A[4] += uxloc * uxloc; A[5] += uyloc * uyloc; A[6] += uzloc * uzloc; A[7] += prloc * prloc;
-          A[8] += uxCell * uyCell; A[9] += uyCell * uzCell; A[10] += uxCell * uzCell;
-          A[11] += uxCell * prloc; A[12] += uyCell * prloc; A[13] += uzCell * prloc;
-          A[14] += uxCell * uxCell * uyCell; A[15] += uyloc * uyloc * uyloc; A[16] += uzCell * uzCell * uyCell;
-          A[17] += uxCell * uyCell * uyCell; A[18] += uxloc * uxloc * uxloc; A[19] += uzloc * uzloc * uzloc;
-          A[20] += uxloc * uxloc * uxloc * uxloc; A[21] += uyloc * uyloc * uyloc * uyloc;
-          A[22] += uzloc * uzloc * uzloc * uzloc;
-          A[23] += prloc * dudx; A[24] += prloc * dvdy; A[25] += prloc * dwdz;
-          A[26] += prloc2 * (dudy + dvdx);
-          A[27] += uxloc * (dudxx + dudyy + dudzz); A[28] += uyloc * (dvdxx + dvdyy + dvdzz);
-          A[29] += uzloc * (dwdxx + dwdyy + dwdzz);
-          A[30] += (dudxC * (dvdxU + dvdx) + (dudyU + dudy) * (uy_xp - uy_xc) * caj) * 0.5;
-          A[31] += dudzC * dvdzC;
-          A[32] += vor_x * vor_x; A[33] += vor_y * vor_y; A[34] += vor_z * vor_z;
+          const double dudxC = (-U(iu, 0, 0) + 8.0 * U(ip, 0, 0) - 8.0 * U(im, 0, 0) + U(is, 0, 0)) * rdxt;
+          const double dvdxU = dx1 * V(is, 1, 0) + dx2 * V(im, 1, 0) + dx3 * V(0, 1, 0) + dx4 * V(ip, 1, 0);
+          const double dudyU = (U(0, 1, 0) - uxloc) * cacU;
+          const double dudzC = (InterpY1 * (-U(0, -1, ku) + 8.0 * U(0, -1, kp) - 8.0 * U(0, -1, km) + U(0, -1, ks)) +
+                                InterpY2 * (-U(0, 0, ku) + 8.0 * U(0, 0, kp) - 8.0 * U(0, 0, km) + U(0, 0, ks))) * rdzt;
+          auto dz4c = [&](int a) { return -V(a, 0, ku) + 8.0 * V(a, 0, kp) - 8.0 * V(a, 0, km) + V(a, 0, ks); };
+          const double dvdzC = (dz4c(is) * in1 + dz4c(im) * in2 + dz4c(0) * in3 + dz4c(ip) * in4) * rdzt;
+          if constexpr (GRP == 0) {
+            A[0] += uxloc; A[1] += uyloc; A[2] += uzloc; A[3] += prloc;
+            A[4] += uxloc * uxloc; A[5] += uyloc * uyloc; A[6] += uzloc * uzloc; A[7] += prloc * prloc;
+            A[8] += uxCell * uyCell; A[9] += uyCell * uzCell; A[10] += uxCell * uzCell;
+            A[11] += uxCell * prloc; A[12] += uyCell * prloc; A[13] += uzCell * prloc;
+            A[14] += uxCell * uxCell * uyCell; A[15] += uyloc * uyloc * uyloc; A[16] += uzCell * uzCell * uyCell;
+            A[17] += uxCell * uyCell * uyCell; A[18] += uxloc * uxloc * uxloc; A[19] += uzloc * uzloc * uzloc;
+            A[20] += uxloc * uxloc * uxloc * uxloc; A[21] += uyloc * uyloc * uyloc * uyloc;
+            A[22] += uzloc * uzloc * uzloc * uzloc;
+          } else {  // A[q] is moment 24 + q
+            A[0] += prloc * dudx; A[1] += prloc * dvdy; A[2] += prloc * dwdz;
+            A[3] += prloc2 * (dudy + dvdx);
+            A[4] += uxloc * (dudxx + dudyy + dudzz); A[5] += uyloc * (dvdxx + dvdyy + dvdzz);
+            A[6] += uzloc * (dwdxx + dwdyy + dwdzz);
+            A[7] += (dudxC * (dvdxU + dvdx) + (dudyU + dudy) * (uy_xp - uy_xc) * caj) * 0.5;
+            A[8] += dudzC * dvdzC;
+            A[9] += vor_x * vor_x; A[10] += vor_y * vor_y; A[11] += vor_z * vor_z;
+          }
         } else {
           // the 24 gradients of SumVec2(3..98) in their order (:496-589); each group takes six
           auto grad = [&](int t) -> double {
             switch (t) {
-              case 0: return dx1 * U(im, j, k) + dx2 * uxloc + dx3 * U(ip, j, k) + dx4 * U(iu, j, k);
+              case 0: return dx1 * U(im, 0, 0) + dx2 * uxloc + dx3 * U(ip, 0, 0) + dx4 * U(iu, 0, 0);
               case 1: return dudy;
-              case 2: return dz1 * U(i, j, ks) + dz2 * U(i, j, km) + dz3 * uxloc + dz4 * U(i, j, kp);
+              case 2: return dz1 * U(0, 0, ks) + dz2 * U(0, 0, km) + dz3 * uxloc + dz4 * U(0, 0, kp);
               case 3: return dvdx;
-              case 4: return (V(i, jp, k) - uyloc) * caj;
-              case 5: return dz1 * V(i, j, ks) + dz2 * V(i, j, km) + dz3 * uyloc + dz4 * V(i, j, kp);
-              case 6: return dx1 * W(is, j, k) + dx2 * W(im, j, k) + dx3 * uzloc + dx4 * W(ip, j, k);
-              case 7: return (uzloc - W(i, jm, k)) * cac;
-              case 8: return dz1 * W(i, j, km) + dz2 * uzloc + dz3 * W(i, j, kp) + dz4 * W(i, j, ku);
-              case 9: return dx1 * P(is, j, k) + dx2 * P(im, j, k) + dx3 * prloc + dx4 * P(ip, j, k);
-              case 10: return (prloc - P(i, jm, k)) * cac;
-              case 11: return dz1 * P(i, j, ks) + dz2 * P(i, j, km) + dz3 * prloc + dz4 * P(i, j, kp);
-              case 12: return dxx1 * U(is, j, k) + dxx2 * U(im, j, k) + dxx3 * uxloc + dxx4 * U(ip, j, k) + dxx5 * U(iu, j, k);
-              case 13: return m.ap2c[jc] * U(i, jp, k) + m.ac2c[jc] * uxloc + m.am2c[jc] * U(i, jm, k);
-              case 14: return dzz1 * U(i, j, ks) + dzz2 * U(i, j, km) + dzz3 * uxloc + dzz4 * U(i, j, kp) + dzz5 * U(i, j, ku);
-              case 15: return dxx1 * V(is, j, k) + dxx2 * V(im, j, k) + dxx3 * uyloc + dxx4 * V(ip, j, k) + dxx5 * V(iu, j, k);
-              case 16: return m.ap2p[jc] * V(i, jp, k) + m.ac2p[jc] * uyloc + m.am2p[jc] * V(i, jm, k);
-              case 17: return dzz1 * V(i, j, ks) + dzz2 * V(i, j, km) + dzz3 * uyloc + dzz4 * V(i, j, kp) + dzz5 * V(i, j, ku);
-              case 18: return dxx1 * W(is, j, k) + dxx2 * W(im, j, k) + dxx3 * uzloc + dxx4 * W(ip, j, k) + dxx5 * W(iu, j, k);
-              case 19: return m.ap2c[jc] * W(i, jp, k) + m.ac2c[jc] * uzloc + m.am2c[jc] * W(i, jm, k);
-              case 20: return dzz1 * W(i, j, ks) + dzz2 * W(i, j, km) + dzz3 * uzloc + dzz4 * W(i, j, kp) + dzz5 * W(i, j, ku);
-              case 21: return dxx1 * P(is, j, k) + dxx2 * P(im, j, k) + dxx3 * prloc + dxx4 * P(ip, j, k) +
-                              dxx5 * (i == nx - 1 ? 0.0 : P(iu, j, k));
-              case 22: return m.ap2c[jc] * P(i, jp, k) + m.ac2c[jc] * prloc + m.am2c[jc] * P(i, jm, k);
-              default: return dzz1 * P(i, j, ks) + dzz2 * P(i, j, km) + dzz3 * prloc + dzz4 * P(i, j, kp) +
-                              dzz5 * (k == nz - 1 ? 0.0 : P(i, j, ku));
+              case 4: return (V(0, 1, 0) - uyloc) * caj;
+              case 5: return dz1 * V(0, 0, ks) + dz2 * V(0, 0, km) + dz3 * uyloc + dz4 * V(0, 0, kp);
+              case 6: return dx1 * W(is, 0, 0) + dx2 * W(im, 0, 0) + dx3 * uzloc + dx4 * W(ip, 0, 0);
+              case 7: return (uzloc - W(0, -1, 0)) * cac;
+              case 8: return dz1 * W(0, 0, km) + dz2 * uzloc + dz3 * W(0, 0, kp) + dz4 * W(0, 0, ku);
+              case 9: return dx1 * P(is, 0, 0) + dx2 * P(im, 0, 0) + dx3 * prloc + dx4 * P(ip, 0, 0);
+              case 10: return (prloc - P(0, -1, 0)) * cac;
+              case 11: return dz1 * P(0, 0, ks) + dz2 * P(0, 0, km) + dz3 * prloc + dz4 * P(0, 0, kp);
+              case 12: return dxx1 * U(is, 0, 0) + dxx2 * U(im, 0, 0) + dxx3 * uxloc + dxx4 * U(ip, 0, 0) + dxx5 * U(iu, 0, 0);
+              case 13: return m.ap2c[jc] * U(0, 1, 0) + m.ac2c[jc] * uxloc + m.am2c[jc] * U(0, -1, 0);
+              case 14: return dzz1 * U(0, 0, ks) + dzz2 * U(0, 0, km) + dzz3 * uxloc + dzz4 * U(0, 0, kp) + dzz5 * U(0, 0, ku);
+              case 15: return dxx1 * V(is, 0, 0) + dxx2 * V(im, 0, 0) + dxx3 * uyloc + dxx4 * V(ip, 0, 0) + dxx5 * V(iu, 0, 0);
+              case 16: return m.ap2p[jc] * V(0, 1, 0) + m.ac2p[jc] * uyloc + m.am2p[jc] * V(0, -1, 0);
+              case 17: return dzz1 * V(0, 0, ks) + dzz2 * V(0, 0, km) + dzz3 * uyloc + dzz4 * V(0, 0, kp) + dzz5 * V(0, 0, ku);
+              case 18: return dxx1 * W(is, 0, 0) + dxx2 * W(im, 0, 0) + dxx3 * uzloc + dxx4 * W(ip, 0, 0) + dxx5 * W(iu, 0, 0);
+              case 19: return m.ap2c[jc] * W(0, 1, 0) + m.ac2c[jc] * uzloc + m.am2c[jc] * W(0, -1, 0);
+              case 20: return dzz1 * W(0, 0, ks) + dzz2 * W(0, 0, km) + dzz3 * uzloc + dzz4 * W(0, 0, kp) + dzz5 * W(0, 0, ku);
+              case 21: return dxx1 * P(is, 0, 0) + dxx2 * P(im, 0, 0) + dxx3 * prloc + dxx4 * P(ip, 0, 0) +
+                              dxx5 * (i == nx - 1 ? 0.0 : P(iu, 0, 0));
+              case 22: return m.ap2c[jc] * P(0, 1, 0) + m.ac2c[jc] * prloc + m.am2c[jc] * P(0, -1, 0);
+              default: return dzz1 * P(0, 0, ks) + dzz2 * P(0, 0, km) + dzz3 * prloc + dzz4 * P(0, 0, kp) +
+                              dzz5 * (k == nz - 1 ? 0.0 : P(0, 0, ku));
             }
           };
           constexpr int T0 = 6 * (GRP - 1), OFF = GRP == 1 ? 2 : 0;
@@ -386,7 +338,6 @@ __global__ void __launch_bounds__(256) k_stats4(Geo<T> g, Geo<double> gd, Metric
             A[OFF + 4 * t + 3] += a * a * a * a;
           }
         }
-      }
     }
   } else {
     // jc = nyp: the row above the last cell (ghost values of SetBC_and_UpdateHalo)
@@ -397,13 +348,13 @@ __global__ void __launch_bounds__(256) k_stats4(Geo<T> g, Geo<double> gd, Metric
         auto P = [&](int a, int b) { return (double)fld(pr, g, 3, a, b, k); };
         const double dudy = ((double)fld(ux, g, 0, i, jt, k) - (double)fld(ux, g, 0, i, jb, k)) * cac;
         const double dwdy = ((double)fld(uz, g, 2, i, jt, k) - (double)fld(uz, g, 2, i, jb, k)) * cac;
-        if constexpr (GRP == 0) {
+        if constexpr (GRP == 5) {
           const double prloc2 = InterpY1 * (in1 * P(is, jb) + in2 * P(im, jb) + in3 * P(i, jb) + in4 * P(ip, jb)) +
                                 InterpY2 * (in1 * P(is, jt) + in2 * P(im, jt) + in3 * P(i, jt) + in4 * P(ip, jt));
           const double vor_x = dwdy, vor_z = -dudy;
-          A[26] += prloc2 * (dudy + 0.0);
-          A[32] += vor_x * vor_x;
-          A[34] += vor_z * vor_z;
+          A[3] += prloc2 * (dudy + 0.0);
+          A[9] += vor_x * vor_x;
+          A[11] += vor_z * vor_z;
         } else if constexpr (GRP == 1) {  // SumVec2(7..10): dudy; SumVec2(31..34) is in group 2
           A[6] += dudy; A[7] += dudy * dudy; A[8] += dudy * dudy * dudy; A[9] += dudy * dudy * dudy * dudy;
         } else if constexpr (GRP == 2) {  // SumVec2(31..34) = group-2 slots 30-26 .. 33-26
@@ -459,6 +410,7 @@ template <class T> static cudaError_t stats4_t(ch3d_ctx* c) {
   double* sumgrad = c->stat + (size_t)35 * (c->ny + 1) + 1;  // after SumStat and PrGradsum
   cudaError_t e;
   if ((e = stats4_group<T, 0>(c, kch, nch, sumstat, 35)) != cudaSuccess) return e;
+  if ((e = stats4_group<T, 5>(c, kch, nch, sumstat, 35)) != cudaSuccess) return e;
   if ((e = stats4_group<T, 1>(c, kch, nch, sumgrad, 98)) != cudaSuccess) return e;
   if ((e = stats4_group<T, 2>(c, kch, nch, sumgrad, 98)) != cudaSuccess) return e;
   if ((e = stats4_group<T, 3>(c, kch, nch, sumgrad, 98)) != cudaSuccess) return e;

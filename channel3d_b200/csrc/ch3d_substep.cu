@@ -53,7 +53,7 @@ struct SubstepPar {
   int ns, begin, last;  // begin: the step starts here; last: the step's diagnostics follow
   double gam, the, alp;
   int iCFL, IsUxConst, order;
-  double CFLc, dtMax, xnu, ubulk, norm_bulk, nxnz, yly;
+  double CFLc, dtMax, xnu, ubulk, norm_bulk, nxnz, yly, visc_wall;
 };
 
 // Elimination factors of the row table for pmBeta (see ch3d_march.cuh), one
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(kSetupThreads) k_substep(DevScalars* sc, const
     sc->divmax1 = 0ull;
     if (p.IsUxConst && p.order == 4) {
       // the partial sums are those of the mean viscous stress (src/CFD_4th/m_TScheme.f90:364-377)
-      const double dpm = p.xnu * s1 / p.nxnz / p.yly;
+      const double dpm = p.xnu * (s1 / p.nxnz + p.visc_wall) / p.yly;
       sc->PrGradNow = dpm;
       sc->dpmdxns = -(sc->pmAlpha * dpm);  // RhsX - pmAlpha*dpmdxns
       sc->PrGradAver = sc->PrGradAver + dpm * p.alp;
@@ -296,6 +296,7 @@ template <class T> static cudaError_t substep_t(ch3d_ctx* c, int ns, bool whole_
   p.norm_bulk = 1.0 / ((double)c->nx * (double)c->nz) / (c->cfg.ybulk2 - c->cfg.ybulk1);
   p.nxnz = (double)(c->nx * c->nz);
   p.yly = c->cfg.yly;
+  p.visc_wall = c->visc_wall;
   TableArgs<T> ta;
   ta.hc = helm_coef(c);
   ta.m = c->cfg.LES_type == 0 ? metrics_of<T>(c) : Metrics<T>();
@@ -311,9 +312,8 @@ template <class T> static cudaError_t substep_t(ch3d_ctx* c, int ns, bool whole_
   ta.r2y = y_periodic(c) ? c->rdy2 : 0.0;
   ta.dtab = ta.tab && (c->march || c->cfg.order == 4) && march_twisted(c) ? march_down_tables<T>(c->mtab, c->ny) : nullptr;
   ta.slots = march_beta_slots(c->mtab, c->ny);
-  // the partials of the bulk sums (projection or k_bulk_partial), or of the
-  // 4th-order viscous sum (k_visc4_partial)
-  const int np = c->cfg.order == 4 ? visc4_npart(c) : (c->march ? c->npart_m : c->npart);
+  // the partials of the bulk sums or of the mean viscous stress (projection or k_bulk_partial)
+  const int np = c->march ? c->npart_m : c->npart;
   const size_t smem = ta.tab && c->ny <= kStagedRows ? (size_t)5 * (c->ny + 1) * sizeof(double) : 0;
   k_substep<T><<<setup_blocks(np), kSetupThreads, smem, c->stream>>>(c->sc, c->part, np, c->red1, p, ta);
   return cudaGetLastError();

@@ -240,11 +240,11 @@ __device__ __forceinline__ void fft_pass_r(int N, int Ns, int nlines, const CT* 
     for (int r = 0; r < R; ++r) store(l, idxD + r * Ns, v[r]);
   }
 }
-// pass p of the plan
+// pass p of the plan; mL: fdiv_magic(nlines), read for LFAST only
 template <class CT, bool LFAST, class LD, class ST>
-__device__ __forceinline__ void fft_pass(const FFTPlanDev& pl, int p, int nlines, const CT* __restrict__ tw, LD load,
-                                         ST store) {
-  const unsigned long long mL = LFAST ? fdiv_magic((unsigned)nlines) : 0ull, mNB = pl.mNB[p], mNs = pl.mNs[p];
+__device__ __forceinline__ void fft_pass(const FFTPlanDev& pl, int p, int nlines, unsigned long long mL,
+                                         const CT* __restrict__ tw, LD load, ST store) {
+  const unsigned long long mNB = pl.mNB[p], mNs = pl.mNs[p];
   const int N = pl.n, Ns = pl.Ns[p];
   switch (pl.radix[p]) {
     case 2: fft_pass_r<CT, 2, LFAST>(N, Ns, nlines, tw, mNB, mNs, mL, load, store); break;
