@@ -10,28 +10,38 @@
 
 namespace ch3d {
 
-constexpr int kSetupThreads = 256;
+constexpr int kSetupThreads = 512;
+constexpr int kSumPer = 8;         // partial sums per thread that one block loads at once
 constexpr int kStagedRows = 1024;  // rows whose coefficient vectors fit in the shared memory of the setup block
 
-// Sum of part[0..n) over the grid, valid in every thread of the block for which
-// the function returns true (the only block, or the last one to finish).
+// Sum of part[0..n) over the grid, valid in thread 0 of the block for which the
+// function returns true (the only block, or the last one to finish).  All loads of
+// a thread are in flight together and the block sums by shuffles: one thread per
+// loop trip with a barrier per halving took 6 us of a launch that is otherwise
+// two round trips to L2.
 __device__ __forceinline__ bool grid_sum(const double* __restrict__ part, int n, double* __restrict__ red,
-                                         unsigned* ticket, double* sh /* kSetupThreads */, double& sum) {
+                                         unsigned* ticket, double* sh /* kSetupThreads / 32 */, double& sum) {
   const int nb = gridDim.x, chunk = (n + nb - 1) / nb;
   const int lo = blockIdx.x * chunk, hi = min(n, lo + chunk);
   auto block_sum = [&](double v) {
-    sh[threadIdx.x] = v;
+    for (int w = 16; w > 0; w >>= 1) v += __shfl_down_sync(0xffffffffu, v, w);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
     __syncthreads();
-    for (int w = kSetupThreads / 2; w > 0; w >>= 1) {
-      if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-      __syncthreads();
+    double r = 0.0;
+    if (threadIdx.x < 32) {
+      r = threadIdx.x < kSetupThreads / 32 ? sh[threadIdx.x] : 0.0;
+      for (int w = kSetupThreads / 64; w > 0; w >>= 1) r += __shfl_down_sync(0xffffffffu, r, w);
     }
-    const double r = sh[0];
-    __syncthreads();
     return r;
   };
   double s = 0.0;
-  for (int q = lo + (int)threadIdx.x; q < hi; q += kSetupThreads) s += part[q];
+  for (int q0 = lo + (int)threadIdx.x; q0 < hi; q0 += kSumPer * kSetupThreads) {
+    double v[kSumPer];
+#pragma unroll
+    for (int u = 0; u < kSumPer; ++u) v[u] = q0 + u * kSetupThreads < hi ? __ldg(part + q0 + u * kSetupThreads) : 0.0;
+#pragma unroll
+    for (int u = 0; u < kSumPer; ++u) s += v[u];
+  }
   sum = block_sum(s);
   if (nb == 1) return true;
   __shared__ bool last;
@@ -40,7 +50,7 @@ __device__ __forceinline__ bool grid_sum(const double* __restrict__ part, int n,
     __threadfence();
     last = atomicInc(ticket, nb - 1) == (unsigned)nb - 1;  // back to 0 for the next launch
   }
-  __syncthreads();
+  __syncthreads();  // also: the first sum's values in sh have been read
   if (!last) return false;
   __threadfence();
   s = 0.0;
@@ -157,52 +167,56 @@ template <class T>
 __global__ void __launch_bounds__(kSetupThreads) k_substep(DevScalars* sc, const double* __restrict__ part, int npart,
                                                            double* __restrict__ red, SubstepPar p, TableArgs<T> ta) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ double sh[kSetupThreads];
+  __shared__ double sh[kSetupThreads / 32];
   __shared__ double beta;
+  // read before the sums, so that thread 0 makes no further round trip to memory
+  const int itime0 = sc->itime;
+  const double uddx = __longlong_as_double((long long)sc->uddx), dt0 = sc->dt, time0 = sc->SimTime,
+               pgaver0 = p.ns == 1 ? 0.0 : sc->PrGradAver;
   if (sc->status) return;
   double s1;
   if (!grid_sum(part, npart, red, &sc->ticket, sh, s1)) return;
   if (threadIdx.x == 0) {
+    double dt = dt0;
     if (p.begin) {  // src/CFD_2nd/m_ChannelSystem.f90:81-88 (CalcMaxCFL result -> cflmp, dt)
-      const double uddx = __longlong_as_double((long long)sc->uddx);
-      sc->itime += 1;
-      sc->cflmp = uddx * sc->dt;
+      sc->itime = itime0 + 1;
+      sc->cflmp = uddx * dt0;
+      dt = p.dtMax;
       if (p.iCFL == 1) {
         const double d = p.CFLc / uddx;
-        sc->dt = d < p.dtMax ? d : p.dtMax;
-      } else {
-        sc->dt = p.dtMax;
+        dt = d < p.dtMax ? d : p.dtMax;
       }
+      sc->dt = dt;
     }
     // src/CFD_2nd/m_Parameters.f90:329-342 (PMcoeUpdate)
-    const double dt = sc->dt;
+    const double pmAlpha = p.alp * dt;
     sc->pmGamma = p.gam * dt;
     sc->pmTheta = p.the * dt;
-    sc->pmAlpha = p.alp * dt;
+    sc->pmAlpha = pmAlpha;
     beta = 0.5 * p.alp * p.xnu * dt;
     sc->pmBeta = beta;
-    sc->SimTime = sc->SimTime + dt * p.alp;
+    sc->SimTime = time0 + dt * p.alp;
     sc->pmAlphaC = p.alp;
     sc->pmBetaT = 0.5 * p.alp * dt;
-    if (p.ns == 1) sc->PrGradAver = 0.0;
     sc->ns = p.ns;
     sc->divmax1 = 0ull;
+    double pg = 0.0;  // this substep's mean pressure gradient
     if (p.IsUxConst && p.order == 4) {
       // the partial sums are those of the mean viscous stress (src/CFD_4th/m_TScheme.f90:364-377)
-      const double dpm = p.xnu * (s1 / p.nxnz + p.visc_wall) / p.yly;
-      sc->PrGradNow = dpm;
-      sc->dpmdxns = -(sc->pmAlpha * dpm);  // RhsX - pmAlpha*dpmdxns
-      sc->PrGradAver = sc->PrGradAver + dpm * p.alp;
+      pg = p.xnu * (s1 / p.nxnz + p.visc_wall) / p.yly;
+      sc->PrGradNow = pg;
+      sc->dpmdxns = -(pmAlpha * pg);  // RhsX - pmAlpha*dpmdxns
     } else if (p.IsUxConst) {
       // the bulk constraint of src/CFD_2nd/m_TSchemePIMP_inc.f90:60-74 from the sums of the current ux
       const double s1tot1 = s1 * p.norm_bulk;
+      pg = (p.ubulk - s1tot1) / dt;
       sc->s1tot1 = s1tot1;
       sc->dpmdxns = p.alp * (p.ubulk - s1tot1);
-      sc->PrGradNow = (p.ubulk - s1tot1) / dt;
-      sc->PrGradAver = sc->PrGradAver + p.alp * sc->PrGradNow;
+      sc->PrGradNow = pg;
     } else {
       sc->dpmdxns = 0.0;
     }
+    sc->PrGradAver = pgaver0 + p.alp * pg;
     if (p.last) {  // the maxima the diagnostics of this step accumulate
       sc->divmax2 = 0ull;
       sc->vmax[0] = sc->vmax[1] = sc->vmax[2] = 0ull;
@@ -235,7 +249,7 @@ __global__ void __launch_bounds__(kSetupThreads) k_substep(DevScalars* sc, const
 __global__ void __launch_bounds__(kSetupThreads) k_step_end(DevScalars* sc, const double* __restrict__ part, int npart,
                                                             double* __restrict__ red, double norm_uxm, double div_limit,
                                                             double vel_limit) {
-  __shared__ double sh[kSetupThreads];
+  __shared__ double sh[kSetupThreads / 32];
   if (sc->status) return;
   double s;
   if (!grid_sum(part, npart, red, &sc->ticket, sh, s) || threadIdx.x != 0) return;
@@ -282,8 +296,8 @@ cudaError_t launch_reduce_partials(ch3d_ctx* c, const double* in, int n, double*
   return cudaGetLastError();
 }
 
-// One block up to 4096 partial sums (16 per thread), else CH3D_NRED.
-static unsigned setup_blocks(int n) { return n <= 16 * kSetupThreads ? 1u : (unsigned)CH3D_NRED; }
+// One block up to 4096 partial sums, all in flight at once, else CH3D_NRED.
+static unsigned setup_blocks(int n) { return n <= kSumPer * kSetupThreads ? 1u : (unsigned)CH3D_NRED; }
 
 template <class T> static cudaError_t substep_t(ch3d_ctx* c, int ns, bool whole_step) {
   SubstepPar p;
@@ -310,7 +324,7 @@ template <class T> static cudaError_t substep_t(ch3d_ctx* c, int ns, bool whole_
   ta.r2x = fimp ? c->rdx2 : 0.0;
   ta.r2z = fimp ? c->rdz2 : 0.0;
   ta.r2y = y_periodic(c) ? c->rdy2 : 0.0;
-  ta.dtab = ta.tab && (c->march || c->cfg.order == 4) && march_twisted(c) ? march_down_tables<T>(c->mtab, c->ny) : nullptr;
+  ta.dtab = ta.tab && ((c->march && !march_rows_path(c)) || c->cfg.order == 4) && march_twisted(c) ? march_down_tables<T>(c->mtab, c->ny) : nullptr;
   ta.slots = march_beta_slots(c->mtab, c->ny);
   // the partials of the bulk sums or of the mean viscous stress (projection or k_bulk_partial)
   const int np = c->march ? c->npart_m : c->npart;

@@ -184,6 +184,11 @@ template <class T> struct SweepArgs {
   __device__ __forceinline__ T* us(int c) const { return c == 0 ? s0 : (c == 1 ? s1 : s2); }
 };
 
+// shared memory of the scans, rounded to the staging's alignment
+template <class R> __host__ __device__ constexpr size_t sweep_scan_bytes(int nwarps, int C) {
+  return ((size_t)(2 * nwarps * C + 2 * nwarps + 2 * C) * sizeof(R) + 15) / 16 * 16;
+}
+
 template <class T, class R, int C, int RPT, int MAXT, int MINB, bool PER, bool ADDU>
 __global__ void __launch_bounds__(MAXT, MINB) k_sweep(SweepArgs<T> A, int nx, int n, long long rs, long long os, int no,
                                                       const double* __restrict__ pf, size_t pfs, const R* __restrict__ tab, int addp,
@@ -196,8 +201,28 @@ __global__ void __launch_bounds__(MAXT, MINB) k_sweep(SweepArgs<T> A, int nx, in
   R* const aggD = aggU + nwarps * C;
   R* const prod = aggD + nwarps * C;
   R* const ends = prod + 2 * nwarps;
+  // the thread's rows of the next line set, [stage][rhs rows, u rows][threads]
+  T* const stg = reinterpret_cast<T*>(smem_raw + sweep_scan_bytes<R>(nwarps, C)) + threadIdx.x;
   const int m = PER ? n - 1 : n;  // rows of the recurrences
   const int j0 = p * RPT;
+  const int i = blockIdx.x * C + c;
+  const bool in = i < nx;
+  T* const r = A.r(comp);
+  const T* const ub = A.u(comp);
+  auto issue = [&](int o, int st) {
+    if (in && o < no) {
+      const long long base = i + os * o + rs * j0;
+      T* const d = stg + (size_t)st * (ADDU ? 2 : 1) * RPT * blockDim.x;
+#pragma unroll
+      for (int u = 0; u < RPT; ++u)
+        if (j0 + u < m) {
+          cp_async_el(d + u * blockDim.x, r + base + rs * u);
+          if (ADDU) cp_async_el(d + (RPT + u) * blockDim.x, ub + base + rs * u);
+        }
+    }
+    cp_async_commit();
+  };
+  issue(blockIdx.y, 0);
   const PtriRows F{pf + pfs * (sc->ns - 1), n};
   const R a = PER ? (R)F.a() : (R)0, cc = PER ? (R)F.c() : (R)0, rden = PER ? (R)(1.0 / F.den()) : (R)0;
   const R* const tb = PER ? nullptr : tab + (size_t)(sc->ns - 1) * n * MT_W + (comp == 1 ? MT_A1 : MT_A0);
@@ -229,23 +254,19 @@ __global__ void __launch_bounds__(MAXT, MINB) k_sweep(SweepArgs<T> A, int nx, in
   fd.init(Ad, prod + nwarps, lane, warp);
   __syncthreads();
   const R add = addp && comp == 0 ? (R)sc->dpmdxns : (R)0;
-  const int i = blockIdx.x * C + c;
-  const bool in = i < nx;
-  T* const r = A.r(comp);
-  const T* const ub = A.u(comp);
-  for (int o = blockIdx.y; o < no; o += gridDim.y) {  // uniform over the block
+  int st = 0;
+  for (int o = blockIdx.y; o < no; o += gridDim.y, st ^= 1) {  // uniform over the block
     const long long base = i + os * o;
-    R v[RPT], uu[ADDU ? RPT : 1], last = (R)0, ulast = (R)0;
-#pragma unroll
-    for (int u = 0; u < RPT; ++u) {
-      const bool ok = in && j0 + u < m;
-      v[u] = ok ? (R)r[base + rs * (j0 + u)] + add : (R)0;
-      if (ADDU) uu[u] = ok ? (R)__ldg(ub + base + rs * (j0 + u)) : (R)0;
-    }
+    R v[RPT], last = (R)0, ulast = (R)0;
     if (PER && in) {
       last = (R)r[base + rs * (n - 1)] + add;
       if (ADDU) ulast = (R)__ldg(ub + base + rs * (n - 1));
     }
+    issue(o + gridDim.y, st ^ 1);  // the next set's rows, while this one is solved
+    cp_async_wait<1>();            // each thread reads only what it copied itself
+    const T* const d0 = stg + (size_t)st * (ADDU ? 2 : 1) * RPT * blockDim.x;
+#pragma unroll
+    for (int u = 0; u < RPT; ++u) v[u] = in && j0 + u < m ? (R)d0[u * blockDim.x] + add : (R)0;
     if (!PER && comp == 1 && p == 0) v[0] = (R)0;  // duy_ym: uy_ym is constant (Update_uy_ym_CH)
     R b = (R)0;
 #pragma unroll
@@ -280,12 +301,12 @@ __global__ void __launch_bounds__(MAXT, MINB) k_sweep(SweepArgs<T> A, int nx, in
         if (p == 0) out[base + rs * (n - 1)] = (T)(ADDU ? ulast + fn : fn);
 #pragma unroll
         for (int u = 0; u < RPT; ++u)
-          if (j0 + u < m) out[base + rs * (j0 + u)] = (T)((ADDU ? uu[u] : (R)0) + (v[u] + fn * w[u]));
+          if (j0 + u < m) out[base + rs * (j0 + u)] = (T)((ADDU ? (R)d0[(RPT + u) * blockDim.x] : (R)0) + (v[u] + fn * w[u]));
       }
     } else if (in) {
 #pragma unroll
       for (int u = 0; u < RPT; ++u)
-        if (j0 + u < m) out[base + rs * (j0 + u)] = (T)((ADDU ? uu[u] : (R)0) + v[u]);
+        if (j0 + u < m) out[base + rs * (j0 + u)] = (T)((ADDU ? (R)d0[(RPT + u) * blockDim.x] : (R)0) + v[u]);
     }
     if (nwarps == 1) __syncwarp();
   }
@@ -363,9 +384,13 @@ static cudaError_t sweep_rows(ch3d_ctx* c, int n, long long rs, long long os, in
     k_sweep_long<T, R, PER, ADDU><<<dim3((c->nx + 127) / 128, no < 65535 ? no : 65535, 3), 128, 0, c->stream>>>(A, c->nx, 1, n, rs, os, no, pf, pfs, tab, addp, c->sc);
     return cudaGetLastError();
   }
-  auto go = [&](auto kern, int C, int RPT) {
+  cudaError_t err = cudaSuccess;
+  auto go = [&](auto kern, PerDevice& site, int C, int RPT, int maxt) {
     const int CW = 32 / C, P = ((n + RPT - 1) / RPT + CW - 1) / CW * CW, threads = C * P, nw = threads / 32;
-    const size_t smem = (size_t)(2 * nw * C + 2 * nw + 2 * C) * sizeof(R);
+    const size_t row = (size_t)2 * (ADDU ? 2 : 1) * RPT * sizeof(T);  // staging per thread
+    const size_t smem = sweep_scan_bytes<R>(nw, C) + row * threads;
+    err = smem_limit_once(site, c->device, kern, sweep_scan_bytes<R>(maxt / 32, C) + row * maxt);
+    if (err != cudaSuccess) return;
     const int gx = (c->nx + C - 1) / C;
     // a few line sets per block, so that their coefficients are formed once, while the GPU stays full
     const long long want = (long long)sm_count(c->device) * (2048 / threads > 0 ? 2048 / threads : 1);
@@ -374,10 +399,12 @@ static cudaError_t sweep_rows(ch3d_ctx* c, int n, long long rs, long long os, in
     if (gy < 1) gy = 1;
     kern<<<dim3(gx, (unsigned)gy, 3), threads, smem, c->stream>>>(A, c->nx, n, rs, os, no, pf, pfs, tab, addp, c->sc);
   };
-  if (n <= 256) go(k_sweep<T, R, 16, 8, 512, 1, PER, ADDU>, 16, 8);
-  else if (n <= 384) go(k_sweep<T, R, 16, 12, 512, 1, PER, ADDU>, 16, 12);
-  else go(k_sweep<T, R, 8, 24, 256, 1, PER, ADDU>, 8, 24);
-  return cudaGetLastError();
+  static PerDevice s8, s8w, s12, s24;  // per template instance
+  if (n <= 128) go(k_sweep<T, R, 16, 8, 256, 2, PER, ADDU>, s8, 16, 8, 256);
+  else if (n <= 256) go(k_sweep<T, R, 8, 8, 256, 2, PER, ADDU>, s8w, 8, 8, 256);
+  else if (n <= 384) go(k_sweep<T, R, 8, 12, 256, 1, PER, ADDU>, s12, 8, 12, 256);
+  else go(k_sweep<T, R, 8, 24, 256, 1, PER, ADDU>, s24, 8, 24, 256);
+  return err != cudaSuccess ? err : cudaGetLastError();
 }
 
 template <class T> static cudaError_t sweep_x(ch3d_ctx* c, const double* pf) {
