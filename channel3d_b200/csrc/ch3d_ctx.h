@@ -67,8 +67,8 @@ struct ch3d_ctx {
   double* red1 = nullptr;    // CH3D_NRED second-level sums of part
   double* red2 = nullptr;    // CH3D_NRED second-level sums of part2
   int npart = 0;
-  bool march = false;        // 2nd-order PIMP without LES: march kernels, npart_m partial sums in part
-  int npart_m = 0;
+  bool march = false;        // 2nd-order PIMP without LES: march kernels
+  int npart_m = 0;           // partial sums of the projection in part (with the diagnostics: part2)
   void* spec2 = nullptr;     // second half spectrum of the 1-D spectra (allocated at their first sample)
   double* specacc = nullptr; // EnergySpecX (nxh, ny, 18) | EnergySpecZ (nz/2+1, ny, 18) sums (FP64)
   int nspectime = 0;

@@ -438,12 +438,16 @@ __global__ void __launch_bounds__(32 * BZ * (TW ? 2 : 1),
 }
 
 // ---------------------------------------------------------------------------
-// FluidVelUpdate (src/CFD_2nd/m_TScheme.f90:281-306) + PressureUpdate_PIMP
-// (src/CFD_2nd/m_TSchemePIMP_inc.f90:852-873) as a march: a thread owns one
-// (i, k) column over a chunk of `rows` rows and keeps phi at j-1, j, j+1 in
-// registers (Neumann ghosts of SetBC_and_UpdateHalo_pr at the walls).  The
-// block's sum of ux * s1coe (the next substep's bulk constraint, clcRhsX_PIMP
-// :60-74) goes to part[block].  mode 1: projection only (pmAlpha = 1, p kept).
+// FluidVelUpdate (src/CFD_2nd/m_TScheme.f90:281-306; 4th order
+// src/CFD_4th/m_TScheme.f90:148-173) + the pressure update as a march: a thread
+// owns one (i, k) column over a chunk of `rows` rows and keeps phi at j-1, j, j+1
+// in registers (Neumann ghosts of SetBC_and_UpdateHalo_pr at the walls, periodic
+// rows without).  The block's sum of ux * s1coe (the next substep's bulk
+// constraint, clcRhsX_PIMP m_TSchemePIMP_inc.f90:60-74, or mean viscous stress)
+// goes to part[block].  mode 1: projection only (pmAlpha = 1, p kept).
+// KIND: 0 PressureUpdate_PIMP (src/CFD_2nd/m_TSchemePIMP_inc.f90:852-873), 1 _FIMP and
+// _FEXP (m_TSchemeFIMP_inc.f90:1371-1386, m_TSchemeFEXP_inc.f90:513-548), 2 the 4th
+// order (PIMP), 3 PressureUpdate_PIMP_LES (m_TSchemePIMP_inc.f90:878-904).
 // ---------------------------------------------------------------------------
 // Rows per block of the march projection: 32 where the grid fills the GPU anyway,
 // else as few as give about four blocks per SM (at least 4: a block's first and
@@ -463,16 +467,16 @@ __device__ __forceinline__ double block_sum128(double v, double* sh /* 4 */) {
   return threadIdx.x == 0 ? (sh[0] + sh[1]) + (sh[2] + sh[3]) : 0.0;
 }
 
-// DIAG (last substep of a step, nx % 32 == 0, nz % 4 == 0 so that no thread
-// idles): CheckDivergence, CalcVmax, the next step's CalcMaxCFL and the
+// DIAG (last substep of a step, 2nd order): CheckDivergence, CalcVmax, the next step's CalcMaxCFL and the
 // CalcUxAver partials (src/CFD_2nd/m_Tools.f90:21-104,250-270) of the new
 // velocity, fused in.  The i+1, j+1 and k+1 neighbours of the new velocity
 // are recomputed from u* and phi with the same expressions their own threads
 // use, so they equal the stored values bit for bit.
-template <class T, bool DIAG>
+template <class T, bool DIAG, int KIND>
 __global__ void __launch_bounds__(128) k_proj_march(Geo<T> g, Metrics<T> m, const T* uxs, const T* uys,
                                                     const T* uzs, T* ux, T* uy, T* uz, T* __restrict__ pr,
-                                                    const T* __restrict__ phi, double* __restrict__ part,
+                                                    const T* __restrict__ phi, const T* __restrict__ nut,
+                                                    double* __restrict__ part,
                                                     double* __restrict__ part2, int mode, int rows,
                                                     DevScalars* __restrict__ sc) {
   __shared__ double red[7][4];
@@ -492,19 +496,25 @@ __global__ void __launch_bounds__(128) k_proj_march(Geo<T> g, Metrics<T> m, cons
     const T pmBeta = (T)sc->pmBeta;
     const T rdxEta2 = g.rdx * pmAlpha, rdzEta2 = g.rdz * pmAlpha;
     const double rdx = g.rdx, rdz = g.rdz;
-    T pm = __ldg(phi + col + (long long)(j0 > 0 ? j0 - 1 : 0) * nx);
+    const bool per = g.bc.lo == 0;  // periodic in y
+    const T pmBetaT = KIND == 3 ? (T)sc->pmBetaT : (T)0;
+    const long long dx2 = i >= 2 ? -2 : nx - 2;
+    const long long dz2 = k >= 2 ? -2 * plane : (long long)(nz - 2) * plane;
+    const C4<T> c4(g);
+    T pm = __ldg(phi + col + (long long)(j0 > 0 ? j0 - 1 : (per ? ny - 1 : 0)) * nx);
     T pc = __ldg(phi + col + (long long)j0 * nx);
     // rows in batches of PB: all loads of a batch before its stores (u* and u may
     // be the same arrays, mode 1, so the compiler cannot reorder them itself)
-    constexpr int PB = DIAG ? 2 : 4;
+    constexpr int PB = DIAG || KIND >= 2 ? 2 : 4;
     for (int jb = j0; jb < j1; jb += PB) {
       T vpp[PB], vpx[PB], vpz[PB], vu[PB], vv[PB], vw[PB], vp[PB], mr[PB], mp[PB], mc[PB], mm[PB], ms[PB];
+      T ex[4][PB];  // KIND 2: phi at i-2, i+1, k-2, k+1; KIND 3: nut at j, j+1, j-1
       T qux[PB], qpx[PB], quz[PB], qpz[PB], quy[PB], qr[PB], qrp[PB], qdy[PB];  // DIAG neighbours, metrics
 #pragma unroll
       for (int b = 0; b < PB; ++b) {
         const int j = jb + b < j1 ? jb + b : j1 - 1;
         const long long idx = col + (long long)j * nx;
-        const int jn = j + 1 < ny ? j + 1 : ny - 1;
+        const int jn = j + 1 < ny ? j + 1 : (per ? 0 : ny - 1);
         vpp[b] = __ldg(phi + col + (long long)jn * nx);
         vpx[b] = __ldg(phi + idx + dxm);
         vpz[b] = __ldg(phi + idx + dzm);
@@ -512,6 +522,18 @@ __global__ void __launch_bounds__(128) k_proj_march(Geo<T> g, Metrics<T> m, cons
         vp[b] = mode == 0 ? pr[idx] : (T)0;
         mr[b] = m.rdyc[j + 1]; mp[b] = m.ap2Pr[j + 1]; mc[b] = m.ac2Pr[j + 1]; mm[b] = m.am2Pr[j + 1];
         ms[b] = m.s1coe[j + 1];
+        if (KIND == 2) {
+          ex[0][b] = __ldg(phi + idx + dx2);
+          ex[1][b] = __ldg(phi + idx + dxp);
+          ex[2][b] = __ldg(phi + idx + dz2);
+          ex[3][b] = __ldg(phi + idx + dzp);
+        }
+        if (KIND == 3 && mode == 0) {
+          ex[0][b] = __ldg(nut + idx);
+          ex[1][b] = j < ny - 1 ? __ldg(nut + idx + nx) : (T)0;
+          ex[2][b] = j > 0 ? __ldg(nut + idx - nx) : (T)0;
+          ex[3][b] = m.rdyc[j + 2];
+        }
         if (DIAG) {
           qux[b] = uxs[idx + dxp]; qpx[b] = __ldg(phi + idx + dxp);
           quz[b] = uzs[idx + dzp]; qpz[b] = __ldg(phi + idx + dzp);
@@ -526,11 +548,28 @@ __global__ void __launch_bounds__(128) k_proj_march(Geo<T> g, Metrics<T> m, cons
         const long long idx = col + (long long)j * nx;
         const T pp = vpp[b];
         const T sucacEta2 = mr[b] * pmAlpha;
-        const T uxn = vu[b] - (pc - vpx[b]) * rdxEta2;
-        const T uyn = vv[b] - (pc - pm) * sucacEta2;
-        const T uzn = vw[b] - (pc - vpz[b]) * rdzEta2;
+        T uxn = vu[b] - (pc - vpx[b]) * rdxEta2;
+        T uyn = vv[b] - (pc - pm) * sucacEta2;
+        T uzn = vw[b] - (pc - vpz[b]) * rdzEta2;
+        if (KIND == 2) {
+          uxn = vu[b] - pmAlpha * (c4.dx1 * ex[0][b] + c4.dx2 * vpx[b] + c4.dx3 * pc + c4.dx4 * ex[1][b]);
+          uyn = vv[b] - pmAlpha * ((pc - pm) * mr[b]);
+          uzn = vw[b] - pmAlpha * (c4.dz1 * ex[2][b] + c4.dz2 * vpz[b] + c4.dz3 * pc + c4.dz4 * ex[3][b]);
+        }
         ux[idx] = uxn; uy[idx] = uyn; uz[idx] = uzn;
-        if (mode == 0) {
+        if (KIND == 1) {
+          if (mode == 0) pr[idx] = vp[b] + pc;
+        } else if (KIND == 3) {
+          if (mode == 0) {
+            const T nc = ex[0][b];
+            const T njp = j < ny - 1 ? ex[1][b] : (g.bc.hi == -1 ? (T)2 * g.xnu - nc : nc);
+            const T njm = j > 0 ? ex[2][b] : (g.bc.lo == -1 ? (T)2 * g.xnu - nc : nc);
+            const T rdyp = m.rdyp[j + 1];
+            const T pmBetap = -pmBetaT * (rdyp * ex[3][b]) * ((T)0.5 * (njp + nc));
+            const T pmBetam = -pmBetaT * (rdyp * mr[b]) * ((T)0.5 * (nc + njm));
+            pr[idx] = vp[b] + pmBetap * pp + (-(pmBetap + pmBetam) + (T)1) * pc + pmBetam * pm;
+          }
+        } else if (mode == 0) {
           const T pmBetap = -pmBeta * mp[b];
           const T pmBetac = -pmBeta * mc[b] + (T)1;
           const T pmBetam = -pmBeta * mm[b];
@@ -541,7 +580,7 @@ __global__ void __launch_bounds__(128) k_proj_march(Geo<T> g, Metrics<T> m, cons
           // the new velocity at i+1, k+1 and j+1, as the threads that own them compute it
           const T uxp = qux[b] - (qpx[b] - pc) * rdxEta2;
           const T uzp = quz[b] - (qpz[b] - pc) * rdzEta2;
-          const T uyp = j + 1 < ny ? quy[b] - (pp - pc) * (qr[b] * pmAlpha) : (T)g.bc.uy_hi;
+          const T uyp = j + 1 < ny || per ? quy[b] - (pp - pc) * (qr[b] * pmAlpha) : (T)g.bc.uy_hi;
           const double a = uxn, bb = uyn, c = uzn, aip = uxp, bjp = uyp, ckp = uzp, rdyp = qrp[b];
           double d = fabs((aip - a) * rdx + (bjp - bb) * rdyp + (ckp - c) * rdz);
           if (!(d == d)) d = INFINITY;  // NaN folded into +inf: a NaN field trips the limits
@@ -823,20 +862,24 @@ int march_npart(const ch3d_ctx* c) {
   return (int)(g.x * g.y * g.z);
 }
 
-bool march_diag_fusable(const ch3d_ctx* c) { return c->march && c->nx % 32 == 0 && c->nz % 4 == 0; }
+bool march_diag_fusable(const ch3d_ctx* c) {
+  // the substituting projection carries them for full tiles only
+  return c->cfg.order == 2 && (!c->gsub || (c->nx % 32 == 0 && c->nz % 4 == 0));
+}
 
 template <class T> static cudaError_t proj_march_t(ch3d_ctx* c, int mode, bool diag) {
   T** f = (T**)c->f;
   T* in[3] = {mode == 1 ? f[0] : f[12], mode == 1 ? f[1] : f[13], mode == 1 ? f[2] : f[14]};
-  if (diag)
-    k_proj_march<T, true><<<march_proj_grid(c), 128, 0, c->stream>>>(make_geo<T>(c), metrics_of<T>(c), in[0], in[1],
-                                                                      in[2], f[0], f[1], f[2], f[3], f[10], c->part,
-                                                                      c->part2, mode, proj_rows(c), c->sc);
-  else
-    k_proj_march<T, false><<<march_proj_grid(c), 128, 0, c->stream>>>(make_geo<T>(c), metrics_of<T>(c), in[0], in[1],
-                                                                       in[2], f[0], f[1], f[2], f[3], f[10], c->part,
-                                                                       c->part2, mode, proj_rows(c), c->sc);
-  return cudaGetLastError();
+  auto go = [&](auto kern) {
+    kern<<<march_proj_grid(c), 128, 0, c->stream>>>(make_geo<T>(c), metrics_of<T>(c), in[0], in[1], in[2], f[0], f[1],
+                                                   f[2], f[3], f[10], f[11], c->part, c->part2, mode, proj_rows(c), c->sc);
+    return cudaGetLastError();
+  };
+  const ch3d_config& q = c->cfg;
+  if (q.order == 4) return go(k_proj_march<T, false, 2>);
+  if (q.IsImplicit != 1) return diag ? go(k_proj_march<T, true, 1>) : go(k_proj_march<T, false, 1>);
+  if (q.LES_type > 0) return diag ? go(k_proj_march<T, true, 3>) : go(k_proj_march<T, false, 3>);
+  return diag ? go(k_proj_march<T, true, 0>) : go(k_proj_march<T, false, 0>);
 }
 cudaError_t launch_proj_march(ch3d_ctx* c, int mode, bool diag) {
   return c->fp32 ? proj_march_t<float>(c, mode, diag) : proj_march_t<double>(c, mode, diag);

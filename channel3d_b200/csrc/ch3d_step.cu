@@ -145,19 +145,6 @@ __global__ void __launch_bounds__(256) k_ysolve(Geo<T> g, Metrics<double> m, con
     spec[kx + (long long)nxh * j + zs * kz] = mk((T)x.x, (T)x.y);
   }
 }
-
-// Block reductions of a 256-thread block with warp shuffles: the result is
-// valid in thread 0 (order of the sums fixed, so results are reproducible).
-__device__ __forceinline__ double block_sum256(double v, double* sh /* 8 */) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int tl = threadIdx.x + blockDim.x * threadIdx.y;
-  if ((tl & 31) == 0) sh[tl >> 5] = v;
-  __syncthreads();
-  double r = 0.0;
-  if (tl == 0)
-    for (int w = 0; w < 8; ++w) r += sh[w];
-  return r;
-}
 __device__ __forceinline__ double block_max256(double v, double* sh /* 8 */) {
   for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
   const int tl = threadIdx.x + blockDim.x * threadIdx.y;
@@ -167,104 +154,6 @@ __device__ __forceinline__ double block_max256(double v, double* sh /* 8 */) {
   if (tl == 0)
     for (int w = 0; w < 8; ++w) r = fmax(r, sh[w]);
   return r;
-}
-
-// ---------------------------------------------------------------------------
-// FluidVelUpdate (src/CFD_2nd/m_TScheme.f90:281-306) + PressureUpdate_PIMP
-// (src/CFD_2nd/m_TSchemePIMP_inc.f90:852-873), phi ghosts from
-// SetBC_and_UpdateHalo_pr (Neumann in y, periodic x,z), plus the block partial
-// sums of ux*dyp used by the next substep's bulk constraint.
-// mode 1: projection only (pmAlpha = 1, no pressure update).
-// ---------------------------------------------------------------------------
-template <class T>
-__global__ void __launch_bounds__(256) k_proj(Geo<T> g, Metrics<T> m, const T* uxs, const T* uys, const T* uzs,
-                                              T* ux, T* uy, T* uz, T* __restrict__ pr, const T* __restrict__ phi,
-                                              double* __restrict__ part, int mode, const DevScalars* __restrict__ sc,
-                                              const T* __restrict__ nut) {
-  __shared__ double red[8];
-  if (sc->status) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = blockIdx.z;
-  const int nx = g.nx, ny = g.ny, nz = g.nz;
-  const int tl = threadIdx.x + blockDim.x * threadIdx.y;
-  double s = 0.0;
-  if (i < nx && j < ny) {
-    const int jc = j + 1;
-    const int im = wrapm(i, nx), km = wrapm(k, nz);
-    const long long idx = i + (long long)nx * (j + (long long)ny * k);
-    const T pmAlpha = mode == 0 ? (T)sc->pmAlpha : (T)1;
-    const T phic = phi[idx];
-    const T phim_x = phi[im + (long long)nx * (j + (long long)ny * k)];
-    const int jm = j > 0 ? j - 1 : (g.bc.lo == 0 ? ny - 1 : 0);  // phi(ic,0,kc): Neumann or periodic halo
-    const T phim_y = phi[i + (long long)nx * (jm + (long long)ny * k)];
-    const T phim_z = phi[i + (long long)nx * (j + (long long)ny * km)];
-    const T rdxEta2 = g.rdx * pmAlpha, rdzEta2 = g.rdz * pmAlpha, sucacEta2 = m.rdyc[jc] * pmAlpha;
-    T uxn = uxs[idx] - (phic - phim_x) * rdxEta2;
-    T uyn = uys[idx] - (phic - phim_y) * sucacEta2;
-    T uzn = uzs[idx] - (phic - phim_z) * rdzEta2;
-    if (g.order == 4) {  // FluidVelUpdate, src/CFD_4th/m_TScheme.f90:148-173
-      const C4<T> c4(g);
-      const Nbr n = make_nbr(g, i, j, k);
-      const T dpdx = c4.dx1 * at(phi, n, n.xm2) + c4.dx2 * phim_x + c4.dx3 * phic + c4.dx4 * at(phi, n, n.xp);
-      const T dpdy = (phic - phim_y) * m.rdyc[jc];
-      const T dpdz = c4.dz1 * at(phi, n, n.zm2) + c4.dz2 * phim_z + c4.dz3 * phic + c4.dz4 * at(phi, n, n.zp);
-      uxn = uxs[idx] - pmAlpha * dpdx;
-      uyn = uys[idx] - pmAlpha * dpdy;
-      uzn = uzs[idx] - pmAlpha * dpdz;
-    }
-    ux[idx] = uxn;
-    uy[idx] = uyn;
-    uz[idx] = uzn;
-    if (mode == 0 && g.les && g.implicit == 1) {  // PressureUpdate_PIMP_LES (src/CFD_2nd/m_TSchemePIMP_inc.f90:878-904)
-      const T phip_y = phi[i + (long long)nx * ((j < ny - 1 ? j + 1 : ny - 1) + (long long)ny * k)];
-      const T nc = nut[idx];
-      const T njp = j < ny - 1 ? nut[idx + nx] : (g.bc.hi == -1 ? (T)2 * g.xnu - nc : nc);
-      const T njm = j > 0 ? nut[idx - nx] : (g.bc.lo == -1 ? (T)2 * g.xnu - nc : nc);
-      const T pmBetaT = (T)sc->pmBetaT;
-      const T metr1 = m.rdyp[jc] * m.rdyc[jc], metr2 = m.rdyp[jc] * m.rdyc[jc + 1];
-      const T visd = (T)0.5 * (njp + nc), visc = (T)0.5 * (nc + njm);
-      const T pmBetap = -pmBetaT * metr2 * visd;
-      const T pmBetam = -pmBetaT * metr1 * visc;
-      const T pmBetac = -(pmBetap + pmBetam) + (T)1;
-      pr[idx] = pr[idx] + pmBetap * phip_y + pmBetac * phic + pmBetam * phim_y;
-    } else if (mode == 0 && (g.implicit == 2 || g.implicit == 0)) {
-      // PressureUpdate_FIMP (src/CFD_2nd/m_TSchemeFIMP_inc.f90:1371-1386), _FEXP and
-      // _FEXP_LES (src/CFD_2nd/m_TSchemeFEXP_inc.f90:513-548)
-      pr[idx] = pr[idx] + phic;
-    } else if (mode == 0) {
-      const int jp = j < ny - 1 ? j + 1 : (g.bc.hi == 0 ? 0 : ny - 1);  // phi(ic,nyp,kc): Neumann or periodic halo
-      const T phip_y = phi[i + (long long)nx * (jp + (long long)ny * k)];
-      const T pmBeta = (T)sc->pmBeta;
-      const T pmBetap = -pmBeta * m.ap2Pr[jc];
-      const T pmBetac = -pmBeta * m.ac2Pr[jc] + (T)1;
-      const T pmBetam = -pmBeta * m.am2Pr[jc];
-      pr[idx] = pr[idx] + pmBetap * phip_y + pmBetac * phic + pmBetam * phim_y;
-    }
-    s = (double)uxn * (double)m.s1coe[jc];
-  }
-  const double bs = block_sum256(s, red);
-  if (tl == 0) part[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)] = bs;
-}
-
-// bulk partial sums of ux*s1coe for a freshly uploaded field
-template <class T>
-__global__ void __launch_bounds__(256) k_bulk_partial(Geo<T> g, Metrics<T> m, const T* __restrict__ ux,
-                                                      double* __restrict__ part) {
-  __shared__ double red[256];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = blockIdx.z;
-  const int tl = threadIdx.x + blockDim.x * threadIdx.y;
-  double s = 0.0;
-  if (i < g.nx && j < g.ny) s = (double)ux[i + (long long)g.nx * (j + (long long)g.ny * k)] * (double)m.s1coe[j + 1];
-  red[tl] = s;
-  __syncthreads();
-  for (int w = blockDim.x * blockDim.y / 2; w > 0; w >>= 1) {
-    if (tl < w) red[tl] += red[tl + w];
-    __syncthreads();
-  }
-  if (tl == 0) part[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)] = red[0];
 }
 
 // CheckDivergence, CalcVmax, CalcMaxCFL of the next step, CalcUxAver partials
@@ -449,23 +338,9 @@ template <class T> static cudaError_t xifft_t(ch3d_ctx* c) {
 }
 cudaError_t launch_xifft(ch3d_ctx* c) { return c->fp32 ? xifft_t<float>(c) : xifft_t<double>(c); }
 
-template <class T> static cudaError_t proj_t(ch3d_ctx* c, int mode) {
-  if (c->march) return launch_proj_march(c, mode, false);
-  T** f = (T**)c->f;
-  T* in[3] = {mode == 1 ? f[0] : f[12], mode == 1 ? f[1] : f[13], mode == 1 ? f[2] : f[14]};
-  k_proj<T><<<cell_grid(c), cell_block(), 0, c->stream>>>(make_geo<T>(c), metrics_of<T>(c), in[0], in[1], in[2], f[0],
-                                                          f[1], f[2], f[3], f[10], c->part, mode, c->sc, f[11]);
-  return cudaGetLastError();
-}
-cudaError_t launch_proj(ch3d_ctx* c, int mode) { return c->fp32 ? proj_t<float>(c, mode) : proj_t<double>(c, mode); }
+cudaError_t launch_proj(ch3d_ctx* c, int mode) { return launch_proj_march(c, mode, false); }
 cudaError_t launch_proj_diag(ch3d_ctx* c) { return launch_proj_march(c, 0, true); }
-template <class T> static cudaError_t bulk_t(ch3d_ctx* c) {
-  if (c->march) return launch_bulk_march(c);
-  T** f = (T**)c->f;
-  k_bulk_partial<T><<<cell_grid(c), cell_block(), 0, c->stream>>>(make_geo<T>(c), metrics_of<T>(c), f[0], c->part);
-  return cudaGetLastError();
-}
-cudaError_t launch_bulk_partials(ch3d_ctx* c) { return c->fp32 ? bulk_t<float>(c) : bulk_t<double>(c); }
+cudaError_t launch_bulk_partials(ch3d_ctx* c) { return launch_bulk_march(c); }
 
 // rows per k_diag block: whole columns when the x-z plane alone gives about
 // eight blocks per SM, shorter chunks on small grids

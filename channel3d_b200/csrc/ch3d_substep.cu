@@ -326,8 +326,8 @@ template <class T> static cudaError_t substep_t(ch3d_ctx* c, int ns, bool whole_
   ta.r2y = y_periodic(c) ? c->rdy2 : 0.0;
   ta.dtab = ta.tab && ((c->march && !march_rows_path(c)) || c->cfg.order == 4) && march_twisted(c) ? march_down_tables<T>(c->mtab, c->ny) : nullptr;
   ta.slots = march_beta_slots(c->mtab, c->ny);
-  // the partials of the bulk sums or of the mean viscous stress (projection or k_bulk_partial)
-  const int np = c->march ? c->npart_m : c->npart;
+  // the partials of the bulk sums or of the mean viscous stress (the projection or k_bulk_march)
+  const int np = c->npart_m;
   const size_t smem = ta.tab && c->ny <= kStagedRows ? (size_t)5 * (c->ny + 1) * sizeof(double) : 0;
   k_substep<T><<<setup_blocks(np), kSetupThreads, smem, c->stream>>>(c->sc, c->part, np, c->red1, p, ta);
   return cudaGetLastError();
