@@ -661,11 +661,11 @@ __global__ void __launch_bounds__(128) k_bulk_march(Geo<T> g, Metrics<T> m, cons
 // |div| into divmax1 (CheckDivergence before the projection).  PB rows of loads
 // in flight: 8 (168 registers, three blocks per SM) where the grid runs many
 // waves anyway, 4 (100 registers) where the column blocks fit in one wave at five.
-template <class T, int PB>
+template <class T, int PB, bool BND>
 __global__ void __launch_bounds__(128) k_div_bsub(Geo<T> g, Metrics<T> m, const T* __restrict__ tab,
                                                   const T* __restrict__ gx, const T* __restrict__ gy,
-                                                  const T* __restrict__ gz, T* __restrict__ dv,
-                                                  DevScalars* __restrict__ sc) {
+                                                  const T* __restrict__ gz, T* __restrict__ dv, T* __restrict__ bnd,
+                                                  int rows, DevScalars* __restrict__ sc) {
   __shared__ double red[4];
   if (sc->status) return;
   const int nx = g.nx, ny = g.ny, nz = g.nz;
@@ -706,6 +706,11 @@ __global__ void __launch_bounds__(128) k_div_bsub(Geo<T> g, Metrics<T> m, const 
         const T r = (axp - ax) * rdx + (ayn - ay) * sy[b] + (azp - az) * rdz;
         if (j >= PB) load(b, j - PB);
         dv[col + (long long)j * nx] = r;
+        if (BND && (j & (rows - 1)) == 0 && j > 0) {  // u* above the chunk of rows that ends here
+          const long long n2 = (long long)nx * nz;
+          T* const q = bnd + 3 * n2 * (j / rows - 1) + i + (long long)nx * k;
+          q[0] = ax; q[n2] = ay; q[2 * n2] = az;
+        }
         dmax = fmax(dmax, fabs((double)r));
         ayn = ay;
       }
@@ -719,15 +724,18 @@ __global__ void __launch_bounds__(128) k_div_bsub(Geo<T> g, Metrics<T> m, const 
 
 // FluidVelUpdate + PressureUpdate_PIMP (m_TScheme.f90:281-306, m_TSchemePIMP_inc.f90:
 // 852-873) from g, as k_proj_march in mode 0; DIAG: the step diagnostics of the
-// last substep (CheckDivergence, CalcVmax, CalcMaxCFL, CalcUxAver).  Partial sums
-// go to the slots of the chunked projection grid (npz row chunks), the unused
+// last substep (CheckDivergence, CalcVmax, CalcMaxCFL, CalcUxAver).  A block walks
+// the whole column where the tiles alone fill the GPU (rows = ny), else the chunk
+// blockIdx.z of `rows` rows from the u* that k_div_bsub left above it (bnd).  Partial
+// sums go to the slots of the chunked projection grid (npz row chunks), the unused
 // chunk slots of each block set to zero.
 template <class T, bool DIAG>
 __global__ void __launch_bounds__(128) k_proj_bsub(Geo<T> g, Metrics<T> m, const T* __restrict__ tab,
                                                    const T* __restrict__ gx, const T* __restrict__ gy,
                                                    const T* __restrict__ gz, T* __restrict__ ux, T* __restrict__ uy,
                                                    T* __restrict__ uz, T* __restrict__ pr, const T* __restrict__ phi,
-                                                   double* __restrict__ part, double* __restrict__ part2, int npz,
+                                                   const T* __restrict__ bnd, double* __restrict__ part,
+                                                   double* __restrict__ part2, int npz, int rows,
                                                    DevScalars* __restrict__ sc) {
   __shared__ double red[7][4];
   if (sc->status) return;
@@ -735,6 +743,7 @@ __global__ void __launch_bounds__(128) k_proj_bsub(Geo<T> g, Metrics<T> m, const
   const long long plane = (long long)nx * ny;
   tab += (size_t)(sc->ns - 1) * ny * MT_W;
   const int i = blockIdx.x * 32 + (threadIdx.x & 31), k = blockIdx.y * 4 + (threadIdx.x >> 5);
+  const int j0 = blockIdx.z * rows, j1 = min(j0 + rows, ny);
   double s = 0.0, s2 = 0.0, dvm = 0.0, v0 = 0.0, v1 = 0.0, v2 = 0.0, cf = 0.0;
   if (i < nx && k < nz) {
     const long long col = i + plane * k;
@@ -746,9 +755,21 @@ __global__ void __launch_bounds__(128) k_proj_bsub(Geo<T> g, Metrics<T> m, const
     const T rdxEta2 = g.rdx * pmAlpha, rdzEta2 = g.rdz * pmAlpha;
     const double rdx = g.rdx, rdz = g.rdz;
     T ax = (T)0, ay = (T)0, az = (T)0, axp = (T)0, azp = (T)0;  // u* of row j+1
-    T pc = __ldg(phi + col + (long long)(ny - 1) * nx);         // phi(j)
+    T pc = __ldg(phi + col + (long long)(j1 - 1) * nx);         // phi(j)
     T pp = pc;                                                   // phi(j+1), clamped at the top row
     T uyp = (T)g.bc.uy_hi;                                       // new uy at j+1 (DIAG)
+    if (j1 < ny) {
+      const long long n2 = (long long)nx * nz;
+      const T* const q = bnd + 3 * n2 * blockIdx.z;
+      const long long cc = i + (long long)nx * k, ck = i + (long long)nx * (k + 1 == nz ? 0 : k + 1);
+      ax = __ldg(q + cc); ay = __ldg(q + n2 + cc); az = __ldg(q + 2 * n2 + cc);
+      pp = __ldg(phi + col + (long long)j1 * nx);
+      if (DIAG) {
+        axp = __ldg(q + cc + dxp);
+        azp = __ldg(q + 2 * n2 + ck);
+        uyp = ay - (pp - pc) * (m.rdyc[j1 + 1] * pmAlpha);
+      }
+    }
     // rows pass through PB register slots, each refilled with the row PB below once consumed
     constexpr int PB = DIAG ? 2 : 4;
     T vx[PB], vy[PB], vz[PB], vp[PB], vpm[PB], vpx[PB], vpz[PB], c0[PB], c1[PB];
@@ -772,12 +793,12 @@ __global__ void __launch_bounds__(128) k_proj_bsub(Geo<T> g, Metrics<T> m, const
       }
     };
 #pragma unroll
-    for (int b = 0; b < PB; ++b) load(b, ny - 1 - b >= 0 ? ny - 1 - b : 0);
-    for (int jb = ny - 1; jb >= 0; jb -= PB) {
+    for (int b = 0; b < PB; ++b) load(b, j1 - 1 - b >= j0 ? j1 - 1 - b : j0);
+    for (int jb = j1 - 1; jb >= j0; jb -= PB) {
 #pragma unroll
       for (int b = 0; b < PB; ++b) {
         const int j = jb - b;
-        if (j < 0) break;
+        if (j < j0) break;
         const long long idx = col + (long long)j * nx;
         ax = vx[b] - c0[b] * ax;
         ay = vy[b] - c1[b] * ay;
@@ -811,15 +832,16 @@ __global__ void __launch_bounds__(128) k_proj_bsub(Geo<T> g, Metrics<T> m, const
           uyp = uyn;
         }
         pp = pc; pc = pm;
-        if (j >= PB) load(b, j - PB);
+        if (j >= j0 + PB) load(b, j - PB);
       }
     }
   }
-  const int bid = blockIdx.x + gridDim.x * blockIdx.y, nb = gridDim.x * gridDim.y;
-  for (int z = 1 + threadIdx.x; z < npz; z += blockDim.x) {  // the chunk slots this grid leaves empty
-    part[bid + (long long)nb * z] = 0.0;
-    if (DIAG) part2[bid + (long long)nb * z] = 0.0;
-  }
+  const int nb = gridDim.x * gridDim.y, bid = blockIdx.x + gridDim.x * blockIdx.y + nb * blockIdx.z;
+  if (gridDim.z == 1)
+    for (int z = 1 + threadIdx.x; z < npz; z += blockDim.x) {  // the chunk slots this grid leaves empty
+      part[bid + (long long)nb * z] = 0.0;
+      if (DIAG) part2[bid + (long long)nb * z] = 0.0;
+    }
   if constexpr (!DIAG) {
     const double bs = block_sum128(s, red[0]);
     if (threadIdx.x == 0) part[bid] = bs;
@@ -892,35 +914,41 @@ template <class T> static cudaError_t bulk_march_t(ch3d_ctx* c) {
 }
 cudaError_t launch_bulk_march(ch3d_ctx* c) { return c->fp32 ? bulk_march_t<float>(c) : bulk_march_t<double>(c); }
 
+// Rows per block of the substituting projection: the whole column, or, in FP64,
+// chunks where the tiles alone are at most six blocks per SM.  Mean of a step's three
+// launches, whole columns / chunks of 32 rows: 256x192x256 FP64 (512 tiles) 217 / 171 us,
+// mixed 115 / 121; 768x384x576 (3456 tiles) 2125 / 2202, mixed 1343 / 1436.
+static int bsub_rows(const ch3d_ctx* c) {
+  const long long tiles = (long long)((c->nx + 31) / 32) * ((c->nz + 3) / 4);
+  return c->fp32 || tiles > 6LL * sm_count(c->device) ? c->ny : proj_rows(c);
+}
 template <class T> static cudaError_t div_bsub_t(ch3d_ctx* c) {
   T** f = (T**)c->f;
   const dim3 grid((c->nx + 31) / 32, (c->nz + 3) / 4);
-  const int nsm = sm_count(c->device);
+  const int rows = bsub_rows(c);
+  T* const bnd = rows < c->ny ? f[7] : nullptr;
+  auto go = [&](auto kern) {
+    kern<<<grid, 128, 0, c->stream>>>(make_geo<T>(c), metrics_of<T>(c), (const T*)c->mtab, f[12], f[13], f[14], f[10],
+                                      bnd, rows, c->sc);
+    return cudaGetLastError();
+  };
   // 256x192x256 (512 blocks): 74 us with 4 rows, 93 with 8; 768x384x576 (3456 blocks):
   // 0.84 ms with 8 rows against 0.88 with 4
-  if ((long long)grid.x * grid.y > 6LL * nsm)
-    k_div_bsub<T, 8><<<grid, 128, 0, c->stream>>>(make_geo<T>(c), metrics_of<T>(c), (const T*)c->mtab, f[12], f[13],
-                                                   f[14], f[10], c->sc);
-  else
-    k_div_bsub<T, 4><<<grid, 128, 0, c->stream>>>(make_geo<T>(c), metrics_of<T>(c), (const T*)c->mtab, f[12], f[13],
-                                                   f[14], f[10], c->sc);
-  return cudaGetLastError();
+  if (bnd) return go(k_div_bsub<T, 4, true>);
+  return (long long)grid.x * grid.y > 6LL * sm_count(c->device) ? go(k_div_bsub<T, 8, false>) : go(k_div_bsub<T, 4, false>);
 }
 cudaError_t launch_div_bsub(ch3d_ctx* c) { return c->fp32 ? div_bsub_t<float>(c) : div_bsub_t<double>(c); }
 
 template <class T> static cudaError_t proj_bsub_t(ch3d_ctx* c, bool diag) {
   T** f = (T**)c->f;
-  const dim3 grid((c->nx + 31) / 32, (c->nz + 3) / 4);
-  const int npz = (int)march_proj_grid(c).z;
-  if (diag)
-    k_proj_bsub<T, true><<<grid, 128, 0, c->stream>>>(make_geo<T>(c), metrics_of<T>(c), (const T*)c->mtab, f[12],
-                                                      f[13], f[14], f[0], f[1], f[2], f[3], f[10], c->part, c->part2,
-                                                      npz, c->sc);
-  else
-    k_proj_bsub<T, false><<<grid, 128, 0, c->stream>>>(make_geo<T>(c), metrics_of<T>(c), (const T*)c->mtab, f[12],
-                                                       f[13], f[14], f[0], f[1], f[2], f[3], f[10], c->part, c->part2,
-                                                       npz, c->sc);
-  return cudaGetLastError();
+  const int rows = bsub_rows(c), npz = (int)march_proj_grid(c).z;
+  const dim3 grid((c->nx + 31) / 32, (c->nz + 3) / 4, (c->ny + rows - 1) / rows);
+  auto go = [&](auto kern) {
+    kern<<<grid, 128, 0, c->stream>>>(make_geo<T>(c), metrics_of<T>(c), (const T*)c->mtab, f[12], f[13], f[14], f[0],
+                                      f[1], f[2], f[3], f[10], f[7], c->part, c->part2, npz, rows, c->sc);
+    return cudaGetLastError();
+  };
+  return diag ? go(k_proj_bsub<T, true>) : go(k_proj_bsub<T, false>);
 }
 cudaError_t launch_proj_bsub(ch3d_ctx* c, bool diag) {
   return c->fp32 ? proj_bsub_t<float>(c, diag) : proj_bsub_t<double>(c, diag);
