@@ -85,8 +85,13 @@ void mesh_section(double* yp1, int id1, int id2, double c1, double c2, int Stret
 }
 
 // Plan of an n-point transform, n a product of 2 and 3: the fewest passes of
-// radix at most 16, the largest radix as small as they allow, smaller radices first.
-bool factor23(int n, FFTPlanDev& pl) {
+// radix at most maxr, the largest radix as small as they allow, smaller radices first.
+// FP64 x transforms stop at 9, a pass more for some lengths but half the registers
+// (ch3d_fft.cu): 96 points as 4 x 4 x 6 76 us, as 8 x 12 82 us (192^3, forward); z
+// transforms, whose passes move more between them, gain nothing (192 points as 12 x 16
+// 34 us, as 4 x 6 x 8 43).
+constexpr int kXRadix64 = 9;
+bool factor23(int n, FFTPlanDev& pl, int maxr) {
   pl.n = n; pl.npass = 0;
   int m = n;
   while (m % 2 == 0) m /= 2;
@@ -95,6 +100,7 @@ bool factor23(int n, FFTPlanDev& pl) {
   static const int radices[] = {2, 3, 4, 6, 8, 9, 12, 16};
   for (int np = 1; n > 1 && pl.npass == 0; ++np)
     for (int top : radices) {  // np ascending radices up to top
+      if (top > maxr) break;
       int r[CH3D_MAX_PASSES] = {0};
       auto search = [&](auto&& self, int p, int rest, int hi) -> bool {
         if (p == 0) return rest == 1;
@@ -626,7 +632,7 @@ int ch3d_create(const ch3d_config* cfg, const double* yp, ch3d_ctx** out) {
   c->NS = (long long)c->nxh * c->ny * c->nz;
   c->fp32 = cfg->precision == CH3D_PREC_MIXED;
   c->device = cfg->device;
-  if (!factor23(c->nx / 2, c->planx) || !factor23(c->nz, c->planz)) {
+  if (!factor23(c->nx / 2, c->planx, c->fp32 ? 16 : kXRadix64) || !factor23(c->nz, c->planz, 16)) {
     delete c;
     return fail(CH3D_ERR_UNSUPPORTED, "nxc/2 and nzc must be products of 2 and 3 (got %d, %d)", cfg->nxc / 2, cfg->nzc);
   }
@@ -1194,7 +1200,7 @@ int ch3d_poisson_noalloc(int nxc, int nyc, int nzc, double xlx, double zlz, cons
   for (int j = 1; j <= nyc; ++j)
     if (!(yp[j] > yp[j - 1])) return fail(CH3D_ERR_INVALID, "yp must increase");
   FFTPlanDev px, pz;
-  if (!factor23(nxc / 2, px) || !factor23(nzc, pz))
+  if (!factor23(nxc / 2, px, kXRadix64) || !factor23(nzc, pz, 16))
     return fail(CH3D_ERR_UNSUPPORTED, "nxc/2 and nzc must be products of 2 and 3");
   const size_t need = noalloc_bytes(nxc, nyc, nzc);
   if (need > (size_t)CH3D_NOALLOC_SCRATCH_BYTES)

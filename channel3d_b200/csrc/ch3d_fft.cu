@@ -9,6 +9,7 @@
 // stores them (k_xfft_g: after the real-to-complex split), so global memory is
 // touched once and shared memory only between passes.
 #include "ch3d_fft.cuh"
+#include <type_traits>
 
 namespace ch3d {
 
@@ -106,14 +107,18 @@ template <class CT> __device__ __forceinline__ CT c2r_unsplit(CT a, CT xb, CT w)
   return cconj(mk(e.x - o.y, e.y + o.x));
 }
 
-// Forward x transform of LPB lines per block.
-template <class T, int SRC>
+// Forward x transform of LPB lines per block.  FP64 forms the source of all lines in
+// shared memory first: in the first pass's registers, next to the butterfly, it took
+// 138 of them (12 warps per SM; 109 us at 192^3, now 76).  FP32 forms it there (80
+// registers; 96 x 65 x 54 step 143 us, 148 with the source first).
+template <class T, int SRC, int MAXR>
 __global__ void __launch_bounds__(256) k_xfft_g(Geo<T> g, Metrics<T> m, const T* __restrict__ ux,
                                                 const T* __restrict__ uy, const T* __restrict__ uz,
                                                 typename CplxOf<T>::type* __restrict__ spec, FFTPlanDev pl,
                                                 const typename CplxOf<T>::type* __restrict__ tw,
                                                 const typename CplxOf<T>::type* __restrict__ twr, int LPB, int LP, int sh,
-                                                unsigned long long mM1, int mode, DevScalars* __restrict__ sc,
+                                                unsigned long long mM, unsigned long long mM1, int mode,
+                                                DevScalars* __restrict__ sc,
                                                 T* __restrict__ pr) {
   typedef typename CplxOf<T>::type CT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -124,11 +129,21 @@ __global__ void __launch_bounds__(256) k_xfft_g(Geo<T> g, Metrics<T> m, const T*
   CT* src = (CT*)smem_raw;
   CT* dst = src + (size_t)LPB * LP;
   XSource<T, SRC> form{g, m, ux, uy, uz, pr, mode, mode == 0 || mode == 3 ? (T)(1.0 / sc->pmAlpha) : (T)1, 0.0};
-  fft_pass<CT, false>(pl, 0, nl, 0ull, tw, [&](int l, int n) { return form(line0 + l, n); },
-                      [&](int l, int n, CT v) { src[l * LP + xpad(n, sh)] = v; });
+  int p = 0;
+  if constexpr (SRC == 2 || sizeof(T) == 4) {
+    p = 1;
+    fft_pass<CT, false, MAXR>(pl, 0, nl, 0ull, tw, [&](int l, int n) { return form(line0 + l, n); },
+                              [&](int l, int n, CT v) { src[l * LP + xpad(n, sh)] = v; });
+  } else {
+#pragma unroll 2
+    for (int t = threadIdx.x; t < nl * M; t += blockDim.x) {
+      const int l = fdiv(t, mM), n = t - l * M;
+      src[l * LP + xpad(n, sh)] = form(line0 + l, n);
+    }
+  }
   __syncthreads();
-  for (int p = 1; p < pl.npass; ++p) {
-    fft_pass<CT, false>(pl, p, nl, 0ull, tw, [&](int l, int n) { return src[l * LP + xpad(n, sh)]; },
+  for (; p < pl.npass; ++p) {
+    fft_pass<CT, false, MAXR>(pl, p, nl, 0ull, tw, [&](int l, int n) { return src[l * LP + xpad(n, sh)]; },
                         [&](int l, int n, CT v) { dst[l * LP + xpad(n, sh)] = v; });
     __syncthreads();
     CT* t = src; src = dst; dst = t;
@@ -143,7 +158,7 @@ __global__ void __launch_bounds__(256) k_xfft_g(Geo<T> g, Metrics<T> m, const T*
 
 // z transform of the spectrum, in place: layout (kx, j, kz), lines over kz.
 // Block = up to TKX consecutive kx at one j; point n of line l at n * TKX + l.
-template <class T>
+template <class T, int MAXR>
 __global__ void __launch_bounds__(256) k_zfft_g(Geo<T> g, typename CplxOf<T>::type* __restrict__ spec, FFTPlanDev pl,
                                                 const typename CplxOf<T>::type* __restrict__ tw, int TKX,
                                                 unsigned long long mT, unsigned long long mTail, int inverse,
@@ -163,21 +178,21 @@ __global__ void __launch_bounds__(256) k_zfft_g(Geo<T> g, typename CplxOf<T>::ty
   auto lds = [&](int l, int n) { return src[n * TKX + l]; };
   const int last = pl.npass - 1;
   if (last == 0) {
-    fft_pass<CT, true>(pl, 0, nl, mL, tw, ldg, stg);
+    fft_pass<CT, true, MAXR>(pl, 0, nl, mL, tw, ldg, stg);
     return;
   }
-  fft_pass<CT, true>(pl, 0, nl, mL, tw, ldg, [&](int l, int n, CT v) { src[n * TKX + l] = v; });
+  fft_pass<CT, true, MAXR>(pl, 0, nl, mL, tw, ldg, [&](int l, int n, CT v) { src[n * TKX + l] = v; });
   __syncthreads();
   for (int p = 1; p < last; ++p) {
-    fft_pass<CT, true>(pl, p, nl, mL, tw, lds, [&](int l, int n, CT v) { dst[n * TKX + l] = v; });
+    fft_pass<CT, true, MAXR>(pl, p, nl, mL, tw, lds, [&](int l, int n, CT v) { dst[n * TKX + l] = v; });
     __syncthreads();
     CT* t = src; src = dst; dst = t;
   }
-  fft_pass<CT, true>(pl, last, nl, mL, tw, lds, stg);
+  fft_pass<CT, true, MAXR>(pl, last, nl, mL, tw, lds, stg);
 }
 
 // inverse x transform (complex-to-real, unnormalised as FFTW's HC2R) * normfft -> phi
-template <class T>
+template <class T, int MAXR>
 __global__ void __launch_bounds__(256) k_xifft_g(Geo<T> g, const typename CplxOf<T>::type* __restrict__ spec,
                                                  T* __restrict__ phi, FFTPlanDev pl,
                                                  const typename CplxOf<T>::type* __restrict__ tw,
@@ -202,17 +217,17 @@ __global__ void __launch_bounds__(256) k_xifft_g(Geo<T> g, const typename CplxOf
   auto lds = [&](int l, int n) { return src[l * LP + xpad(n, sh)]; };
   const int last = pl.npass - 1;
   if (last == 0) {
-    fft_pass<CT, false>(pl, 0, nl, 0ull, tw, unsplit, out);
+    fft_pass<CT, false, MAXR>(pl, 0, nl, 0ull, tw, unsplit, out);
     return;
   }
-  fft_pass<CT, false>(pl, 0, nl, 0ull, tw, unsplit, [&](int l, int n, CT v) { src[l * LP + xpad(n, sh)] = v; });
+  fft_pass<CT, false, MAXR>(pl, 0, nl, 0ull, tw, unsplit, [&](int l, int n, CT v) { src[l * LP + xpad(n, sh)] = v; });
   __syncthreads();
   for (int p = 1; p < last; ++p) {
-    fft_pass<CT, false>(pl, p, nl, 0ull, tw, lds, [&](int l, int n, CT v) { dst[l * LP + xpad(n, sh)] = v; });
+    fft_pass<CT, false, MAXR>(pl, p, nl, 0ull, tw, lds, [&](int l, int n, CT v) { dst[l * LP + xpad(n, sh)] = v; });
     __syncthreads();
     CT* t = src; src = dst; dst = t;
   }
-  fft_pass<CT, false>(pl, last, nl, 0ull, tw, lds, out);
+  fft_pass<CT, false, MAXR>(pl, last, nl, 0ull, tw, lds, out);
 }
 
 // ---------------------------------------------------------------------------
@@ -220,20 +235,29 @@ __global__ void __launch_bounds__(256) k_xifft_g(Geo<T> g, const typename CplxOf
 // ---------------------------------------------------------------------------
 constexpr int kFftSmemLimit = 200 * 1024;
 
-template <class T> static cudaError_t limits_t() {
+template <class T, int MAXR> static cudaError_t limits_t() {
   const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  cudaError_t r = cudaFuncSetAttribute(k_xfft_g<T, 0>, a, kFftSmemLimit);
-  if (r == cudaSuccess) r = cudaFuncSetAttribute(k_xfft_g<T, 1>, a, kFftSmemLimit);
-  if (r == cudaSuccess) r = cudaFuncSetAttribute(k_xfft_g<T, 2>, a, kFftSmemLimit);
-  if (r == cudaSuccess) r = cudaFuncSetAttribute(k_zfft_g<T>, a, kFftSmemLimit);
-  if (r == cudaSuccess) r = cudaFuncSetAttribute(k_xifft_g<T>, a, kFftSmemLimit);
+  cudaError_t r = cudaFuncSetAttribute(k_xfft_g<T, 0, MAXR>, a, kFftSmemLimit);
+  if (r == cudaSuccess) r = cudaFuncSetAttribute(k_xfft_g<T, 1, MAXR>, a, kFftSmemLimit);
+  if (r == cudaSuccess) r = cudaFuncSetAttribute(k_xfft_g<T, 2, MAXR>, a, kFftSmemLimit);
+  if (r == cudaSuccess) r = cudaFuncSetAttribute(k_zfft_g<T, MAXR>, a, kFftSmemLimit);
+  if (r == cudaSuccess) r = cudaFuncSetAttribute(k_xifft_g<T, MAXR>, a, kFftSmemLimit);
   return r;
+}
+// Runs go with the radices to compile in: FP64 plans up to radix 9 have kernels of 72
+// to 74 registers, those with the 12- and 16-point butterflies 118 to 128 (64^3 step
+// 145 / 141 us); in FP32 (44 / 64) the smaller ones were no faster (96 x 65 x 54 143 / 146).
+template <class T, class F> static void with_radices(const FFTPlanDev& pl, F go) {
+  if constexpr (sizeof(T) == 8)
+    if (pl.npass == 0 || pl.radix[pl.npass - 1] <= 9) return go(std::integral_constant<int, 9>{});  // radices ascend
+  go(std::integral_constant<int, 16>{});
 }
 cudaError_t fft_generic_setup(int device) {
   static PerDevice site;
   return once_per_device(site, device, [] {
-    const cudaError_t r = limits_t<double>();
-    return r == cudaSuccess ? limits_t<float>() : r;
+    cudaError_t r = limits_t<double, 9>();
+    if (r == cudaSuccess) r = limits_t<double, 16>();
+    return r == cudaSuccess ? limits_t<float, 16>() : r;
   });
 }
 
@@ -260,11 +284,13 @@ cudaError_t xfft_generic(const Geo<T>& g, const Metrics<T>& m, const T* a, const
   const XShape s = x_shape<T>(g.nx / 2, pl.radix[0]);
   const int nlines = g.ny * g.nz, grid = (nlines + s.LPB - 1) / s.LPB;
   auto go = [&](auto kern) {
-    kern<<<grid, s.threads, s.smem, st>>>(g, m, a, b, c, spec, pl, tw, twr, s.LPB, s.LP, s.sh, fdiv_magic(g.nx / 2 + 1), mode, sc, pr);
+    kern<<<grid, s.threads, s.smem, st>>>(g, m, a, b, c, spec, pl, tw, twr, s.LPB, s.LP, s.sh, fdiv_magic(g.nx / 2), fdiv_magic(g.nx / 2 + 1), mode, sc, pr);
   };
-  if (mode >= 2) go(k_xfft_g<T, 2>);
-  else if (g.order == 4) go(k_xfft_g<T, 1>);
-  else go(k_xfft_g<T, 0>);
+  with_radices<T>(pl, [&](auto R) {
+    if (mode >= 2) go(k_xfft_g<T, 2, R.value>);
+    else if (g.order == 4) go(k_xfft_g<T, 1, R.value>);
+    else go(k_xfft_g<T, 0, R.value>);
+  });
   return cudaGetLastError();
 }
 
@@ -278,8 +304,11 @@ cudaError_t zfft_generic(const Geo<T>& g, typename CplxOf<T>::type* spec, const 
   int TKX = sizeof(T) == 8 || g.nz > 256 ? 8 : 16;
   while (TKX > 1 && (size_t)nbuf * TKX * g.nz * sizeof(CT) > (size_t)kFftSmemLimit / 2) TKX >>= 1;
   const int tail = g.nxh % TKX;
-  k_zfft_g<T><<<dim3((g.nxh + TKX - 1) / TKX, g.ny), g.nz > 256 ? 256 : 128, (size_t)nbuf * TKX * g.nz * sizeof(CT), st>>>(
-      g, spec, pl, tw, TKX, fdiv_magic(TKX), fdiv_magic(tail > 0 ? tail : 1), inverse, sc);
+  auto go = [&](auto kern) {
+    kern<<<dim3((g.nxh + TKX - 1) / TKX, g.ny), g.nz > 256 ? 256 : 128, (size_t)nbuf * TKX * g.nz * sizeof(CT), st>>>(
+        g, spec, pl, tw, TKX, fdiv_magic(TKX), fdiv_magic(tail > 0 ? tail : 1), inverse, sc);
+  };
+  with_radices<T>(pl, [&](auto R) { go(k_zfft_g<T, R.value>); });
   return cudaGetLastError();
 }
 
@@ -289,7 +318,10 @@ cudaError_t xifft_generic(const Geo<T>& g, const typename CplxOf<T>::type* spec,
                           const DevScalars* sc, cudaStream_t st) {
   const XShape s = x_shape<T>(g.nx / 2, pl.radix[0]);
   const int nlines = g.ny * g.nz;
-  k_xifft_g<T><<<(nlines + s.LPB - 1) / s.LPB, s.threads, s.smem, st>>>(g, spec, phi, pl, tw, twr, s.LPB, s.LP, s.sh, normfft, sc);
+  auto go = [&](auto kern) {
+    kern<<<(nlines + s.LPB - 1) / s.LPB, s.threads, s.smem, st>>>(g, spec, phi, pl, tw, twr, s.LPB, s.LP, s.sh, normfft, sc);
+  };
+  with_radices<T>(pl, [&](auto R) { go(k_xifft_g<T, R.value>); });
   return cudaGetLastError();
 }
 

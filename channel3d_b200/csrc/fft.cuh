@@ -240,8 +240,9 @@ __device__ __forceinline__ void fft_pass_r(int N, int Ns, int nlines, const CT* 
     for (int r = 0; r < R; ++r) store(l, idxD + r * Ns, v[r]);
   }
 }
-// pass p of the plan; mL: fdiv_magic(nlines), read for LFAST only
-template <class CT, bool LFAST, class LD, class ST>
+// pass p of the plan; mL: fdiv_magic(nlines), read for LFAST only.  MAXR: radices compiled in
+// (9 or 16: the larger butterflies cost every pass of a kernel their registers)
+template <class CT, bool LFAST, int MAXR, class LD, class ST>
 __device__ __forceinline__ void fft_pass(const FFTPlanDev& pl, int p, int nlines, unsigned long long mL,
                                          const CT* __restrict__ tw, LD load, ST store) {
   const unsigned long long mNB = pl.mNB[p], mNs = pl.mNs[p];
@@ -253,8 +254,12 @@ __device__ __forceinline__ void fft_pass(const FFTPlanDev& pl, int p, int nlines
     case 6: fft_pass_r<CT, 6, LFAST>(N, Ns, nlines, tw, mNB, mNs, mL, load, store); break;
     case 8: fft_pass_r<CT, 8, LFAST>(N, Ns, nlines, tw, mNB, mNs, mL, load, store); break;
     case 9: fft_pass_r<CT, 9, LFAST>(N, Ns, nlines, tw, mNB, mNs, mL, load, store); break;
-    case 12: fft_pass_r<CT, 12, LFAST>(N, Ns, nlines, tw, mNB, mNs, mL, load, store); break;
-    case 16: fft_pass_r<CT, 16, LFAST>(N, Ns, nlines, tw, mNB, mNs, mL, load, store); break;
+    case 12:
+      if constexpr (MAXR >= 12) fft_pass_r<CT, 12, LFAST>(N, Ns, nlines, tw, mNB, mNs, mL, load, store);
+      break;
+    case 16:
+      if constexpr (MAXR >= 16) fft_pass_r<CT, 16, LFAST>(N, Ns, nlines, tw, mNB, mNs, mL, load, store);
+      break;
   }
 }
 
