@@ -934,8 +934,11 @@ template <class T> static cudaError_t div_bsub_t(ch3d_ctx* c) {
   };
   // 256x192x256 (512 blocks): 74 us with 4 rows, 93 with 8; 768x384x576 (3456 blocks):
   // 0.84 ms with 8 rows against 0.88 with 4
-  if (bnd) return go(k_div_bsub<T, 4, true>);
-  return (long long)grid.x * grid.y > 6LL * sm_count(c->device) ? go(k_div_bsub<T, 8, false>) : go(k_div_bsub<T, 4, false>);
+  if constexpr (sizeof(T) == 8)
+    if (bnd) return go(k_div_bsub<T, 4, true>);
+  // FP32: 8 rows always (256x192x256 with the x transform 93 / 86 us, 768x384x576 the same)
+  if constexpr (sizeof(T) == 4) return go(k_div_bsub<T, 8, false>);
+  else return (long long)grid.x * grid.y > 6LL * sm_count(c->device) ? go(k_div_bsub<T, 8, false>) : go(k_div_bsub<T, 4, false>);
 }
 cudaError_t launch_div_bsub(ch3d_ctx* c) { return c->fp32 ? div_bsub_t<float>(c) : div_bsub_t<double>(c); }
 

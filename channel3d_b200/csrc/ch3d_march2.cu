@@ -7,7 +7,9 @@
 // the columns i and i+1 and works on pairs of FP32 values: the sm_100
 // instructions add, mul and fma .f32x2 take two operands in a 64-bit register,
 // and aligned pairs of the staged rows are single 8-byte reads.  The arithmetic
-// is that of rhs2_cell, with the constants folded.
+// is that of rhs2_cell, with the constants folded.  The old Hist of a thread's columns
+// comes through shared memory as well, D + 1 rows ahead: two rows ahead in registers
+// 256x192x256 took 193 us per launch, now 150; 768x384x576 1.81 ms, now 1.75.
 #include "ch3d_march.cuh"
 
 namespace ch3d {
@@ -54,20 +56,25 @@ __device__ __forceinline__ F2 fma(F2 a, F2 b, F2 c) {
 }
 
 // Tile of 64 x 4 columns, 128 threads; rows staged in 16-byte vectors with the x
-// halo rounded up to 4 points, three rows ahead (four blocks per SM).
-constexpr int M2_BZ = 4, M2_D = 3, M2_RS = M2_D + 4, M2_SX = 64 + 8, M2_PL = M2_SX * (M2_BZ + 2);
+// halo rounded up to 4 points, D rows ahead.
+constexpr int M2_BZ = 4, M2_SX = 64 + 8, M2_PL = M2_SX * (M2_BZ + 2);
 constexpr int M2_NS = (M2_PL / 4 + 127) / 128;  // staging vectors per thread and field
-constexpr size_t M2_SMEM = (size_t)4 * M2_RS * M2_PL * sizeof(float) + (size_t)M2_RS * MT_W * sizeof(F2);
+// rows, table entries, old Hist
+constexpr size_t m2_smem(int D) {
+  return (size_t)4 * (D + 4) * M2_PL * sizeof(float) + (size_t)(D + 4) * MT_W * sizeof(F2) + (size_t)3 * (D + 1) * 128 * sizeof(F2);
+}
 
+template <int D>
 __global__ void __launch_bounds__(128, 4)
     k_rhs_march2(Geo<float> g, const float* __restrict__ tab, const float* __restrict__ ux,
                  const float* __restrict__ uy, const float* __restrict__ uz, const float* __restrict__ pr,
                  float* __restrict__ hx, float* __restrict__ hy, float* __restrict__ hz, float* __restrict__ gx,
                  float* __restrict__ gy, float* __restrict__ gz, const DevScalars* __restrict__ sc) {
-  constexpr int SX = M2_SX, PL = M2_PL, D = M2_D, RS = M2_RS, NT = 128;
+  constexpr int SX = M2_SX, PL = M2_PL, RS = D + 4, NT = 128;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float (*ring)[RS][PL] = reinterpret_cast<float (*)[RS][PL]>(smem_raw);
   F2 (*trs)[MT_W] = reinterpret_cast<F2 (*)[MT_W]>(smem_raw + (size_t)4 * RS * PL * sizeof(float));  // entries twice
+  unsigned long long (*hring)[3][NT] = reinterpret_cast<unsigned long long (*)[3][NT]>(&trs[RS][0]);  // the thread's own old Hist
   if (sc->status) return;
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const long long plane = (long long)nx * ny;
@@ -135,30 +142,32 @@ __global__ void __launch_bounds__(128, 4)
       if (kg < 0) kg += nz;
       so[q] = s < PL ? ig + plane * kg : 0;
     }
+    long long idx = act ? i + plane * k : 0;
+    const bool hread = act && (float)sc->pmTheta != 0.f;  // pmTheta = 0: the old Hist does not enter
+    auto issue_hist = [&](int r, int hsl, long long o) {
+      if (hread && r < ny) {
+        cp_async_el(&hring[hsl][0][tid], reinterpret_cast<const unsigned long long*>(hx + o));
+        cp_async_el(&hring[hsl][1][tid], reinterpret_cast<const unsigned long long*>(hy + o));
+        cp_async_el(&hring[hsl][2][tid], reinterpret_cast<const unsigned long long*>(hz + o));
+      }
+    };
 #pragma unroll
     for (int r = 0; r <= D + 1; ++r) {
       if (r < ny) issue_row(r);
+      if (r > 0) issue_hist(r - 1, r - 1, idx + (long long)(r - 1) * nx);
       cp_async_commit();
     }
-    long long idx = act ? i + plane * k : 0;
     F2 e0 = f2(0.f), e1 = f2(0.f), e2 = f2(0.f);  // eliminated right-hand sides of the previous row
-    const bool hread = act && (float)sc->pmTheta != 0.f;  // pmTheta = 0: the old Hist does not enter
-    auto ldp = [](const float* a, long long o) { return F2{*reinterpret_cast<const unsigned long long*>(a + o)}; };
     auto stp = [](float* a, long long o, F2 v) { *reinterpret_cast<unsigned long long*>(a + o) = v.v; };
-    F2 ho0 = f2(0.f), ho1 = f2(0.f), ho2 = f2(0.f), hb0 = f2(0.f), hb1 = f2(0.f), hb2 = f2(0.f);
-    if (hread) {
-      ho0 = ldp(hx, idx); ho1 = ldp(hy, idx); ho2 = ldp(hz, idx);
-      hb0 = ldp(hx, idx + nx); hb1 = ldp(hy, idx + nx); hb2 = ldp(hz, idx + nx);
-    }
+    int hsl = 0;  // Hist slot of row j
     for (int j = 0; j < ny; ++j, idx += nx) {
       cp_async_wait<D>();  // this thread's copies of rows <= j+1 are done
       if (j + 1 == ny) ghost_row(ny);
       if (j == 0) ghost_row(-1);
       __syncthreads();
       if (j + D + 2 < ny) issue_row(j + D + 2);
-      cp_async_commit();
-      F2 hn0 = f2(0.f), hn1 = f2(0.f), hn2 = f2(0.f);
-      if (hread && j + 2 < ny) { hn0 = ldp(hx, idx + 2 * nx); hn1 = ldp(hy, idx + 2 * nx); hn2 = ldp(hz, idx + 2 * nx); }
+      F2 ho0 = f2(0.f), ho1 = f2(0.f), ho2 = f2(0.f);
+      if (hread) { ho0.v = hring[hsl][0][tid]; ho1.v = hring[hsl][1][tid]; ho2.v = hring[hsl][2][tid]; }
       if (act) {
         const int s0 = slot(j - 1), s1 = slot(j), s2 = slot(j + 1);
         const F2* tr = trs[s1];
@@ -229,24 +238,33 @@ __global__ void __launch_bounds__(128, 4)
         stp(gy, idx, fma(tr[MT_CP1], vjp, v + e1));
         stp(gz, idx, fma(tr[MT_CP0], wjp, w + e2));
       }
-      ho0 = hb0; ho1 = hb1; ho2 = hb2;
-      hb0 = hn0; hb1 = hn1; hb2 = hn2;
+      issue_hist(j + D + 1, hsl, idx + (long long)(D + 1) * nx);  // the slot just used
+      cp_async_commit();
+      hsl = hsl == D ? 0 : hsl + 1;
     }
     cp_async_wait<0>();
     __syncthreads();  // the ring is refilled by the next tile's prologue
   }
 }
 
-// nx a multiple of 4 (16-byte row vectors)
-cudaError_t launch_rhs_march2(ch3d_ctx* c) {
-  static PerDevice site;
-  const cudaError_t e = smem_limit_once(site, c->device, k_rhs_march2, M2_SMEM);
+template <int D> static cudaError_t march2_t(ch3d_ctx* c, long long ntiles, int bps) {
+  static PerDevice site;  // per instance
+  const cudaError_t e = smem_limit_once(site, c->device, k_rhs_march2<D>, m2_smem(D));
   if (e != cudaSuccess) return e;
   float** f = (float**)c->f;
-  const long long ntiles = (long long)((c->nx + 63) / 64) * ((c->nz + M2_BZ - 1) / M2_BZ);
-  const long long cap = 4LL * sm_count(c->device);  // persistent blocks
-  k_rhs_march2<<<(unsigned)(ntiles < cap ? ntiles : cap), 128, M2_SMEM, c->stream>>>(make_geo<float>(c), (const float*)c->mtab, f[0], f[1], f[2], f[3], f[4], f[5], f[6], f[12], f[13], f[14], c->sc);
+  const long long cap = (long long)bps * sm_count(c->device);  // persistent blocks
+  k_rhs_march2<D><<<(unsigned)(ntiles < cap ? ntiles : cap), 128, m2_smem(D), c->stream>>>(
+      make_geo<float>(c), (const float*)c->mtab, f[0], f[1], f[2], f[3], f[4], f[5], f[6], f[12], f[13], f[14], c->sc);
   return cudaGetLastError();
+}
+// nx is a multiple of 128 here (x lengths with a register plan), so rows are whole 16-byte
+// vectors.  Three rows ahead and three blocks per SM, or two and four where that takes
+// fewer rounds of tiles: 256 tiles 150 / 162 us (256x192x256), 512 tiles 108 / 98
+// (512x64x256), 864 tiles 147 / 163 (768x64x288), 1728 tiles 1767 / 1748 (768x384x576).
+cudaError_t launch_rhs_march2(ch3d_ctx* c) {
+  const long long ntiles = (long long)((c->nx + 63) / 64) * ((c->nz + M2_BZ - 1) / M2_BZ), nsm = sm_count(c->device);
+  const long long rounds3 = (ntiles + 3 * nsm - 1) / (3 * nsm), rounds4 = (ntiles + 4 * nsm - 1) / (4 * nsm);
+  return rounds3 <= rounds4 ? march2_t<3>(c, ntiles, 3) : march2_t<2>(c, ntiles, 4);
 }
 
 }  // namespace ch3d

@@ -1,19 +1,17 @@
-// ch3d_step.cu -- sm_100a kernels of the 2nd-order partially implicit RK3
-// step (src/CFD_2nd/m_ChannelSystem.f90:73-154 with the PIMP procedures of
-// src/CFD_2nd/m_TSchemePIMP_inc.f90) and the pressure Poisson pipeline
-// (src/CFD_2nd/m_Poisson.f90:1078-1201).  FP64 and FP32 (mixed) instances.
+// ch3d_step.cu -- the pressure Poisson pipeline (src/CFD_2nd/m_Poisson.f90:1078-
+// 1201), the diagnostics and the 2nd-order statistics, and the solve without
+// allocations.  FP64 and FP32 (mixed) instances.
 //
 // Per substep the device runs:
-//   substep_setup  PMcoeUpdate + bulk-velocity reduction (clcRhsX_PIMP :60-74)
-//   rhs + uhat     clcRhsX/Y/Z_PIMP and clcU1/2/3Hat_PIMP as one column march
-//                  (ch3d_march.cu); the stage entry points run them separately
-//                  (k_rhs_pimp, k_uhat_pimp: partitioned tridiagonal)
+//   substep_setup  PMcoeUpdate + bulk-velocity reduction (ch3d_substep.cu)
+//   ustar          right-hand sides and Crank-Nicolson solves (ch3d_march.cu, or
+//                  ch3d_rhs.cu and ch3d_sweep.cu)
 //   prsrc_xfft     clcPrSrcOther fused with the forward x R2C FFT
 //   spectral       z FFT, y tridiagonal per (kx,kz) with the (0,0) pin, z iFFT
 //   xifft          x C2R FFT * normfft -> phi
-//   proj           FluidVelUpdate + PressureUpdate_PIMP + next bulk partial sums
-// and per step: step_begin (CalcMaxCFL/dt), diag (CheckDivergence, CalcVmax,
-// CalcUxAver, next CFL), step_end (limit checks).
+//   proj           FluidVelUpdate + the pressure update + next bulk partial sums,
+//                  in the last substep the step's diagnostics
+// and per step: step_end (limit checks).
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -29,7 +27,7 @@ namespace ch3d {
 // y tridiagonal per (kx,kz) (src/CFD_2nd/m_Poisson.f90:1114-1156):
 // [am2Pr, ac2Pr + WaveNumX + WaveNumZ, ap2Pr], with the (kx,kz)=(0,0) system's
 // first row replaced by the identity and zero right-hand side.  Solved in FP64
-// in shared memory (also in the mixed path), partitioned as in k_uhat_pimp
+// in shared memory (also in the mixed path), partitioned over the block's threads
 // but with per-system factors.  Block = TS consecutive kx at one kz.
 // ---------------------------------------------------------------------------
 template <class T>
