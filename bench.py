@@ -44,17 +44,11 @@ ALG_ARRAYS_PER_SUBSTEP = {"pimp": 32, "order4": 32, "fimp": 47, "les": 32}
 #  4: inverse x FFT: read spectrum, write phi;
 #  5: projection + pressure update: read phi u* x3 p, write u x3 p)
 GROUP_ARRAYS = {0: 13, 2: 4, 3: 6, 4: 2, 5: 9}
-GROUP_NAMES = {0: "rhs", 1: "y_solves", 2: "k_prsrc_xfft", 3: "k_zfft+k_ysolve2+k_zfft", 4: "k_xifft",
-               5: "k_proj", 6: "scalar_kernels_per_step"}
-# the group-0 kernel of each scheme (RHS, fused with the y solves for pimp and order4)
-GROUP0_KERNEL = {"pimp": "k_rhs_march", "order4": "k_rhs_march", "fimp": "k_rhs_fimp", "les": "k_rhs_les"}
-# CUDA kernels launched per step by the step graph (ch3d_api.cu record_step):
-# step_begin 1 + per substep (reduce_partials + substep_setup 2, march table (pimp) or
-# helm_factors 1, rhs+uhat 1, prsrc_xfft 1, zfft + ysolve2 + zfft 3 (the mixed path's FP64
-# low modes inside the same y-solve kernel), xifft 1, proj 1) + diag_reset + diag 2
-# (the diag kernel only where the last projection does not carry the diagnostics)
-# + reduce_partials + step_end 2
-LAUNCHES_PER_SUBSTEP = {"fp64": 10, "mixed": 10}
+GROUP_NAMES = {0: "rhs", 1: "y_solves", 2: "k_prsrc_xfft", 3: "k_zfft+k_yscan+k_zfft", 4: "k_xifft",
+               5: "k_proj_march", 6: "scalar_kernels_per_step"}
+# the group-0 kernels of each scheme: one column march, or right-hand sides and line solves
+GROUP0_KERNEL = {"pimp": "k_rhs_march", "order4": "k_rhs_march", "fimp": "k_rhs_rows+k_sweep", "les": "k_rhs_les+k_uhat_les"}
+GROUP0_ROWS = "k_rhs_rows+k_sweep"
 
 
 def parse():
@@ -261,19 +255,27 @@ def profile_traffic(kernel, precision):
     return None, None
 
 
-def launches_per_step(cfg, key, precision, gsub):
+def rows_path(cfg, key, path):
+    """The partially implicit step of grids with few columns forms the right-hand
+    sides by rows and sweeps in y (march_rows_path, ch3d_march.cu)."""
+    import torch
+    sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+    return key == "pimp" and "gsub" not in path and cfg.nxc * cfg.nzc <= 120 * sms
+
+
+def launches_per_step(cfg, key, path, rows):
     """Kernel launches of one graph-replayed step (ch3d_api.cu record_step)."""
-    launches = 1 + 3 * LAUNCHES_PER_SUBSTEP[precision] + 4
-    if key == "pimp" and cfg.nxc % 32 == 0 and cfg.nzc % 4 == 0:
-        launches -= 1  # the last projection carries the step diagnostics (no diag kernel)
-    if gsub:
-        launches += 3  # divergence march + x FFT in place of the fused divergence/x FFT kernel
-    if key == "order4":
-        launches += 3 * 2        # mean viscous stress partials, interpolated velocities
-    elif key == "fimp":
-        launches += 3 * 4        # RHS and y solve unfused, x/z periodic sweeps + their factors
-    elif key == "les":
-        launches += 3 * 1 + 1 + (1 if cfg.LES_type == 10 else 0)  # RHS/y solve unfused, eddy viscosity (+ wall shear)
+    gsub = "gsub" in path
+    # u -> u*: the march, or right-hand sides with the y sweep (les: with its y solves),
+    # ADI with the x and z sweeps too
+    ustar = {"pimp": 2 if rows else 1, "order4": 1, "fimp": 4, "les": 2}[key]
+    # k_substep, u*, divergence (on its own when it substitutes) with x FFT, z FFT + y systems + z FFT, x iFFT, projection
+    launches = 3 * (1 + ustar + (2 if gsub else 1) + 3 + 1 + 1)
+    launches += 1  # k_step_end
+    if key == "order4" or (gsub and (cfg.nxc % 32 or cfg.nzc % 4)):
+        launches += 1  # k_diag: the last projection does not carry the diagnostics
+    if key == "les":  # wall shear, network and stress divergence; wall shear and eddy viscosity; eddy viscosity
+        launches += {11: 3, 10: 2}.get(cfg.LES_type, 1)
     return launches
 
 
@@ -322,10 +324,13 @@ def measure(args, ws, rank, local, precision, want_e2e):
     key = scheme_key(cfg)
     names = dict(GROUP_NAMES)
     names[0] = GROUP0_KERNEL[key]
-    if key == "pimp":
-        names[5] = "k_proj_march"
     path = sorted(s.path_flags())
     gsub = "gsub" in path
+    rows = rows_path(cfg, key, path)
+    if rows or (key == "les" and cfg.LES_type == 11):
+        names[0] = GROUP0_ROWS
+    elif gsub and precision == "mixed":
+        names[0] = "k_rhs_march2"
     if gsub:  # the march stops at g; the divergence and projection marches substitute u*
         names[2] = "k_div_bsub+k_prsrc_xfft"
         names[5] = "k_proj_bsub"
@@ -345,7 +350,7 @@ def measure(args, ws, rank, local, precision, want_e2e):
     traffic = tpp * cfg.npoints if tpp is not None else None
     step_alg = ALG_ARRAYS_PER_SUBSTEP[key] * 3 * word * cfg.npoints
     step_achieved = step_alg / (ms_per_step * 1e-3) / 1e9
-    launches = launches_per_step(cfg, key, precision, gsub)
+    launches = launches_per_step(cfg, key, path, rows)
 
     # end-to-end through the public API: pinned host arrays -> upload -> K steps -> download
     e2e = None

@@ -1,0 +1,81 @@
+"""The scalar work between the field kernels (channel3d_b200/csrc/ch3d_substep.cu, and
+the projection's last block on grids with up to 4096 partial sums) when the time
+step changes from step to step (iCFL = 1), so that every substep's coefficient
+tables are formed anew, against the oracle's steps: the grids on both sides of the
+line, the schemes with row tables and with periodic factor blocks, and a stage
+sequence after fused steps.
+
+Tolerance: whole steps 1e-10 as elsewhere; dt and the CFL number follow the
+velocities, 1e-9; pressure 4 eps U (L / 2 pi) / (2/15 dt) over its rms where larger."""
+import numpy as np
+import pytest
+
+from helpers import rel_l2, small_channel
+
+pytestmark = pytest.mark.gpu
+EPS = np.finfo(np.float64).eps
+
+
+def _cfg(scheme, shape):
+    from channel3d_b200 import workloads
+    nx, ny, nz = shape
+    if scheme == "periodic_adi":
+        cfg = workloads.taylor_green_periodic(16).copy(nxc=nx, nyc=ny, nzc=nz, nycSection=[ny], IsImplicit=2)
+    elif scheme == "wall":
+        cfg = small_channel(nx, ny, nz)
+    else:
+        cfg, _ = workloads.get({"adi": "channel128_re5600_fimp", "4th": "channel128_re5600_4th"}[scheme])
+        cfg = cfg.copy(nxc=nx, nyc=ny, nzc=nz, nycSection=[ny // 2, ny - ny // 2])
+    return cfg.copy(iCFL=1, CFLc=0.3, dtMax=1.0)
+
+
+@pytest.mark.parametrize("scheme,shape", [("wall", (36, 17, 18)), ("adi", (36, 17, 18)), ("4th", (36, 17, 18)),
+                                          ("periodic_adi", (36, 17, 18)), ("wall", (256, 16, 162)), ("adi", (768, 33, 192))])
+def test_variable_time_step(built, scheme, shape):
+    from channel3d_b200 import ChannelSolver, initfield, mesh_y
+    from oracle import oracle as O
+    cfg = _cfg(scheme, shape)
+    yp = mesh_y(cfg)
+    rng = np.random.default_rng(5)
+    if scheme == "periodic_adi":
+        f = [a + 0.05 * rng.standard_normal(cfg.shape) for a in initfield.taylor_green(cfg, yp=yp)]
+    else:
+        f = list(initfield.laminar_noise(cfg, yp=yp, seed=5))
+        f[3] = 0.01 * rng.standard_normal(cfg.shape)
+    o = O.Oracle(cfg)
+    o.set_state(*f)
+    with ChannelSolver(cfg, yp=yp) as s:
+        s.upload(*f)
+        for _ in range(3):
+            di, do = s.step(1), o.step(1)
+            for k in ("cflmp", "uxm"):
+                assert abs(di[k] - do[k]) <= 1e-9 * max(1.0, abs(do[k])), (k, di[k], do[k])
+        gs, go = s.download(), o.get_state()
+        for k in ("ux", "uy", "uz"):
+            assert rel_l2(gs[k], go[k]) < 1e-10, (k, rel_l2(gs[k], go[k]))
+        dt = di["dt"] if "dt" in di else 1e-3
+        ptol = 4 * EPS * np.abs(go["ux"]).max() * cfg.xlx / (2 * np.pi) / (2 / 15 * dt) / np.sqrt(np.mean(go["p"] ** 2))
+        assert rel_l2(gs["p"], go["p"]) < max(1e-10, ptol), rel_l2(gs["p"], go["p"])
+
+
+def test_stages_after_steps(built):
+    from channel3d_b200 import ChannelSolver, initfield, mesh_y
+    from oracle import oracle as O
+    cfg = small_channel(36, 17, 18)
+    yp = mesh_y(cfg)
+    f = initfield.laminar_noise(cfg, yp=yp, seed=6)
+    o = O.Oracle(cfg)
+    o.set_state(*f)
+    with ChannelSolver(cfg, yp=yp) as s:
+        s.upload(*f)
+        s.step(2)
+        o.step(2)
+        for ns in (1, 2, 3):
+            for q in range(7):
+                s.stage(q, ns)
+                o.stage(q, ns)
+        s.step(1)
+        o.step(1)
+        gs, go = s.download(), o.get_state()
+    for k in ("ux", "uy", "uz"):
+        assert rel_l2(gs[k], go[k]) < 1e-10, (k, rel_l2(gs[k], go[k]))
