@@ -7,7 +7,9 @@
 // the columns i and i+1 and works on pairs of FP32 values: the sm_100
 // instructions add, mul and fma .f32x2 take two operands in a 64-bit register,
 // and aligned pairs of the staged rows are single 8-byte reads.  The arithmetic
-// is that of rhs2_cell, with the constants folded.  The old Hist of a thread's columns
+// is that of rhs2_cell, with the constants folded; the two face fluxes of a term are
+// subtracted before they are scaled and added, so that the sum never holds a single
+// flux (adding them one by one raised the pressure error of 768x384x576 runs by a fifth and more).  The old Hist of a thread's columns
 // comes through shared memory as well, D + 1 rows ahead: two rows ahead in registers
 // 256x192x256 took 193 us per launch, now 150; 768x384x576 1.81 ms, now 1.75.
 #include "ch3d_march.cuh"
@@ -126,8 +128,8 @@ __global__ void __launch_bounds__(128, 4)
   const F2 dpm = f2((float)sc->dpmdxns);
   const F2 nax = f2(-pmA * g.rdx), naz = f2(-pmA * g.rdz), na = f2(-pmA);
   const F2 q1 = f2(0.25f * g.rdx), q3 = f2(0.25f * g.rdz), nq1 = f2(-0.25f * g.rdx), nq3 = f2(-0.25f * g.rdz);
-  const F2 d1 = f2(0.5f * g.rdx), d3 = f2(0.5f * g.rdz), nd1 = f2(-0.5f * g.rdx), nd3 = f2(-0.5f * g.rdz);
-  const F2 nux = f2(g.xnu * g.rdx2), nuz = f2(g.xnu * g.rdz2), m2 = f2(-2.f), p2 = f2(2.f);
+  const F2 d1 = f2(0.5f * g.rdx), d3 = f2(0.5f * g.rdz);
+  const F2 nux = f2(g.xnu * g.rdx2), nuz = f2(g.xnu * g.rdz2), m1 = f2(-1.f), m2 = f2(-2.f), p2 = f2(2.f);
   const int c0 = (tz + 1) * SX + 4 + 2 * tx;
   const int ntx = (nx + 63) / 64, ntiles = ntx * ((nz + M2_BZ - 1) / M2_BZ);
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -185,7 +187,7 @@ __global__ void __launch_bounds__(128, 4)
         const F2 p = at(3, s1, 0), pim = left(3, s1, 0, p), pjm = at(3, s0, 0), pkm = at(3, s1, -SX);
         const F2 IY1 = tr[MT_IY1], IY3 = tr[MT_IY3], one = f2(1.f);
         const F2 IY2 = one - IY1, IY4 = one - IY3;
-        const F2 suc = f2(0.5f) * tr[MT_RDYP], nsuc = f2(-0.5f) * tr[MT_RDYP];
+        const F2 suc = f2(0.5f) * tr[MT_RDYP];
         // velocities interpolated in y at the lower and upper faces
         const F2 ul = fma(IY1, ujm, IY2 * u), uu = fma(IY3, u, IY4 * ujp);
         const F2 wl = fma(IY1, wjm, IY2 * w), wu = fma(IY3, w, IY4 * wjp);
@@ -195,10 +197,8 @@ __global__ void __launch_bounds__(128, 4)
           F2 c = fma(nux, fma(m2, u, sx), f2(g.g1));
           c = fma(nuz, fma(m2, u, ukp + ukm), c);
           c = fma((uip - uim) * fma(p2, u, sx), nq1, c);  // (u_ip + u)^2 - (u + u_im)^2
-          c = fma((v + vim) * ul, suc, c);
-          c = fma((vjp + vimjp) * uu, nsuc, c);
-          c = fma((w + wim) * (u + ukm), q3, c);
-          c = fma((wkp + wimkp) * (ukp + u), nq3, c);
+          c = fma(fma(v + vim, ul, m1 * ((vjp + vimjp) * uu)), suc, c);
+          c = fma(fma(w + wim, u + ukm, m1 * ((wkp + wimkp) * (ukp + u))), q3, c);
           const F2 d22 = fma(tr[MT_AP2C], ujp, fma(tr[MT_AC2C], u, tr[MT_AM2C] * ujm));
           r0 = fma(gam, c, fma(the, ho0, fma(beta2, d22, fma(nax, p - pim, dpm))));
           stp(hx, idx, c);
@@ -208,11 +208,9 @@ __global__ void __launch_bounds__(128, 4)
           const F2 rc = tr[MT_RDYC], qrc = f2(-0.25f) * rc;
           F2 c = fma(nux, fma(m2, v, sx), f2(g.g2));
           c = fma(nuz, fma(m2, v, vkp + vkm), c);
-          c = fma(ul * (v + vim), d1, c);
-          c = fma(fma(IY1, uipjm, IY2 * uip) * (vip + v), nd1, c);
+          c = fma(fma(ul, v + vim, m1 * (fma(IY1, uipjm, IY2 * uip) * (vip + v))), d1, c);
           c = fma((vjp - vjm) * fma(p2, v, vjp + vjm), qrc, c);
-          c = fma(wl * (v + vkm), d3, c);
-          c = fma(fma(IY1, wjmkp, IY2 * wkp) * (vkp + v), nd3, c);
+          c = fma(fma(wl, v + vkm, m1 * (fma(IY1, wjmkp, IY2 * wkp) * (vkp + v))), d3, c);
           const F2 d22 = fma(tr[MT_AP2P], vjp, fma(tr[MT_AC2P], v, tr[MT_AM2P] * vjm));
           r1 = fma(gam, c, fma(the, ho1, fma(beta2, d22, (na * rc) * (p - pjm))));
           stp(hy, idx, c);
@@ -221,10 +219,8 @@ __global__ void __launch_bounds__(128, 4)
           const F2 sz = wkp + wkm;
           F2 c = fma(nux, fma(m2, w, wip + wim), f2(g.g3));
           c = fma(nuz, fma(m2, w, sz), c);
-          c = fma((u + ukm) * (w + wim), q1, c);
-          c = fma((uip + uipkm) * (wip + w), nq1, c);
-          c = fma((v + vkm) * wl, suc, c);
-          c = fma((vjp + vjpkm) * wu, nsuc, c);
+          c = fma(fma(u + ukm, w + wim, m1 * ((uip + uipkm) * (wip + w))), q1, c);
+          c = fma(fma(v + vkm, wl, m1 * ((vjp + vjpkm) * wu)), suc, c);
           c = fma((wkp - wkm) * fma(p2, w, sz), nq3, c);  // (w_kp + w)^2 - (w + w_km)^2
           const F2 d22 = fma(tr[MT_AP2C], wjp, fma(tr[MT_AC2C], w, tr[MT_AM2C] * wjm));
           r2 = fma(gam, c, fma(the, ho2, fma(beta2, d22, naz * (p - pkm))));
