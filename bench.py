@@ -329,8 +329,6 @@ def measure(args, ws, rank, local, precision, want_e2e):
     rows = rows_path(cfg, key, path)
     if rows or (key == "les" and cfg.LES_type == 11):
         names[0] = GROUP0_ROWS
-    elif gsub and precision == "mixed":
-        names[0] = "k_rhs_march2"
     if gsub:  # the march stops at g; the divergence and projection marches substitute u*
         names[2] = "k_div_bsub+k_prsrc_xfft"
         names[5] = "k_proj_bsub"

@@ -103,7 +103,6 @@ cudaError_t launch_ustar_fexp(ch3d_ctx* c);            // explicit scheme: right
 cudaError_t launch_rhs_les_const(ch3d_ctx* c);         // learned closure: constant viscosity and the stress force
 cudaError_t launch_uhat(ch3d_ctx* c);                  // stage path: Rhs arrays -> u*
 // 2nd-order PIMP step: RHS + y solves as a column march (ch3d_march.cu)
-cudaError_t launch_rhs_march2(ch3d_ctx* c);            // FP32 march that stops at g, two columns per thread (ch3d_march2.cu)
 cudaError_t launch_rhs_march(ch3d_ctx* c);             // u -> u*, Hist
 bool march_rows_path(const ch3d_ctx* c);               // few columns: right-hand sides by chunks of rows, then the y sweep
 size_t march_table_bytes(int ny);

@@ -7,7 +7,10 @@
 //   k_xifft_g  inverse x C2R transform * normfft -> phi (m_Poisson.f90:1194-1200)
 // The first pass forms or loads its points in registers and the last one
 // stores them (k_xfft_g: after the real-to-complex split), so global memory is
-// touched once and shared memory only between passes.
+// touched once and shared memory only between passes.  At 192^3 in FP64 the
+// forward x transform takes 76 us (102 with radix 2 and 3 passes), z 34 each (55),
+// the inverse x 35 (50), for 0.23, 0.11 and 0.11 GB: latency at 16 to 24 warps per
+// SM, part of it the fetch of the unrolled butterflies' code.
 #include "ch3d_fft.cuh"
 #include <type_traits>
 
@@ -235,15 +238,6 @@ __global__ void __launch_bounds__(256) k_xifft_g(Geo<T> g, const typename CplxOf
 // ---------------------------------------------------------------------------
 constexpr int kFftSmemLimit = 200 * 1024;
 
-template <class T, int MAXR> static cudaError_t limits_t() {
-  const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  cudaError_t r = cudaFuncSetAttribute(k_xfft_g<T, 0, MAXR>, a, kFftSmemLimit);
-  if (r == cudaSuccess) r = cudaFuncSetAttribute(k_xfft_g<T, 1, MAXR>, a, kFftSmemLimit);
-  if (r == cudaSuccess) r = cudaFuncSetAttribute(k_xfft_g<T, 2, MAXR>, a, kFftSmemLimit);
-  if (r == cudaSuccess) r = cudaFuncSetAttribute(k_zfft_g<T, MAXR>, a, kFftSmemLimit);
-  if (r == cudaSuccess) r = cudaFuncSetAttribute(k_xifft_g<T, MAXR>, a, kFftSmemLimit);
-  return r;
-}
 // Runs go with the radices to compile in: FP64 plans up to radix 9 have kernels of 72
 // to 74 registers, those with the 12- and 16-point butterflies 118 to 128 (64^3 step
 // 145 / 141 us); in FP32 (44 / 64) the smaller ones were no faster (96 x 65 x 54 143 / 146).
@@ -252,13 +246,31 @@ template <class T, class F> static void with_radices(const FFTPlanDev& pl, F go)
     if (pl.npass == 0 || pl.radix[pl.npass - 1] <= 9) return go(std::integral_constant<int, 9>{});  // radices ascend
   go(std::integral_constant<int, 16>{});
 }
-cudaError_t fft_generic_setup(int device) {
-  static PerDevice site;
-  return once_per_device(site, device, [] {
-    cudaError_t r = limits_t<double, 9>();
-    if (r == cudaSuccess) r = limits_t<double, 16>();
-    return r == cudaSuccess ? limits_t<float, 16>() : r;
+// Shared-memory limits of the kernels that transforms with these plans use, each once
+// per process and device (setting one loads the kernel).
+template <class T> static cudaError_t setup_t(int device, const FFTPlanDev& planx, const FFTPlanDev& planz) {
+  cudaError_t e = cudaSuccess;
+  with_radices<T>(planx, [&](auto R) {
+    static PerDevice site;  // per precision and radix set
+    e = once_per_device(site, device, [] {
+      const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+      cudaError_t r = cudaFuncSetAttribute(k_xfft_g<T, 0, decltype(R)::value>, a, kFftSmemLimit);
+      if (r == cudaSuccess) r = cudaFuncSetAttribute(k_xfft_g<T, 1, decltype(R)::value>, a, kFftSmemLimit);
+      if (r == cudaSuccess) r = cudaFuncSetAttribute(k_xfft_g<T, 2, decltype(R)::value>, a, kFftSmemLimit);
+      return r == cudaSuccess ? cudaFuncSetAttribute(k_xifft_g<T, decltype(R)::value>, a, kFftSmemLimit) : r;
+    });
   });
+  if (e != cudaSuccess) return e;
+  with_radices<T>(planz, [&](auto R) {
+    static PerDevice site;
+    e = once_per_device(site, device, [] {
+      return cudaFuncSetAttribute(k_zfft_g<T, decltype(R)::value>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFftSmemLimit);
+    });
+  });
+  return e;
+}
+cudaError_t fft_generic_setup(int device, bool fp32, const FFTPlanDev& planx, const FFTPlanDev& planz) {
+  return fp32 ? setup_t<float>(device, planx, planz) : setup_t<double>(device, planx, planz);
 }
 
 // Lines per x block: one round of 128 tasks in the first pass, at most 16 lines.

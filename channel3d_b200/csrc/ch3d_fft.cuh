@@ -1,5 +1,5 @@
 // ch3d_fft.cuh -- launchers of the generic-length Poisson transforms
-// (ch3d_fft.cu); fft_generic_setup(device) once before the first launch.
+// (ch3d_fft.cu); fft_generic_setup(...) once before the first launch.
 #pragma once
 #include "ch3d_dev.cuh"
 
@@ -10,7 +10,7 @@ struct XShape {
   size_t smem;
 };
 
-cudaError_t fft_generic_setup(int device);
+cudaError_t fft_generic_setup(int device, bool fp32, const FFTPlanDev& planx, const FFTPlanDev& planz);
 size_t fft_generic_smem(const FFTPlanDev& planx, const FFTPlanDev& planz);
 // mode: 0 div(u*)/pmAlpha of (a, b, c), 1 div(u), 2 source in a, 3 divergence in a, /pmAlpha, 4 field in a
 template <class T>

@@ -1000,7 +1000,7 @@ template <class T, bool O4> static cudaError_t rhs_march_t(ch3d_ctx* c) {
   cudaError_t e = once_per_device(site, c->device, [&] {
     const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
     cudaError_t r = cudaFuncSetAttribute(kern, a, (int)smem);
-    if constexpr (!O4 && sizeof(T) == 8) {
+    if constexpr (!O4) {
       if (r == cudaSuccess) r = cudaFuncSetAttribute(k_rhs_march<T, O4, false, false, BZ, D, RS>, a, (int)smem);
     }
     return r;
@@ -1021,8 +1021,8 @@ template <class T, bool O4> static cudaError_t rhs_march_t(ch3d_ctx* c) {
     const long long cap = !O4 ? (long long)nsm * S::bps : ntiles;
     const unsigned grid = (unsigned)(ntiles < cap ? ntiles : cap);
     bool done = false;
-    if constexpr (!O4 && sizeof(T) == 8) {
-      if (c->gsub) {  // stops at g: the divergence and projection marches substitute (FP32: ch3d_march2.cu)
+    if constexpr (!O4) {
+      if (c->gsub) {  // stops at g: the divergence and projection marches substitute
         args(k_rhs_march<T, O4, false, false, BZ, D, RS>, grid, 32 * BZ, smem);
         done = true;
       }
@@ -1039,7 +1039,6 @@ bool march_rows_path(const ch3d_ctx* c) {
   return c->march && (long long)c->nx * c->nz <= 120LL * sm_count(c->device);
 }
 cudaError_t launch_rhs_march(ch3d_ctx* c) {
-  if (c->fp32 && c->gsub) return launch_rhs_march2(c);  // two columns per thread; such nx are multiples of 128
   if (c->cfg.order == 4) return c->fp32 ? rhs_march_t<float, true>(c) : rhs_march_t<double, true>(c);
   return c->fp32 ? rhs_march_t<float, false>(c) : rhs_march_t<double, false>(c);
 }

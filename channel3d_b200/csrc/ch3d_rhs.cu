@@ -10,7 +10,9 @@
 // row's table entries), copied two (FP64) or four (FP32) rows ahead; each thread
 // forms the three right-hand sides of its cell from rows j-1, j, j+1 of the ring.
 // One thread per cell and component, with the stencil read from global memory,
-// was bound by its loads: 157 us at 128^3 (87 with a warm L2).
+// was bound by its loads: 157 us at 128^3 (87 with a warm L2).  Now 50 us there for
+// 0.22 GB (ADI; 44% of the DRAM bandwidth) and 9 us at 64^3, bound by the latency of a
+// row with 16 warps per SM: the registers allow four blocks of 128 threads.
 #include "ch3d_march.cuh"
 
 namespace ch3d {

@@ -301,7 +301,7 @@ template <class T> static cudaError_t prsrc_t(ch3d_ctx* c, int mode) {
   typedef typename CplxOf<T>::type CT;
   cudaError_t e;
   if (launch_prsrc_xfft_r(c, mode, &e)) return e;
-  if ((e = fft_generic_setup(c->device)) != cudaSuccess) return e;
+  if ((e = fft_generic_setup(c->device, c->fp32, c->planx, c->planz)) != cudaSuccess) return e;
   T** f = (T**)c->f;
   const T* a = mode >= 2 ? f[10] : (mode == 1 ? f[0] : f[12]);
   return xfft_generic<T>(make_geo<T>(c), metrics_of<T>(c), a, mode == 1 ? f[1] : f[13], mode == 1 ? f[2] : f[14],
@@ -313,7 +313,7 @@ template <class T> static cudaError_t zfft_t(ch3d_ctx* c, int inverse) {
   typedef typename CplxOf<T>::type CT;
   cudaError_t e;
   if (launch_zfft_r(c, inverse, &e)) return e;
-  if ((e = fft_generic_setup(c->device)) != cudaSuccess) return e;
+  if ((e = fft_generic_setup(c->device, c->fp32, c->planx, c->planz)) != cudaSuccess) return e;
   return zfft_generic<T>(make_geo<T>(c), (CT*)c->spec, c->planz, (const CT*)c->twz, inverse, c->sc, c->stream);
 }
 static cudaError_t zfft(ch3d_ctx* c, int inverse) { return c->fp32 ? zfft_t<float>(c, inverse) : zfft_t<double>(c, inverse); }
@@ -330,7 +330,7 @@ template <class T> static cudaError_t xifft_t(ch3d_ctx* c) {
   typedef typename CplxOf<T>::type CT;
   cudaError_t e;
   if (launch_xifft_r(c, &e)) return e;
-  if ((e = fft_generic_setup(c->device)) != cudaSuccess) return e;
+  if ((e = fft_generic_setup(c->device, c->fp32, c->planx, c->planz)) != cudaSuccess) return e;
   return xifft_generic<T>(make_geo<T>(c), (const CT*)c->spec, (T*)c->f[10], c->planx, (const CT*)c->twx,
                           (const CT*)c->twr, (T)c->normfft, c->sc, c->stream);
 }
@@ -570,14 +570,18 @@ size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 }  // namespace
 
 // Once per device (that device current): looks up the array's device address
-// and sets the dynamic shared-memory limit of the four kernels the solve runs.
+// and sets the dynamic shared-memory limits of the kernels the solve runs.
 cudaError_t noalloc_scratch_address(int dev, void** out) {
   cudaError_t e = once_per_device(g_noalloc_site, dev, [&] {
     void* p = nullptr;
     cudaError_t r = cudaGetSymbolAddress(&p, g_noalloc_scratch);
     if (r != cudaSuccess) return r;
     const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    if ((r = fft_generic_setup(dev)) != cudaSuccess) return r;
+    FFTPlanDev p9 = {}, p16 = {};  // FP64 x plans stop at radix 9, z plans may hold the larger ones
+    p16.npass = 1;
+    p16.radix[0] = 16;
+    if ((r = fft_generic_setup(dev, false, p9, p9)) != cudaSuccess) return r;
+    if ((r = fft_generic_setup(dev, false, p9, p16)) != cudaSuccess) return r;
     if ((r = cudaFuncSetAttribute(k_ysolve<double>, a, kNoallocSmemLimit)) != cudaSuccess) return r;
     g_noalloc_addr[dev] = p;
     return cudaSuccess;

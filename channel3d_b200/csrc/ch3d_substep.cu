@@ -6,6 +6,8 @@
 // Few partial sums are reduced by one block; many by CH3D_NRED blocks, the
 // last of which to finish sums the blocks' results in block order and does the
 // scalar work, so the result does not depend on the order the blocks run in.
+// Letting the projection's last block do this work instead, without a launch, took
+// 4 us more of the projection and 145 against 141 us per step at 64^3.
 #include "ch3d_march.cuh"
 
 namespace ch3d {

@@ -1,5 +1,5 @@
-"""The FP32 march of two columns per thread (channel3d_b200/csrc/ch3d_march2.cu:
-mixed path, grids whose march stops at g) at its edges, whole steps against the
+"""The FP32 march that stops at g (channel3d_b200/csrc/ch3d_march.cu, mixed path)
+at its edges, whole steps against the
 FP64 oracle within the mixed path's 1e-4: fewer rows than the march keeps in
 flight, ragged tiles in z, several and single rounds of the persistent blocks,
 and every x length with a register plan that the layout takes."""
