@@ -491,6 +491,7 @@ int init_scalars(ch3d_ctx* c) {
   DevScalars s;
   std::memset(&s, 0, sizeof(s));
   s.dt = c->cfg.dtMax;
+  s.ns = 1;  // the substep whose tables a stage reads before any set-up
   CU(cudaMemcpyAsync(c->sc, &s, sizeof(s), cudaMemcpyHostToDevice, c->stream));
   CU(launch_bulk_partials(c));
   CU(launch_diag(c));
@@ -866,10 +867,12 @@ int ch3d_stage(ch3d_ctx* c, int stage, int ns) {
       CU(launch_substep_setup(c, ns, false));
       break;
     case 1:
+      CU(launch_tables(c));
       if (c->cfg.LES_type > 0) CU(launch_rhs_les(c));
       else CU(c->cfg.order == 4 ? launch_rhs4(c) : launch_rhs(c));
       break;
     case 2:
+      CU(launch_tables(c));
       if (c->cfg.IsImplicit == 0) { CU(launch_uhat_fexp(c)); break; }
       if (c->cfg.LES_type > 0) { CU(launch_uhat_les(c)); break; }
       if (c->cfg.order == 2 && c->cfg.IsImplicit == 2) CU(launch_ptri_xz(c));

@@ -97,6 +97,7 @@ inline bool les_const(const ch3d_ctx* c) { return c->cfg.LES_type == CH3D_LES_ML
 // launchers (ch3d_step.cu)
 cudaError_t launch_substep_setup(ch3d_ctx* c, int ns, bool whole_step);  // whole_step: with the step's CFL and dt (ns 1)
                                                                          // and the reset of its maxima (last ns)
+cudaError_t launch_tables(ch3d_ctx* c);                // stage path: the coefficient tables of the current scalars
 cudaError_t launch_step_end(ch3d_ctx* c);
 cudaError_t launch_rhs(ch3d_ctx* c);                   // 2nd order: the scheme's right-hand sides -> RhsX/Y/Z
 cudaError_t launch_ustar_fexp(ch3d_ctx* c);            // explicit scheme: right-hand sides and u* in one pass

@@ -165,6 +165,39 @@ template <class T> struct TableArgs {
   unsigned long long* slots;  // pmBeta the tables of each substep hold (all ones: none)
 };
 
+// The tables of substep ns for pmBeta, by the whole block; left as they are when
+// they hold those already.  smem: 5 (ny + 1) values up to kStagedRows rows.
+template <class T>
+__device__ void update_tables(const TableArgs<T>& ta, int ns, double pmBeta, unsigned char* smem) {
+  const int q = ns - 1;
+  const unsigned long long bits = (unsigned long long)__double_as_longlong(pmBeta);
+  if (ta.slots[q] == bits) return;  // uniform: every thread reads it before thread 0 writes below
+  __syncthreads();
+  if (ta.pf && threadIdx.x >= 128 && (threadIdx.x & 31) == 0) {  // warps 4, 5, 6: the x, z and y blocks
+    const int d = (threadIdx.x >> 5) - 4;
+    const double r2 = d == 0 ? ta.r2x : d == 1 ? ta.r2z : d == 2 ? ta.r2y : 0.0;
+    double* F = ta.pf + (size_t)q * ptri_doubles(ta.nx, ta.ny, ta.nz);
+    if (r2 > 0.0)
+      update_ptri_block(d == 0 ? F : d == 1 ? F + ptri_stride(ta.nx) : F + ptri_stride(ta.nx) + ptri_stride(ta.nz),
+                        d == 0 ? ta.nx : d == 1 ? ta.nz : ta.ny, r2, pmBeta);
+  }
+  update_row_table(ta.hc, ta.m, ta.ny, ta.tab + (size_t)q * ta.ny * MT_W,
+                   ta.dtab ? ta.dtab + (size_t)q * ta.ny * MD_W : nullptr, pmBeta,
+                   ta.ny <= kStagedRows ? reinterpret_cast<double*>(smem) : nullptr);
+  __syncthreads();
+  if (threadIdx.x == 0) ta.slots[q] = bits;
+}
+
+// The tables that belong to the current scalars, for the stage entry points: a host
+// may call a stage whose substep's coefficients were never set up (after an upload
+// they are zero and ns is 1).
+template <class T>
+__global__ void __launch_bounds__(kSetupThreads) k_tables(const DevScalars* __restrict__ sc, TableArgs<T> ta) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  if (sc->status) return;
+  update_tables(ta, sc->ns, sc->pmBeta, smem_raw);
+}
+
 template <class T>
 __global__ void __launch_bounds__(kSetupThreads) k_substep(DevScalars* sc, const double* __restrict__ part, int npart,
                                                            double* __restrict__ red, SubstepPar p, TableArgs<T> ta) {
@@ -227,23 +260,7 @@ __global__ void __launch_bounds__(kSetupThreads) k_substep(DevScalars* sc, const
   }
   if (!ta.tab) return;
   __syncthreads();
-  const int q = p.ns - 1;
-  const unsigned long long bits = (unsigned long long)__double_as_longlong(beta);
-  if (ta.slots[q] == bits) return;  // uniform: every thread reads it before thread 0 writes below
-  __syncthreads();
-  if (ta.pf && threadIdx.x >= 128 && (threadIdx.x & 31) == 0) {  // warps 4, 5, 6: the x, z and y blocks
-    const int d = (threadIdx.x >> 5) - 4;
-    const double r2 = d == 0 ? ta.r2x : d == 1 ? ta.r2z : d == 2 ? ta.r2y : 0.0;
-    double* F = ta.pf + (size_t)q * ptri_doubles(ta.nx, ta.ny, ta.nz);
-    if (r2 > 0.0)
-      update_ptri_block(d == 0 ? F : d == 1 ? F + ptri_stride(ta.nx) : F + ptri_stride(ta.nx) + ptri_stride(ta.nz),
-                        d == 0 ? ta.nx : d == 1 ? ta.nz : ta.ny, r2, beta);
-  }
-  update_row_table(ta.hc, ta.m, ta.ny, ta.tab + (size_t)q * ta.ny * MT_W,
-                   ta.dtab ? ta.dtab + (size_t)q * ta.ny * MD_W : nullptr, beta,
-                   ta.ny <= kStagedRows ? reinterpret_cast<double*>(smem_raw) : nullptr);
-  __syncthreads();
-  if (threadIdx.x == 0) ta.slots[q] = bits;
+  update_tables(ta, p.ns, beta, smem_raw);
 }
 
 // src/CFD_2nd/m_ChannelSystem.f90:127-130 (limit checks after the step) and
@@ -301,18 +318,7 @@ cudaError_t launch_reduce_partials(ch3d_ctx* c, const double* in, int n, double*
 // One block up to 4096 partial sums, all in flight at once, else CH3D_NRED.
 static unsigned setup_blocks(int n) { return n <= kSumPer * kSetupThreads ? 1u : (unsigned)CH3D_NRED; }
 
-template <class T> static cudaError_t substep_t(ch3d_ctx* c, int ns, bool whole_step) {
-  SubstepPar p;
-  p.ns = ns;
-  p.begin = whole_step && ns == 1;
-  p.last = whole_step && ns == c->iadvance;
-  p.gam = c->gam[ns - 1]; p.the = c->the[ns - 1]; p.alp = c->alp[ns - 1];
-  p.iCFL = c->cfg.iCFL; p.IsUxConst = c->cfg.IsUxConst; p.order = c->cfg.order;
-  p.CFLc = c->cfg.CFLc; p.dtMax = c->cfg.dtMax; p.xnu = c->cfg.xnu; p.ubulk = c->cfg.ubulk;
-  p.norm_bulk = 1.0 / ((double)c->nx * (double)c->nz) / (c->cfg.ybulk2 - c->cfg.ybulk1);
-  p.nxnz = (double)(c->nx * c->nz);
-  p.yly = c->cfg.yly;
-  p.visc_wall = c->visc_wall;
+template <class T> static TableArgs<T> table_args(ch3d_ctx* c) {
   TableArgs<T> ta;
   ta.hc = helm_coef(c);
   ta.m = c->cfg.LES_type == 0 ? metrics_of<T>(c) : Metrics<T>();
@@ -328,15 +334,43 @@ template <class T> static cudaError_t substep_t(ch3d_ctx* c, int ns, bool whole_
   ta.r2y = y_periodic(c) ? c->rdy2 : 0.0;
   ta.dtab = ta.tab && ((c->march && !march_rows_path(c)) || c->cfg.order == 4) && march_twisted(c) ? march_down_tables<T>(c->mtab, c->ny) : nullptr;
   ta.slots = march_beta_slots(c->mtab, c->ny);
+  return ta;
+}
+template <class T> static size_t table_smem(const ch3d_ctx* c, const TableArgs<T>& ta) {
+  return ta.tab && c->ny <= kStagedRows ? (size_t)5 * (c->ny + 1) * sizeof(double) : 0;
+}
+
+template <class T> static cudaError_t substep_t(ch3d_ctx* c, int ns, bool whole_step) {
+  SubstepPar p;
+  p.ns = ns;
+  p.begin = whole_step && ns == 1;
+  p.last = whole_step && ns == c->iadvance;
+  p.gam = c->gam[ns - 1]; p.the = c->the[ns - 1]; p.alp = c->alp[ns - 1];
+  p.iCFL = c->cfg.iCFL; p.IsUxConst = c->cfg.IsUxConst; p.order = c->cfg.order;
+  p.CFLc = c->cfg.CFLc; p.dtMax = c->cfg.dtMax; p.xnu = c->cfg.xnu; p.ubulk = c->cfg.ubulk;
+  p.norm_bulk = 1.0 / ((double)c->nx * (double)c->nz) / (c->cfg.ybulk2 - c->cfg.ybulk1);
+  p.nxnz = (double)(c->nx * c->nz);
+  p.yly = c->cfg.yly;
+  p.visc_wall = c->visc_wall;
+  const TableArgs<T> ta = table_args<T>(c);
   // the partials of the bulk sums or of the mean viscous stress (the projection or k_bulk_march)
   const int np = c->npart_m;
-  const size_t smem = ta.tab && c->ny <= kStagedRows ? (size_t)5 * (c->ny + 1) * sizeof(double) : 0;
-  k_substep<T><<<setup_blocks(np), kSetupThreads, smem, c->stream>>>(c->sc, c->part, np, c->red1, p, ta);
+  k_substep<T><<<setup_blocks(np), kSetupThreads, table_smem(c, ta), c->stream>>>(c->sc, c->part, np, c->red1, p, ta);
   return cudaGetLastError();
 }
 cudaError_t launch_substep_setup(ch3d_ctx* c, int ns, bool whole_step) {
   // LES: FP64 coefficients on either field type
   return c->fp32 && c->cfg.LES_type == 0 ? substep_t<float>(c, ns, whole_step) : substep_t<double>(c, ns, whole_step);
+}
+
+template <class T> static cudaError_t tables_t(ch3d_ctx* c) {
+  const TableArgs<T> ta = table_args<T>(c);
+  if (!ta.tab) return cudaSuccess;
+  k_tables<T><<<1, kSetupThreads, table_smem(c, ta), c->stream>>>(c->sc, ta);
+  return cudaGetLastError();
+}
+cudaError_t launch_tables(ch3d_ctx* c) {
+  return c->fp32 && c->cfg.LES_type == 0 ? tables_t<float>(c) : tables_t<double>(c);
 }
 
 cudaError_t launch_step_end(ch3d_ctx* c) {

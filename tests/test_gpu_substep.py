@@ -79,3 +79,49 @@ def test_stages_after_steps(built):
         gs, go = s.download(), o.get_state()
     for k in ("ux", "uy", "uz"):
         assert rel_l2(gs[k], go[k]) < 1e-10, (k, rel_l2(gs[k], go[k]))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("scheme", ["wall", "adi", "4th", "explicit", "periodic", "periodic_adi", "les"])
+def test_stages_before_any_set_up(built, scheme, precision):
+    """Right-hand sides and solves called first, or after an array was set (both leave the
+    substep's coefficients zero): the right-hand sides are zero, Hist is the convective term
+    of the state, and the solves return u* = u + Rhs, exactly."""
+    from channel3d_b200 import ChannelSolver, initfield, mesh_y, workloads
+    if precision == "mixed" and scheme in ("explicit", "periodic", "periodic_adi"):
+        pytest.skip("periodic y runs in FP64")
+    shape = (36, 17, 18)
+    if scheme in ("explicit", "periodic"):
+        cfg = _cfg("periodic_adi", shape).copy(IsImplicit=0 if scheme == "explicit" else 1)
+    elif scheme == "les":
+        cfg, _ = workloads.get("channel48_les")
+        cfg = cfg.copy(nxc=36, nyc=17, nzc=18, nycSection=[8, 9], LES_type=2, Cs=0.1)
+    else:
+        cfg = _cfg(scheme, shape)
+    cfg = cfg.copy(precision=precision)
+    yp = mesh_y(cfg)
+    rng = np.random.default_rng(8)
+    f = [rng.standard_normal(cfg.shape).astype(np.float32).astype(np.float64) for _ in range(4)]
+    if cfg.BcOption[2] != 0:
+        f[1][:, 0, :] = 0.0
+    with ChannelSolver(cfg, yp=yp) as s, ChannelSolver(cfg, yp=yp) as ref:
+        s.upload(*f)
+        ref.upload(*f)
+        ref.stage(0, 1)
+        ref.stage(1, 1)
+        s.stage(1, 1)
+        for h in (s.HISTX, s.HISTY, s.HISTZ):
+            assert np.array_equal(s.get_array(h), ref.get_array(h)), h
+        for r in (s.RHSX, s.RHSY, s.RHSZ):
+            assert not s.get_array(r).any(), r
+        s.stage(0, 2)
+        rhs = [rng.standard_normal(cfg.shape).astype(np.float32).astype(np.float64) for _ in range(3)]
+        for q, r in zip((s.RHSX, s.RHSY, s.RHSZ), rhs):
+            s.set_array(q, r)
+        s.stage(2, 2)
+        if cfg.BcOption[2] != 0 and cfg.IsImplicit != 0:
+            rhs[1][:, 0, :] = 0.0  # the wall row of uy is held
+        word = np.float32 if precision == "mixed" else np.float64
+        for q in range(3):
+            want = f[q].astype(word) + rhs[q].astype(word)
+            assert np.array_equal(s.get_array(12 + q), want.astype(np.float64)), q
