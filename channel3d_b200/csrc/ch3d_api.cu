@@ -561,6 +561,14 @@ int build_graph(ch3d_ctx* c) {
   return CH3D_OK;
 }
 
+// the next step records anew
+void drop_graph(ch3d_ctx* c) {
+  if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
+  if (c->graph) cudaGraphDestroy(c->graph);
+  c->graph_exec = nullptr;
+  c->graph = nullptr;
+}
+
 int fetch_info(ch3d_ctx* c, ch3d_step_info* info) {
   DevScalars s;
   CU(cudaMemcpyAsync(&s, c->sc, sizeof(s), cudaMemcpyDeviceToHost, c->stream));
@@ -748,8 +756,7 @@ int ch3d_create(const ch3d_config* cfg, const double* yp, ch3d_ctx** out) {
 int ch3d_destroy(ch3d_ctx* c) {
   if (!c) return CH3D_OK;
   cudaSetDevice(c->device);
-  if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
-  if (c->graph) cudaGraphDestroy(c->graph);
+  drop_graph(c);
   for (int q = 0; q < 15; ++q) if (c->f[q]) cudaFree(c->f[q]);
   for (int q = 0; q < 6; ++q) if (c->ih[q]) cudaFree(c->ih[q]);
   if (c->pfac) cudaFree(c->pfac);
@@ -930,6 +937,13 @@ int ch3d_set_array(ch3d_ctx* c, int which, const double* host) {
                    : upload_field<double>(c, q, CH3D_LAYOUT_INTERIOR, host, q == 1 ? 1 : -1);
   if (rc) return rc;
   c->scalars_ready = false;
+  if (which == 10 && c->cfg.LES_type == CH3D_LES_MLP) {  // the constant-viscosity kernels hold for xnu only
+    bool set = false;
+    for (long long n = 0; n < c->N && !set; ++n)
+      set = c->fp32 ? (float)host[n] != (float)c->cfg.xnu : host[n] != c->cfg.xnu;
+    if (set != c->nut_set) drop_graph(c);
+    c->nut_set = set;
+  }
   return CH3D_OK;
 }
 
@@ -974,8 +988,7 @@ int ch3d_project(ch3d_ctx* c, double* divmax_before, double* divmax_after) {
 int ch3d_set_dt(ch3d_ctx* c, double dt) {
   if (!c || !(dt > 0)) return fail(CH3D_ERR_INVALID, "bad dt");
   c->cfg.dtMax = dt;
-  if (c->graph_exec) { cudaGraphExecDestroy(c->graph_exec); c->graph_exec = nullptr; }
-  if (c->graph) { cudaGraphDestroy(c->graph); c->graph = nullptr; }
+  drop_graph(c);
   CU(cudaMemcpyAsync(&c->sc->dt, &dt, sizeof(double), cudaMemcpyHostToDevice, c->stream));
   CU(cudaStreamSynchronize(c->stream));
   return CH3D_OK;
@@ -1103,8 +1116,7 @@ int ch3d_sgs_mlp_set(ch3d_ctx* c, const float* params, const float* norm) {
   CU(cudaStreamSynchronize(c->stream));
   std::memcpy(c->mlp_norm, norm, sizeof(c->mlp_norm));
   c->mlp_ready = true;
-  if (c->graph_exec) { cudaGraphExecDestroy(c->graph_exec); c->graph_exec = nullptr; }  // the norm is a kernel argument
-  if (c->graph) { cudaGraphDestroy(c->graph); c->graph = nullptr; }
+  drop_graph(c);  // the norm is a kernel argument
   return CH3D_OK;
 }
 

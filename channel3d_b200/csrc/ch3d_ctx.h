@@ -51,6 +51,7 @@ struct ch3d_ctx {
   double* yRM64 = nullptr;   // mixed path: FP64 factors of the low modes (kx < TSy, |kz| <= KL)
   double* ylow = nullptr;    // mixed path, columns beyond the chunked solve: FP64 sweep scratch of the low modes
   double* yA2 = nullptr;     // periodic y: the Poisson cyclic solve's closure vector per mode
+  bool nut_set = false;      // learned closure: the total viscosity is the host's, not xnu
   bool gsub = false;         // the march stops at g; divergence and projection substitute u*
   int KL = 8;
   int TSy = 8;               // kx extent of the FP64 low modes
@@ -92,8 +93,11 @@ namespace ch3d {
 
 // y periodic (BcOption(3:4) = 0): the triply periodic steps (FIMP_000, PIMP_0)
 inline bool y_periodic(const ch3d_ctx* c) { return c->cfg.BcOption[2] == 0; }
-// learned closure with the partially implicit step: the total viscosity is xnu everywhere
-inline bool les_const(const ch3d_ctx* c) { return c->cfg.LES_type == CH3D_LES_MLP && c->cfg.IsImplicit == 1; }
+// learned closure with the partially implicit step: the total viscosity is xnu everywhere,
+// unless the host has set another one (ch3d_set_array 10)
+inline bool les_const(const ch3d_ctx* c) {
+  return c->cfg.LES_type == CH3D_LES_MLP && c->cfg.IsImplicit == 1 && !c->nut_set;
+}
 // launchers (ch3d_step.cu)
 cudaError_t launch_substep_setup(ch3d_ctx* c, int ns, bool whole_step);  // whole_step: with the step's CFL and dt (ns 1)
                                                                          // and the reset of its maxima (last ns)

@@ -175,7 +175,9 @@ CH3D_API int ch3d_stage(ch3d_ctx* ctx, int stage, int ns);
    total viscosity of Clc_SGS_Vis, xnu included), 11 RhsZ, 12..14 the
    velocity after the Helmholtz solves (u*), 15..20 (CH3D_LES_MLP, read
    only) the SGS stresses tau_11 tau_12 tau_13 tau_22 tau_23 tau_33 at the
-   cell centres of the last ch3d_sgs_viscosity or step. */
+   cell centres of the last ch3d_sgs_viscosity or step.  Setting 10: an
+   eddy-viscosity model forms it anew in each step; with CH3D_LES_MLP (where
+   it is xnu) the steps keep what was set. */
 CH3D_API int ch3d_get_array(ch3d_ctx* ctx, int which, double* host);
 CH3D_API int ch3d_set_array(ch3d_ctx* ctx, int which, const double* host);
 

@@ -154,3 +154,49 @@ def test_learned_closure_mixed_precision(built):
     info = m.step(20)
     assert info["status"] == 0 and info["divmax2"] < 1e-4
     m.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_total_viscosity_set_by_the_host(built, precision):
+    """With a total viscosity set by the host (array 10, before any step and after recorded
+    ones), whole steps are the stages', and back at xnu those of a context that never had
+    another: FP64 1e-11 (max norm, as one step above); mixed 1e-5 (16 FP32 ulp of velocities
+    whose y derivatives enter with the viscosity)."""
+    from channel3d_b200 import ChannelSolver
+    from oracle import mlp_oracle as M
+    cfg = _cfg().copy(precision=precision)
+    tol = 1e-11 if precision == "fp64" else 1e-5
+    rng = np.random.default_rng(21)
+    nut = cfg.xnu * (1.0 + 20.0 * rng.random(cfg.shape))
+    _, a, yp, _ = _pair(cfg)
+    st = a.download()
+    solvers = [a] + [ChannelSolver(cfg, yp=yp) for _ in range(2)]
+    for s in solvers:
+        s.sgs_mlp_set(M.init_params(1), _norm(1e30, -1e30))
+    _, b, c = solvers
+
+    def restart(s, v):
+        s.upload(*(st[k] for k in ("ux", "uy", "uz", "p")))
+        if v is not None:
+            s.set_array(s.NUT, v)
+
+    for first in (True, False):  # nothing recorded yet; steps with xnu recorded
+        for s in (a, b):
+            restart(s, nut)
+        a.step(1)
+        b.sgs_viscosity()
+        for ns in (1, 2, 3):
+            for q in range(7):
+                b.stage(q, ns)
+        ga, gb = a.download(), b.download()
+        for k in ("ux", "uy", "uz"):
+            assert rel_max(ga[k], gb[k]) < tol, (first, k, rel_max(ga[k], gb[k]))
+        restart(a, np.full(cfg.shape, cfg.xnu))
+        restart(c, None)
+        a.step(3)
+        c.step(3)
+        ga, gc = a.download(), c.download()
+        for k in ("ux", "uy", "uz", "p"):
+            assert np.array_equal(ga[k], gc[k]), (first, k)
+    for s in solvers:
+        s.close()
