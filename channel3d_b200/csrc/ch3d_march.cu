@@ -24,8 +24,10 @@
 
 namespace ch3d {
 
-// Positions of a staged row of a 32 x BZ tile with a halo of H cells
-constexpr int march_pl(int H, int BZ) { return (32 + 2 * H) * (BZ + 2 * H); }
+// Staging geometry: x halo H rounded up to whole copy vectors of VW points, and
+// points per staged row of a 32 x BZ tile.
+constexpr int march_hx(int H, int VW) { return (H + VW - 1) / VW * VW; }
+constexpr int march_pl(int H, int VW, int BZ) { return (32 + 2 * march_hx(H, VW)) * (BZ + 2 * H); }
 
 // Shared memory of one thread group of the march: RS row slots of the four
 // staged fields (PL points each) and of the row table (MT_W values).
@@ -52,16 +54,25 @@ template <class T> constexpr size_t march_group_smem(int RS, int PL) {
 // u* = g - cp u*_{j+1} themselves while they walk each column downwards, so u*
 // is never stored and g is never read back here (6 arrays less traffic).
 //
-template <class T, bool O4, bool TW, bool BS, int BZ, int D, int RS>
+// VW: rows staged in copy vectors of VW elements, 4 (16-byte copies of FP32 rows, the
+// x halo rounded up to 4 points) where the FP32 march stops at g, which takes lines of
+// whole vectors only, else 1.  That march is bound by instruction issue, so a quarter of
+// the copy instructions and a sixth block per SM count: 2.08 ms per launch at 768x384x576
+// and 194 us at 256x192x256, element by element with five blocks 2.28 ms and 201 us (the
+// same bits).
+template <class T, bool O4, bool TW, bool BS, int VW, int BZ, int D, int RS>
 __global__ void __launch_bounds__(32 * BZ * (TW ? 2 : 1),
-                                  (O4 ? 384 : (sizeof(T) == 4 ? 640 : 512)) / (32 * BZ * (TW ? 2 : 1)))
+                                  VW == 4 ? 6 : (O4 ? 384 : (sizeof(T) == 4 ? 640 : 512)) / (32 * BZ * (TW ? 2 : 1)))
     k_rhs_march(Geo<T> g, const T* __restrict__ tab, const T* __restrict__ dtab, const T* __restrict__ ux, const T* __restrict__ uy,
                 const T* __restrict__ uz, const T* __restrict__ pr, T* __restrict__ hx, T* __restrict__ hy,
                 T* __restrict__ hz, T* __restrict__ uxs, T* __restrict__ uys, T* __restrict__ uzs,
                 const DevScalars* __restrict__ sc) {
   constexpr int H = O4 ? 3 : 1;  // x/z halo
-  constexpr int BX = 32, NT = BX * BZ, SX = BX + 2 * H, PL = march_pl(H, BZ);
-  constexpr int NS = (PL + NT - 1) / NT;  // staging slots per thread and array
+  constexpr int HX = march_hx(H, VW);  // staged x halo
+  constexpr int BX = 32, NT = BX * BZ, SX = BX + 2 * HX, PL = march_pl(H, VW, BZ);
+  constexpr int NS = (PL / VW + NT - 1) / NT;  // staging vectors per thread and array
+  static_assert(VW == 1 || (VW == 4 && sizeof(T) == 4), "16-byte vectors of FP32 rows only");
+  typedef typename std::conditional<VW == 4, float4, T>::type VT;
   static_assert(RS >= D + 4, "ring too small for the prefetch distance");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int hf = TW ? (int)threadIdx.x / NT : 0;  // thread group: 0 lower (or the only one), 1 upper
@@ -95,12 +106,12 @@ __global__ void __launch_bounds__(32 * BZ * (TW ? 2 : 1),
     const int sl = slot(r);
 #pragma unroll
     for (int q = 0; q < NS; ++q) {
-      const int s = tid + q * NT;
+      const int s = (tid + q * NT) * VW;
       if (s < PL) {
-        cp_async_el(&ring[0][sl][s], ux + so[q] + ro);
-        cp_async_el(&ring[1][sl][s], uy + so[q] + ro);
-        cp_async_el(&ring[2][sl][s], uz + so[q] + ro);
-        cp_async_el(&ring[3][sl][s], pr + so[q] + ro);
+        cp_async_el(reinterpret_cast<VT*>(&ring[0][sl][s]), reinterpret_cast<const VT*>(ux + so[q] + ro));
+        cp_async_el(reinterpret_cast<VT*>(&ring[1][sl][s]), reinterpret_cast<const VT*>(uy + so[q] + ro));
+        cp_async_el(reinterpret_cast<VT*>(&ring[2][sl][s]), reinterpret_cast<const VT*>(uz + so[q] + ro));
+        cp_async_el(reinterpret_cast<VT*>(&ring[3][sl][s]), reinterpret_cast<const VT*>(pr + so[q] + ro));
       }
     }
     // the row's table entries (MT_W values, 16-byte copies) in the same copy group
@@ -112,8 +123,8 @@ __global__ void __launch_bounds__(32 * BZ * (TW ? 2 : 1),
   auto ghost_row = [&](int r) {
     const int sl = slot(r);
 #pragma unroll
-    for (int q = 0; q < NS; ++q) {
-      const int s = tid + q * NT;
+    for (int qv = 0; qv < NS * VW; ++qv) {  // the elements of this thread's staging vectors
+      const int s = (tid + (qv / VW) * NT) * VW + qv % VW;
       if (s >= PL) continue;
       if (r < 0) {
         const T u = ring[0][slot(0)][s], w = ring[2][slot(0)][s], v1 = ring[1][slot(1)][s];
@@ -137,7 +148,7 @@ __global__ void __launch_bounds__(32 * BZ * (TW ? 2 : 1),
   const T rdx = g.rdx, rdz = g.rdz, rdx2 = g.rdx2, rdz2 = g.rdz2, xnu = g.xnu;
   const T pmGamma = (T)sc->pmGamma, pmTheta = (T)sc->pmTheta, pmAlpha = (T)sc->pmAlpha, pmBeta = (T)sc->pmBeta;
   const T dpm = (T)sc->dpmdxns;
-  const int c0 = (tz + H) * SX + tx + H;
+  const int c0 = (tz + H) * SX + tx + HX;
   const int ntx = (nx + BX - 1) / BX, ntiles = ntx * ((nz + BZ - 1) / BZ);
 
   // Persistent blocks walk tiles of 32 x BZ columns.  The back substitution of
@@ -153,8 +164,8 @@ __global__ void __launch_bounds__(32 * BZ * (TW ? 2 : 1),
   // staging slots: s = tid + q NT -> halo-tile position (s % SX, s / SX), periodic in x and z
 #pragma unroll
   for (int q = 0; q < NS; ++q) {
-    const int s = tid + q * NT;
-    int ig = (i0 - H + s % SX) % nx, kg = (k0 - H + s / SX) % nz;
+    const int s = (tid + q * NT) * VW;  // a vector never wraps: nx and i0 - HX are multiples of VW
+    int ig = (i0 - HX + s % SX) % nx, kg = (k0 - H + s / SX) % nz;
     if (ig < 0) ig += nx;
     if (kg < 0) kg += nz;
     so[q] = s < PL ? ig + plane * kg : 0;
@@ -961,15 +972,19 @@ cudaError_t launch_proj_bsub(ch3d_ctx* c, bool diag) {
 // two-group blocks.
 template <class T, bool O4> struct MarchShape {
   static constexpr int BZ = 4, D = sizeof(T) == 8 ? 2 : 4, RS = D + 4;
-  static constexpr int bps = sizeof(T) == 8 ? 4 : 5;  // resident blocks per SM of the 2nd-order kernel
-  static constexpr int H = O4 ? 3 : 1, PL = march_pl(H, BZ);
-  static constexpr size_t smem = march_group_smem<T>(RS, PL);
+  // resident blocks per SM of the 2nd-order kernel
+  static constexpr int bps(bool stops_at_g) { return sizeof(T) == 8 ? 4 : (stops_at_g ? 6 : 5); }
+  static constexpr int H = O4 ? 3 : 1;
+  static constexpr size_t smem = march_group_smem<T>(RS, march_pl(H, 1, BZ));
+  // the march that stops at g (lines of multiples of 128 points): copy vectors
+  static constexpr int GW = sizeof(T) == 4 ? 4 : 1;
+  static constexpr size_t smem_g = march_group_smem<T>(RS, march_pl(H, GW, BZ));
 };
 template <class T, bool O4> static bool march_twisted_t(const ch3d_ctx* c) {
   typedef MarchShape<T, O4> S;
   static PerDevice site;                  // per instance: the twisted kernel's limit and occupancy
   static int occ_dev[kMaxDevices] = {};   // twisted blocks per SM, written once per device under the set-up lock
-  auto kern_tw = k_rhs_march<T, O4, true, true, S::BZ, S::D, S::RS>;
+  auto kern_tw = k_rhs_march<T, O4, true, true, 1, S::BZ, S::D, S::RS>;
   const cudaError_t e = once_per_device(site, c->device, [&] {
     cudaError_t r = cudaFuncSetAttribute(kern_tw, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * S::smem));
     if (r != cudaSuccess) return r;
@@ -993,15 +1008,15 @@ template <class T, bool O4> static cudaError_t rhs_march_t(ch3d_ctx* c) {
   constexpr int BZ = S::BZ, D = S::D, RS = S::RS;
   const size_t smem = S::smem;
   T** f = (T**)c->f;
-  auto kern = k_rhs_march<T, O4, false, true, BZ, D, RS>;
-  auto kern_tw = k_rhs_march<T, O4, true, true, BZ, D, RS>;
+  auto kern = k_rhs_march<T, O4, false, true, 1, BZ, D, RS>;
+  auto kern_tw = k_rhs_march<T, O4, true, true, 1, BZ, D, RS>;
   const bool tw = march_twisted_t<T, O4>(c);  // also sets the twisted kernel's shared-memory limit
   static PerDevice site;  // per instance: the one-directional kernels' limits
   cudaError_t e = once_per_device(site, c->device, [&] {
     const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
     cudaError_t r = cudaFuncSetAttribute(kern, a, (int)smem);
     if constexpr (!O4) {
-      if (r == cudaSuccess) r = cudaFuncSetAttribute(k_rhs_march<T, O4, false, false, BZ, D, RS>, a, (int)smem);
+      if (r == cudaSuccess) r = cudaFuncSetAttribute(k_rhs_march<T, O4, false, false, S::GW, BZ, D, RS>, a, (int)S::smem_g);
     }
     return r;
   });
@@ -1018,12 +1033,12 @@ template <class T, bool O4> static cudaError_t rhs_march_t(ch3d_ctx* c) {
   } else {
     // 2nd order: persistent blocks (back substitution, if any, overlapped with the next
     // tile's march); 4th order: one tile per block
-    const long long cap = !O4 ? (long long)nsm * S::bps : ntiles;
+    const long long cap = !O4 ? (long long)nsm * S::bps(c->gsub) : ntiles;
     const unsigned grid = (unsigned)(ntiles < cap ? ntiles : cap);
     bool done = false;
     if constexpr (!O4) {
       if (c->gsub) {  // stops at g: the divergence and projection marches substitute
-        args(k_rhs_march<T, O4, false, false, BZ, D, RS>, grid, 32 * BZ, smem);
+        args(k_rhs_march<T, O4, false, false, S::GW, BZ, D, RS>, grid, 32 * BZ, S::smem_g);
         done = true;
       }
     }

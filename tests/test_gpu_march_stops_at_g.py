@@ -1,18 +1,23 @@
 """The FP32 march that stops at g (channel3d_b200/csrc/ch3d_march.cu, mixed path)
-at its edges, whole steps against the
-FP64 oracle within the mixed path's 1e-4: fewer rows than the march keeps in
-flight, ragged tiles in z, several and single rounds of the persistent blocks,
-and every x length with a register plan that the layout takes."""
+at its edges, whole steps against the FP64 oracle: fewer rows than the march keeps
+in flight, ragged tiles in z, several and single rounds of the persistent blocks,
+and every x length with a register plan that the layout takes.
+
+Tolerance: velocities within the mixed path's 1e-4.  Pressure: u* is rounded to
+FP32, and a rounding of eps U from cell to cell is corrected by a pressure
+difference of eps U dx / (alpha dt) over the substep, alpha >= 2/15; that over the
+pressure's rms (4e-3 to 4e-2 here, measured 3e-4 to 8e-4)."""
 import numpy as np
 import pytest
 
 from helpers import rel_l2, small_channel
 
 pytestmark = pytest.mark.gpu
+EPS32 = np.finfo(np.float32).eps
 
 
 @pytest.mark.parametrize("shape", [(768, 4, 162), (768, 5, 216), (512, 9, 243), (256, 33, 486), (128, 8, 972)])
-def test_two_column_march(built, shape):
+def test_march_stops_at_g(built, shape):
     from channel3d_b200 import ChannelSolver, initfield, mesh_y
     from oracle import oracle as O
     cfg = small_channel(*shape, precision="mixed")
@@ -30,3 +35,5 @@ def test_two_column_march(built, shape):
     go = o.get_state()
     for k in ("ux", "uy", "uz"):
         assert rel_l2(gs[k], go[k]) < 1e-4, (k, rel_l2(gs[k], go[k]))
+    ptol = EPS32 * np.abs(go["ux"]).max() * cfg.xlx / cfg.nxc / (2 / 15 * cfg.dtMax) / np.sqrt(np.mean(go["p"] ** 2))
+    assert rel_l2(gs["p"], go["p"]) < ptol, (rel_l2(gs["p"], go["p"]), ptol)
