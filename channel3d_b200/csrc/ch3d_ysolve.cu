@@ -329,77 +329,72 @@ __device__ __forceinline__ void thomas_column(int ny, bool pin, const R* __restr
   }
   store(ny - 1, dx, dy);
   for (int j1 = ny - 2; j1 >= 0; j1 -= YB) {
-    R ex[YB], ey[YB], c[YB];
+    R ex[YB], ey[YB], r[YB], c[YB];
 #pragma unroll
     for (int u = 0; u < YB; ++u) {
       const int j = j1 - u;
       if (j >= 0) {
         const CT v = load_d(j);
         ex[u] = (R)v.x; ey[u] = (R)v.y;
-        c[u] = pin && j == 0 ? (R)0 : (R)__ldg(ap + j + 1) * __ldg(rm + fst * j);
+        r[u] = __ldg(rm + fst * j);  // multiplied below: the product here waits for each row's loads (32x1024x32 397 us, 228)
+        c[u] = (R)__ldg(ap + j + 1);
       }
     }
 #pragma unroll
     for (int u = 0; u < YB; ++u) {
       const int j = j1 - u;
       if (j >= 0) {
-        dx = ex[u] - c[u] * dx;
-        dy = ey[u] - c[u] * dy;
+        const R cp = pin && j == 0 ? (R)0 : c[u] * r[u];
+        dx = ex[u] - cp * dx;
+        dy = ey[u] - cp * dy;
         store(j, dx, dy);
       }
     }
   }
 }
 
-// All columns in the precision of the field (FP64 path), or in the mixed
-// path the FP32 columns: the low modes kx < KX, |kz| <= KL are skipped
-// (KX = 0: none) and solved by k_ythomas_low.
+// All columns in the precision of the field; in the mixed path the blocks from nhi on
+// solve the low modes kx < KX, |kz| <= KL (column zi = kz for kz <= KL, KL + nz - kz
+// above) in FP64 beside the FP32 columns, their forward sweep kept in the FP64 scratch
+// scr, [j][low column].  With both z transforms 384 us for 32x800x32 mixed, 857 with the
+// low modes in a launch before the others.
 template <class T>
 __global__ void __launch_bounds__(128) k_ythomas(Geo<T> g, Metrics<double> m, const T* __restrict__ RMf,
-                                                 typename CplxOf<T>::type* __restrict__ spec, int KL, int KX,
-                                                 const DevScalars* __restrict__ sc) {
+                                                 typename CplxOf<T>::type* __restrict__ spec, int nhi,
+                                                 const double* __restrict__ RM64, double2* __restrict__ scr, int KL,
+                                                 int KX, const DevScalars* __restrict__ sc) {
   typedef typename CplxOf<T>::type CT;
   if (sc->status) return;
   const int nxh = g.nxh, ny = g.ny, nz = g.nz;
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)nxh * nz) return;
-  const int kx = (int)(t % nxh), kz = (int)(t / nxh);
-  const int kzh = kz <= nz - kz ? kz : nz - kz;
-  if (kx < KX && kzh <= KL) return;
   const size_t st = (size_t)nxh;
-  CT* col = spec + kx + st * ny * kz;
-  auto load = [&](int j) { return col[st * j]; };
-  auto store = [&](int j, T x, T y) { col[st * j] = mk(x, y); };
-  thomas_column<T, CT, 16>(ny, kx == 0 && kz == 0, RMf + (size_t)kzh * ny * st + kx, st, m.am2Pr, m.ap2Pr, load, store,
-                           store, load);
-}
-
-// Mixed path: the low modes kx < KX, |kz| <= KL (column zi = kz for kz <= KL,
-// KL + nz - kz above) in FP64 with FP64 factors, their forward sweep kept in
-// the FP64 scratch [j][low column].
-__global__ void __launch_bounds__(128) k_ythomas_low(Geo<float> g, Metrics<double> m, const double* __restrict__ RM64,
-                                                     float2* __restrict__ spec, double2* __restrict__ scr, int KL,
-                                                     int KX, const DevScalars* __restrict__ sc) {
-  typedef float T;
-  typedef float2 CT;
-  if (sc->status) return;
-  const int nxh = g.nxh, ny = g.ny, nz = g.nz;
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= (2 * KL + 1) * KX) return;
-  const int zi = q / KX, kx = q - zi * KX;
-  const int kz = zi <= KL ? zi : nz - (zi - KL);
-  if (kx >= nxh || (zi > KL && kz <= KL)) return;
-  const int kzh = kz <= nz - kz ? kz : nz - kz;
-  const size_t st = (size_t)nxh;
-  CT* col = spec + kx + st * ny * kz;
-  const size_t nlow = (size_t)(2 * KL + 1) * KX;
-  double2* w = scr + (size_t)zi * KX + kx;  // [j][low column]
-  auto load = [&](int j) { const CT v = col[st * j]; return make_double2(v.x, v.y); };
-  auto store = [&](int j, double x, double y) { col[st * j] = mk((T)x, (T)y); };
-  auto store_d = [&](int j, double x, double y) { w[nlow * j] = make_double2(x, y); };
-  auto load_d = [&](int j) { return w[nlow * j]; };
-  thomas_column<double, double2, 16>(ny, kx == 0 && kz == 0, RM64 + (size_t)kzh * ny * KX + kx, (size_t)KX, m.am2Pr,
-                                     m.ap2Pr, load, store, store_d, load_d);
+  if (sizeof(T) == 8 || (int)blockIdx.x < nhi) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (long long)nxh * nz) return;
+    const int kx = (int)(t % nxh), kz = (int)(t / nxh);
+    const int kzh = kz <= nz - kz ? kz : nz - kz;
+    if (sizeof(T) == 4 && kx < KX && kzh <= KL) return;
+    CT* col = spec + kx + st * ny * kz;
+    auto load = [&](int j) { return col[st * j]; };
+    auto store = [&](int j, T x, T y) { col[st * j] = mk(x, y); };
+    thomas_column<T, CT, 16>(ny, kx == 0 && kz == 0, RMf + (size_t)kzh * ny * st + kx, st, m.am2Pr, m.ap2Pr, load,
+                             store, store, load);
+  } else if constexpr (sizeof(T) == 4) {
+    const int q = ((int)blockIdx.x - nhi) * blockDim.x + threadIdx.x;
+    if (q >= (2 * KL + 1) * KX) return;
+    const int zi = q / KX, kx = q - zi * KX;
+    const int kz = zi <= KL ? zi : nz - (zi - KL);
+    if (kx >= nxh || (zi > KL && kz <= KL)) return;
+    const int kzh = kz <= nz - kz ? kz : nz - kz;
+    CT* col = spec + kx + st * ny * kz;
+    const size_t nlow = (size_t)(2 * KL + 1) * KX;
+    double2* w = scr + (size_t)zi * KX + kx;  // [j][low column]
+    auto load = [&](int j) { const CT v = col[st * j]; return make_double2(v.x, v.y); };
+    auto store = [&](int j, double x, double y) { col[st * j] = mk((T)x, (T)y); };
+    auto store_d = [&](int j, double x, double y) { w[nlow * j] = make_double2(x, y); };
+    auto load_d = [&](int j) { return w[nlow * j]; };
+    thomas_column<double, double2, 16>(ny, kx == 0 && kz == 0, RM64 + (size_t)kzh * ny * KX + kx, (size_t)KX, m.am2Pr,
+                                       m.ap2Pr, load, store, store_d, load_d);
+  }
 }
 
 // One thread per (kx, kz) column of the (kx, j, kz) spectrum (kx fastest, so
@@ -543,15 +538,12 @@ cudaError_t launch_ysolve(ch3d_ctx* c) {
                                                      (const double*)c->yCP, c->yA2, (double2*)c->spec, c->sc);
   } else if (!c->fp32) {
     k_ythomas<double><<<gy, 128, 0, c->stream>>>(make_geo<double>(c), c->m64full, (const double*)c->yRM,
-                                                 (double2*)c->spec, 0, 0, c->sc);
+                                                 (double2*)c->spec, (int)gy, nullptr, nullptr, 0, 0, c->sc);
   } else {
     const int nlow = (2 * c->KL + 1) * c->TSy;
-    k_ythomas_low<<<(nlow + 127) / 128, 128, 0, c->stream>>>(make_geo<float>(c), c->m64full, c->yRM64,
-                                                             (float2*)c->spec, (double2*)c->ylow, c->KL, c->TSy, c->sc);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    k_ythomas<float><<<gy, 128, 0, c->stream>>>(make_geo<float>(c), c->m64full, (const float*)c->yRM,
-                                                (float2*)c->spec, c->KL, c->TSy, c->sc);
+    k_ythomas<float><<<gy + (nlow + 127) / 128, 128, 0, c->stream>>>(
+        make_geo<float>(c), c->m64full, (const float*)c->yRM, (float2*)c->spec, (int)gy, c->yRM64, (double2*)c->ylow,
+        c->KL, c->TSy, c->sc);
   }
   return cudaGetLastError();
 }
