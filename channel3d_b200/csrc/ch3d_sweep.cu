@@ -369,21 +369,26 @@ __global__ void __launch_bounds__(128) k_sweep_long(SweepArgs<T> A, int ni, long
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-constexpr int kSweepMaxRows = 768;  // 32 chunks of 24 rows
+constexpr int kSweepXMax = 768;      // points of a line held by a warp, 24 per lane
+constexpr int kSweepMaxRows = 6144;  // 256 chunks of 24 rows
 
 template <class T> static SweepArgs<T> sweep_args(const ch3d_ctx* c) {
   T** f = (T**)c->f;
   return {f[7], f[8], f[9], f[0], f[1], f[2], f[12], f[13], f[14]};
 }
 
-// rows of length n at stride rs, `no` line sets at stride os
+// rows of length n at stride rs, `no` sets of ni lines at stride os.  Up to 768 rows a
+// block's 8 or 16 lines fill whole 32-byte sectors of both precisions; longer lines take
+// the chunks of 4, 2 or 1 lines a block of 256 threads can hold.  ADI's x and z sweeps at
+// 1024x32x32 60 us together and at 32x32x1024 93 (one thread per line 500 and 450), all
+// solves of 32x1024x32 85 us (one thread per line 890).
 template <class T, class R, bool PER, bool ADDU>
-static cudaError_t sweep_rows(ch3d_ctx* c, int n, long long rs, long long os, int no, const double* pf, int addp) {
+static cudaError_t sweep_rows(ch3d_ctx* c, int ni, int n, long long rs, long long os, int no, const double* pf, int addp) {
   const SweepArgs<T> A = sweep_args<T>(c);
   const R* tab = (const R*)c->mtab;
   const size_t pfs = ptri_doubles(c->nx, c->ny, c->nz);
   if (n > kSweepMaxRows) {
-    k_sweep_long<T, R, PER, ADDU><<<dim3((c->nx + 127) / 128, no < 65535 ? no : 65535, 3), 128, 0, c->stream>>>(A, c->nx, 1, n, rs, os, no, pf, pfs, tab, addp, c->sc);
+    k_sweep_long<T, R, PER, ADDU><<<dim3((ni + 127) / 128, no < 65535 ? no : 65535, 3), 128, 0, c->stream>>>(A, ni, 1, n, rs, os, no, pf, pfs, tab, addp, c->sc);
     return cudaGetLastError();
   }
   cudaError_t err = cudaSuccess;
@@ -393,29 +398,35 @@ static cudaError_t sweep_rows(ch3d_ctx* c, int n, long long rs, long long os, in
     const size_t smem = sweep_scan_bytes<R>(nw, C) + row * threads;
     err = smem_limit_once(site, c->device, kern, sweep_scan_bytes<R>(maxt / 32, C) + row * maxt);
     if (err != cudaSuccess) return;
-    const int gx = (c->nx + C - 1) / C;
+    const int gx = (ni + C - 1) / C;
     // a few line sets per block, so that their coefficients are formed once, while the GPU stays full
     const long long want = (long long)sm_count(c->device) * (2048 / threads > 0 ? 2048 / threads : 1);
     long long gy = (want + 3LL * gx - 1) / (3LL * gx);
     if (gy > no) gy = no;
     if (gy < 1) gy = 1;
-    kern<<<dim3(gx, (unsigned)gy, 3), threads, smem, c->stream>>>(A, c->nx, n, rs, os, no, pf, pfs, tab, addp, c->sc);
+    if (gy > 65535) gy = 65535;
+    kern<<<dim3(gx, (unsigned)gy, 3), threads, smem, c->stream>>>(A, ni, n, rs, os, no, pf, pfs, tab, addp, c->sc);
   };
-  static PerDevice s8, s8w, s12, s24;  // per template instance
+  static PerDevice s8, s8w, s12, s24, s4, s2, s1, sx;  // per template instance
+  if constexpr (PER && !ADDU)  // lines along x: one line a block, consecutive points
+    if (ni == 1 && n <= 2048) {
+      go(k_sweep<T, R, 1, 8, 256, 2, PER, ADDU>, sx, 1, 8, 256);
+      return err != cudaSuccess ? err : cudaGetLastError();
+    }
   if (n <= 128) go(k_sweep<T, R, 16, 8, 256, 2, PER, ADDU>, s8, 16, 8, 256);
   else if (n <= 256) go(k_sweep<T, R, 8, 8, 256, 2, PER, ADDU>, s8w, 8, 8, 256);
   else if (n <= 384) go(k_sweep<T, R, 8, 12, 256, 1, PER, ADDU>, s12, 8, 12, 256);
-  else go(k_sweep<T, R, 8, 24, 256, 1, PER, ADDU>, s24, 8, 24, 256);
+  else if (n <= 768) go(k_sweep<T, R, 8, 24, 256, 1, PER, ADDU>, s24, 8, 24, 256);
+  else if (n <= 1536) go(k_sweep<T, R, 4, 24, 256, 1, PER, ADDU>, s4, 4, 24, 256);
+  else if (n <= 3072) go(k_sweep<T, R, 2, 24, 256, 1, PER, ADDU>, s2, 2, 24, 256);
+  else go(k_sweep<T, R, 1, 24, 256, 1, PER, ADDU>, s1, 1, 24, 256);
   return err != cudaSuccess ? err : cudaGetLastError();
 }
 
 template <class T> static cudaError_t sweep_x(ch3d_ctx* c, const double* pf) {
   T** f = (T**)c->f;
   const long long nlines = (long long)c->ny * c->nz;
-  if (c->nx > kSweepMaxRows) {
-    k_sweep_long<T, T, true, false><<<dim3((c->ny + 127) / 128, c->nz < 65535 ? c->nz : 65535, 3), 128, 0, c->stream>>>(sweep_args<T>(c), c->ny, c->nx, c->nx, 1, (long long)c->nx * c->ny, c->nz, pf, ptri_doubles(c->nx, c->ny, c->nz), (const T*)nullptr, 0, c->sc);
-    return cudaGetLastError();
-  }
+  if (c->nx > kSweepXMax) return sweep_rows<T, T, true, false>(c, 1, c->nx, 1, c->nx, (int)nlines, pf, 0);
   const long long nb = (nlines + 3) / 4, cap = (long long)sm_count(c->device) * 6;
   const dim3 grid((unsigned)(nb < cap ? nb : cap), 3);
   auto go = [&](auto kern) { kern<<<grid, 128, 0, c->stream>>>(c->nx, nlines, pf, ptri_doubles(c->nx, c->ny, c->nz), f[7], f[8], f[9], c->sc); };
@@ -430,21 +441,21 @@ template <class T> static cudaError_t sweep_x(ch3d_ctx* c, const double* pf) {
 template <class T> static cudaError_t ptri_xz_t(ch3d_ctx* c) {
   const cudaError_t e = sweep_x<T>(c, ptri_block(c, 0));
   if (e != cudaSuccess) return e;
-  return sweep_rows<T, T, true, false>(c, c->nz, (long long)c->nx * c->ny, c->nx, c->ny, ptri_block(c, 1), 0);
+  return sweep_rows<T, T, true, false>(c, c->nx, c->nz, (long long)c->nx * c->ny, c->nx, c->ny, ptri_block(c, 1), 0);
 }
 cudaError_t launch_ptri_xz(ch3d_ctx* c) { return c->fp32 ? ptri_xz_t<float>(c) : ptri_xz_t<double>(c); }
 
 // periodic y: u* = u + solution; the partially implicit RhsX gets the mean
 // pressure gradient first (clcRhsX_PIMP adds it; the FIMP RhsX carries it already)
 template <class T> static cudaError_t ptri_y_t(ch3d_ctx* c) {
-  return sweep_rows<T, T, true, true>(c, c->ny, c->nx, (long long)c->nx * c->ny, c->nz, ptri_block(c, 2),
+  return sweep_rows<T, T, true, true>(c, c->nx, c->ny, c->nx, (long long)c->nx * c->ny, c->nz, ptri_block(c, 2),
                                    c->cfg.IsImplicit == 1);
 }
 cudaError_t launch_ptri_y(ch3d_ctx* c) { return c->fp32 ? ptri_y_t<float>(c) : ptri_y_t<double>(c); }
 
 // y between walls: u* = u + solution; the 4th-order, FIMP and LES RhsX already carry the forcing
 template <class T, class R> static cudaError_t uhat_t(ch3d_ctx* c) {
-  return sweep_rows<T, R, false, true>(c, c->ny, c->nx, (long long)c->nx * c->ny, c->nz, nullptr,
+  return sweep_rows<T, R, false, true>(c, c->nx, c->ny, c->nx, (long long)c->nx * c->ny, c->nz, nullptr,
                                        c->cfg.order != 4 && c->cfg.IsImplicit != 2 && c->cfg.LES_type == 0);
 }
 cudaError_t launch_uhat(ch3d_ctx* c) {

@@ -3,8 +3,9 @@ line solves that follow them (ch3d_sweep.cu), whole steps against the oracle:
 
 - ny at the edges of the chunks (8, 16, 32 rows) and of the march's ring, ragged
   tiles in x and z, walls and periodic y, the three implicit schemes;
-- sweep lengths at the edges of their forms: 64, 128, 256, 384, 768 points of an x
-  line, 128, 256, 384, 768 rows of a z or y line, and one thread per line beyond;
+- sweep lengths at the edges of their forms: 64, 128, 256, 384, 768, 2048, 6144 points
+  of an x line, 128, 256, 384, 768, 1536, 3072, 6144 rows of a z or y line, and one
+  thread per line beyond;
 - grids with more columns than the rows take, where the march runs twisted
   (18432 columns, 160 tiles), FP64 and mixed.
 
@@ -95,3 +96,24 @@ def test_sweep_lengths_y(built, ny, periodic):
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 def test_twisted_march_above_the_rows(built, precision):
     _check(small_channel(144, 25, 128, precision=precision), mixed=precision == "mixed")
+
+
+@pytest.mark.parametrize("shape", [(2048, 4, 4), (2304, 5, 6), (6144, 4, 4), (6912, 4, 4), (8, 5, 1536), (8, 5, 1728),
+                                   (6, 4, 3456)])
+def test_long_sweeps_xz(built, shape):
+    _check(_fimp(*shape), 1)
+
+
+@pytest.mark.parametrize("ny", [1000, 1536, 1537, 3072, 3073, 6144, 6145])
+@pytest.mark.parametrize("scheme", ["wall", "adi", "periodic", "periodic_adi"])
+def test_long_sweeps_y(built, scheme, ny):
+    if scheme.startswith("periodic"):
+        cfg = _periodic(18, ny, 6, 2 if scheme == "periodic_adi" else 1)
+    else:
+        cfg = small_channel(18, ny, 6) if scheme == "wall" else _fimp(18, ny, 6)
+    _check(cfg.copy(dtMax=cfg.dtMax * 769 / ny), 1)  # the convective limit of a shorter cell
+
+
+def test_long_sweeps_y_mixed(built):
+    cfg = small_channel(18, 1537, 6, precision="mixed")
+    _check(cfg.copy(dtMax=cfg.dtMax / 2), 1, mixed=True)
