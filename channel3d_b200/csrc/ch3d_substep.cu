@@ -68,63 +68,37 @@ struct SubstepPar {
   double CFLc, dtMax, xnu, ubulk, norm_bulk, nxnz, yly, visc_wall;
 };
 
-// Elimination factors of the row table for pmBeta (see ch3d_march.cuh), one
-// thread per Helmholtz set and direction, sequential in j; skipped when the
-// table already holds those of this pmBeta (constant dt).  The coefficient
-// vectors come through shared memory (co, 5 (ny + 1) values) where they fit: read
-// from global memory row by row they cost 49 us at 64 rows.
+// Elimination factors of the row table for pmBeta (see ch3d_march.cuh) of one
+// Helmholtz set, upwards: a, 1/m, c/m
 template <class T>
-__device__ void update_row_table(const HelmCoef& hg, const Metrics<T>& m, int ny, T* __restrict__ tab,
-                                 T* __restrict__ dtab, double pmBeta, double* co) {
-  HelmCoef hc = hg;
-  if (co) {
-    const double* src[5] = {hg.ap2cForCN, hg.am2cForCN, hg.ap2p, hg.ac2p, hg.am2p};
-    const double** dst[5] = {&hc.ap2cForCN, &hc.am2cForCN, &hc.ap2p, &hc.ac2p, &hc.am2p};
-    for (int v = 0; v < 5; ++v) {
-      double* o = co + (size_t)v * (ny + 1);
-      for (int q = threadIdx.x; q <= ny; q += blockDim.x) o[q] = src[v][q];
-      *dst[v] = o;
-    }
-    __syncthreads();
+__device__ void update_row_factors(const HelmCoef& hc, int set, int ny, double pmBeta, T* __restrict__ tab) {
+  T* col = tab + (set ? MT_A1 : MT_A0);
+  double cpp = 0.0;
+  for (int j = 0; j < ny; ++j) {
+    double a, b, c;
+    helm_abc(hc, set, pmBeta, j, a, b, c);
+    const double rm = 1.0 / (j == 0 ? b : b - a * cpp);
+    const double cp = c * rm;
+    col[(size_t)j * MT_W + 0] = (T)a;
+    col[(size_t)j * MT_W + 1] = (T)rm;
+    col[(size_t)j * MT_W + 2] = j == ny - 1 ? (T)0 : (T)cp;
+    cpp = cp;
   }
-  const int who = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0 && who < 4) {
-    const int set = who & 1;
-    if (who < 2) {  // upwards: a, 1/m, c/m
-      T* col = tab + (set ? MT_A1 : MT_A0);
-      double cpp = 0.0;
-      for (int j = 0; j < ny; ++j) {
-        double a, b, c;
-        helm_abc(hc, set, pmBeta, j, a, b, c);
-        const double rm = 1.0 / (j == 0 ? b : b - a * cpp);
-        const double cp = c * rm;
-        col[(size_t)j * MT_W + 0] = (T)a;
-        col[(size_t)j * MT_W + 1] = (T)rm;
-        col[(size_t)j * MT_W + 2] = j == ny - 1 ? (T)0 : (T)cp;
-        cpp = cp;
-      }
-    } else if (dtab) {  // downwards (twisted march): c, 1/m', a/m'
-      T* col = dtab + (set ? MD_C1 : MD_C0);
-      double aqn = 0.0;
-      for (int j = ny - 1; j >= 0; --j) {
-        double a, b, c;
-        helm_abc(hc, set, pmBeta, j, a, b, c);
-        const double rq = 1.0 / (j == ny - 1 ? b : b - c * aqn);
-        const double aq = a * rq;
-        col[(size_t)j * MD_W + 0] = (T)c;
-        col[(size_t)j * MD_W + 1] = (T)rq;
-        col[(size_t)j * MD_W + 2] = (T)aq;
-        aqn = aq;
-      }
-    }
-  }
-  for (int j = threadIdx.x; j < ny; j += blockDim.x) {
-    const int jc = j + 1;
-    T* row = tab + (size_t)j * MT_W;
-    row[MT_IY1] = m.yinterp[jc]; row[MT_IY3] = m.yinterp[jc + 1];
-    row[MT_RDYP] = m.rdyp[jc]; row[MT_RDYC] = m.rdyc[jc];
-    row[MT_AP2C] = m.ap2c[jc]; row[MT_AC2C] = m.ac2c[jc]; row[MT_AM2C] = m.am2c[jc];
-    row[MT_AP2P] = m.ap2p[jc]; row[MT_AC2P] = m.ac2p[jc]; row[MT_AM2P] = m.am2p[jc];
+}
+// and downwards (twisted march): c, 1/m', a/m'
+template <class T>
+__device__ void update_down_factors(const HelmCoef& hc, int set, int ny, double pmBeta, T* __restrict__ dtab) {
+  T* col = dtab + (set ? MD_C1 : MD_C0);
+  double aqn = 0.0;
+  for (int j = ny - 1; j >= 0; --j) {
+    double a, b, c;
+    helm_abc(hc, set, pmBeta, j, a, b, c);
+    const double rq = 1.0 / (j == ny - 1 ? b : b - c * aqn);
+    const double aq = a * rq;
+    col[(size_t)j * MD_W + 0] = (T)c;
+    col[(size_t)j * MD_W + 1] = (T)rq;
+    col[(size_t)j * MD_W + 2] = (T)aq;
+    aqn = aq;
   }
 }
 
@@ -159,6 +133,7 @@ template <class T> struct TableArgs {
   Metrics<T> m;
   int nx, ny, nz;
   T* tab;                     // row tables of the substeps (null: none)
+  bool walls;                 // y solves between walls: their factors in the row tables
   T* dtab;                    // their downward tables (null: not used)
   double* pf;                 // periodic factor blocks of the substeps (null: none)
   double r2x, r2y, r2z;       // 1/h^2 of the x, y and z sweeps; 0: no such sweep
@@ -166,24 +141,57 @@ template <class T> struct TableArgs {
 };
 
 // The tables of substep ns for pmBeta, by the whole block; left as they are when
-// they hold those already.  smem: 5 (ny + 1) values up to kStagedRows rows.
+// they hold those already (constant dt).  Every chain of factors, sequential in its
+// direction, has a warp: 0 to 3 the Helmholtz sets upwards and downwards, 4 to 6 the
+// periodic blocks.  The Helmholtz coefficients come through shared memory (smem, 5
+// (ny + 1) values) up to kStagedRows rows: read from global memory row by row they
+// cost 49 us at 64 rows.  A scheme forms the factors its solves read: none for the
+// explicit one, whose table holds the metrics alone (key 0).  Steps with a changing
+// time step, before with all factors and the walls' chain after the periodic ones: ADI
+// at 128^3 829 -> 807 us, periodic at 64^3 191 -> 166, explicit there 164 -> 120.
 template <class T>
 __device__ void update_tables(const TableArgs<T>& ta, int ns, double pmBeta, unsigned char* smem) {
-  const int q = ns - 1;
-  const unsigned long long bits = (unsigned long long)__double_as_longlong(pmBeta);
+  const int q = ns - 1, ny = ta.ny;
+  const bool factors = ta.walls || ta.r2x > 0.0 || ta.r2y > 0.0 || ta.r2z > 0.0;
+  const unsigned long long bits = (unsigned long long)__double_as_longlong(factors ? pmBeta : 0.0);
   if (ta.slots[q] == bits) return;  // uniform: every thread reads it before thread 0 writes below
-  __syncthreads();
-  if (ta.pf && threadIdx.x >= 128 && (threadIdx.x & 31) == 0) {  // warps 4, 5, 6: the x, z and y blocks
-    const int d = (threadIdx.x >> 5) - 4;
-    const double r2 = d == 0 ? ta.r2x : d == 1 ? ta.r2z : d == 2 ? ta.r2y : 0.0;
-    double* F = ta.pf + (size_t)q * ptri_doubles(ta.nx, ta.ny, ta.nz);
-    if (r2 > 0.0)
-      update_ptri_block(d == 0 ? F : d == 1 ? F + ptri_stride(ta.nx) : F + ptri_stride(ta.nx) + ptri_stride(ta.nz),
-                        d == 0 ? ta.nx : d == 1 ? ta.nz : ta.ny, r2, pmBeta);
+  HelmCoef hc = ta.hc;
+  if (ta.walls && ny <= kStagedRows) {
+    double* const co = reinterpret_cast<double*>(smem);
+    const double* src[5] = {ta.hc.ap2cForCN, ta.hc.am2cForCN, ta.hc.ap2p, ta.hc.ac2p, ta.hc.am2p};
+    const double** dst[5] = {&hc.ap2cForCN, &hc.am2cForCN, &hc.ap2p, &hc.ac2p, &hc.am2p};
+    for (int v = 0; v < 5; ++v) {
+      double* o = co + (size_t)v * (ny + 1);
+      for (int j = threadIdx.x; j <= ny; j += blockDim.x) o[j] = src[v][j];
+      *dst[v] = o;
+    }
   }
-  update_row_table(ta.hc, ta.m, ta.ny, ta.tab + (size_t)q * ta.ny * MT_W,
-                   ta.dtab ? ta.dtab + (size_t)q * ta.ny * MD_W : nullptr, pmBeta,
-                   ta.ny <= kStagedRows ? reinterpret_cast<double*>(smem) : nullptr);
+  __syncthreads();
+  T* const tab = ta.tab + (size_t)q * ny * MT_W;
+  if ((threadIdx.x & 31) == 0) {
+    const int who = threadIdx.x >> 5, set = who & 1;
+    if (who < 2) {
+      if (ta.walls) update_row_factors(hc, set, ny, pmBeta, tab);
+    } else if (who < 4) {
+      if (ta.dtab) update_down_factors(hc, set, ny, pmBeta, ta.dtab + (size_t)q * ny * MD_W);
+    } else if (ta.pf) {
+      const int d = who - 4;  // x, z, y
+      const double r2 = d == 0 ? ta.r2x : d == 1 ? ta.r2z : d == 2 ? ta.r2y : 0.0;
+      double* F = ta.pf + (size_t)q * ptri_doubles(ta.nx, ny, ta.nz);
+      if (r2 > 0.0)
+        update_ptri_block(d == 0 ? F : d == 1 ? F + ptri_stride(ta.nx) : F + ptri_stride(ta.nx) + ptri_stride(ta.nz),
+                          d == 0 ? ta.nx : d == 1 ? ta.nz : ny, r2, pmBeta);
+    }
+  }
+  const Metrics<T>& m = ta.m;
+  for (int j = threadIdx.x; j < ny; j += blockDim.x) {
+    const int jc = j + 1;
+    T* row = tab + (size_t)j * MT_W;
+    row[MT_IY1] = m.yinterp[jc]; row[MT_IY3] = m.yinterp[jc + 1];
+    row[MT_RDYP] = m.rdyp[jc]; row[MT_RDYC] = m.rdyc[jc];
+    row[MT_AP2C] = m.ap2c[jc]; row[MT_AC2C] = m.ac2c[jc]; row[MT_AM2C] = m.am2c[jc];
+    row[MT_AP2P] = m.ap2p[jc]; row[MT_AC2P] = m.ac2p[jc]; row[MT_AM2P] = m.am2p[jc];
+  }
   __syncthreads();
   if (threadIdx.x == 0) ta.slots[q] = bits;
 }
@@ -331,13 +339,14 @@ template <class T> static TableArgs<T> table_args(ch3d_ctx* c) {
   const bool fimp = c->cfg.order == 2 && c->cfg.IsImplicit == 2;
   ta.r2x = fimp ? c->rdx2 : 0.0;
   ta.r2z = fimp ? c->rdz2 : 0.0;
-  ta.r2y = y_periodic(c) ? c->rdy2 : 0.0;
+  ta.r2y = y_periodic(c) && c->cfg.IsImplicit != 0 ? c->rdy2 : 0.0;
+  ta.walls = ta.tab && !y_periodic(c) && c->cfg.IsImplicit != 0;
   ta.dtab = ta.tab && ((c->march && !march_rows_path(c)) || c->cfg.order == 4) && march_twisted(c) ? march_down_tables<T>(c->mtab, c->ny) : nullptr;
   ta.slots = march_beta_slots(c->mtab, c->ny);
   return ta;
 }
 template <class T> static size_t table_smem(const ch3d_ctx* c, const TableArgs<T>& ta) {
-  return ta.tab && c->ny <= kStagedRows ? (size_t)5 * (c->ny + 1) * sizeof(double) : 0;
+  return ta.walls && c->ny <= kStagedRows ? (size_t)5 * (c->ny + 1) * sizeof(double) : 0;
 }
 
 template <class T> static cudaError_t substep_t(ch3d_ctx* c, int ns, bool whole_step) {

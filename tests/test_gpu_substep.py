@@ -19,8 +19,9 @@ EPS = np.finfo(np.float64).eps
 def _cfg(scheme, shape):
     from channel3d_b200 import workloads
     nx, ny, nz = shape
-    if scheme == "periodic_adi":
-        cfg = workloads.taylor_green_periodic(16).copy(nxc=nx, nyc=ny, nzc=nz, nycSection=[ny], IsImplicit=2)
+    if scheme in ("explicit", "periodic", "periodic_adi"):
+        cfg = workloads.taylor_green_periodic(16).copy(nxc=nx, nyc=ny, nzc=nz, nycSection=[ny])
+        cfg = cfg.copy(IsImplicit=("explicit", "periodic", "periodic_adi").index(scheme))
     elif scheme == "wall":
         cfg = small_channel(nx, ny, nz)
     else:
@@ -30,6 +31,7 @@ def _cfg(scheme, shape):
 
 
 @pytest.mark.parametrize("scheme,shape", [("wall", (36, 17, 18)), ("adi", (36, 17, 18)), ("4th", (36, 17, 18)),
+                                          ("explicit", (36, 17, 18)), ("periodic", (36, 17, 18)),
                                           ("periodic_adi", (36, 17, 18)), ("wall", (256, 16, 162)), ("adi", (768, 33, 192))])
 def test_variable_time_step(built, scheme, shape):
     from channel3d_b200 import ChannelSolver, initfield, mesh_y
@@ -37,7 +39,7 @@ def test_variable_time_step(built, scheme, shape):
     cfg = _cfg(scheme, shape)
     yp = mesh_y(cfg)
     rng = np.random.default_rng(5)
-    if scheme == "periodic_adi":
+    if cfg.BcOption[2] == 0:
         f = [a + 0.05 * rng.standard_normal(cfg.shape) for a in initfield.taylor_green(cfg, yp=yp)]
     else:
         f = list(initfield.laminar_noise(cfg, yp=yp, seed=5))
@@ -91,9 +93,7 @@ def test_stages_before_any_set_up(built, scheme, precision):
     if precision == "mixed" and scheme in ("explicit", "periodic", "periodic_adi"):
         pytest.skip("periodic y runs in FP64")
     shape = (36, 17, 18)
-    if scheme in ("explicit", "periodic"):
-        cfg = _cfg("periodic_adi", shape).copy(IsImplicit=0 if scheme == "explicit" else 1)
-    elif scheme == "les":
+    if scheme == "les":
         cfg, _ = workloads.get("channel48_les")
         cfg = cfg.copy(nxc=36, nyc=17, nzc=18, nycSection=[8, 9], LES_type=2, Cs=0.1)
     else:
