@@ -255,14 +255,6 @@ def profile_traffic(kernel, precision):
     return None, None
 
 
-def rows_path(cfg, key, path):
-    """The partially implicit step of grids with few columns forms the right-hand
-    sides by rows and sweeps in y (march_rows_path, ch3d_march.cu)."""
-    import torch
-    sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
-    return key == "pimp" and "gsub" not in path and cfg.nxc * cfg.nzc <= 120 * sms
-
-
 def launches_per_step(cfg, key, path, rows):
     """Kernel launches of one graph-replayed step (ch3d_api.cu record_step)."""
     gsub = "gsub" in path
@@ -326,7 +318,7 @@ def measure(args, ws, rank, local, precision, want_e2e):
     names[0] = GROUP0_KERNEL[key]
     path = sorted(s.path_flags())
     gsub = "gsub" in path
-    rows = rows_path(cfg, key, path)
+    rows = key == "pimp" and "march" not in path  # few columns: right-hand sides by rows, then a y sweep
     if rows or (key == "les" and cfg.LES_type == 11):
         names[0] = GROUP0_ROWS
     if gsub:  # the march stops at g; the divergence and projection marches substitute u*

@@ -1261,8 +1261,8 @@ int ch3d_last_step_ms(ch3d_ctx* c, double* ms) {
 int ch3d_path_flags(ch3d_ctx* c, int* flags) {
   if (!c || !flags) return fail(CH3D_ERR_INVALID, "NULL argument");
   CU(cudaSetDevice(c->device));
-  const bool march = march_path(c) || c->cfg.order == 4;
-  *flags = (march ? CH3D_PATH_MARCH : 0) | (march && !march_rows_path(c) && march_twisted(c) ? CH3D_PATH_TWISTED : 0) |
+  const bool march = (march_path(c) && !march_rows_path(c)) || c->cfg.order == 4;
+  *flags = (march ? CH3D_PATH_MARCH : 0) | (march && march_twisted(c) ? CH3D_PATH_TWISTED : 0) |
            (c->gsub ? CH3D_PATH_GSUB : 0);
   return CH3D_OK;
 }

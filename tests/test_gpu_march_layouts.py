@@ -102,3 +102,17 @@ def test_gsub_mixed(built):
     for k in ("ux", "uy", "uz"):
         assert rel_l2(gs[k], go[k]) < 1e-4, (k, rel_l2(gs[k], go[k]))
     assert di["divmax2"] < 1e-4
+
+
+@pytest.mark.parametrize("scheme,shape,flags", [
+    ("rows", (64, 48, 48), set()), ("twisted", (144, 24, 128), {"march", "twisted"}),
+    ("gsub", (256, 16, 162), {"march", "gsub"}), ("adi", (48, 32, 36), set()), ("4th", (48, 24, 36), {"march", "twisted"})])
+def test_layout_flags(built, scheme, shape, flags):
+    """The layout flags say which kernels run: no march where the right-hand sides go by rows."""
+    from channel3d_b200 import ChannelSolver, mesh_y, workloads
+    cfg = small_channel(*shape)
+    if scheme in ("adi", "4th"):
+        cfg, _ = workloads.get({"adi": "channel128_re5600_fimp", "4th": "channel128_re5600_4th"}[scheme])
+        cfg = cfg.copy(nxc=shape[0], nyc=shape[1], nzc=shape[2], nycSection=[shape[1] // 2, shape[1] - shape[1] // 2])
+    with ChannelSolver(cfg, yp=mesh_y(cfg)) as s:
+        assert s.path_flags() == flags
