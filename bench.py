@@ -38,7 +38,8 @@ sys.path.insert(0, ROOT)
 # 4th order: 32 arrays per substep; fully implicit (ADI): 47.
 ALG_ARRAYS_PER_SUBSTEP = {"pimp": 32, "order4": 32, "fimp": 47, "les": 32}
 # per-launch algorithmic arrays of each kernel group of ch3d_kernel_times
-# (0: RHS + y Helmholtz solve, fused: read u v w p Hist x3, write Hist x3 u* x3;
+# (0: RHS, with the y Helmholtz solve where they are one kernel: read u v w p Hist x3,
+#  write Hist x3 and RHS or u* x3;
 #  2: divergence + forward x FFT: read u* x3, write the half spectrum;
 #  3: z FFT, y Poisson solve, inverse z FFT: 3 x (read + write) of the spectrum;
 #  4: inverse x FFT: read spectrum, write phi;
@@ -46,9 +47,10 @@ ALG_ARRAYS_PER_SUBSTEP = {"pimp": 32, "order4": 32, "fimp": 47, "les": 32}
 GROUP_ARRAYS = {0: 13, 2: 4, 3: 6, 4: 2, 5: 9}
 GROUP_NAMES = {0: "rhs", 1: "y_solves", 2: "k_prsrc_xfft", 3: "k_zfft+k_yscan+k_zfft", 4: "k_xifft",
                5: "k_proj_march", 6: "scalar_kernels_per_step"}
-# the group-0 kernels of each scheme: one column march, or right-hand sides and line solves
-GROUP0_KERNEL = {"pimp": "k_rhs_march", "order4": "k_rhs_march", "fimp": "k_rhs_rows+k_sweep", "les": "k_rhs_les+k_uhat_les"}
-GROUP0_ROWS = "k_rhs_rows+k_sweep"
+# the kernels of groups 0 and 1 by scheme: one column march, or right-hand sides and line solves
+GROUP01_KERNEL = {"pimp": ("k_rhs_march", None), "order4": ("k_rhs_march", None), "fimp": ("k_rhs_rows", "k_sweep_x+k_sweep"),
+                  "les": ("k_rhs_les", "k_uhat_les")}
+GROUP01_ROWS = ("k_rhs_rows", "k_sweep")
 
 
 def parse():
@@ -315,12 +317,10 @@ def measure(args, ws, rank, local, precision, want_e2e):
     word = 4 if precision == "mixed" else 8
     key = scheme_key(cfg)
     names = dict(GROUP_NAMES)
-    names[0] = GROUP0_KERNEL[key]
     path = sorted(s.path_flags())
     gsub = "gsub" in path
     rows = key == "pimp" and "march" not in path  # few columns: right-hand sides by rows, then a y sweep
-    if rows or (key == "les" and cfg.LES_type == 11):
-        names[0] = GROUP0_ROWS
+    names[0], names[1] = GROUP01_ROWS if rows or (key == "les" and cfg.LES_type == 11) else GROUP01_KERNEL[key]
     if gsub:  # the march stops at g; the divergence and projection marches substitute u*
         names[2] = "k_div_bsub+k_prsrc_xfft"
         names[5] = "k_proj_bsub"

@@ -506,20 +506,28 @@ static bool march_path(const ch3d_ctx* c) {
   return c->cfg.LES_type == 0 && c->cfg.order == 2 && c->cfg.IsImplicit == 1 && !y_periodic(c);
 }
 
-// u -> u* of one substep: right-hand sides, Hist and the Crank-Nicolson solves
-cudaError_t launch_ustar(ch3d_ctx* c) {
+// u -> u* of one substep, in two parts: the right-hand sides with Hist, then the
+// Crank-Nicolson solves.  One kernel does both where columns march and in the explicit
+// scheme without LES; the second part is then empty.
+bool ustar_fused(const ch3d_ctx* c) {
   const ch3d_config& g = c->cfg;
-  cudaError_t e;
-  if (c->march && !march_rows_path(c)) return launch_rhs_march(c);  // one column march
-  if (g.order == 4) return launch_rhs_march(c);  // the same with the 4th-order stencils
-  if (les_const(c)) return (e = launch_rhs_les_const(c)) != cudaSuccess ? e : launch_uhat(c);
-  if (g.LES_type > 0) {  // the LES y solves form their own coefficients (FEXP: none)
-    if ((e = launch_rhs_les(c)) != cudaSuccess) return e;
+  return g.order == 4 || (c->march && !march_rows_path(c)) || (g.IsImplicit == 0 && g.LES_type == 0);
+}
+cudaError_t launch_ustar_rhs(ch3d_ctx* c) {
+  const ch3d_config& g = c->cfg;
+  if (ustar_fused(c)) return g.IsImplicit == 0 ? launch_ustar_fexp(c) : launch_rhs_march(c);
+  if (les_const(c)) return launch_rhs_les_const(c);
+  return g.LES_type > 0 ? launch_rhs_les(c) : launch_rhs(c);
+}
+cudaError_t launch_ustar_solve(ch3d_ctx* c) {
+  const ch3d_config& g = c->cfg;
+  if (ustar_fused(c)) return cudaSuccess;
+  if (g.LES_type > 0 && !les_const(c))  // the LES y solves form their own coefficients (FEXP: none)
     return g.IsImplicit == 0 ? launch_uhat_fexp(c) : launch_uhat_les(c);
+  if (g.IsImplicit == 2) {
+    const cudaError_t e = launch_ptri_xz(c);
+    if (e != cudaSuccess) return e;
   }
-  if (g.IsImplicit == 0) return launch_ustar_fexp(c);  // explicit right-hand sides, u* = u + Rhs
-  if ((e = launch_rhs(c)) != cudaSuccess) return e;
-  if (g.IsImplicit == 2 && (e = launch_ptri_xz(c)) != cudaSuccess) return e;
   return y_periodic(c) ? launch_ptri_y(c) : launch_uhat(c);  // FIMP_000 or PIMP_0, else between walls
 }
 
@@ -527,7 +535,8 @@ int record_step(ch3d_ctx* c) {
   if (c->cfg.LES_type > 0) CU(launch_sgs_nut(c));  // once per step (m_ChannelSystem.f90:89)
   for (int ns = 1; ns <= c->iadvance; ++ns) {
     CU(launch_substep_setup(c, ns, true));
-    CU(launch_ustar(c));
+    CU(launch_ustar_rhs(c));
+    CU(launch_ustar_solve(c));
     if (c->gsub) {
       CU(launch_div_bsub(c));
       CU(launch_prsrc_xfft(c, 3));
@@ -1153,13 +1162,14 @@ int ch3d_memory_bytes(ch3d_ctx* c, long long* bytes) {
 // Runs `nsteps` steps kernel group by kernel group with CUDA events between
 // the groups on the context's stream; out[q] = mean milliseconds per launch of
 // group q: 0 rhs, 1 uhat, 2 prsrc+x FFT, 3 z FFT + y solve + z iFFT,
-// 4 x iFFT, 5 projection, 6 scalar/reduction kernels.  Group 0 holds u -> u*.
+// 4 x iFFT, 5 projection, 6 scalar/reduction kernels.  Group 1 is 0 where group 0
+// holds the solves (ustar_fused).
 int ch3d_kernel_times(ch3d_ctx* c, int nsteps, double* out, int nout) {
   if (!c || !out || nout < 7 || nsteps < 1) return fail(CH3D_ERR_INVALID, "bad argument");
   CU(cudaSetDevice(c->device));
   if (!c->scalars_ready) { int rc = init_scalars(c); if (rc) return rc; }
   const int G = 7;
-  const int per_step = 1 + 7 * c->iadvance + 1;  // timed groups per step
+  const int per_step = 1 + (ustar_fused(c) ? 6 : 7) * c->iadvance + 1;  // timed groups per step
   std::vector<cudaEvent_t> ev((size_t)2 * per_step * nsteps, nullptr);
   for (auto& e : ev) CU(cudaEventCreate(&e));
   std::vector<int> grp;
@@ -1172,8 +1182,8 @@ int ch3d_kernel_times(ch3d_ctx* c, int nsteps, double* out, int nout) {
       CU(mark(6));
       CU(launch_substep_setup(c, ns, true));
       CU(done());
-      CU(mark(0)); CU(launch_ustar(c)); CU(done());
-      CU(mark(1)); CU(done());
+      CU(mark(0)); CU(launch_ustar_rhs(c)); CU(done());
+      if (!ustar_fused(c)) { CU(mark(1)); CU(launch_ustar_solve(c)); CU(done()); }
       if (c->gsub) {
         CU(mark(2)); CU(launch_div_bsub(c)); CU(launch_prsrc_xfft(c, 3)); CU(done());
       } else {

@@ -269,7 +269,9 @@ CH3D_API int ch3d_memory_bytes(ch3d_ctx* ctx, long long* bytes);
 
 /* Runs `nsteps` steps launching kernel groups one by one, with CUDA events
    between them on the context's stream, and returns in out[0..5] the mean time
-   (ms) per substep of each group: 0 RHS stencils, 1 y Helmholtz solves,
+   (ms) per substep of each group: 0 RHS stencils, 1 Helmholtz solves (0 where
+   one kernel does both and group 0 holds it: CH3D_PATH_MARCH, and the explicit
+   scheme without LES),
    2 divergence + forward x FFT, 3 z FFT + y Poisson solve + inverse z FFT,
    4 inverse x FFT, 5 projection + pressure update; out[6] is the time per step
    of the scalar and reduction kernels (CFL, substep coefficients,

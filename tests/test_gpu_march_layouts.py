@@ -116,3 +116,36 @@ def test_layout_flags(built, scheme, shape, flags):
         cfg = cfg.copy(nxc=shape[0], nyc=shape[1], nzc=shape[2], nycSection=[shape[1] // 2, shape[1] - shape[1] // 2])
     with ChannelSolver(cfg, yp=mesh_y(cfg)) as s:
         assert s.path_flags() == flags
+
+
+@pytest.mark.parametrize("scheme,shape,fused", [
+    ("rows", (64, 48, 48), False), ("twisted", (144, 24, 128), True), ("gsub", (256, 16, 162), True),
+    ("adi", (48, 32, 36), False), ("4th", (48, 24, 36), True), ("explicit", (32, 24, 32), True),
+    ("periodic", (32, 24, 32), False), ("les", (48, 24, 32), False), ("les_explicit", (48, 24, 32), False)])
+def test_kernel_groups(built, scheme, shape, fused):
+    """Group times keep right-hand sides and solves apart unless one kernel does both (then
+    group 1 is 0), and the steps taken are steps."""
+    from channel3d_b200 import ChannelSolver, initfield, mesh_y, workloads
+    nx, ny, nz = shape
+    if scheme in ("explicit", "periodic"):
+        cfg = workloads.taylor_green_periodic(16).copy(nxc=nx, nyc=ny, nzc=nz, nycSection=[ny],
+                                                       IsImplicit=0 if scheme == "explicit" else 1)
+    elif scheme in ("rows", "twisted", "gsub"):
+        cfg = small_channel(*shape)
+    else:
+        cfg, _ = workloads.get({"adi": "channel128_re5600_fimp", "4th": "channel128_re5600_4th"}.get(scheme, "channel48_les"))
+        cfg = cfg.copy(nxc=nx, nyc=ny, nzc=nz, nycSection=[ny // 2, ny - ny // 2])
+        if scheme.startswith("les"):
+            cfg = cfg.copy(LES_type=2, Cs=0.1, IsImplicit=0 if scheme == "les_explicit" else 1)
+    yp = mesh_y(cfg)
+    f = initfield.taylor_green(cfg, yp=yp) if cfg.FlowType == 3 else initfield.laminar_noise(cfg, yp=yp, seed=3)
+    with ChannelSolver(cfg, yp=yp) as s, ChannelSolver(cfg, yp=yp) as ref:
+        s.upload(*f)
+        ref.upload(*f)
+        t = s.kernel_times(2)
+        ref.step(2)
+        a, b = s.download(), ref.download()
+    assert (t[[0, 2, 3, 4, 5, 6]] > 0).all(), t
+    assert (t[1] == 0) if fused else (t[1] > 0), t
+    for k in ("ux", "uy", "uz", "p"):
+        assert np.array_equal(a[k], b[k]), k
