@@ -11,6 +11,7 @@
 #include <string>
 #include <vector>
 #include "../../include/ch3d_mlp.h"
+#include "ch3d_fft.cuh"
 #include "ch3d_march.cuh"
 
 using namespace ch3d;
@@ -86,11 +87,6 @@ void mesh_section(double* yp1, int id1, int id2, double c1, double c2, int Stret
 
 // Plan of an n-point transform, n a product of 2 and 3: the fewest passes of
 // radix at most maxr, the largest radix as small as they allow, smaller radices first.
-// FP64 x transforms stop at 9, a pass more for some lengths but half the registers
-// (ch3d_fft.cu): 96 points as 4 x 4 x 6 76 us, as 8 x 12 82 us (192^3, forward); z
-// transforms, whose passes move more between them, gain nothing (192 points as 12 x 16
-// 34 us, as 4 x 6 x 8 43).
-constexpr int kXRadix64 = 9;
 bool factor23(int n, FFTPlanDev& pl, int maxr) {
   pl.n = n; pl.npass = 0;
   int m = n;

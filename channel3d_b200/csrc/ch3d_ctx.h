@@ -121,7 +121,7 @@ bool march_diag_fusable(const ch3d_ctx* c);            // the step diagnostics c
 cudaError_t launch_bulk_march(ch3d_ctx* c);            // bulk partials of an uploaded field
 int march_npart(const ch3d_ctx* c);
 cudaError_t launch_prsrc_xfft(ch3d_ctx* c, int mode);  // mode 0: div(u*)/pmAlpha, 1: div(u), 2: source in phi,
-                                                       // 3: div(u*) in phi's array, /pmAlpha (register FFT only)
+                                                       // 3: div(u*) in phi's array, /pmAlpha (x lengths with a register plan)
 cudaError_t launch_poisson_spectral(ch3d_ctx* c);      // z fwd, y solve, z inv
 cudaError_t launch_ysolve(ch3d_ctx* c);                // the y systems (ch3d_ysolve.cu)
 bool ysolve_chunked(int ny);                           // they run as the chunked kernel (no scratch)

@@ -22,8 +22,8 @@ __device__ __forceinline__ int xpad(int n, int sh) { return n + (n >> sh); }
 
 // The source of the forward transform, packed as z_n = src_2n + i src_2n+1:
 // div(u)/pmAlpha (modes 0, 1), with its largest magnitude in dmax.
-// SRC: 0 2nd-order divergence, 1 4th-order divergence, 2 the source (mode 2), the
-// divergence (mode 3) or a field (mode 4) as it stands in the first array.
+// SRC: 0 2nd-order divergence, 1 4th-order divergence, 2 the source (mode 2) or a
+// field (mode 4) as it stands in the first array.
 template <class T, int SRC> struct XSource {
   typedef typename CplxOf<T>::type CT;
   const Geo<T>& g;
@@ -78,9 +78,9 @@ template <class T, int SRC> struct XSource {
     dmax = fmax(dmax, fmax(fabs((double)r0), fabs((double)r1)));
     return mk(sudtal * r0, sudtal * r1);
   }
-  // the block's largest |div| into sc->divmax1 (modes 0 to 2; mode 3: it was taken where the divergence was formed)
+  // the block's largest |div| into sc->divmax1 (modes 0 to 2)
   __device__ __forceinline__ void finish(DevScalars* sc) {
-    if (mode >= 3) return;
+    if (mode == 4) return;
     __shared__ double wred[16];
     for (int o = 16; o > 0; o >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
     if ((threadIdx.x & 31) == 0) wred[threadIdx.x >> 5] = dmax;
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(256) k_xfft_g(Geo<T> g, Metrics<T> m, const T*
   const int nl = min(LPB, g.ny * g.nz - line0);
   CT* src = (CT*)smem_raw;
   CT* dst = src + (size_t)LPB * LP;
-  XSource<T, SRC> form{g, m, ux, uy, uz, pr, mode, mode == 0 || mode == 3 ? (T)(1.0 / sc->pmAlpha) : (T)1, 0.0};
+  XSource<T, SRC> form{g, m, ux, uy, uz, pr, mode, mode == 0 ? (T)(1.0 / sc->pmAlpha) : (T)1, 0.0};
   int p = 0;
   if constexpr (SRC == 2 || sizeof(T) == 4) {
     p = 1;
@@ -238,39 +238,39 @@ __global__ void __launch_bounds__(256) k_xifft_g(Geo<T> g, const typename CplxOf
 // ---------------------------------------------------------------------------
 constexpr int kFftSmemLimit = 200 * 1024;
 
-// Runs go with the radices to compile in: FP64 plans up to radix 9 have kernels of 72
-// to 74 registers, those with the 12- and 16-point butterflies 118 to 128 (64^3 step
-// 145 / 141 us); in FP32 (44 / 64) the smaller ones were no faster (96 x 65 x 54 143 / 146).
-template <class T, class F> static void with_radices(const FFTPlanDev& pl, F go) {
+// Radices compiled in.  FP64 kernels up to radix 9 have 72 to 74 registers, those with
+// the 12- and 16-point butterflies 118 to 128 (64^3 step 145 / 141 us): x plans stop at
+// 9, and z plans up to 9 have kernels of their own.  In FP32 (44 / 64) the smaller ones
+// were no faster (96 x 65 x 54 143 / 146).
+template <class T> constexpr int x_radices() { return sizeof(T) == 8 ? kXRadix64 : 16; }
+template <class T, class F> static void with_z_radices(const FFTPlanDev& pl, F go) {
   if constexpr (sizeof(T) == 8)
     if (pl.npass == 0 || pl.radix[pl.npass - 1] <= 9) return go(std::integral_constant<int, 9>{});  // radices ascend
   go(std::integral_constant<int, 16>{});
 }
 // Shared-memory limits of the kernels that transforms with these plans use, each once
 // per process and device (setting one loads the kernel).
-template <class T> static cudaError_t setup_t(int device, const FFTPlanDev& planx, const FFTPlanDev& planz) {
-  cudaError_t e = cudaSuccess;
-  with_radices<T>(planx, [&](auto R) {
-    static PerDevice site;  // per precision and radix set
-    e = once_per_device(site, device, [] {
-      const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-      cudaError_t r = cudaFuncSetAttribute(k_xfft_g<T, 0, decltype(R)::value>, a, kFftSmemLimit);
-      if (r == cudaSuccess) r = cudaFuncSetAttribute(k_xfft_g<T, 1, decltype(R)::value>, a, kFftSmemLimit);
-      if (r == cudaSuccess) r = cudaFuncSetAttribute(k_xfft_g<T, 2, decltype(R)::value>, a, kFftSmemLimit);
-      return r == cudaSuccess ? cudaFuncSetAttribute(k_xifft_g<T, decltype(R)::value>, a, kFftSmemLimit) : r;
-    });
+template <class T> static cudaError_t setup_t(int device, const FFTPlanDev& planz) {
+  static PerDevice xsite;  // per precision
+  cudaError_t e = once_per_device(xsite, device, [] {
+    constexpr int R = x_radices<T>();
+    const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t r = cudaFuncSetAttribute(k_xfft_g<T, 0, R>, a, kFftSmemLimit);
+    if (r == cudaSuccess) r = cudaFuncSetAttribute(k_xfft_g<T, 1, R>, a, kFftSmemLimit);
+    if (r == cudaSuccess) r = cudaFuncSetAttribute(k_xfft_g<T, 2, R>, a, kFftSmemLimit);
+    return r == cudaSuccess ? cudaFuncSetAttribute(k_xifft_g<T, R>, a, kFftSmemLimit) : r;
   });
   if (e != cudaSuccess) return e;
-  with_radices<T>(planz, [&](auto R) {
-    static PerDevice site;
+  with_z_radices<T>(planz, [&](auto R) {
+    static PerDevice site;  // per precision and radix set
     e = once_per_device(site, device, [] {
       return cudaFuncSetAttribute(k_zfft_g<T, decltype(R)::value>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFftSmemLimit);
     });
   });
   return e;
 }
-cudaError_t fft_generic_setup(int device, bool fp32, const FFTPlanDev& planx, const FFTPlanDev& planz) {
-  return fp32 ? setup_t<float>(device, planx, planz) : setup_t<double>(device, planx, planz);
+cudaError_t fft_generic_setup(int device, bool fp32, const FFTPlanDev& planz) {
+  return fp32 ? setup_t<float>(device, planz) : setup_t<double>(device, planz);
 }
 
 // Lines per x block: one round of 128 tasks in the first pass, at most 16 lines.
@@ -298,11 +298,10 @@ cudaError_t xfft_generic(const Geo<T>& g, const Metrics<T>& m, const T* a, const
   auto go = [&](auto kern) {
     kern<<<grid, s.threads, s.smem, st>>>(g, m, a, b, c, spec, pl, tw, twr, s.LPB, s.LP, s.sh, fdiv_magic(g.nx / 2), fdiv_magic(g.nx / 2 + 1), mode, sc, pr);
   };
-  with_radices<T>(pl, [&](auto R) {
-    if (mode >= 2) go(k_xfft_g<T, 2, R.value>);
-    else if (g.order == 4) go(k_xfft_g<T, 1, R.value>);
-    else go(k_xfft_g<T, 0, R.value>);
-  });
+  constexpr int R = x_radices<T>();
+  if (mode >= 2) go(k_xfft_g<T, 2, R>);
+  else if (g.order == 4) go(k_xfft_g<T, 1, R>);
+  else go(k_xfft_g<T, 0, R>);
   return cudaGetLastError();
 }
 
@@ -320,7 +319,7 @@ cudaError_t zfft_generic(const Geo<T>& g, typename CplxOf<T>::type* spec, const 
     kern<<<dim3((g.nxh + TKX - 1) / TKX, g.ny), g.nz > 256 ? 256 : 128, (size_t)nbuf * TKX * g.nz * sizeof(CT), st>>>(
         g, spec, pl, tw, TKX, fdiv_magic(TKX), fdiv_magic(tail > 0 ? tail : 1), inverse, sc);
   };
-  with_radices<T>(pl, [&](auto R) { go(k_zfft_g<T, R.value>); });
+  with_z_radices<T>(pl, [&](auto R) { go(k_zfft_g<T, R.value>); });
   return cudaGetLastError();
 }
 
@@ -330,10 +329,7 @@ cudaError_t xifft_generic(const Geo<T>& g, const typename CplxOf<T>::type* spec,
                           const DevScalars* sc, cudaStream_t st) {
   const XShape s = x_shape<T>(g.nx / 2, pl.radix[0]);
   const int nlines = g.ny * g.nz;
-  auto go = [&](auto kern) {
-    kern<<<(nlines + s.LPB - 1) / s.LPB, s.threads, s.smem, st>>>(g, spec, phi, pl, tw, twr, s.LPB, s.LP, s.sh, normfft, sc);
-  };
-  with_radices<T>(pl, [&](auto R) { go(k_xifft_g<T, R.value>); });
+  k_xifft_g<T, x_radices<T>()><<<(nlines + s.LPB - 1) / s.LPB, s.threads, s.smem, st>>>(g, spec, phi, pl, tw, twr, s.LPB, s.LP, s.sh, normfft, sc);
   return cudaGetLastError();
 }
 

@@ -143,16 +143,6 @@ __global__ void __launch_bounds__(256) k_ysolve(Geo<T> g, Metrics<double> m, con
     spec[kx + (long long)nxh * j + zs * kz] = mk((T)x.x, (T)x.y);
   }
 }
-__device__ __forceinline__ double block_max256(double v, double* sh /* 8 */) {
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  const int tl = threadIdx.x + blockDim.x * threadIdx.y;
-  if ((tl & 31) == 0) sh[tl >> 5] = v;
-  __syncthreads();
-  double r = 0.0;
-  if (tl == 0)
-    for (int w = 0; w < 8; ++w) r = fmax(r, sh[w]);
-  return r;
-}
 
 // CheckDivergence, CalcVmax, CalcMaxCFL of the next step, CalcUxAver partials
 // (src/CFD_2nd/m_Tools.f90:21-104,250-270).  A thread walks `rows` rows of
@@ -301,7 +291,7 @@ template <class T> static cudaError_t prsrc_t(ch3d_ctx* c, int mode) {
   typedef typename CplxOf<T>::type CT;
   cudaError_t e;
   if (launch_prsrc_xfft_r(c, mode, &e)) return e;
-  if ((e = fft_generic_setup(c->device, c->fp32, c->planx, c->planz)) != cudaSuccess) return e;
+  if ((e = fft_generic_setup(c->device, c->fp32, c->planz)) != cudaSuccess) return e;
   T** f = (T**)c->f;
   const T* a = mode >= 2 ? f[10] : (mode == 1 ? f[0] : f[12]);
   return xfft_generic<T>(make_geo<T>(c), metrics_of<T>(c), a, mode == 1 ? f[1] : f[13], mode == 1 ? f[2] : f[14],
@@ -313,7 +303,7 @@ template <class T> static cudaError_t zfft_t(ch3d_ctx* c, int inverse) {
   typedef typename CplxOf<T>::type CT;
   cudaError_t e;
   if (launch_zfft_r(c, inverse, &e)) return e;
-  if ((e = fft_generic_setup(c->device, c->fp32, c->planx, c->planz)) != cudaSuccess) return e;
+  if ((e = fft_generic_setup(c->device, c->fp32, c->planz)) != cudaSuccess) return e;
   return zfft_generic<T>(make_geo<T>(c), (CT*)c->spec, c->planz, (const CT*)c->twz, inverse, c->sc, c->stream);
 }
 static cudaError_t zfft(ch3d_ctx* c, int inverse) { return c->fp32 ? zfft_t<float>(c, inverse) : zfft_t<double>(c, inverse); }
@@ -330,7 +320,7 @@ template <class T> static cudaError_t xifft_t(ch3d_ctx* c) {
   typedef typename CplxOf<T>::type CT;
   cudaError_t e;
   if (launch_xifft_r(c, &e)) return e;
-  if ((e = fft_generic_setup(c->device, c->fp32, c->planx, c->planz)) != cudaSuccess) return e;
+  if ((e = fft_generic_setup(c->device, c->fp32, c->planz)) != cudaSuccess) return e;
   return xifft_generic<T>(make_geo<T>(c), (const CT*)c->spec, (T*)c->f[10], c->planx, (const CT*)c->twx,
                           (const CT*)c->twr, (T)c->normfft, c->sc, c->stream);
 }
@@ -577,11 +567,11 @@ cudaError_t noalloc_scratch_address(int dev, void** out) {
     cudaError_t r = cudaGetSymbolAddress(&p, g_noalloc_scratch);
     if (r != cudaSuccess) return r;
     const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    FFTPlanDev p9 = {}, p16 = {};  // FP64 x plans stop at radix 9, z plans may hold the larger ones
+    FFTPlanDev p9 = {}, p16 = {};  // both radix sets of z plans
     p16.npass = 1;
     p16.radix[0] = 16;
-    if ((r = fft_generic_setup(dev, false, p9, p9)) != cudaSuccess) return r;
-    if ((r = fft_generic_setup(dev, false, p9, p16)) != cudaSuccess) return r;
+    if ((r = fft_generic_setup(dev, false, p9)) != cudaSuccess) return r;
+    if ((r = fft_generic_setup(dev, false, p16)) != cudaSuccess) return r;
     if ((r = cudaFuncSetAttribute(k_ysolve<double>, a, kNoallocSmemLimit)) != cudaSuccess) return r;
     g_noalloc_addr[dev] = p;
     return cudaSuccess;

@@ -108,7 +108,6 @@ template <int NCOLS> __device__ __forceinline__ void tmem_ld(uint32_t taddr, flo
 #pragma unroll
   for (int q = 0; q < NCOLS; ++q) v[q] = __uint_as_float(r[q]);
 }
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) { tmem_ld<16>(taddr, v); }
 
 // shared-memory matrix descriptor: canonical K-major, no swizzle
 __device__ __forceinline__ uint64_t sdesc(const void* base, uint32_t lbo, uint32_t sbo) {
@@ -128,9 +127,6 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
 // byte offset of element (r, k) of a K-major tile with R rows
 __device__ __forceinline__ uint32_t koff(int r, int k, int R) {
   return (uint32_t)((k >> 3) * (16 * R) + (r >> 3) * 128 + (r & 7) * 16 + (k & 7) * 2);
-}
-__device__ __forceinline__ void st_bf16(unsigned char* tile, int r, int k, int R, float v) {
-  *(__nv_bfloat16*)(tile + koff(r, k, R)) = __float2bfloat16_rn(v);
 }
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);  // lo at the lower address
