@@ -2,10 +2,11 @@
 channel3d_b200/csrc/ch3d_march.cu) in each of its launch layouts, whole steps
 against the oracle within the 1e-10 relative bound:
 
-- twisted blocks (few column tiles: two thread groups per tile, the lower
-  eliminating upwards and the upper downwards, meeting in the middle), with
-  odd ny so the groups march different numbers of rows, ragged tiles in x and
-  z, and the smallest ny the layout takes;
+- twisted blocks (few column tiles, more columns than the rows take: two thread
+  groups per tile, the lower eliminating upwards and the upper downwards, meeting
+  in the middle), with odd ny so the groups march different numbers of rows, even
+  ny, ragged tiles in x and z, and the smallest ny the layout takes;
+- grids of fewer columns, whose right-hand sides go by rows;
 - one tile per plain block (more tiles than twisted blocks fit on the GPU, fewer
   than the resident persistent blocks), with a ragged last z tile;
 - the 4th-order march both ways (128 column tiles twisted, 384 plain);
@@ -43,9 +44,26 @@ def _check(go, gs, tol=1e-10):
         assert e < tol, (k, e)
 
 
-@pytest.mark.parametrize("shape", [(48, 25, 18), (32, 5, 16), (64, 24, 48)])
+def _flags(cfg):
+    from channel3d_b200 import ChannelSolver, mesh_y
+    with ChannelSolver(cfg, yp=mesh_y(cfg)) as s:
+        return s.path_flags()
+
+
+@pytest.mark.parametrize("shape", [(144, 25, 162), (128, 5, 162), (96, 24, 192), (108, 4, 192), (144, 7, 128)])
 def test_twisted_march(built, shape):
-    go, gs, di = _run(small_channel(*shape), 4)
+    cfg = small_channel(*shape)
+    assert _flags(cfg) == {"march", "twisted"}
+    go, gs, di = _run(cfg, 4)
+    _check(go, gs)
+    assert di["divmax2"] < 1e-12
+
+
+@pytest.mark.parametrize("shape", [(48, 25, 18), (32, 5, 16), (64, 24, 48)])
+def test_few_columns(built, shape):
+    cfg = small_channel(*shape)
+    assert not _flags(cfg)
+    go, gs, di = _run(cfg, 4)
     _check(go, gs)
     assert di["divmax2"] < 1e-12
 
@@ -56,9 +74,13 @@ def test_plain_blocks_one_tile_each(built):
     _check(go, gs)
 
 
-def test_twisted_march_mixed(built):
-    """FP32 twisted march (mixed path) within the mixed path's 1e-4 bound."""
-    go, gs, _ = _run(small_channel(48, 25, 18, precision="mixed"), 4)
+@pytest.mark.parametrize("shape,twisted", [((144, 25, 162), True), ((128, 5, 162), True), ((48, 25, 18), False)])
+def test_twisted_march_mixed(built, shape, twisted):
+    """FP32 twisted march (mixed path), and the rows of fewer columns, within the mixed
+    path's 1e-4 bound."""
+    cfg = small_channel(*shape, precision="mixed")
+    assert ("twisted" in _flags(cfg)) == twisted
+    go, gs, _ = _run(cfg, 4)
     for k in ("ux", "uy", "uz"):
         assert rel_l2(gs[k], go[k]) < 1e-4, (k, rel_l2(gs[k], go[k]))
 

@@ -2,7 +2,8 @@
 diagnostics that ride on the last one (channel3d_b200/csrc/ch3d_march.cu), on ragged
 tiles and chunks: after steps of each scheme the reported divergence, velocity
 maxima and bulk mean are those of the downloaded field (the sums in another order:
-1e-12), and fields and diagnostics match the oracle's steps (1e-10)."""
+1e-12; the divergence, a difference of terms whose products may be contracted, 8 eps
+of their sum), and fields and diagnostics match the oracle's steps (1e-10)."""
 import numpy as np
 import pytest
 
@@ -59,3 +60,52 @@ def test_projection_and_diagnostics(built, scheme, shape):
     for k in ("uxm", "cflmp"):
         assert abs(di[k] - do[k]) <= 1e-9 * max(1.0, abs(do[k])), (k, di[k], do[k])
     assert di["divmax2"] < 1e-11
+
+
+def _divergence(f, cfg, yp, word):
+    """(div, sum of its terms' magnitudes) of the staggered field, with metrics of the field's precision."""
+    m = lambda v: np.asarray(v, dtype=word).astype(np.float64)  # noqa: E731
+    rdx, rdz, rdyp = m(cfg.nxc / cfg.xlx), m(cfg.nzc / cfg.zlz), m(1.0 / np.diff(yp))[None, :, None]
+    v = f["uy"]
+    vp = np.roll(v, -1, 1)
+    if cfg.BcOption[2] != 0:
+        vp[:, -1, :] = cfg.uyBcValue[3]
+
+    def d(a, axis, r):
+        u = lambda n: np.roll(a, -n, axis)  # noqa: E731
+        if cfg.order == 4:
+            return r * ((u(-1) - u(2)) / 24 + 1.125 * (u(1) - a)), abs(r) * (abs(u(-1)) + abs(u(2)) + abs(u(1)) + abs(a))
+        return (u(1) - a) * r, (abs(u(1)) + abs(a)) * r
+
+    (dx, sx), (dz, sz) = d(f["ux"], 2, rdx), d(f["uz"], 0, rdz)
+    return dx + (vp - v) * rdyp + dz, sx + (abs(vp) + abs(v)) * rdyp + sz
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("scheme,shape", [(q, s) for q in ("wall", "adi", "4th", "les", "free_slip_explicit")
+                                          for s in ((36, 9, 18), (96, 33, 54))] +
+                         [("periodic%d" % q, (36, 9, 18)) for q in (0, 1, 2)] +
+                         [("wall", (144, 9, 128)), ("wall", (256, 16, 162)), ("wall", (256, 16, 192)), ("wall", (128, 9, 486))])
+def test_reported_divergence(built, scheme, shape, precision):
+    """The divergence that the diagnostics report is that of the downloaded field: rows,
+    twisted and substituting projections, ragged tiles and whole ones."""
+    from channel3d_b200 import ChannelSolver, initfield, mesh_y
+    if precision == "mixed" and scheme.startswith("periodic"):
+        pytest.skip("periodic y runs in FP64")
+    cfg = _cfg(scheme, *shape).copy(precision=precision)
+    yp = mesh_y(cfg)
+    f = initfield.taylor_green(cfg, yp=yp) if cfg.FlowType == 3 else initfield.laminar_noise(cfg, yp=yp, seed=4)
+    with ChannelSolver(cfg, yp=yp) as s:
+        s.upload(*f)
+        di = s.step(2)
+        gs = s.download()
+    word = np.float32 if precision == "mixed" else np.float64
+    div, terms = _divergence(gs, cfg, yp, word)
+    want = np.abs(div).max()
+    bound = 8 * np.finfo(np.float64).eps * terms.max()
+    if scheme == "4th" and precision == "mixed":  # its divergence is formed in the field's precision
+        bound = 8 * np.finfo(np.float32).eps * terms.max()
+    assert want > 0 and di["divmax2"] > 0
+    assert abs(di["divmax2"] - want) <= bound, (di["divmax2"], want, bound)
+    if precision == "mixed" and scheme != "4th":
+        assert want > 100 * bound  # far above what the comparison leaves open

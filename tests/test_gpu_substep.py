@@ -1,9 +1,8 @@
-"""The scalar work between the field kernels (channel3d_b200/csrc/ch3d_substep.cu, and
-the projection's last block on grids with up to 4096 partial sums) when the time
-step changes from step to step (iCFL = 1), so that every substep's coefficient
-tables are formed anew, against the oracle's steps: the grids on both sides of the
-line, the schemes with row tables and with periodic factor blocks, and a stage
-sequence after fused steps.
+"""The scalar work between the field kernels (channel3d_b200/csrc/ch3d_substep.cu) when
+the time step changes from step to step (iCFL = 1), so that every substep's
+coefficient tables are formed anew, against the oracle's steps: one block's partial
+sums (up to 4096) and many blocks', the schemes with row tables and with periodic
+factor blocks, a stage sequence after fused steps, and stages before any set-up.
 
 Tolerance: whole steps 1e-10 as elsewhere; dt and the CFL number follow the
 velocities, 1e-9; pressure 4 eps U (L / 2 pi) / (2/15 dt) over its rms where larger."""
@@ -30,13 +29,25 @@ def _cfg(scheme, shape):
     return cfg.copy(iCFL=1, CFLc=0.3, dtMax=1.0)
 
 
+def _partial_sums(cfg):
+    """Partial sums of the projection (its tiles times its chunks of rows)."""
+    import torch
+    cols = -(-cfg.nxc // 32) * -(-cfg.nzc // 4)
+    rows = 32
+    while rows > 4 and cols * -(-cfg.nyc // rows) < 4 * torch.cuda.get_device_properties(0).multi_processor_count:
+        rows //= 2
+    return cols * -(-cfg.nyc // rows)
+
+
 @pytest.mark.parametrize("scheme,shape", [("wall", (36, 17, 18)), ("adi", (36, 17, 18)), ("4th", (36, 17, 18)),
                                           ("explicit", (36, 17, 18)), ("periodic", (36, 17, 18)),
-                                          ("periodic_adi", (36, 17, 18)), ("wall", (256, 16, 162)), ("adi", (768, 33, 192))])
+                                          ("periodic_adi", (36, 17, 18)), ("wall", (256, 16, 162)), ("adi", (768, 33, 192)),
+                                          ("wall", (768, 9, 768)), ("adi", (768, 9, 768)), ("4th", (768, 9, 768))])
 def test_variable_time_step(built, scheme, shape):
     from channel3d_b200 import ChannelSolver, initfield, mesh_y
     from oracle import oracle as O
     cfg = _cfg(scheme, shape)
+    assert (_partial_sums(cfg) > 4096) == (shape == (768, 9, 768))
     yp = mesh_y(cfg)
     rng = np.random.default_rng(5)
     if cfg.BcOption[2] == 0:
