@@ -925,13 +925,16 @@ template <class T> static cudaError_t bulk_march_t(ch3d_ctx* c) {
 }
 cudaError_t launch_bulk_march(ch3d_ctx* c) { return c->fp32 ? bulk_march_t<float>(c) : bulk_march_t<double>(c); }
 
-// Rows per block of the substituting projection: the whole column, or, in FP64,
-// chunks where the tiles alone are at most six blocks per SM.  Mean of a step's three
-// launches, whole columns / chunks of 32 rows: 256x192x256 FP64 (512 tiles) 217 / 171 us,
-// mixed 115 / 121; 768x384x576 (3456 tiles) 2125 / 2202, mixed 1343 / 1436.
+// Rows per block of the substituting projection: the whole column, or, in FP64, chunks
+// where the tiles, three blocks per SM, leave more than a fifth of their waves' slots
+// empty (on 148 SMs below 356 tiles, 445 to 710, 889 to 1065 and 1333 to 1420).  Steps of
+// 192 rows, whole columns / chunks of 32: 384 tiles 1794 / 1833 us, 512 2419 / 2277, 648
+// 3418 / 3367, 768 3606 / 3620, 864 4095 / 4143, 1024 4821 / 4718, 1152 5486 / 5461, 1296
+// 6070 / 6241.  Mixed, the launch: 512 tiles 115 / 121 us, 3456 1343 / 1436.
 static int bsub_rows(const ch3d_ctx* c) {
   const long long tiles = (long long)((c->nx + 31) / 32) * ((c->nz + 3) / 4);
-  return c->fp32 || tiles > 6LL * sm_count(c->device) ? c->ny : proj_rows(c);
+  const long long slots = 3LL * sm_count(c->device), waves = (tiles + slots - 1) / slots;
+  return c->fp32 || 5 * tiles >= 4 * waves * slots ? c->ny : proj_rows(c);
 }
 template <class T> static cudaError_t div_bsub_t(ch3d_ctx* c) {
   T** f = (T**)c->f;
@@ -1049,7 +1052,10 @@ template <class T, bool O4> static cudaError_t rhs_march_t(ch3d_ctx* c) {
 // Grids with few columns: a column march's time is set by its dependent rows per
 // thread, however few columns there are; the right-hand sides by chunks of rows
 // and the y sweep as its own pass cost 6 more arrays of (L2) traffic instead.
-// 64^3 (4096 columns): 50 us against 19; 192^3 (36864): 224 us against 335.
+// 64^3 (4096 columns): 50 us against 19; 192^3 (36864): 224 us against 335.  Steps of 128
+// rows, rows / march: 16384 columns 535 / 587 us, 18432 706 / 740, 24576 813 / 810, 31104
+// 1054 / 993; mixed 376 / 421, 466 / 520, 611 / 589, 760 / 695.  With 48 rows they meet
+// near 14000 (16384: 251 / 251, mixed 177 / 172), with 256 near 25000.
 bool march_rows_path(const ch3d_ctx* c) {
   return c->march && (long long)c->nx * c->nz <= 120LL * sm_count(c->device);
 }

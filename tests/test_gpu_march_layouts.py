@@ -118,6 +118,17 @@ def test_gsub_step_info(built):
     assert di["divmax2"] < 1e-12
 
 
+@pytest.mark.parametrize("shape", [(256, 16, 192), (128, 9, 486), (256, 33, 162)])
+def test_gsub_projection_chunks(built, shape):
+    """The substituting projection over whole columns (384 tiles, 0.86 of a wave) and over
+    chunks of rows (488 and 328 tiles; ny below, at and above a chunk)."""
+    cfg = small_channel(*shape)
+    assert _flags(cfg) == {"march", "gsub"}
+    go, gs, di = _run(cfg, 3)
+    _check(go, gs)
+    assert di["divmax2"] < 1e-12
+
+
 def test_gsub_mixed(built):
     """Mixed path with the march stopping at g (8 x 81 = 648 tiles)."""
     go, gs, di = _run(small_channel(256, 24, 324, precision="mixed"), 3)
